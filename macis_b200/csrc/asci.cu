@@ -48,6 +48,11 @@ struct CoreData {
   const double* VT;       // V with its index pairs swapped (ham_vt): the
                           // opposite-spin elements of one outer pair are a
                           // contiguous row
+  const double2* GG;      // GG[x + y n] = (G2_red(x, y), G2_red(y, x))
+  const double* V2T;      // V2T[x + y n] = V2_red(y, x)
+  const uint8_t* full;    // per outer pair p = a + i n: 1 when every inner
+                          // same-spin element passes the threshold, [n^2 + p]
+                          // the same for the opposite-spin elements
 };
 
 // udet[u] = c for the units u of core det c (one warp per det): one load
@@ -62,28 +67,55 @@ __global__ void unit_owner_fill_k(const int64_t* uoff, size_t ncdets,
       udet[u] = int32_t(c);
 }
 
-// Outer-pair integral bounds (macis_b200_ham::pairmax). G rows are
-// contiguous (warp per pair); V is read with one thread per pair so that a
-// warp's loads are consecutive.
-__global__ void pairmax_g_k(const double* G, int n, double* out) {
+// Outer-pair integral bounds (macis_b200_ham::pairmax): the largest magnitude
+// of each row of G or of the pair-swapped V (one warp per contiguous row).
+__global__ void pairmax_k(const double* rows, int n, double* out) {
   const int lane = threadIdx.x & 31;
   const size_t n2 = size_t(n) * n;
   for(size_t p = size_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
       p < n2; p += size_t(gridDim.x) * (blockDim.x >> 5)) {
     double m = 0.0;
-    for(size_t q = lane; q < n2; q += 32) m = fmax(m, fabs(G[p * n2 + q]));
+    for(size_t q = lane; q < n2; q += 32) m = fmax(m, fabs(rows[p * n2 + q]));
     for(int o = 16; o > 0; o >>= 1)
       m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
     if(lane == 0) out[p] = m;
   }
 }
-__global__ void pairmax_v_k(const double* V, int n, double* out) {
+
+// Per outer pair p = (a, i), a != i: whether every inner pair (b, j) with
+// b != a, j != i passes the threshold test of the contributions, out[p] for
+// G(a,i,b,j) (b != j) and out[n^2 + p] for V(a,i,b,j) (any b != j). Units of
+// such a pair keep all their contributions, so the count pass need not
+// evaluate them: on the synthetic and molecular integrals without spatial
+// symmetry these are all pairs. One warp per row (rows are contiguous in G
+// and in the pair-swapped V).
+__global__ void pair_full_k(const double* G, const double* VT, int n,
+                            double tol, uint8_t* out) {
+  const int lane = threadIdx.x & 31;
   const size_t n2 = size_t(n) * n;
-  for(size_t p = size_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n2;
-      p += size_t(gridDim.x) * blockDim.x) {
-    double m = 0.0;
-    for(size_t q = 0; q < n2; ++q) m = fmax(m, fabs(V[p + q * n2]));
-    out[p] = m;
+  for(size_t r = size_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+      r < 2 * n2; r += size_t(gridDim.x) * (blockDim.x >> 5)) {
+    const bool os = r >= n2;
+    const int p = int(os ? r - n2 : r), a = p % n, i = p / n;
+    const double* row = (os ? VT : G) + size_t(p) * n2;
+    bool ok = a != i;
+    for(int q = lane; ok && q < n * n; q += 32) {
+      const int b = q % n, j = q / n;
+      const bool used = b != j && (os || (b != a && j != i && b != i && j != a));
+      if(used && fabs(row[q]) < tol) ok = false;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if(lane == 0) out[r] = ok ? 1 : 0;
+  }
+}
+
+__global__ void pair_tables_k(const double* G2, const double* V2, int n,
+                              double2* GG, double* V2T) {
+  for(int q = blockIdx.x * blockDim.x + threadIdx.x; q < n * n;
+      q += gridDim.x * blockDim.x) {
+    const int x = q % n, y = q / n;
+    GG[q] = make_double2(G2[q], G2[y + size_t(x) * n]);
+    V2T[q] = V2[y + size_t(x) * n];
   }
 }
 
@@ -364,7 +396,6 @@ struct RankBinGroup {
 };
 
 #define G2R(p, q) __ldg(I.G2_red + (p) + size_t(q) * n)
-#define V2R(p, q) __ldg(I.V2_red + (p) + size_t(q) * n)
 
 // A unit of core det c: t = 0 / 1 alpha / beta singles; then the (ii, aa)
 // outer pairs of the same-spin alpha doubles, of the same-spin beta doubles
@@ -409,7 +440,7 @@ __device__ __forceinline__ UnitDesc decode_unit(int nA, int nB, int nvA,
 // 1 / d: (q + 0.5) / d is at least 0.5 / d away from an integer, far above
 // the float rounding error (< 2^-22 q / d), so truncation gives the quotient
 // without a 64-bit integer division per contribution.
-__device__ __forceinline__ int small_div(int64_t q, float rd) {
+__device__ __forceinline__ int small_div(int q, float rd) {
   return int((float(q) + 0.5f) * rd);
 }
 
@@ -512,6 +543,55 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
     qlist = al.q + al.base[row] + e0;
     nloop = int64_t(rr[al.g + 1]) - e0;
   }
+  // Everything that is fixed for the unit. The pair tables are read with the
+  // inner orbitals as the fast index (GG holds both orders of a pair, V2T is
+  // V2_red transposed), so that the 32 lanes, whose inner virtuals b are
+  // neighbours, read neighbouring entries: with V2_red / G2_red themselves
+  // four of a contribution's loads went to 32 different lines, and the
+  // generation of 2.7e9 contributions (n = 48) was bound by them. The sums
+  // keep the reference's order of terms.
+  const int S = kind == 1 || kind == 3 ? 1 : 0;  // spin of the inner pair
+  const int SI = kind == 4 ? 1 : S;
+  const uint8_t* occI = SI ? occB : occA;
+  const uint8_t* virI = SI ? virB : virA;
+  const double* epsO = S ? epsB : epsA;   // spin of the outer pair
+  const double* epsI = SI ? epsB : epsA;
+  int i = 0, a = 0;
+  if(kind >= 2) {
+    i = (S ? occB : occA)[ii];
+    a = (S ? virB : virA)[aa];
+  }
+  const int jj0 = kind == 2 || kind == 3 ? ii + 1 : 0;
+  const int bb0 = kind == 2 || kind == 3 ? aa + 1 : 0;
+  const int span = (SI ? nvB : nvA) - bb0;
+  const float rspan = 1.0f / float(span > 0 ? span : 1);
+  if(MODE == 0 && kind >= 2 && !chk && !chkb && !(hist && kind == 2) &&
+     cd.full[(kind == 4 ? size_t(n) * n : 0) + a + size_t(i) * n]) {
+    // no contribution of this outer pair is below the threshold
+    if(lane == 0) {
+      *count_out = nloop;
+      if(hist && nloop) atomicAdd(hist + ubin, (unsigned long long)nloop);
+    }
+    return;
+  }
+  const size_t ai = size_t(a) + size_t(i) * n;
+  const double* row4 = (kind == 4 ? cd.VT : I.G) + ai * n * n;
+  const double2* GGi = cd.GG + size_t(i) * n;
+  const double2* GGa = cd.GG + size_t(a) * n;
+  const double* Vi = cd.V2T + size_t(i) * n;
+  const double* Va = cd.V2T + size_t(a) * n;
+  double hia = 0, eI = 0, gai = 0, gia = 0;
+  int par0 = 0;  // parity of the outer pair's part of the sign
+  if(MODE >= 1 && kind >= 2) {
+    hia = hii + epsO[a];
+    eI = epsO[i];
+    const double2 g = __ldg(GGi + a);
+    gai = g.x;
+    gia = g.y;
+    // occupied orbitals strictly between an occupied i (the ii-th) and a
+    // virtual a (the aa-th): a - aa occupied lie below a
+    par0 = (a - aa) ^ ii ^ int(a > i);
+  }
   for(int64_t q0 = 0; q0 < nloop; q0 += 32) {
     const int64_t qi = q0 + lane;
     bool keep = false;
@@ -519,57 +599,44 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
     uint64_t ex[D::NW];
     uint64_t rkey = 0;
     if(qi < nloop) {
-      const int64_t q = qlist ? int64_t(qlist[qi]) : qi;
+      const int q = qlist ? int(qlist[qi]) : int(qi);
+      const int qd = small_div(q, rspan);
+      const int jj = jj0 + qd, bb = bb0 + (q - qd * span);
+      const int j = occI[jj], b = virI[bb];
       if(kind <= 1) {
         // append_singles_asci_contributions (determinant_contributions.hpp:25-66)
-        const int S = kind;
-        const int nS = S ? nB : nA, nvS = S ? nvB : nvA;
-        const uint8_t* occS = S ? occB : occA;
-        const uint8_t* virS = S ? virB : virA;
-        const int nO = S ? nA : nB;
+        const int nS = S ? nB : nA, nO = S ? nA : nB;
         const uint8_t* occO = S ? occA : occB;
-        const int qd = small_div(q, 1.0f / float(nvS));
-        const int i = occS[qd], a = virS[int(q) - qd * nvS];
         uint32_t cbin = 0;
         if(S == 0 && (chk || hist))
-          cbin = alpha_bin<NSW>(sp_flip(sp_flip(sA, i), a));
+          cbin = alpha_bin<NSW>(sp_flip(sp_flip(sA, j), b));
         bool inr = !chk || (cbin >= blo && cbin < bhi);
         if(chkb)  // S == 1
-          inr = beta_sub<NSW>(sp_flip(sp_flip(sB, i), a), nsub) == sub;
+          inr = beta_sub<NSW>(sp_flip(sp_flip(sB, j), b), nsub) == sub;
         double h = 0;
         if(inr) {
-          h = __ldg(I.T + a + size_t(i) * n);
-          const double* Gov = I.G_red + size_t(a) * n + size_t(i) * n * n;
-          const double* Vov = I.V_red + size_t(a) * n + size_t(i) * n * n;
-          for(int p = 0; p < nS; ++p) h += __ldg(Gov + occS[p]);
+          h = __ldg(I.T + b + size_t(j) * n);
+          const double* Gov = I.G_red + size_t(b) * n + size_t(j) * n * n;
+          const double* Vov = I.V_red + size_t(b) * n + size_t(j) * n * n;
+          for(int p = 0; p < nS; ++p) h += __ldg(Gov + occI[p]);
           for(int p = 0; p < nO; ++p) h += __ldg(Vov + occO[p]);
         }
         keep = inr && !(fabs(h) < tol);
         if(MODE == 0 && hist && S == 0 && keep) atomicAdd(hist + cbin, 1ull);
         if(MODE >= 1 && keep) {
-          const double* eps = S ? epsB : epsA;
-          h *= ex_sign(S ? sB : sA, a, i);
-          const double hd = hii + eps[a] - eps[i] - G2R(a, i) - G2R(i, a);
+          h *= ex_sign(S ? sB : sA, b, j);
+          const double hd = hii + epsI[b] - epsI[j] - G2R(b, j) - G2R(j, b);
           h /= (E0 - hd);
           r = coeff * h;
           if constexpr(MODE == 1) {
 #pragma unroll
             for(int w = 0; w < D::NW; ++w) ex[w] = det[w];
-            det_flip<NBITS>(ex, S, i);
-            det_flip<NBITS>(ex, S, a);
+            det_flip<NBITS>(ex, S, j);
+            det_flip<NBITS>(ex, S, b);
           }
         }
-        (void)nS;
       } else if(kind <= 3) {
         // append_ss_doubles_asci_contributions (determinant_contributions.hpp:68-120)
-        const int S = kind - 2;
-        const int nvS = S ? nvB : nvA;
-        const uint8_t* occS = S ? occB : occA;
-        const uint8_t* virS = S ? virB : virA;
-        const int span = nvS - 1 - aa;
-        const int qd = small_div(q, 1.0f / float(span));
-        const int jj = ii + 1 + qd, bb = aa + 1 + (int(q) - qd * span);
-        const int i = occS[ii], a = virS[aa], j = occS[jj], b = virS[bb];
         uint32_t cbin = 0;
         if(S == 0 && (chk || hist))
           cbin = alpha_bin<NSW>(
@@ -579,21 +646,21 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
           inr = beta_sub<NSW>(
                     sp_flip(sp_flip(sp_flip(sp_flip(sB, i), j), a), b), nsub) ==
                 sub;
-        const double Gv =
-            inr ? __ldg(I.G + size_t(a + size_t(i) * n) * n * n + b + size_t(j) * n)
-                : 0.0;
+        const double Gv = inr ? __ldg(row4 + b + j * n) : 0.0;
         keep = inr && !(fabs(Gv) < tol);
         if(MODE == 0 && hist && S == 0 && keep) atomicAdd(hist + cbin, 1ull);
         if(MODE >= 1 && keep) {
-          const Spin<NSW> st = S ? sB : sA;
-          Spin<NSW> fx = sp_flip(sp_flip(sp_flip(sp_flip(sp_zero<NSW>(), i), j), a), b);
-          const uint32_t e = double_ex(st, st ^ fx);
-          double h = ex_sgn(e) * Gv;
-          const double* eps = S ? epsB : epsA;
-          const double hd = hii + eps[a] + eps[b] - eps[i] - eps[j] + G2R(i, j) +
-                            G2R(j, i) + G2R(a, b) + G2R(b, a) - G2R(a, i) -
-                            G2R(i, a) - G2R(b, i) - G2R(i, b) - G2R(a, j) -
-                            G2R(j, a) - G2R(b, j) - G2R(j, b);
+          // double_ex's sign (i < j, a < b): i <-> a in the string without
+          // j and with b, then j <-> b in the string itself
+          const int par = par0 ^ (b - bb) ^ jj ^ int(b > j) ^
+                          int(a > i ? j < a : b < i);
+          const double2 gji = __ldg(GGi + j), gba = __ldg(GGa + b),
+                        gbi = __ldg(GGi + b), gja = __ldg(GGa + j),
+                        gbj = __ldg(cd.GG + b + j * n);
+          double h = (par & 1) ? -Gv : Gv;
+          const double hd = hia + epsI[b] - eI - epsI[j] + gji.y + gji.x +
+                            gba.y + gba.x - gai - gia - gbi.x - gbi.y -
+                            gja.y - gja.x - gbj.x - gbj.y;
           h /= (E0 - hd);
           r = coeff * h;
           if constexpr(MODE == 1) {
@@ -607,23 +674,18 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
         }
       } else {
         // append_os_doubles_asci_contributions (determinant_contributions.hpp:122-160)
-        const int i = occA[ii], a = virA[aa];
-        const int qd = small_div(q, 1.0f / float(nvB));
-        const int j = occB[qd], b = virB[int(q) - qd * nvB];
         const bool inr =
             !chkb || beta_sub<NSW>(sp_flip(sp_flip(sB, j), b), nsub) == sub;
-        // V(a,i,b,j) from row (a,i) of the pair-swapped copy: consecutive
-        // inner indices read neighbouring addresses
-        const double Vv =
-            inr ? __ldg(cd.VT + size_t(a + size_t(i) * n) * n * n + b + size_t(j) * n)
-                : 0.0;
+        // V(a,i,b,j) from row (a,i) of the pair-swapped copy
+        const double Vv = inr ? __ldg(row4 + b + j * n) : 0.0;
         keep = inr && !(fabs(Vv) < tol);
         if(MODE >= 1 && keep) {
-          const double sign = ex_sign(sA, a, i) * ex_sign(sB, b, j);
-          double h = sign * Vv;
-          const double hd = hii + epsA[a] + epsB[b] - epsA[i] - epsB[j] +
-                            V2R(i, j) + V2R(a, b) - G2R(a, i) - G2R(i, a) -
-                            G2R(b, j) - G2R(j, b) - V2R(a, j) - V2R(i, b);
+          const int par = par0 ^ (b - bb) ^ jj ^ int(b > j);
+          const double2 gbj = __ldg(cd.GG + b + j * n);
+          double h = (par & 1) ? -Vv : Vv;
+          const double hd = hia + epsI[b] - eI - epsI[j] + __ldg(Vi + j) +
+                            __ldg(Va + b) - gai - gia - gbj.x - gbj.y -
+                            __ldg(Va + j) - __ldg(Vi + b);
           h /= (E0 - hd);
           r = coeff * h;
           if constexpr(MODE == 1) {
@@ -665,7 +727,6 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
   }
 }
 #undef G2R
-#undef V2R
 
 // Units [u0, u1) of the batch, a warp at a time over runs of 32
 // consecutive units: the lanes read the 32 units' masks, counts, owners and
@@ -788,7 +849,7 @@ __global__ void __launch_bounds__(256)
     const int span = nvA - 1 - aa;
     const int64_t ninner = int64_t(nA - 1 - ii) * span;
     for(int64_t q = lane; q < ninner; q += 32) {
-      const int qd = small_div(q, 1.0f / float(span));
+      const int qd = small_div(int(q), 1.0f / float(span));
       const int j = occA[ii + 1 + qd], b = virA[aa + 1 + (int(q) - qd * span)];
       const double Gv =
           __ldg(I.G + size_t(a + size_t(i) * n) * n * n + b + size_t(j) * n);
@@ -849,7 +910,7 @@ __global__ void __launch_bounds__(256)
       const int64_t q = q0 + lane;
       unsigned g = 0xFFFFu;
       if(q < ninner) {
-        const int qd = small_div(q, 1.0f / float(span));
+        const int qd = small_div(int(q), 1.0f / float(span));
         const int j = occA[ii + 1 + qd],
                   b = virA[aa + 1 + (int(q) - qd * span)];
         const double Gv =
@@ -1259,11 +1320,12 @@ double ms_since(std::chrono::steady_clock::time_point t) {
 }
 }  // namespace
 
-// Core-det precompute and unit offsets; returns the unit count.
+// Core-det precompute and unit offsets; returns the unit count. bounds: also
+// the outer-pair bounds, which the network's inputs need.
 template <int NBITS>
 static int64_t core_setup(macis_b200_ham* h, Arena& A, const uint64_t* cdets,
                           size_t ncdets, const double* C, int just_singles,
-                          CoreData& cd) {
+                          bool bounds, CoreData& cd) {
   cudaStream_t s = h->stream;
   const int n = h->norb;
   const int sms = num_sms();
@@ -1279,17 +1341,25 @@ static int64_t core_setup(macis_b200_ham* h, Arena& A, const uint64_t* cdets,
   cd.hd = A.get<double>(ncdets + 1);
   int64_t* units = A.get<int64_t>(ncdets + 1);
   cd.uoff = A.get<int64_t>(ncdets + 1);
-  if(!h->pairmax) {
+  cd.VT = ham_vt(h);
+  if(bounds && !h->pairmax) {
     const size_t n2 = size_t(n) * n;
     MB_CUDA(dev_malloc(&h->pairmax, 2 * n2 * sizeof(double)));
-    pairmax_g_k<<<grid_for(n2 * 32, 256, 16 * sms), 256, 0, s>>>(
-        h->G, n, h->pairmax), note_launch();
-    pairmax_v_k<<<grid_for(n2, 128, 4 * sms), 128, 0, s>>>(
-        h->V, n, h->pairmax + n2), note_launch();
+    const unsigned g = grid_for(n2 * 32, 256, 16 * sms);
+    pairmax_k<<<g, 256, 0, s>>>(h->G, n, h->pairmax), note_launch();
+    pairmax_k<<<g, 256, 0, s>>>(cd.VT, n, h->pairmax + n2), note_launch();
     MB_CUDA(cudaGetLastError());
   }
   cd.pairmax = h->pairmax;
-  cd.VT = ham_vt(h);
+  {
+    const size_t n2 = size_t(n) * n;
+    double2* GG = A.get<double2>(n2);
+    double* V2T = A.get<double>(n2);
+    pair_tables_k<<<grid_for(n2, 256, 4 * sms), 256, 0, s>>>(
+        h->G2_red, h->V2_red, n, GG, V2T), note_launch();
+    cd.GG = GG;
+    cd.V2T = V2T;
+  }
   if(ncdets) {
     core_prep_k<NBITS><<<grid_for(ncdets * 32, 256, 16 * sms), 256, 0, s>>>(
         h->ints(), cd, just_singles, units), note_launch();
@@ -1531,7 +1601,8 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
 
   // ------------------------------------------------ core precompute
   CoreData cd{};
-  const int64_t U = core_setup<NBITS>(h, A, cdets, ncdets, C, st.just_singles, cd);
+  const int64_t U = core_setup<NBITS>(h, A, cdets, ncdets, C, st.just_singles,
+                                       scr && scr->net, cd);
 
   // ------------------------------------------------ learned screening
   macis_b200_mlp* net = scr ? scr->net : nullptr;
@@ -1607,22 +1678,30 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
   }
   stats.screen_ms = ms_since(t_scr);
 
-  // unit counts of the whole search (count pass over all units at once)
+  {
+    const size_t n2 = size_t(h->norb) * h->norb;
+    uint8_t* full = A.get<uint8_t>(2 * n2);
+    pair_full_k<<<grid_for(2 * n2 * 32, 256, 16 * sms), 256, 0, s>>>(
+        h->G, cd.VT, h->norb, st.h_el_tol, full), note_launch();
+    cd.full = full;
+  }
+  // unit counts of the whole search (count pass over all units at once);
+  // with a histogram also the contributions per alpha-string bin, which only
+  // searches of several ranges or parts need
   int64_t* ucnt = A.get<int64_t>(U + 1);
-  auto* dhist = A.get<unsigned long long>(ASCI_BINS);
-  MB_CUDA(cudaMemsetAsync(dhist, 0, ASCI_BINS * 8, s));
-  if(U) {
-    const size_t hbytes = ASCI_BINS * sizeof(unsigned long long);
+  auto count_units = [&](unsigned long long* hist) {
+    const size_t hbytes = hist ? ASCI_BINS * sizeof(unsigned long long) : 0;
     MB_CUDA(cudaFuncSetAttribute(units_k<NBITS, 0>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(hbytes)));
+                                 int(ASCI_BINS * sizeof(unsigned long long))));
     units_k<NBITS, 0><<<grid_for(size_t(U), 256, 32 * sms), 256, hbytes,
                         s>>>(I, cd, 0, U, 0, ncdets, E0, st.h_el_tol, ucnt,
                              nullptr, nullptr, nullptr, umask, nullptr, 0u,
-                             ASCI_BINS, 0u, 0u, dhist, AlphaLists{},
+                             ASCI_BINS, 0u, 0u, hist, AlphaLists{},
                              RankTables{}),
         note_launch();
-  }
+  };
+  if(U) count_units(nullptr);
   int64_t* uout = A.get<int64_t>(U + 1);
   exclusive_scan<int64_t, int64_t>(ucnt, uout, size_t(U), uout + U, A);
   const int64_t Ptot = U ? to_host(uout + U, s) : 0;
@@ -1720,7 +1799,11 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
   std::vector<unsigned long long> hh;
   auto load_hist = [&] {
     if(!hh.empty()) return;
-    hh.resize(ASCI_BINS);
+    hh.assign(ASCI_BINS, 0);
+    if(!U) return;
+    auto* dhist = A.get<unsigned long long>(ASCI_BINS);
+    MB_CUDA(cudaMemsetAsync(dhist, 0, ASCI_BINS * 8, s));
+    count_units(dhist);
     MB_CUDA(cudaMemcpyAsync(hh.data(), dhist, ASCI_BINS * 8,
                             cudaMemcpyDeviceToHost, s));
     MB_CUDA(cudaStreamSynchronize(s));
@@ -2315,7 +2398,7 @@ static int64_t unit_features_impl(macis_b200_ham* h, const uint64_t* cdets,
                                   size_t first, size_t n, uint16_t* X) {
   Arena A(h->stream);
   CoreData cd{};
-  const int64_t U = core_setup<NBITS>(h, A, cdets, ncdets, C, 0, cd);
+  const int64_t U = core_setup<NBITS>(h, A, cdets, ncdets, C, 0, true, cd);
   if(X && n) {
     MB_REQUIRE(first + n <= size_t(U), MACIS_B200_EINVAL,
                "unit range outside the search's units");
