@@ -7,8 +7,9 @@
 //     a count pass over "units" (singles of a spin, or one (i,a) outer pair
 //     of a double loop) and a fill pass writing every (det, rv) record at its
 //     exact position -- so the raw list is the reference push_back order
-//  3. stable radix sort by determinant and a sequential per-segment sum:
-//     duplicates are added in generation order (sort_and_accumulate_asci_pairs,
+//  3. stable grouping by determinant (group.cuh; a full sort where the list
+//     itself is the result) and a sequential sum per group: duplicates are
+//     added in generation order (sort_and_accumulate_asci_pairs,
 //     determinant_sort.hpp:40-83)
 //  4. drop core dets and zero scores (keep_only_largest_copy_asci_pairs +
 //     partition, determinant_sort.hpp:86-120, determinant_search.hpp:528-544)
@@ -25,6 +26,7 @@
 #include <cstdlib>
 
 #include "internal.hpp"
+#include "group.cuh"
 #include "mlp.cuh"
 #include "primitives.cuh"
 
@@ -225,19 +227,6 @@ __device__ __forceinline__ uint32_t alpha_bin(const Spin<NSW>& a) {
   return uint32_t(h >> 52);  // 12 bits: ASCI_BINS
 }
 
-// Sort group of a candidate record of a range: groups are runs of the
-// range's alpha-string bins (gtab: bin -> group), so that equal
-// determinants share a group.
-template <int NBITS>
-struct BinGroup {
-  const uint8_t* gtab;  // ASCI_BINS entries
-  __device__ __forceinline__ unsigned operator()(
-      const Key<DetTraits<NBITS>::NW>& k) const {
-    using D = DetTraits<NBITS>;
-    return gtab[alpha_bin<D::NSW>(D::alpha(k.w))];
-  }
-};
-
 // Alpha lists of a partitioned search. The bins of the contributions of an
 // alpha same-spin double unit (kind 2) depend only on the core det's alpha
 // string, and so does their threshold test (|G| against the tolerance):
@@ -288,7 +277,6 @@ struct RankTables {
   int bits_a = 0;
   const uint64_t* La = nullptr;  // distinct candidate alpha strings (NSW words)
   const uint64_t* Lb = nullptr;
-  const uint16_t* bin_a = nullptr;  // per alpha rank: its bin
 };
 // First double of row ii * nv + aa among the doubles of a string with ne
 // electrons and nv virtuals (rows before it hold (ne-1-ii')(nv-1-aa') each).
@@ -355,14 +343,16 @@ __global__ void rank_scatter_k(const uint64_t* cand, const uint32_t* idx,
     }
   }
 }
-template <int NSW>
-__global__ void string_bins_k(const uint64_t* L, size_t n, uint16_t* bin) {
-  for(size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-      i += size_t(gridDim.x) * blockDim.x) {
-    Spin<NSW> st;
-#pragma unroll
-    for(int j = 0; j < NSW; ++j) st.w[j] = L[i * NSW + j];
-    bin[i] = uint16_t(alpha_bin<NSW>(st));
+// Ranked keys of the core dets in the order `ord` (each core string is the
+// first candidate of its own table row).
+__global__ void rank_core_k(RankTables rt, const uint32_t* ord, size_t nc,
+                            uint64_t* rk) {
+  for(size_t c = size_t(blockIdx.x) * blockDim.x + threadIdx.x; c < nc;
+      c += size_t(gridDim.x) * blockDim.x) {
+    const uint32_t d = ord[c];
+    const uint64_t ra = rt.a.R[size_t(rt.a.idx[d]) * size_t(rt.a.M)];
+    const uint64_t rb = rt.b.R[size_t(rt.b.idx[d]) * size_t(rt.b.M)];
+    rk[c] = (rb << rt.bits_a) | ra;
   }
 }
 // Ranked keys back to determinants.
@@ -385,16 +375,6 @@ __global__ void unrank_k(const uint64_t* rk, size_t n, RankTables rt,
     D::make(dets + i * D::NW, a, b);
   }
 }
-// Sort group of a ranked key: the group of its alpha string's bin.
-struct RankBinGroup {
-  const uint8_t* gtab;
-  const uint16_t* bin_a;
-  uint64_t mask_a;
-  __device__ __forceinline__ unsigned operator()(const Key<1>& k) const {
-    return gtab[bin_a[k.w[0] & mask_a]];
-  }
-};
-
 #define G2R(p, q) __ldg(I.G2_red + (p) + size_t(q) * n)
 
 // A unit of core det c: t = 0 / 1 alpha / beta singles; then the (ii, aa)
@@ -1306,7 +1286,16 @@ __global__ void tie_select_k(const uint64_t* keys, const uint32_t* gt,
     f[i] = gt[i] || (eq[i] && key_cmp<NW>(load_key<NW>(keys, i), Kmax) <= 0);
 }
 
+__global__ void iota_k(uint32_t* x, size_t n) {
+  for(size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+      i += size_t(gridDim.x) * blockDim.x)
+    x[i] = uint32_t(i);
+}
+
 // ----------------------------------------------------------------- driver
+// A range's score threshold is sampled from one part in GROUP_SAMPLE of it.
+constexpr size_t GROUP_SAMPLE = 32;
+
 namespace {
 struct Pairs {
   uint64_t* keys = nullptr;
@@ -1541,7 +1530,7 @@ static int build_ranks(const SpinPlan& pa, const SpinPlan& pb, size_t ncdets,
   const size_t na = build_spin_ranks<NBITS>(pa, A, s, ra, &La);
   const size_t nb = build_spin_ranks<NBITS>(pb, A, s, rb, &Lb);
   const int ba = bits_for(na), bb = bits_for(nb);
-  const double strings = (8.0 * NSW + 2.0) * double(na) + 8.0 * NSW * double(nb);
+  const double strings = 8.0 * NSW * (double(na) + double(nb));
   if(ba + bb > 64 || tables + strings > 0.15 * avail) {
     for(const void* q : {static_cast<const void*>(ra.R),
                          static_cast<const void*>(rb.R),
@@ -1550,9 +1539,6 @@ static int build_ranks(const SpinPlan& pa, const SpinPlan& pb, size_t ncdets,
       A.release(const_cast<void*>(q));
     return 0;
   }
-  uint16_t* bin = A.get<uint16_t>(na + 1);
-  string_bins_k<NSW><<<grid_for(na, 256, 4 * num_sms()), 256, 0, s>>>(
-      La, na, bin), note_launch();
   int32_t* ai = A.get<int32_t>(ncdets);
   int32_t* bi = A.get<int32_t>(ncdets);
   MB_CUDA(cudaMemcpyAsync(ai, pa.idx.data(), ncdets * 4,
@@ -1567,7 +1553,6 @@ static int build_ranks(const SpinPlan& pa, const SpinPlan& pb, size_t ncdets,
   rt.bits_a = ba;
   rt.La = La;
   rt.Lb = Lb;
-  rt.bin_a = bin;
   return ba + bb;
 }
 
@@ -1749,19 +1734,21 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
       stats.rank_ms = ms_since(t_rk);
     }
   }
-  // bytes of a sorted record, and of a candidate with its determinant
-  // (the unique candidates of a range, the survivors)
+  // bytes of a record, and of a candidate with its determinant
   const double rs = ranked ? 16.0 : double(NW * 8 + 8);
   const double rf = double(NW * 8 + 8);
-  // per raw contribution while a range is processed, whichever phase holds
-  // more: record + sort copy, flags and radix tables (sort); or the unique
-  // candidates as determinants, their flags and kept copy and the running
-  // top-k concatenation (few duplicates: unique ~ raw; 128 B at 256 bits,
-  // more than a ranked-key record's sort)
-  const double per_pair = std::max(4.0 * rs + 20.0, 3.0 * rf + 8.0);
+  // per raw contribution while a range is processed: the record, its copy
+  // and the digit counts of the partition
+  const double per_pair = 2.0 * rs + 2.0;
   const size_t topk = ndets_max - ncdets;   // size_t arithmetic (:547)
+  // the running top-k with its copies, and the candidates a range leaves
+  // above its sampled threshold (about GROUP_SAMPLE times the wanted ones)
+  // as determinants with their flags and kept copy
   const double keep_reserve =
-      6.0 * rf * double(std::min<uint64_t>(topk, uint64_t(Ptot)));
+      6.0 * rf * double(std::min<uint64_t>(topk, uint64_t(Ptot))) +
+      (2.0 * rf + 16.0) *
+          std::min(2.0 * GROUP_SAMPLE * (double(topk) + double(ncdets)),
+                   double(Ptot));
   // MACIS_B200_ASCI_BATCH_PAIRS caps the raw pairs per range (exercises the
   // partitioned path on small problems).
   int64_t cap = 0;
@@ -1774,14 +1761,6 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
     cap = std::min<int64_t>(std::max<int64_t>(cap, int64_t(1) << 20),
                             int64_t(1) << 31);
   }
-  // records per sort group of a range (MACIS_B200_ASCI_SORT_GROUP). Only
-  // determinant keys are grouped by default: with ranked keys (16-byte
-  // records) a range sorted whole was measured as fast as or faster than
-  // any grouping (n = 48: 1e4 core dets 246 against 276 ms, 1e5 core dets
-  // 3.48 s against 3.35-5.9 s for groups of 5e8-1.07e9 records)
-  uint64_t sort_group_cap = ranked ? ~uint64_t(0) : uint64_t(4) << 28;
-  if(const char* e = getenv("MACIS_B200_ASCI_SORT_GROUP"))
-    sort_group_cap = std::max<uint64_t>(1, uint64_t(atoll(e)));
   // ranges: consecutive alpha-string bins packed up to the cap from the
   // measured bin loads (a single bin above the cap is a range of its own)
   // (a bin above the cap is split into beta-hash classes)
@@ -1976,14 +1955,24 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
   }
   stats.pairs_ms = ms_since(t_all);
 
-  // sorted core dets (dropped from the candidates)
+  // sorted core dets (dropped from the candidates), and their record keys
   uint64_t* core = A.get<uint64_t>(ncdets * NW + NW);
+  uint64_t* core_key = core;
   if(ncdets) {
     uint64_t* ct = A.get<uint64_t>(ncdets * NW + NW);
+    uint32_t* ord = A.get<uint32_t>(2 * ncdets);
     MB_CUDA(cudaMemcpyAsync(core, cdets, ncdets * NW * 8,
                             cudaMemcpyDeviceToDevice, s));
-    radix_sort<NW, uint32_t>(core, nullptr, ct, nullptr, ncdets, A);
+    iota_k<<<grid_for(ncdets, 256, 8 * sms), 256, 0, s>>>(ord, ncdets),
+        note_launch();
+    radix_sort<NW, uint32_t>(core, ord, ct, ord + ncdets, ncdets, A);
+    if(ranked) {
+      core_key = A.get<uint64_t>(ncdets);
+      rank_core_k<<<grid_for(ncdets, 256, 8 * sms), 256, 0, s>>>(
+          rt, ord, ncdets, core_key), note_launch();
+    }
     A.release(ct);
+    A.release(ord);
   }
 
   // MSD radix select on |rv| bits: the bits T of the topk-th largest score
@@ -2089,100 +2078,112 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
     MB_CUDA(cudaStreamSynchronize(s));
     pair_ms += ms_since(tb);
     tb = std::chrono::steady_clock::now();
-    // sort + accumulate (stable: duplicates summed in generation order)
+    // group + accumulate (stable: duplicates summed in generation order)
     Pairs uq;
+    uint64_t nuniq = 0, nscored = 0, npruned = 0;
     uint64_t* k2 = nullptr;
     double* r2 = nullptr;
-    // KW key words per record; group(dg) the sort-group functor of a bin ->
-    // group table
-    auto accumulate = [&](auto kw, auto group) {
+    auto accumulate = [&](auto kw) {  // KW key words per record
       constexpr int KW = decltype(kw)::value;
       k2 = B.get<uint64_t>(size_t(P) * KW + KW);
       r2 = B.get<double>(size_t(P) + 1);
-      // a large range is first split by bin into groups that are sorted
-      // one at a time: the digit passes of a sort over fewer records run
-      // faster (measured: 12 passes over 6e8 records at 1.7x the rate of
-      // 1.3e9), and equal determinants share a bin, so each group's sums
-      // are complete and in generation order
-      std::vector<size_t> goff{0, size_t(P)};
-      if(!pairs_only && rns[rr] == 0 && rhi[rr] - rlo[rr] > 1 &&
-         uint64_t(P) > sort_group_cap) {
-        load_hist();
-        std::vector<uint8_t> gt(ASCI_BINS, 0);
-        int g = 0;
-        unsigned long long acc = 0;
-        for(uint32_t b = rlo[rr]; b < rhi[rr]; ++b) {
-          if(acc && acc + hh[b] > sort_group_cap && g < 255) {
-            ++g;
-            acc = 0;
-          }
-          gt[b] = uint8_t(g);
-          acc += hh[b];
-        }
-        if(g > 0) {
-          uint8_t* dg = B.get<uint8_t>(ASCI_BINS);
-          MB_CUDA(cudaMemcpyAsync(dg, gt.data(), ASCI_BINS,
-                                  cudaMemcpyHostToDevice, s));
-          goff = stable_partition<KW, double>(keys, rv, k2, r2, size_t(P),
-                                              g + 1, group(dg), B);
-          std::swap(keys, k2);
-          std::swap(rv, r2);
-          stats.sort_pass_items += uint64_t(P);
-        }
-      }
-      for(size_t gi = 0; gi + 1 < goff.size(); ++gi) {
-        const size_t a = goff[gi], m = goff[gi + 1] - a;
+      const size_t n = size_t(P);
+      if(pairs_only) {  // the list in ascending order: a full sort
         stats.sort_pass_items +=
-            uint64_t(radix_sort<KW, double>(keys + a * KW, rv + a,
-                                            k2 + a * KW, r2 + a, m, B)) *
-            uint64_t(m);
+            uint64_t(radix_sort<KW, double>(keys, rv, k2, r2, n, B)) * n;
+        uint32_t* f = B.get<uint32_t>(n + 1);
+        uint32_t* fx = B.get<uint32_t>(n + 1);
+        seg_flags_k<KW><<<grid_for(n, 256, 16 * sms), 256, 0, s>>>(
+            keys, n, f), note_launch();
+        exclusive_scan<uint32_t, uint32_t>(f, fx, n, fx + n, B);
+        uq.n = nuniq = to_host(fx + n, s);
+        int64_t* start = B.get<int64_t>(uq.n + 1);
+        // unique keys into k2, sums into r2
+        seg_starts_k<KW><<<grid_for(n, 256, 16 * sms), 256, 0, s>>>(
+            f, fx, n, start, keys, k2), note_launch();
+        seg_sum_k<<<grid_for(uq.n, 256, 16 * sms), 256, 0, s>>>(
+            start, uq.n, n, rv, r2), note_launch();
+        for(void* q : {static_cast<void*>(f), static_cast<void*>(fx),
+                       static_cast<void*>(start)})
+          B.release(q);
+      } else {
+        const int np = group_digits(n);
+        const int sh = 32 - 8 * np;
+        {
+          DigitPasses<KW, double> passes(n, B);
+          for(int p = 0; p < np; ++p) {
+            passes.run(keys, rv, k2, r2, HashDigit<KW>{sh + 8 * p});
+            std::swap(keys, k2);
+            std::swap(rv, r2);
+          }
+          passes.release();
+        }
+        stats.sort_pass_items += uint64_t(np) * n;
+        auto* gc = B.get<GroupCounts>(1);
+        auto run = [&](size_t n1, uint64_t tout) {
+          MB_CUDA(cudaMemsetAsync(gc, 0, sizeof(GroupCounts), s));
+          group_sum_k<KW><<<grid_for(n1, GS_TILE, 8 * sms), GS_THREADS, 0, s>>>(
+              keys, rv, n, 0, n1, sh, tcut, tout, st.rv_prune_tol, k2, r2, gc),
+              note_launch();
+          MB_CUDA(cudaGetLastError());
+        };
+        // A bound below the k-th score of the range: the k-th score of its
+        // first 1 / GROUP_SAMPLE (buckets are in hash order, so these are a
+        // random sample of the candidates; up to ncdets of the scores may be
+        // core dets'). With it the pass over the whole range writes about
+        // GROUP_SAMPLE k candidates instead of all.
+        uint64_t tout = 0;
+        if(topk < n) {
+          const size_t want = topk + ncdets;
+          const size_t n1 = std::max<size_t>(n / GROUP_SAMPLE, 8 * want);
+          if(want && n1 < n / 4) {
+            run(n1, 0);
+            const size_t c1 = size_t(to_host(&gc->out, s));
+            uint64_t need = 0;
+            if(c1 > want) tout = kth_bits(r2, c1, want, &need);
+          }
+        }
+        run(n, tout);
+        GroupCounts hc = to_host(gc, s);
+        uq.n = size_t(hc.out);
+        nuniq = hc.unique;
+        if(ncdets) {
+          MB_CUDA(cudaMemsetAsync(gc, 0, sizeof(GroupCounts), s));
+          group_core_k<KW><<<grid_for(ncdets, 128, 16 * sms), 128, 0, s>>>(
+              keys, rv, n, sh, tcut, st.rv_prune_tol, core_key, ncdets, gc),
+              note_launch();
+          const GroupCounts cc = to_host(gc, s);
+          hc.scored -= cc.scored;
+          hc.pruned -= cc.pruned;
+        }
+        nscored = hc.scored;
+        npruned = hc.pruned;
       }
-      uint32_t* f = B.get<uint32_t>(size_t(P) + 1);
-      uint32_t* fx = B.get<uint32_t>(size_t(P) + 1);
-      seg_flags_k<KW><<<grid_for(size_t(P), 256, 16 * sms), 256, 0, s>>>(
-          keys, size_t(P), f), note_launch();
-      exclusive_scan<uint32_t, uint32_t>(f, fx, size_t(P), fx + P, B);
-      const uint32_t nu = to_host(fx + P, s);
-      int64_t* start = B.get<int64_t>(nu + 1);
-      // unique keys into k2, sums into r2
-      seg_starts_k<KW><<<grid_for(size_t(P), 256, 16 * sms), 256, 0, s>>>(
-          f, fx, size_t(P), start, keys, k2), note_launch();
-      seg_sum_k<<<grid_for(nu, 256, 16 * sms), 256, 0, s>>>(
-          start, nu, size_t(P), rv, r2), note_launch();
       // the raw records are summed: release them before the keep / top-k
-      for(void* q : {static_cast<void*>(f), static_cast<void*>(fx),
-                     static_cast<void*>(start), static_cast<void*>(keys),
-                     static_cast<void*>(rv)})
-        B.release(q);
-      return nu;
+      B.release(keys);
+      B.release(rv);
     };
     if(P) {
-      uint32_t nu = 0;
       if(ranked) {
-        nu = accumulate(std::integral_constant<int, 1>{},
-                        [&](const uint8_t* dg) {
-                          return RankBinGroup{
-                              dg, rt.bin_a, (uint64_t(1) << rt.bits_a) - 1};
-                        });
+        accumulate(std::integral_constant<int, 1>{});
         // ranked keys back to determinants
-        uint64_t* kd = B.get<uint64_t>(size_t(nu) * NW + NW);
-        if(nu)
-          unrank_k<NBITS><<<grid_for(nu, 256, 16 * sms), 256, 0, s>>>(
-              k2, nu, rt, kd), note_launch();
+        uint64_t* kd = B.get<uint64_t>(uq.n * NW + NW);
+        if(uq.n)
+          unrank_k<NBITS><<<grid_for(uq.n, 256, 16 * sms), 256, 0, s>>>(
+              k2, uq.n, rt, kd), note_launch();
         B.release(k2);
         k2 = kd;
       } else {
-        nu = accumulate(std::integral_constant<int, NW>{},
-                        [&](const uint8_t* dg) { return BinGroup<NBITS>{dg}; });
+        accumulate(std::integral_constant<int, NW>{});
       }
       uq.keys = k2;
       uq.rv = r2;
-      uq.n = nu;
     }
-    uniq_total += uq.n;
+    uniq_total += nuniq;
     // pruning when the accumulated lists outgrow pair_size_max
     // (determinant_search.hpp:121-137)
-    if(uq.n && uniq_total > st.pair_size_max) {
+    const bool prune = nuniq && uniq_total > st.pair_size_max;
+    if(prune && uq.n) {
       uint32_t* f = B.get<uint32_t>(uq.n + 1);
       prune_flags_k<<<grid_for(uq.n, 256, 16 * sms), 256, 0, s>>>(
           uq.rv, uq.n, st.rv_prune_tol, f), note_launch();
@@ -2214,7 +2215,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
           uq.keys, uq.rv, uq.n, core, ncdets, tcut, f), note_launch();
       kept = compact_to(B, uq.keys, uq.rv, uq.n, f);
     }
-    kept_total += kept.n;
+    kept_total += prune ? npruned : nscored;
     // running top-k: survivors + this range, cut at the topk-th score (all
     // entries tied with it stay)
     Pairs cat;
@@ -2303,7 +2304,14 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
   }
   if(part) {
     // the part's running top-k, ties at its cut included: the union over
-    // the parts holds the whole search's top-k
+    // the parts holds the whole search's top-k (ascending determinants)
+    if(surv.n) {
+      uint64_t* kt = A.get<uint64_t>(surv.n * NW + NW);
+      double* rt2 = A.get<double>(surv.n + 1);
+      radix_sort<NW, double>(surv.keys, surv.rv, kt, rt2, surv.n, A);
+      A.release(kt);
+      A.release(rt2);
+    }
     h->part_states.resize(surv.n * NW);
     h->part_scores.resize(surv.n);
     if(surv.n) {

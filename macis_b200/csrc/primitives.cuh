@@ -258,9 +258,9 @@ __device__ __forceinline__ unsigned digit_of(const Key<NW>& k, int shift) {
   return unsigned(w >> (shift & 63)) & 255u;
 }
 
-template <int NW>
+template <int NW, class Digit>
 __global__ void __launch_bounds__(RS_THREADS)
-    radix_hist_k(const uint64_t* keys, size_t n, int shift, uint32_t* counts,
+    radix_hist_k(const uint64_t* keys, size_t n, Digit digit, uint32_t* counts,
                  unsigned nblocks) {
   __shared__ uint32_t h[256];
   h[threadIdx.x] = 0;
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(RS_THREADS)
 #pragma unroll 4
   for(int r = 0; r < RS_IPT; ++r) {
     size_t i = base + size_t(r) * RS_THREADS + threadIdx.x;
-    if(i < n) atomicAdd(&h[digit_of<NW>(load_key<NW>(keys, i), shift)], 1u);
+    if(i < n) atomicAdd(&h[digit(load_key<NW>(keys, i))], 1u);
   }
   __syncthreads();
   counts[size_t(threadIdx.x) * nblocks + blockIdx.x] = h[threadIdx.x];
@@ -376,17 +376,16 @@ __device__ __forceinline__ void rs_tile_pass(const uint64_t* keys,
 }
 
 // One digit pass with per-block bucket offsets from radix_hist_k + scan.
-template <int NW, typename P>
+template <int NW, typename P, class Digit>
 __global__ void __launch_bounds__(RS_THREADS, 4)
-    radix_scatter_k(const uint64_t* keys, const P* vals, size_t n, int shift,
+    radix_scatter_k(const uint64_t* keys, const P* vals, size_t n, Digit digit,
                     const uint64_t* offsets, unsigned nblocks,
                     uint64_t* keys_out, P* vals_out) {
   // issued before the ranking: its latency hides behind the tile loads
   const uint64_t my_off =
       offsets[size_t(threadIdx.x) * nblocks + blockIdx.x];
-  rs_tile_pass<NW, P>(keys, vals, n, ShiftDigit<NW>{shift},
-                      size_t(blockIdx.x) * RS_TILE, keys_out, vals_out,
-                      [&](int, uint32_t) { return my_off; });
+  rs_tile_pass<NW, P>(keys, vals, n, digit, size_t(blockIdx.x) * RS_TILE,
+                      keys_out, vals_out, [&](int, uint32_t) { return my_off; });
 }
 
 // ------------------------------------------------------ one-sweep passes
@@ -478,6 +477,45 @@ __global__ void __launch_bounds__(RS_THREADS, 4)
       });
 }
 
+// Classic digit passes (per-block histogram, scan, scatter) over n records,
+// with their scratch.
+template <int NW, typename P>
+struct DigitPasses {
+  size_t n;
+  Arena& A;
+  unsigned nblocks;
+  uint32_t* counts = nullptr;
+  uint64_t* offs = nullptr;
+  DigitPasses(size_t n_, Arena& A_)
+      : n(n_), A(A_), nblocks(unsigned((n_ + RS_TILE - 1) / RS_TILE)) {}
+  template <class Digit>
+  void run(const uint64_t* kin, const P* vin, uint64_t* kout, P* vout,
+           Digit digit) {
+    constexpr size_t stage = rs_stage_bytes<NW, P>();
+    if(!counts) {
+      MB_CUDA(cudaFuncSetAttribute(radix_scatter_k<NW, P, Digit>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(stage)));
+      counts = A.get<uint32_t>(size_t(256) * nblocks);
+      offs = A.get<uint64_t>(size_t(256) * nblocks);
+    }
+    radix_hist_k<NW><<<nblocks, RS_THREADS, 0, A.s>>>(kin, n, digit, counts,
+                                                      nblocks), note_launch();
+    exclusive_scan<uint32_t, uint64_t>(counts, offs, size_t(256) * nblocks,
+                                       nullptr, A);
+    radix_scatter_k<NW, P><<<nblocks, RS_THREADS, stage, A.s>>>(
+        kin, vin, n, digit, offs, nblocks, kout, vout), note_launch();
+  }
+  void release() {
+    if(counts) {
+      A.release(counts);
+      A.release(offs);
+    }
+    counts = nullptr;
+    offs = nullptr;
+  }
+};
+
 // Stable sort of n keys (NW words each) with optional payload. The sorted
 // result ends in (keys, vals); keys_alt/vals_alt are scratch of the same
 // size. Returns the number of digit passes run.
@@ -494,9 +532,6 @@ int radix_sort(uint64_t* keys, P* vals, uint64_t* keys_alt, P* vals_alt,
   MB_CUDA(cudaStreamSynchronize(A.s));
   const unsigned nblocks = unsigned((n + RS_TILE - 1) / RS_TILE);
   constexpr size_t stage = rs_stage_bytes<NW, P>();
-  MB_CUDA(cudaFuncSetAttribute(radix_scatter_k<NW, P>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(stage)));
   int passes = 0;
   std::vector<int> shifts;
   for(int w = 0; w < NW; ++w)
@@ -505,20 +540,9 @@ int radix_sort(uint64_t* keys, P* vals, uint64_t* keys_alt, P* vals_alt,
   const int np = int(shifts.size());
   uint64_t *kin = keys, *kout = keys_alt;
   P *vin = vals, *vout = vals_alt;
-  uint32_t* counts = nullptr;
-  uint64_t* offs = nullptr;
-  // classic pass: per-block histogram, scan, scatter
+  DigitPasses<NW, P> classic(n, A);
   auto classic_pass = [&](int shift) {
-    if(!counts) {
-      counts = A.get<uint32_t>(size_t(256) * nblocks);
-      offs = A.get<uint64_t>(size_t(256) * nblocks);
-    }
-    radix_hist_k<NW><<<nblocks, RS_THREADS, 0, A.s>>>(kin, n, shift, counts,
-                                                      nblocks), note_launch();
-    exclusive_scan<uint32_t, uint64_t>(counts, offs, size_t(256) * nblocks,
-                                       nullptr, A);
-    radix_scatter_k<NW, P><<<nblocks, RS_THREADS, stage, A.s>>>(
-        kin, vin, n, shift, offs, nblocks, kout, vout), note_launch();
+    classic.run(kin, vin, kout, vout, ShiftDigit<NW>{shift});
   };
   // The one-sweep passes are opt-in (MACIS_B200_SORT_ONESWEEP=1): measured
   // on the n = 48 ASCI searches with bin-grouped ranges, the classic passes
@@ -591,75 +615,6 @@ int radix_sort(uint64_t* keys, P* vals, uint64_t* keys_alt, P* vals_alt,
       MB_CUDA(cudaMemcpyAsync(vals, vin, n * sizeof(P), cudaMemcpyDeviceToDevice, A.s));
   }
   return passes;
-}
-
-// Counts of each digit value (< nbuckets <= 256) of a functor over the keys.
-template <int NW, class Digit>
-__global__ void __launch_bounds__(RS_THREADS)
-    rs_hist_fn_k(const uint64_t* keys, size_t n, Digit digit,
-                 unsigned long long* hist) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  for(size_t i = size_t(blockIdx.x) * RS_THREADS + threadIdx.x; i < n;
-      i += size_t(gridDim.x) * RS_THREADS)
-    atomicAdd(&h[digit(load_key<NW>(keys, i))], 1u);
-  __syncthreads();
-  if(h[threadIdx.x])
-    atomicAdd(hist + threadIdx.x, (unsigned long long)h[threadIdx.x]);
-}
-
-// Stable partition of (keys, vals) into (keys_out, vals_out) by the bucket
-// digit(key) < nbuckets <= 256 (one histogram read, one one-sweep pass;
-// the classic passes if a look-back gives up). Returns the nbuckets + 1
-// bucket offsets.
-template <int NW, typename P, class Digit>
-std::vector<size_t> stable_partition(const uint64_t* keys, const P* vals,
-                                     uint64_t* keys_out, P* vals_out,
-                                     size_t n, int nbuckets, Digit digit,
-                                     Arena& A) {
-  std::vector<size_t> off(size_t(nbuckets) + 1, 0);
-  if(n == 0) return off;
-  auto* hist = A.get<unsigned long long>(256);
-  MB_CUDA(cudaMemsetAsync(hist, 0, 256 * 8, A.s));
-  rs_hist_fn_k<NW><<<grid_for(n, RS_THREADS, 4 * size_t(num_sms())),
-                     RS_THREADS, 0, A.s>>>(keys, n, digit, hist), note_launch();
-  std::vector<unsigned long long> h(256);
-  MB_CUDA(cudaMemcpyAsync(h.data(), hist, 256 * 8, cudaMemcpyDeviceToHost,
-                          A.s));
-  MB_CUDA(cudaStreamSynchronize(A.s));
-  unsigned long long acc = 0;
-  for(int d = 0; d < 256; ++d) {
-    const unsigned long long c = h[d];
-    h[d] = acc;
-    acc += c;
-    if(d < nbuckets) off[size_t(d) + 1] = size_t(acc);
-  }
-  MB_REQUIRE(acc == n, MACIS_B200_EINVAL, "partition digit out of range");
-  auto* bucket = A.get<unsigned long long>(256);
-  MB_CUDA(cudaMemcpyAsync(bucket, h.data(), 256 * 8, cudaMemcpyHostToDevice,
-                          A.s));
-  const unsigned nblocks = unsigned((n + RS_TILE - 1) / RS_TILE);
-  constexpr size_t stage = rs_stage_bytes<NW, P>();
-  MB_CUDA(cudaFuncSetAttribute(rs_onesweep_k<NW, P, Digit>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(stage)));
-  uint64_t* status = A.get<uint64_t>(size_t(nblocks) * 256);
-  unsigned* counter = A.get<unsigned>(1);
-  int* err = A.get<int>(1);
-  MB_CUDA(cudaMemsetAsync(status, 0, size_t(nblocks) * 256 * 8, A.s));
-  MB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), A.s));
-  MB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), A.s));
-  rs_onesweep_k<NW, P, Digit><<<nblocks, RS_THREADS, stage, A.s>>>(
-      keys, vals, n, digit, bucket, status, counter, err, keys_out, vals_out,
-      RS_SPIN_LIMIT), note_launch();
-  int e = 0;
-  MB_CUDA(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, A.s));
-  MB_CUDA(cudaStreamSynchronize(A.s));
-  MB_REQUIRE(e == 0, MACIS_B200_ETIMEOUT,
-             "partition pass: a look-back wait gave up");
-  A.release(status);
-  return off;
 }
 
 // Device bytes that allocations can still obtain: free memory plus what the

@@ -347,3 +347,42 @@ def test_ranked_keys_and_alpha_lists_match_plain_search(monkeypatch, nbits, n,
                 assert got[3]["alpha_strings"] == 3
             assert (got[3]["key_bits"] > 0) == (ranks == "1")
             same(got, plain)
+@pytest.mark.parametrize("nbits,n,k,ncore", [(64, 24, 6, 40), (128, 48, 12, 12),
+                                             (256, 70, 8, 8)])
+def test_grouped_candidates_match_accumulated_list(monkeypatch, nbits, n, k,
+                                                   ncore):
+    """The search's grouping of contributions by key hash, with the score
+    threshold it samples from a part of the range, against the top-k taken
+    from the fully sorted accumulated list (asci_pairs): 1 to 3 hash digits,
+    with ranked and determinant keys, one range and several, cuts from one
+    determinant up to more than there are (no threshold, every candidate
+    written). A single core determinant gives pairs of equal scores."""
+    from cases import core_set
+    T, V = mb.synthetic_integrals(n, 3)
+    cd, C = core_set(n, k, ncore, nbits)
+    H = mb.HamiltonianGenerator(T, V, nbits)
+    E0 = float(H.matrix_element(cd[:1], cd[:1])) - 0.5
+    for nc in (1, 3, ncore):
+        core, c = cd[:nc], C[:nc]
+        st, rv = mb.asci_pairs(_settings(), core, E0, c, H)
+        W = nbits // 64
+        iscore = np.zeros(len(st), dtype=bool)
+        for d in core:
+            iscore |= (st == d).all(axis=1)
+        ok = (rv != 0) & ~iscore
+        st, rv = st[ok], np.abs(rv[ok])
+        order = np.lexsort(tuple(st[:, w] for w in range(W)) + (-rv,))
+        for ranks, cap in (("0", None), ("1", None), ("1", "200000")):
+            monkeypatch.setenv("MACIS_B200_ASCI_RANKS", ranks)
+            if cap:
+                monkeypatch.setenv("MACIS_B200_ASCI_BATCH_PAIRS", cap)
+            else:
+                monkeypatch.delenv("MACIS_B200_ASCI_BATCH_PAIRS", raising=False)
+            for top in (1, 100, 2047, len(st) // 3, len(st) + 5):
+                got = mb.asci_search(_settings(), top + nc, core, E0, c, n, H)
+                stat = mb.last_search_stats(H)
+                sel = st[order[:top]]
+                sel = sel[np.lexsort(tuple(sel[:, w] for w in range(W)))]
+                assert np.array_equal(got, np.concatenate([sel, core]))
+                if stat["batches"] == 1:
+                    assert stat["kept_pairs"] == len(st)
