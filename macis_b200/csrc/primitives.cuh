@@ -131,6 +131,37 @@ __global__ void scan_apply_k(const TI* in, size_t n, TO* out,
   }
 }
 
+// Short inputs in one block and one launch, the total included: below
+// SCAN_SMALL the 3 to 5 launches of the two-level scan cost more than one
+// block's passes over the input (about 1.5 us per 8192 items).
+constexpr size_t SCAN_SMALL = 32768;
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(1024)
+    scan_small_k(const TI* in, size_t n, TO* out, TO* total) {
+  __shared__ TO sh[33];
+  TO carry = 0;
+  for(size_t base = 0; base < n; base += 1024 * SCAN_IPT) {
+    TO v[SCAN_IPT];
+    TO acc = 0;
+#pragma unroll
+    for(int i = 0; i < SCAN_IPT; ++i) {
+      const size_t j = base + size_t(threadIdx.x) * SCAN_IPT + i;
+      v[i] = j < n ? TO(in[j]) : TO(0);
+      acc += v[i];
+    }
+    TO tot;
+    TO pre = carry + block_excl_scan<TO>(acc, sh, &tot);
+#pragma unroll
+    for(int i = 0; i < SCAN_IPT; ++i) {
+      const size_t j = base + size_t(threadIdx.x) * SCAN_IPT + i;
+      if(j < n) out[j] = pre;
+      pre += v[i];
+    }
+    carry += tot;
+  }
+  if(total && threadIdx.x == 0) *total = carry;
+}
+
 // out[i] = sum_{j<i} in[j]; out may alias in. If total != nullptr the grand
 // total is written to *total (device pointer). Returns nothing; sync-free.
 template <typename TI, typename TO>
@@ -139,14 +170,11 @@ void exclusive_scan(const TI* in, TO* out, size_t n, TO* total, Arena& A) {
     if(total) MB_CUDA(cudaMemsetAsync(total, 0, sizeof(TO), A.s));
     return;
   }
-  size_t nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-  if(nb == 1) {
-    TO* sums = A.get<TO>(2);
-    scan_reduce_k<TI, TO><<<1, SCAN_THREADS, 0, A.s>>>(in, n, sums), note_launch();
-    if(total) MB_CUDA(cudaMemcpyAsync(total, sums, sizeof(TO), cudaMemcpyDeviceToDevice, A.s));
-    scan_apply_k<TI, TO><<<1, SCAN_THREADS, 0, A.s>>>(in, n, out, nullptr), note_launch();
+  if(n <= SCAN_SMALL) {
+    scan_small_k<TI, TO><<<1, 1024, 0, A.s>>>(in, n, out, total), note_launch();
     return;
   }
+  size_t nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
   TO* sums = A.get<TO>(nb + 1);
   scan_reduce_k<TI, TO><<<unsigned(nb), SCAN_THREADS, 0, A.s>>>(in, n, sums), note_launch();
   exclusive_scan<TO, TO>(sums, sums, nb, total, A);
