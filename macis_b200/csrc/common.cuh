@@ -254,6 +254,28 @@ __device__ __forceinline__ double me_os_double(const Ints& I, uint32_t ea,
   return sign *
          __ldg(I.V + idx4(ex_v1(ea), ex_o1(ea), ex_v1(eb), ex_o1(eb), I.n));
 }
+// The element of a double excitation of any class (same-spin alpha or beta,
+// opposite-spin): the same instructions for all three, so that a warp whose
+// lanes hold different classes does not run them one after another.
+template <int NSW>
+__device__ __forceinline__ double me_double(const Ints& I, Spin<NSW> ba,
+                                            Spin<NSW> bb, Spin<NSW> ka,
+                                            Spin<NSW> kb) {
+  const Spin<NSW> ea = ba ^ ka, eb = bb ^ kb;
+  const int ca = sp_popc(ea);
+  const bool os = ca == 2, beta = ca == 0;
+  // first excitation: alpha, or beta when only beta differs
+  Spin<NSW> k = beta ? kb : ka, e = beta ? eb : ea;
+  const int o1 = sp_lowest(k & e), v1 = sp_lowest((k ^ e) & e);
+  int par = o1 < v1 ? sp_count_between(k, o1, v1) : sp_count_between(k, v1, o1);
+  // second: the beta one, or what is left of the same spin
+  k = os ? kb : sp_flip(sp_flip(k, o1), v1);
+  e = os ? eb : sp_flip(sp_flip(e, o1), v1);
+  const int o2 = sp_lowest(k & e), v2 = sp_lowest((k ^ e) & e);
+  par += o2 < v2 ? sp_count_between(k, o2, v2) : sp_count_between(k, v2, o2);
+  const double v = __ldg((os ? I.V : I.G) + idx4(v1, o1, v2, o2, I.n));
+  return (par & 1) ? -v : v;
+}
 // matrix_element_diag (matrix_elements.hpp:98-125), reference summation
 // order.
 template <int NSW>

@@ -1272,17 +1272,71 @@ __device__ __forceinline__ void gen_enumerate(const GenData& g, int32_t rg,
         }
         continue;
       }
-      for(int64_t base = m0; base < m1; base += 32) {
-        const int64_t m = base + lane;
-        bool act = m < m1;
-        int pb = 99;
-        if(act) pb = sp_popc(ld_spin<NSW>(g.sbeta, m) ^ bb);
-        act = act && pb <= limit;
-        emit(act, m, gg, ppa, pb);
+      // four loads in flight: groups are a few hundred members, and the loop
+      // waits for each load
+      for(int64_t base = m0; base < m1; base += 128) {
+        int pb[4];
+#pragma unroll
+        for(int u = 0; u < 4; ++u) {
+          const int64_t m = base + 32 * u + lane;
+          pb[u] = m < m1 ? sp_popc(ld_spin<NSW>(g.sbeta, m) ^ bb) : 99;
+        }
+#pragma unroll
+        for(int u = 0; u < 4; ++u)
+          if(base + 32 * u < m1)
+            emit(pb[u] <= limit, base + 32 * u + lane, gg, ppa, pb[u]);
       }
     }
   }
 }
+
+// The connected kets of a row are a few of the members that gen_enumerate
+// tests (1.5 % on an n = 48 list of 1.5e5 determinants), so its chunks of 32
+// hold one or two each. gen_pairs queues them and calls eval(on, m, ket
+// group, is_double) with 32 at a time, doubles and the rest (singles, the
+// diagonal, lists of mixed electron counts) apart: an element then costs a
+// lane's share of the warp's instructions and not all of them. q: 128
+// entries of shared memory per warp.
+template <int NSW, class F>
+__device__ __forceinline__ void gen_pairs(const GenData& g, int32_t rg,
+                                          Spin<NSW> ba, Spin<NSW> bb,
+                                          uint8_t* ov, uint64_t* q, F&& eval) {
+  const int lane = threadIdx.x & 31;
+  int n[2] = {0, 0};  // queued: others, doubles
+  auto run = [&](int c, int cnt) {
+    const bool on = lane < cnt;
+    const uint64_t e = on ? q[64 * c + lane] : 0;
+    eval(on, int64_t(e & 0xffffffffu), int32_t(e >> 32), c == 1);
+  };
+  gen_enumerate<NSW>(g, rg, ba, bb, ov,
+                     [&](bool act, int64_t m, int32_t kg, int pa, int pb) {
+    if(!__any_sync(0xffffffffu, act)) return;
+    const bool dbl = pa + pb == 4 && !(pa & 1);
+#pragma unroll
+    for(int c = 0; c < 2; ++c) {
+      const bool mine = act && dbl == (c == 1);
+      const unsigned msk = __ballot_sync(0xffffffffu, mine);
+      if(mine)
+        q[64 * c + n[c] + __popc(msk & lanemask_lt())] =
+            (uint64_t(uint32_t(kg)) << 32) | uint32_t(m);
+      n[c] += __popc(msk);
+      if(n[c] >= 32) {
+        __syncwarp();
+        run(c, 32);
+        n[c] -= 32;
+        const uint64_t t = lane < n[c] ? q[64 * c + 32 + lane] : 0;
+        __syncwarp();
+        if(lane < n[c]) q[64 * c + lane] = t;
+      }
+    }
+  });
+  __syncwarp();
+#pragma unroll
+  for(int c = 0; c < 2; ++c)
+    if(n[c]) run(c, n[c]);
+  __syncwarp();
+}
+constexpr int GEN_SCRATCH = 256 + 128 * 8;  // bytes per warp: ov, q
 
 template <int NBITS>
 __global__ void __launch_bounds__(HB_THREADS)
@@ -1324,7 +1378,7 @@ __global__ void __launch_bounds__(HB_THREADS)
   constexpr int NSW = D::NSW;
   __shared__ uint32_t s_col[HB_WARPS][GEN_CAP];
   __shared__ double s_val[HB_WARPS][GEN_CAP];
-  // orbital lists of the bra beta, 256 bytes per warp: dynamic, since the
+  // orbital lists of the bra beta and the pair queues: dynamic, since the
   // candidate buffers take the whole static allowance
   extern __shared__ __align__(16) uint8_t gen_ov[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1348,14 +1402,17 @@ __global__ void __launch_bounds__(HB_THREADS)
     const Spin<NSW> ba = D::alpha(bd), bb = D::beta(bd);
     const double hd = hdiag[row];
     int64_t c = 0;
-    gen_enumerate<NSW>(g, rg, ba, bb, gen_ov + wid * 256, [&](bool act, int64_t m,
-                                                 int32_t kg, int pa, int pb) {
+    gen_pairs<NSW>(g, rg, ba, bb, gen_ov + wid * GEN_SCRATCH,
+                   reinterpret_cast<uint64_t*>(gen_ov + wid * GEN_SCRATCH + 256),
+                   [&](bool act, int64_t m, int32_t kg, bool dbl) {
       double h = 0;
       uint32_t col = 0;
       if(act) {
         const Spin<NSW> ka = ld_spin<NSW>(g.kalpha, kg);
         const Spin<NSW> kb = ld_spin<NSW>(g.sbeta, m);
-        if(pa == 0 && pb == 0)
+        if(dbl)
+          h = me_double(I, ba, bb, ka, kb);
+        else if(ka == ba && kb == bb)
           h = hd;
         else
           h = me_generic(I, ba, bb, ka, kb);
@@ -1929,7 +1986,7 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     // what is free; short rows of the chunk are written by the same launch.
     int64_t lchunk = int64_t(0.7 * double(device_bytes_available()) / 32.0);
     lchunk = std::max<int64_t>(lchunk, int64_t(1) << 20);
-    constexpr int gen_dyn = HB_WARPS * 256;
+    constexpr int gen_dyn = HB_WARPS * GEN_SCRATCH;
     MB_CUDA(cudaFuncSetAttribute(gen_fill_k<NBITS, CI, VT>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  gen_dyn));
@@ -2108,16 +2165,20 @@ __global__ void __launch_bounds__(HB_THREADS)
       const uint64_t* bd = dets + row * D::NW;
       const Spin<NSW> ba = D::alpha(bd), bb = D::beta(bd);
       const double hd = hdiag[row];
-      gen_enumerate<NSW>(g, rg, ba, bb, gen_ov + wid * 256,
-                         [&](bool act, int64_t m, int32_t kg, int pa, int pb) {
+      gen_pairs<NSW>(g, rg, ba, bb, gen_ov + wid * GEN_SCRATCH,
+                     reinterpret_cast<uint64_t*>(gen_ov + wid * GEN_SCRATCH + 256),
+                     [&](bool act, int64_t m, int32_t kg, bool dbl) {
         if(act) {
           const uint32_t col = g.sidx[m];
+          const Spin<NSW> ka = ld_spin<NSW>(g.kalpha, kg);
+          const Spin<NSW> kb = ld_spin<NSW>(g.sbeta, m);
           double h;
-          if(pa == 0 && pb == 0)
+          if(dbl)
+            h = me_double(I, ba, bb, ka, kb);
+          else if(ka == ba && kb == bb)
             h = hd;
           else
-            h = me_generic(I, ba, bb, ld_spin<NSW>(g.kalpha, kg),
-                           ld_spin<NSW>(g.sbeta, m));
+            h = me_generic(I, ba, bb, ka, kb);
           if(fabs(h) > thresh) {
             if(mixed && int64_t(col) != row) h = double(float(h));
             acc += h * x[col];
@@ -2188,7 +2249,7 @@ void hop_apply(const macis_b200_hop* op, double alpha, const double* x,
                double beta, double* y) {
   cudaStream_t s = op->stream;
   const unsigned gr = grid_for(size_t(op->n), HB_WARPS, size_t(num_sms()) * 16);
-  constexpr int dyn = HB_WARPS * 256;
+  constexpr int dyn = HB_WARPS * GEN_SCRATCH;
   const Ints I = op->I;
 #define MB_HOP_APPLY(NB)                                                     \
   gen_apply_k<NB><<<gr, HB_THREADS, dyn, s>>>(I, op->g, op->dets, op->n,     \
@@ -2361,7 +2422,7 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
   cudaStream_t s = h->stream;
   Arena A(s);
   const unsigned gr = grid_for(n, HB_WARPS, size_t(num_sms()) * 16);
-  constexpr int dyn = HB_WARPS * 256;
+  constexpr int dyn = HB_WARPS * GEN_SCRATCH;
 #define MB_RDM(NB)                                                          \
   {                                                                         \
     const GenData g = gen_plan<NB>(h, dets, n, dets, n, true, 0, A);        \
