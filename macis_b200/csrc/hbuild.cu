@@ -2290,105 +2290,74 @@ __device__ __forceinline__ void rdm_add(double* a, size_t i, double v) {
   atomicAdd(a + i, v);
 }
 
-// Contributions of one (bra, ket) pair: rdm_contributions and its parts
-// (include/macis/util/rdms.hpp:15-131), dispatched in the same order (the
-// two-body branches only when trdm is given). ordm(p,q) = ordm[p + q n],
-// trdm(p,q,r,s) = trdm[p + n (q + n (r + n s))].
+// Sums of rdm_contributions (include/macis/util/rdms.hpp:15-131) over all
+// (bra, ket) pairs, one entry for what the reference adds to several: a pair
+// costs 1 atomic instead of 2 (opposite-spin doubles), 1 instead of 4 (same
+// spin), and a single 1 per occupied orbital instead of 4 or 2; rdm_expand_k
+// then forms every element of the 2-RDM from the entries that reach it.
+// Indices as the 2-RDM's, (p,q,r,s) at p + n (q + n (r + n s)).
+struct RdmSums {
+  double* os;     // n^4: (v1, o1, v2, o2), alpha and beta excitation
+  double* ss;     // n^4: (v1, o1, v2, o2) of double_ex, both spins
+  double* ss1;    // n^3: (v1, o1, p), p occupied in the excited spin
+  double* os1;    // n^3: (v1, o1, p), p occupied in the other spin
+  double* diag;   // per row: the sum over its pairs with itself
+  double* dss;    // n^2: (p, q) both occupied in one spin, over both spins
+  double* dos;    // n^2: p occupied in alpha, q in beta
+};
+
+// One pair with at least two determinants apart by an even count, in the
+// reference's dispatch (:15-66); pairs of the diagonal branch return true.
 template <int NSW>
-__device__ void rdm_pair(Spin<NSW> ba, Spin<NSW> bb, Spin<NSW> ka,
-                         Spin<NSW> kb, double val, int n, double* ordm,
-                         double* trdm) {
+__device__ __forceinline__ bool rdm_pair(Spin<NSW> ba, Spin<NSW> bb,
+                                         Spin<NSW> ka, Spin<NSW> kb,
+                                         double val, int n, double* ordm,
+                                         bool two, const RdmSums& S) {
   const int ca = sp_popc(ba ^ ka), cb = sp_popc(bb ^ kb);
-  if(ca + cb > 4) return;
-  auto t4 = [&](int p, int q, int r, int s, double v) {
-    rdm_add(trdm, size_t(p) + size_t(n) * (q + size_t(n) * (r + size_t(n) * s)),
-            v);
-  };
-  if((ca == 4 || cb == 4) && trdm) {  // rdm_contributions_4, :15-25
+  if(ca + cb > 4) return false;
+  auto at = [n](int p, int q, int r) { return size_t(p) + size_t(n) * (q + size_t(n) * r); };
+  if((ca == 4 || cb == 4) && two) {  // rdm_contributions_4, :15-25
     const uint32_t e = ca == 4 ? double_ex(ba, ka) : double_ex(bb, kb);
-    const int o1 = ex_o1(e), v1 = ex_v1(e), o2 = ex_o2(e), v2 = ex_v2(e);
-    const double v = val * (ex_sgn(e) * 0.5);
-    t4(v1, o1, v2, o2, v);
-    t4(v2, o1, v1, o2, -v);
-    t4(v1, o2, v2, o1, -v);
-    t4(v2, o2, v1, o1, v);
-  } else if(ca == 2 && cb == 2 && trdm) {  // rdm_contributions_22, :27-41
+    rdm_add(S.ss, at(ex_v1(e), ex_o1(e), ex_v2(e)) + size_t(n) * n * n * ex_o2(e),
+            val * ex_sgn(e));
+  } else if(ca == 2 && cb == 2 && two) {  // rdm_contributions_22, :27-41
     const uint32_t ea = single_ex(ba, ka), eb = single_ex(bb, kb);
-    const double v = val * (ex_sgn(ea) * ex_sgn(eb) * 0.5);
-    t4(ex_v1(ea), ex_o1(ea), ex_v1(eb), ex_o1(eb), v);
-    t4(ex_v1(eb), ex_o1(eb), ex_v1(ea), ex_o1(ea), v);
+    rdm_add(S.os, at(ex_v1(ea), ex_o1(ea), ex_v1(eb)) + size_t(n) * n * n * ex_o1(eb),
+            val * (ex_sgn(ea) * ex_sgn(eb)));
   } else if(ca == 2 || cb == 2) {  // rdm_contributions_2, :43-66
     const bool a = ca == 2;
     const uint32_t e = a ? single_ex(ba, ka) : single_ex(bb, kb);
-    const Spin<NSW> occ_s = a ? ba : bb, occ_o = a ? bb : ba;
     const int o1 = ex_o1(e), v1 = ex_v1(e);
-    const double sg = ex_sgn(e);
-    rdm_add(ordm, size_t(v1) + size_t(n) * o1, sg * val);
-    if(trdm) {
-      const double v = val * (sg * 0.5);
-      for(Spin<NSW> s = occ_s; sp_popc(s);) {
+    const double v = ex_sgn(e) * val;
+    rdm_add(ordm, size_t(v1) + size_t(n) * o1, v);
+    if(two) {
+      for(Spin<NSW> s = a ? ba : bb; sp_popc(s);) {
         const int p = sp_lowest(s);
         s = sp_flip(s, p);
-        t4(v1, o1, p, p, v);
-        t4(p, p, v1, o1, v);
-        t4(v1, p, p, o1, -v);
-        t4(p, o1, v1, p, -v);
+        rdm_add(S.ss1, at(v1, o1, p), v);
       }
-      for(Spin<NSW> s = occ_o; sp_popc(s);) {
+      for(Spin<NSW> s = a ? bb : ba; sp_popc(s);) {
         const int p = sp_lowest(s);
         s = sp_flip(s, p);
-        t4(v1, o1, p, p, v);
-        t4(p, p, v1, o1, v);
+        rdm_add(S.os1, at(v1, o1, p), v);
       }
     }
-  } else {  // rdm_contributions_diag, :68-99
-    for(Spin<NSW> s = ba; sp_popc(s);) {
-      const int p = sp_lowest(s);
-      s = sp_flip(s, p);
-      rdm_add(ordm, size_t(p) * (n + 1), val);
-    }
-    for(Spin<NSW> s = bb; sp_popc(s);) {
-      const int p = sp_lowest(s);
-      s = sp_flip(s, p);
-      rdm_add(ordm, size_t(p) * (n + 1), val);
-    }
-    if(trdm) {
-      const double v = val * 0.5;
-      for(int spin = 0; spin < 2; ++spin) {
-        const Spin<NSW> o = spin ? bb : ba;
-        for(Spin<NSW> sq = o; sp_popc(sq);) {
-          const int q = sp_lowest(sq);
-          sq = sp_flip(sq, q);
-          for(Spin<NSW> sp = o; sp_popc(sp);) {
-            const int p = sp_lowest(sp);
-            sp = sp_flip(sp, p);
-            t4(p, p, q, q, v);
-            t4(p, q, p, q, -v);
-          }
-        }
-      }
-      for(Spin<NSW> sq = bb; sp_popc(sq);) {
-        const int q = sp_lowest(sq);
-        sq = sp_flip(sq, q);
-        for(Spin<NSW> sp = ba; sp_popc(sp);) {
-          const int p = sp_lowest(sp);
-          sp = sp_flip(sp, p);
-          t4(p, p, q, q, v);
-          t4(q, q, p, p, v);
-        }
-      }
-    }
+  } else {
+    return true;  // rdm_contributions_diag, :68-99
   }
+  return false;
 }
 
 // form_rdms (double_loop.hpp:117-165) over one determinant list: every
 // (bra, ket) pair within four spin-orbital differences with |C_i C_j| >
 // 1e-16 adds its contributions. One warp per bra row; the pairs come from
-// the general build's enumeration; sums are atomic (order not fixed).
+// the general build's enumeration; sums are atomic (order not fixed). The
+// contributions of the diagonal branch depend on the bra alone: their sum
+// per row goes to S.diag.
 template <int NBITS>
 __global__ void __launch_bounds__(HB_THREADS)
     rdm_k(GenData g, const uint64_t* dets, int64_t n, const double* C,
-          int norb, double* ordm, double* trdm) {
+          int norb, double* ordm, int two, RdmSums S) {
   using D = DetTraits<NBITS>;
   constexpr int NSW = D::NSW;
   extern __shared__ __align__(16) uint8_t gen_ov[];
@@ -2397,18 +2366,88 @@ __global__ void __launch_bounds__(HB_THREADS)
   for(int64_t row = int64_t(blockIdx.x) * HB_WARPS + wid; row < n;
       row += nwarp) {
     const int32_t rg = g.rowgroup[row];
-    if(rg < 0) continue;
-    const uint64_t* bd = dets + row * D::NW;
-    const Spin<NSW> ba = D::alpha(bd), bb = D::beta(bd);
-    const double ci = C[row];
-    gen_enumerate<NSW>(g, rg, ba, bb, gen_ov + wid * 256,
-                       [&](bool act, int64_t m, int32_t kg, int, int) {
-      if(!act) return;
-      const double val = ci * C[g.sidx[m]];
-      if(!(fabs(val) > 1e-16)) return;
-      rdm_pair<NSW>(ba, bb, ld_spin<NSW>(g.kalpha, kg),
-                    ld_spin<NSW>(g.sbeta, m), val, norb, ordm, trdm);
-    });
+    double dsum = 0.0;
+    if(rg >= 0) {
+      const uint64_t* bd = dets + row * D::NW;
+      const Spin<NSW> ba = D::alpha(bd), bb = D::beta(bd);
+      const double ci = C[row];
+      gen_pairs<NSW>(g, rg, ba, bb, gen_ov + wid * GEN_SCRATCH,
+                     reinterpret_cast<uint64_t*>(gen_ov + wid * GEN_SCRATCH + 256),
+                     [&](bool act, int64_t m, int32_t kg, bool) {
+        if(!act) return;
+        const double val = ci * C[g.sidx[m]];
+        if(!(fabs(val) > 1e-16)) return;
+        if(rdm_pair<NSW>(ba, bb, ld_spin<NSW>(g.kalpha, kg),
+                         ld_spin<NSW>(g.sbeta, m), val, norb, ordm, two != 0, S))
+          dsum += val;
+      });
+#pragma unroll
+      for(int o = 16; o > 0; o >>= 1)
+        dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
+    }
+    if((threadIdx.x & 31) == 0) S.diag[row] = dsum;
+  }
+}
+
+// Diagonal branch: the rows' sums over the pairs of orbitals occupied in
+// them. A block takes DG_ROWS rows, its threads the orbital pairs, and adds
+// one partial sum per pair: atomics per orbital pair and block, not per row
+// (every row adds to the pairs of the deepest orbitals).
+constexpr int DG_ROWS = 128;
+template <int NBITS>
+__global__ void rdm_diag_k(const uint64_t* dets, int64_t n, const double* w,
+                           int norb, double* ordm, int two, RdmSums S) {
+  using D = DetTraits<NBITS>;
+  constexpr int NSW = D::NSW;
+  __shared__ uint64_t sd[DG_ROWS * D::NW];
+  __shared__ double sw[DG_ROWS];
+  const int64_t r0 = int64_t(blockIdx.x) * DG_ROWS;
+  const int nr = int(n - r0 < DG_ROWS ? n - r0 : DG_ROWS);
+  for(int i = threadIdx.x; i < nr * D::NW; i += blockDim.x)
+    sd[i] = dets[r0 * D::NW + i];
+  for(int i = threadIdx.x; i < nr; i += blockDim.x) sw[i] = w[r0 + i];
+  __syncthreads();
+  const int npair = two ? norb * norb : norb;
+  for(int x = threadIdx.x; x < npair; x += blockDim.x) {
+    const int p = two ? x % norb : x, q = two ? x / norb : x;
+    double one = 0.0, ss = 0.0, os = 0.0;
+    for(int r = 0; r < nr; ++r) {
+      const double v = sw[r];
+      const Spin<NSW> a = D::alpha(sd + r * D::NW), b = D::beta(sd + r * D::NW);
+      const int ap = sp_test(a, p), bp = sp_test(b, p);
+      const int aq = sp_test(a, q), bq = sp_test(b, q);
+      if(p == q) one += double(ap + bp) * v;
+      ss += double((ap & aq) + (bp & bq)) * v;
+      if(ap & bq) os += v;
+    }
+    if(p == q && one != 0.0) rdm_add(ordm, size_t(p) * (norb + 1), one);
+    if(two) {
+      if(ss != 0.0) rdm_add(S.dss, size_t(x), ss);
+      if(os != 0.0) rdm_add(S.dos, size_t(x), os);
+    }
+  }
+}
+
+// trdm += the elements formed from the sums (rdms.hpp:15-99 gathered by
+// target element instead of scattered by pair).
+__global__ void rdm_expand_k(RdmSums S, int n, double* trdm) {
+  const size_t n2 = size_t(n) * n, n4 = n2 * n2;
+  for(size_t x = size_t(blockIdx.x) * blockDim.x + threadIdx.x; x < n4;
+      x += size_t(gridDim.x) * blockDim.x) {
+    const int p = int(x % n), q = int(x / n % n), r = int(x / n2 % n),
+              s = int(x / n2 / n);
+    auto a4 = [n](int i, int j, int k, int l) { return idx4(i, j, k, l, n); };
+    auto a3 = [n](int i, int j, int k) { return size_t(i) + size_t(n) * (j + size_t(n) * k); };
+    double v = S.os[x] + S.os[a4(r, s, p, q)];
+    v += S.ss[x] + S.ss[a4(r, s, p, q)] - S.ss[a4(r, q, p, s)] - S.ss[a4(p, s, r, q)];
+    if(r == s) v += S.ss1[a3(p, q, r)] + S.os1[a3(p, q, r)];
+    if(p == q) v += S.ss1[a3(r, s, p)] + S.os1[a3(r, s, p)];
+    if(q == r) v -= S.ss1[a3(p, s, q)];
+    if(p == s) v -= S.ss1[a3(r, q, p)];
+    if(p == q && r == s)
+      v += S.dss[p + n * r] + S.dos[p + n * r] + S.dos[r + n * p];
+    if(p == r && q == s) v -= S.dss[p + n * q];
+    trdm[x] += 0.5 * v;
   }
 }
 
@@ -2423,11 +2462,30 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
   Arena A(s);
   const unsigned gr = grid_for(n, HB_WARPS, size_t(num_sms()) * 16);
   constexpr int dyn = HB_WARPS * GEN_SCRATCH;
+  const size_t n1 = size_t(h->norb), n3 = n1 * n1 * n1, n4 = n3 * n1;
+  RdmSums S{};
+  S.diag = A.get<double>(n);
+  if(trdm) {
+    const size_t tot = 2 * n4 + 2 * n3 + 2 * n1 * n1;
+    double* z = A.get<double>(tot);
+    MB_CUDA(cudaMemsetAsync(z, 0, tot * 8, s));
+    S.os = z;
+    S.ss = S.os + n4;
+    S.ss1 = S.ss + n4;
+    S.os1 = S.ss1 + n3;
+    S.dss = S.os1 + n3;
+    S.dos = S.dss + n1 * n1;
+  }
+  const int two = trdm ? 1 : 0;
+  const unsigned gd = grid_for(n, DG_ROWS);
 #define MB_RDM(NB)                                                          \
   {                                                                         \
     const GenData g = gen_plan<NB>(h, dets, n, dets, n, true, 0, A);        \
     rdm_k<NB><<<gr, HB_THREADS, dyn, s>>>(g, dets, int64_t(n), C, h->norb,  \
-                                         ordm, trdm),                       \
+                                         ordm, two, S),                     \
+        note_launch();                                                      \
+    rdm_diag_k<NB><<<gd, 256, 0, s>>>(dets, int64_t(n), S.diag, h->norb,    \
+                                      ordm, two, S),                        \
         note_launch();                                                      \
   }
   if(h->nbits == 64) {
@@ -2437,6 +2495,9 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
   } else {
     MB_RDM(256)
   }
+  if(trdm)
+    rdm_expand_k<<<grid_for(n4, 256, 16 * num_sms()), 256, 0, s>>>(
+        S, h->norb, trdm), note_launch();
 #undef MB_RDM
   MB_CUDA(cudaGetLastError());
   MB_CUDA(cudaStreamSynchronize(s));
