@@ -12,8 +12,8 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libmacis_b200.so")
-SOURCES = ["ham.cu", "hbuild.cu", "spmv.cu", "davidson.cu", "asci.cu", "mlp.cu",
-           "capi.cu"]
+SOURCES = ["ham.cu", "hbuild.cu", "spmv.cu", "davidson.cu", "eig.cpp", "asci.cu",
+           "mlp.cu", "capi.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
@@ -36,7 +36,7 @@ def build(verbose=False, jobs=None):
     objs, procs = [], []
     for src in SOURCES:
         s = os.path.join(CSRC, src)
-        o = os.path.join(objdir, src.replace(".cu", ".o"))
+        o = os.path.join(objdir, os.path.splitext(src)[0] + ".o")
         objs.append(o)
         if _stale(o, [s] + headers):
             cmd = [NVCC] + ARCH + FLAGS + ["-c", s, "-o", o]

@@ -671,6 +671,7 @@ int macis_b200_hop_davidson(const macis_b200_hop* op,
     dop.n = n;
     dop.diag = hop_diag(op);
     dop.s = s;
+    dop.pinned = hop_pinned(op);
     dop.apply = [op](const double* xin, double* y) {
       hop_apply(op, 1.0, xin, 0.0, y);
     };

@@ -3,17 +3,25 @@
 //
 // Basis V and A*V live in HBM (N x (max_m+1) FP64 each). Per iteration:
 //   AV_i = H V_i                                  (spmv.cu)
-//   row i of the Rayleigh matrix V^T AV           (multi-dot, FP64)
-//   k x k symmetric eigenproblem on the host      (cyclic Jacobi, FP64)
-//   X = V c, R = AV c - lambda X, |R|, W = -R/(D - lambda)   (one fused pass)
-//   CGS2 of W against V, normalise                (davidson.hpp:111-126)
+//   row i of the Rayleigh matrix V^T AV           (multidot_k, FP64)
+//   k x k symmetric eigenproblem on the host      (eig.cpp, lowest pair)
+//   X = V c, R = AV c - lambda X, |R|, W = -R/(D - lambda), then CGS2 of W
+//   against V and its norm (davidson.hpp:111-126) (dav_step_k, one launch)
 // The reference recomputes the full k x k product with gemm every
 // iteration; only its lower triangle enters syev (rayleigh_ritz.hpp:73-75),
 // and the entries of earlier rows do not change, so only the new row is
 // formed. Reductions are two-stage with a fixed order (deterministic).
+//
+// For a basis that L2 holds, an iteration is bound by launches and by the
+// two round trips to the host, so it is three launches (product, Rayleigh
+// row, step), the kernels write what the host needs (the row, |R|^2, phase
+// times) to page-locked memory with a sequence number that the host polls,
+// and the host decides on convergence while the step still orthonormalises.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "internal.hpp"
@@ -25,14 +33,27 @@ constexpr int DV_THREADS = 512;
 constexpr int DV_WARPS = DV_THREADS / 32;
 constexpr int DV_CHUNK = 8;  // columns held by one multi-dot block
 
-// The vector kernels of one iteration form a chain of short launches (for a
-// basis that L2 holds, each runs 2-4 us, about a launch latency), so they
-// are launched with programmatic serialization: the launch work of a kernel
-// overlaps its predecessor and dav_wait holds its first access back until
-// the predecessor has completed and its writes are visible.
+// Waits for the preceding kernel of the stream: these kernels are launched
+// with programmatic serialization, so that their launch work overlaps it.
 __device__ __forceinline__ void dav_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+__device__ __forceinline__ unsigned long long gpu_time_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// What the kernels report to the host, in page-locked host memory.
+struct DavReport {
+  volatile unsigned row_seq;   // the Rayleigh row of this number is there
+  volatile unsigned res_seq;   // |R|^2 of this number is there
+  volatile unsigned err;       // a grid barrier gave up
+  volatile double rn2;
+  // phase boundaries, ns: the row's kernel, the step's residual, its end
+  volatile unsigned long long t_row0, t_row1, t_res0, t_res1, t_end;
+  volatile double row[1];      // max_m + 1 entries
+};
 
 // Sum of acc[c] over the warp for 8 values at once: each step halves the
 // values a lane holds, 9 shuffles instead of 40. Lane l ends with the sum of
@@ -90,16 +111,19 @@ __device__ __forceinline__ double warp_sum_partials(const double* p, int nb,
   return a;
 }
 
-// out[c] = A[:, c] . v for c < ncol: block (x, y) sums rows x, x + gridDim.x,
-// ... (in units of DV_THREADS) of the DV_CHUNK columns from DV_CHUNK y, and
-// the last block of a chunk adds the chunk's partial sums in a fixed order
-// (one launch instead of two per 8 columns). HBM-bound for long vectors.
+// rep->row[c] = A[:, c] . v for c < ncol: block (x, y) sums rows x, x +
+// gridDim.x, ... (in units of DV_THREADS) of the DV_CHUNK columns from
+// DV_CHUNK y, the last block of a chunk adds the chunk's partial sums in a
+// fixed order, and the last chunk reports. HBM-bound for long vectors.
+// done: one counter per chunk, one for the chunks; t0: scratch.
 __global__ void __launch_bounds__(DV_THREADS)
     multidot_k(const double* __restrict__ A, int64_t lda, int ncol,
                const double* __restrict__ v, int64_t n, double* partial,
-               unsigned* done, double* out) {
+               unsigned* done, unsigned long long* t0, DavReport* rep,
+               unsigned seq) {
   __shared__ double sh[DV_WARPS][DV_CHUNK];
   dav_wait();
+  if(blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *t0 = gpu_time_ns();
   const int c0 = int(blockIdx.y) * DV_CHUNK;
   const int nc = ncol - c0 < DV_CHUNK ? ncol - c0 : DV_CHUNK;
   const double* Ac = A + c0 * lda;
@@ -124,60 +148,18 @@ __global__ void __launch_bounds__(DV_THREADS)
     for(int w = 0; w < DV_WARPS; ++w) t += sh[w][threadIdx.x];
     pc[blockIdx.x * DV_CHUNK + threadIdx.x] = t;
   }
-  if(last_block(done + blockIdx.y, gridDim.x) && wid < nc) {
+  if(!last_block(done + blockIdx.y, gridDim.x)) return;
+  if(wid < nc) {
     const double t = warp_sum_partials(pc + wid, int(gridDim.x), DV_CHUNK);
-    if(lane == 0) out[c0 + wid] = t;
+    if(lane == 0) rep->row[c0 + wid] = t;
   }
-}
-
-// Block sum of acc into partial[blockIdx.x]; the last block writes the total.
-__device__ __forceinline__ void grid_sum(double acc, double* partial,
-                                         unsigned* done, double* out) {
-  __shared__ double sh[DV_WARPS];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for(int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if(lane == 0) sh[wid] = acc;
-  __syncthreads();
-  if(threadIdx.x == 0) {
-    double t = 0;
-    for(int w = 0; w < DV_WARPS; ++w) t += sh[w];
-    partial[blockIdx.x] = t;
+  __threadfence_system();  // before the report of the last chunk
+  if(last_block(done + gridDim.y, gridDim.y) && threadIdx.x == 0) {
+    rep->t_row0 = *static_cast<volatile unsigned long long*>(t0);
+    rep->t_row1 = gpu_time_ns();
+    __threadfence_system();
+    rep->row_seq = seq;
   }
-  if(last_block(done, gridDim.x) && wid == 0) {
-    const double t = warp_sum_partials(partial, int(gridDim.x), 1);
-    if(lane == 0) *out = t;
-  }
-}
-
-// v -= A[:, 0:k] coef; with norm2 != nullptr also *norm2 = v . v after it.
-__global__ void __launch_bounds__(DV_THREADS)
-    cgs_update_k(const double* __restrict__ A, int64_t lda, int k,
-                 const double* __restrict__ coef, double* v, int64_t n,
-                 double* partial, unsigned* done, double* norm2) {
-  __shared__ double cf[1024];
-  dav_wait();
-  for(int c = threadIdx.x; c < k; c += blockDim.x) cf[c] = coef[c];
-  __syncthreads();
-  double acc = 0;
-  for(int64_t i = int64_t(blockIdx.x) * DV_THREADS + threadIdx.x; i < n;
-      i += int64_t(gridDim.x) * DV_THREADS) {
-    double s = 0;
-#pragma unroll 8
-    for(int c = 0; c < k; ++c) s += A[i + c * lda] * cf[c];
-    const double x = v[i] - s;
-    v[i] = x;
-    acc += x * x;
-  }
-  if(norm2) grid_sum(acc, partial, done, norm2);
-}
-
-__global__ void scale_k(double* v, int64_t n, const double* nrm2) {
-  dav_wait();
-  const double inv = 1. / sqrt(*nrm2);
-  for(int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-      i += int64_t(gridDim.x) * blockDim.x)
-    v[i] *= inv;
 }
 
 // Ritz coefficients passed with the launch (no copy to the device) up to
@@ -188,33 +170,175 @@ struct RitzCoef {
   const double* dev;  // used when not null
 };
 
-// X = V c; R = AV c - lam X; *rn2 = |R|^2; W = -R / (D - lam) into W.
-__global__ void __launch_bounds__(DV_THREADS)
-    ritz_residual_k(const double* __restrict__ V, const double* __restrict__ AV,
-                    int64_t n, int k, const __grid_constant__ RitzCoef rc,
-                    double lam, const double* __restrict__ D,
-                    double* __restrict__ X, double* __restrict__ W,
-                    double* partial, unsigned* done, double* rn2) {
-  __shared__ double cf[1024];
-  dav_wait();
-  for(int j = threadIdx.x; j < k; j += blockDim.x)
-    cf[j] = rc.dev ? rc.dev[j] : rc.c[j];
+struct StepArgs {
+  const double* V;
+  const double* AV;
+  int64_t n;
+  int k;             // basis vectors
+  int ritz;          // form X and the correction W (else W is given)
+  int ortho;         // CGS2 and normalise W
+  double lam;
+  const double* D;
+  double* X;
+  double* W;
+  double* partial;   // 2 x k x blocks, then 2 x blocks
+  unsigned* done;    // arrival counter
+  unsigned* bar;     // barrier counter, grows by `blocks` per barrier
+  unsigned bar0;     // its value before this launch
+  DavReport* rep;
+  unsigned seq;
+};
+
+// Barrier over the blocks of a cooperative launch (they are all resident).
+// The wait is bounded: a block that gives up reports it and the kernel ends.
+constexpr int DV_SPIN_LIMIT = 1 << 24;  // polls of about 0.5 us
+__device__ __forceinline__ bool grid_barrier(const StepArgs& a,
+                                             unsigned& target) {
+  __shared__ bool ok;
+  target += gridDim.x;
   __syncthreads();
-  double acc = 0;
-  for(int64_t i = int64_t(blockIdx.x) * DV_THREADS + threadIdx.x; i < n;
-      i += int64_t(gridDim.x) * DV_THREADS) {
-    double x = 0, av = 0;
-#pragma unroll 8
-    for(int j = 0; j < k; ++j) {
-      x += V[i + j * n] * cf[j];
-      av += AV[i + j * n] * cf[j];
+  if(gridDim.x == 1) return true;
+  if(threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(a.bar, 1u);
+    ok = false;
+    for(int t = 0; t < DV_SPIN_LIMIT; ++t) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+      if(int(v - target) >= 0) {
+        ok = true;
+        break;
+      }
     }
-    const double r = av - lam * x;
-    X[i] = x;
-    W[i] = -r / (D[i] - lam);
-    acc += r * r;
+    if(!ok) a.rep->err = 1;
   }
-  grid_sum(acc, partial, done, rn2);
+  __syncthreads();
+  return ok;
+}
+
+__device__ __forceinline__ double block_sum(double acc, double* sh) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for(int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  __syncthreads();
+  if(lane == 0) sh[wid] = acc;
+  __syncthreads();
+  double t = 0;
+  for(int w = 0; w < DV_WARPS; ++w) t += sh[w];
+  return t;
+}
+
+// One step behind the Rayleigh row: Ritz vector, residual and correction,
+//   X = V c; R = AV c - lam X; |R|^2; W = -R / (D - lam),
+// then gram_schmidt (davidson.hpp:111-126), W -= V (V^T W) twice and W /= |W|.
+// A thread keeps its rows through all phases; the column sums meet at three
+// grid barriers (their partial sums added by every block in the same order).
+// One cooperative launch: as five launches the same work took 2 to 4 us each
+// on a basis of 63,504 x 40, about a launch latency, whatever its size.
+// For long vectors it streams V three times and AV once from HBM.
+__global__ void __launch_bounds__(DV_THREADS, 2)
+    dav_step_k(StepArgs a, const __grid_constant__ RitzCoef rc) {
+  __shared__ double cf[1024];
+  __shared__ double shc[2][DV_WARPS][DV_CHUNK];
+  __shared__ double shb[DV_WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t n = a.n;
+  const int k = a.k, nb = int(gridDim.x);
+  const int64_t i0 = int64_t(blockIdx.x) * DV_THREADS + threadIdx.x;
+  const int64_t di = int64_t(nb) * DV_THREADS;
+  const double* __restrict__ V = a.V;
+  double* W = a.W;
+  double* pn = a.partial + size_t(2) * k * nb;  // |R|^2, then |W|^2
+  unsigned target = a.bar0;
+  if(blockIdx.x == 0 && threadIdx.x == 0 && a.ritz) a.rep->t_res0 = gpu_time_ns();
+  if(a.ritz) {
+    for(int j = threadIdx.x; j < k; j += DV_THREADS)
+      cf[j] = rc.dev ? rc.dev[j] : rc.c[j];
+    __syncthreads();
+    const double* __restrict__ AV = a.AV;
+    double acc = 0;
+    for(int64_t i = i0; i < n; i += di) {
+      double x = 0, av = 0;
+#pragma unroll 8
+      for(int j = 0; j < k; ++j) {
+        x += V[i + j * n] * cf[j];
+        av += AV[i + j * n] * cf[j];
+      }
+      const double r = av - a.lam * x;
+      a.X[i] = x;
+      W[i] = -r / (a.D[i] - a.lam);
+      acc += r * r;
+    }
+    const double t = block_sum(acc, shb);
+    if(threadIdx.x == 0) pn[blockIdx.x] = t;
+    if(last_block(a.done, unsigned(nb)) && wid == 0) {
+      const double s = warp_sum_partials(pn, nb, 1);
+      if(lane == 0) {
+        a.rep->rn2 = s;
+        a.rep->t_res1 = gpu_time_ns();
+        __threadfence_system();
+        a.rep->res_seq = a.seq;
+      }
+    }
+  }
+  if(a.ortho) {
+    for(int pass = 0; pass < 2; ++pass) {
+      // column sums of V^T W over this block's rows
+      double* pc = a.partial + size_t(pass) * k * nb;
+      for(int c0 = 0; c0 < k; c0 += DV_CHUNK) {
+        double acc[DV_CHUNK];
+#pragma unroll
+        for(int c = 0; c < DV_CHUNK; ++c) acc[c] = 0;
+        for(int64_t i = i0; i < n; i += di) {
+          const double x = W[i];
+#pragma unroll
+          for(int c = 0; c < DV_CHUNK; ++c)
+            if(c0 + c < k) acc[c] += V[i + (c0 + c) * n] * x;
+        }
+        double (*sh)[DV_CHUNK] = shc[(c0 / DV_CHUNK) & 1];
+        const double t = warp_sum8(acc);
+        if((lane & 3) == 0)
+          sh[wid][(lane >> 4) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = t;
+        __syncthreads();
+        if(threadIdx.x < DV_CHUNK && c0 + int(threadIdx.x) < k) {
+          double u = 0;
+#pragma unroll
+          for(int w = 0; w < DV_WARPS; ++w) u += sh[w][threadIdx.x];
+          pc[size_t(c0 + threadIdx.x) * nb + blockIdx.x] = u;
+        }
+      }
+      if(!grid_barrier(a, target)) return;
+      for(int c = wid; c < k; c += DV_WARPS) {
+        const double u = warp_sum_partials(pc + size_t(c) * nb, nb, 1);
+        if(lane == 0) cf[c] = u;
+      }
+      __syncthreads();
+      double acc = 0;
+      for(int64_t i = i0; i < n; i += di) {
+        double s = 0;
+#pragma unroll 8
+        for(int c = 0; c < k; ++c) s += V[i + c * n] * cf[c];
+        const double x = W[i] - s;
+        W[i] = x;
+        acc += x * x;
+      }
+      if(pass) {
+        const double t = block_sum(acc, shb);
+        if(threadIdx.x == 0) pn[nb + blockIdx.x] = t;
+      } else {
+        __syncthreads();  // cf is rewritten behind the next barrier
+      }
+    }
+    if(!grid_barrier(a, target)) return;
+    if(wid == 0) {
+      const double s = warp_sum_partials(pn + nb, nb, 1);
+      if(lane == 0) shb[0] = 1. / sqrt(s);
+    }
+    __syncthreads();
+    const double inv = shb[0];
+    for(int64_t i = i0; i < n; i += di) W[i] *= inv;
+  }
+  if(blockIdx.x == 0 && threadIdx.x == 0) a.rep->t_end = gpu_time_ns();
 }
 
 // X = unit vector at the first minimum of D (diagonal_guess,
@@ -253,144 +377,6 @@ __global__ void __launch_bounds__(1024)
   }
 }
 
-// Lowest `nwant` eigenpairs of the k x k Rayleigh matrix, given by its lower
-// triangle (column-major, ld k) as dsyev with Uplo::Lower reads it
-// (lobpcgxx/rayleigh_ritz.hpp:75). Householder reduction to tridiagonal
-// form, Sturm-sequence bisection for each wanted eigenvalue, inverse
-// iteration on the tridiagonal matrix, back-transformation and modified
-// Gram-Schmidt among the returned vectors. W ascending; Vec columns.
-void small_syev_lowest(int k, const double* lower, int nwant, double* W,
-                       double* Vec) {
-  std::vector<double> a(size_t(k) * k);
-  for(int j = 0; j < k; ++j)
-    for(int i = j; i < k; ++i) a[i + size_t(j) * k] = a[j + size_t(i) * k] = lower[i + size_t(j) * k];
-  std::vector<double> d(k), e(k, 0.0);
-  std::vector<std::vector<double>> refl;  // Householder vectors (length k)
-  // tridiagonalise: A <- H A H with H = I - 2 v v^T acting on rows/cols j+1..
-  for(int j = 0; j + 2 < k; ++j) {
-    double nrm = 0;
-    for(int i = j + 1; i < k; ++i) nrm += a[i + size_t(j) * k] * a[i + size_t(j) * k];
-    nrm = std::sqrt(nrm);
-    std::vector<double> v(k, 0.0);
-    const double x0 = a[j + 1 + size_t(j) * k];
-    if(nrm == 0) {
-      refl.push_back(v);
-      continue;
-    }
-    const double alpha = x0 > 0 ? -nrm : nrm;
-    v[j + 1] = x0 - alpha;
-    for(int i = j + 2; i < k; ++i) v[i] = a[i + size_t(j) * k];
-    double vn = 0;
-    for(int i = j + 1; i < k; ++i) vn += v[i] * v[i];
-    vn = std::sqrt(vn);
-    if(vn == 0) {
-      refl.push_back(std::vector<double>(k, 0.0));
-      continue;
-    }
-    for(int i = j + 1; i < k; ++i) v[i] /= vn;
-    // p = A v ; K = v.p ; q = p - K v ; A <- A - 2 v q^T - 2 q v^T
-    std::vector<double> p(k, 0.0);
-    for(int c = j; c < k; ++c) {  // column c (= row c: a is symmetric)
-      const double* ac = a.data() + size_t(c) * k;
-      double s4[4] = {0, 0, 0, 0};  // four chains: the sum is latency-bound
-      int r = j + 1;
-      for(; r + 3 < k; r += 4)
-        for(int q = 0; q < 4; ++q) s4[q] += ac[r + q] * v[r + q];
-      for(; r < k; ++r) s4[0] += ac[r] * v[r];
-      p[c] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-    }
-    double K = 0;
-    for(int r = j + 1; r < k; ++r) K += v[r] * p[r];
-    for(int r = j; r < k; ++r) p[r] -= K * v[r];
-    for(int c = j; c < k; ++c)
-      for(int r = j; r < k; ++r)
-        a[r + size_t(c) * k] -= 2 * (v[r] * p[c] + p[r] * v[c]);
-    refl.push_back(v);
-  }
-  for(int i = 0; i < k; ++i) d[i] = a[i + size_t(i) * k];
-  for(int i = 0; i + 1 < k; ++i) e[i] = a[i + 1 + size_t(i) * k];
-  // Gershgorin bounds
-  double lo = d[0], hi = d[0];
-  for(int i = 0; i < k; ++i) {
-    const double r = (i ? std::fabs(e[i - 1]) : 0) + (i + 1 < k ? std::fabs(e[i]) : 0);
-    lo = std::min(lo, d[i] - r);
-    hi = std::max(hi, d[i] + r);
-  }
-  const double span = std::max({hi - lo, std::fabs(lo), std::fabs(hi), 1e-30});
-  lo -= 1e-12 * span;
-  hi += 1e-12 * span;
-  const double tiny = 1e-15 * span;  // pivot floor of the shifted solves
-  auto count_below = [&](double x) {  // Sturm count of eigenvalues < x
-    int c = 0;
-    double q = d[0] - x;
-    if(q < 0) ++c;
-    for(int i = 1; i < k; ++i) {
-      if(q == 0) q = 1e-300;
-      q = d[i] - x - e[i - 1] * e[i - 1] / q;
-      if(q < 0) ++c;
-    }
-    return c;
-  };
-  nwant = std::min(nwant, k);
-  std::vector<std::vector<double>> ztri;  // eigenvectors of the tridiagonal
-  for(int m = 0; m < nwant; ++m) {
-    double l = lo, h = hi;  // the m-th eigenvalue has count_below(x) > m
-    for(int it = 0; it < 200 && h - l > 4e-16 * std::max(std::fabs(l), std::fabs(h)) + 1e-300; ++it) {
-      const double mid = 0.5 * (l + h);
-      if(count_below(mid) > m)
-        h = mid;
-      else
-        l = mid;
-    }
-    W[m] = 0.5 * (l + h);
-    // inverse iteration on T - lambda I (tridiagonal LU with pivoting-free
-    // elimination, shifted slightly to stay regular)
-    const double lam = W[m] + 1e-14 * span;
-    auto floor_piv = [&](double x) {
-      return std::fabs(x) < tiny ? (x < 0 ? -tiny : tiny) : x;
-    };
-    // start vector: deterministic, different per wanted pair
-    std::vector<double> z(k), w2(k);
-    for(int i = 0; i < k; ++i)
-      z[i] = 1.0 + 0.5 * std::sin(0.7 * (i + 1) * (m + 1) + 0.3 * m);
-    for(int it = 0; it < 5; ++it) {
-      std::vector<double> dd(k), rhs = z;
-      dd[0] = floor_piv(d[0] - lam);
-      for(int i = 1; i < k; ++i) {
-        const double f = e[i - 1] / dd[i - 1];
-        dd[i] = floor_piv(d[i] - lam - f * e[i - 1]);
-        rhs[i] -= f * rhs[i - 1];
-      }
-      w2[k - 1] = rhs[k - 1] / dd[k - 1];
-      for(int i = k - 2; i >= 0; --i) w2[i] = (rhs[i] - e[i] * w2[i + 1]) / dd[i];
-      // keep it orthogonal to the vectors of (nearly) equal eigenvalues
-      for(int p = 0; p < m; ++p) {
-        if(std::fabs(W[p] - W[m]) > 1e-7 * span) continue;
-        double s2 = 0;
-        for(int i = 0; i < k; ++i) s2 += ztri[p][i] * w2[i];
-        for(int i = 0; i < k; ++i) w2[i] -= s2 * ztri[p][i];
-      }
-      double nn = 0;
-      for(double x : w2) nn += x * x;
-      nn = std::sqrt(nn);
-      if(!(nn > 0) || !std::isfinite(nn)) break;
-      for(int i = 0; i < k; ++i) z[i] = w2[i] / nn;
-    }
-    ztri.push_back(z);
-    // back-transform: y = H_0 H_1 ... H_{k-3} z
-    for(int r = int(refl.size()) - 1; r >= 0; --r) {
-      const auto& v = refl[r];
-      double s2 = 0;
-      for(int i = 0; i < k; ++i) s2 += v[i] * z[i];
-      for(int i = 0; i < k; ++i) z[i] -= 2 * s2 * v[i];
-    }
-    double nn = 0;
-    for(double x : z) nn += x * x;
-    nn = std::sqrt(nn);
-    for(int i = 0; i < k; ++i) Vec[i + size_t(m) * k] = z[i] / nn;
-  }
-}
-
 // out[:, j] = A[:, 0:k] Q[:, j] for j < keep (Q column-major, ld k): a thread
 // keeps 8 output columns of its row in registers while it reads the row once.
 // out may be A when keep <= 8 (a row is read whole before it is written).
@@ -424,72 +410,44 @@ static thread_local macis_b200_davidson_stats g_dav_stats{};
 const macis_b200_davidson_stats& davidson_last_stats() { return g_dav_stats; }
 
 namespace {
-// Device time per phase, summed over the solve: marks recorded on the solver
-// stream at the phase boundaries of an iteration, read at the next
-// synchronisation behind them.
-struct PhaseMarks {
-  static constexpr int N = 6;
-  struct Set {  // the marks of one iteration
-    cudaEvent_t e[N];
-    double* acc[N] = {};  // where the time from mark i to mark i + 1 goes
-  } set[2];
-  int cur = 0;
-  cudaStream_t s;
-  explicit PhaseMarks(cudaStream_t st) : s(st) {
-    for(auto& x : set)
-      for(auto& y : x.e) cudaEventCreate(&y);
-  }
-  PhaseMarks(const PhaseMarks&) = delete;
-  ~PhaseMarks() {
-    for(auto& x : set)
-      for(auto& y : x.e) cudaEventDestroy(y);
-  }
-  void mark(int i, double* into) {
-    cudaEventRecord(set[cur].e[i], s);
-    set[cur].acc[i] = into;
-  }
-  void wait(int i) const { MB_CUDA(cudaEventSynchronize(set[cur].e[i])); }
-  // adds the phases of a set; its marks must have completed
-  void collect(int which) {
-    Set& x = set[which];
-    for(int i = 0; i + 1 < N; ++i) {
-      float ms = 0.f;
-      if(x.acc[i] && cudaEventElapsedTime(&ms, x.e[i], x.e[i + 1]) == cudaSuccess)
-        *x.acc[i] += ms;
-      x.acc[i] = nullptr;
-    }
-  }
-};
-
-// Page-locked host memory the kernels write the few numbers into that the
-// host needs each iteration.
-struct HostResults {
-  double* p = nullptr;
-  cudaStream_t s;
-  HostResults(size_t n, cudaStream_t st) : s(st) {
-    MB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), n * 8, cudaHostAllocMapped));
-  }
-  HostResults(const HostResults&) = delete;
-  ~HostResults() {
-    cudaStreamSynchronize(s);  // kernels in flight may still write here
-    cudaFreeHost(p);
-  }
-};
-
 struct DavCtx {
   cudaStream_t s;
   int64_t n;
-  unsigned nb;      // row blocks of the vector kernels
+  unsigned nb;            // row blocks
+  unsigned step_blocks;   // blocks of a step (all resident)
   double* partial;
-  unsigned* done;   // arrival counters: one per column chunk, and one more
-  double* dots;     // up to 1024 coefficients, then a norm
-  DavCtx(cudaStream_t st, int64_t nn, int ncol, Arena& A) : s(st), n(nn) {
+  unsigned* done;         // arrival counters: per column chunk, of the chunks
+  unsigned* bar;
+  unsigned long long* t0;
+  unsigned nbar = 0;      // barrier arrivals so far
+  unsigned seq = 0;
+  DavReport* rep = nullptr;
+  std::shared_ptr<PinnedPool> pool;
+  DavCtx(cudaStream_t st, int64_t nn, int ncol, Arena& A,
+         const std::shared_ptr<PinnedPool>& pin)
+      : s(st), n(nn), pool(pin ? pin : std::make_shared<PinnedPool>()) {
     nb = grid_for(size_t(nn), DV_THREADS, size_t(num_sms()) * 4);
+    int per_sm = 0;
+    MB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dav_step_k,
+                                                          DV_THREADS, 0));
+    step_blocks = std::min(nb, unsigned(num_sms() * std::min(2, std::max(1, per_sm))));
     const size_t chunks = size_t(ncol + DV_CHUNK - 1) / DV_CHUNK;
-    partial = A.get<double>(size_t(nb) * DV_CHUNK * (chunks + 1));
-    done = A.get<unsigned>(chunks + 1);
-    MB_CUDA(cudaMemsetAsync(done, 0, (chunks + 1) * sizeof(unsigned), st));
-    dots = A.get<double>(1026);
+    partial = A.get<double>(std::max(size_t(nb) * DV_CHUNK * chunks,
+                                     (size_t(2) * ncol + 2) * step_blocks));
+    done = A.get<unsigned>(chunks + 3);
+    bar = done + chunks + 2;
+    MB_CUDA(cudaMemsetAsync(done, 0, (chunks + 3) * sizeof(unsigned), st));
+    t0 = A.get<unsigned long long>(1);
+    const size_t bytes = sizeof(DavReport) + size_t(ncol) * 8;
+    MB_REQUIRE(bytes <= PinnedPool::BYTES, MACIS_B200_EINVAL,
+               "Davidson: subspace too large");
+    rep = static_cast<DavReport*>(pool->take());
+    memset(static_cast<void*>(rep), 0, bytes);
+  }
+  DavCtx(const DavCtx&) = delete;
+  ~DavCtx() {
+    cudaStreamSynchronize(s);  // kernels in flight may still report
+    if(rep) pool->give(rep);
   }
   template <class... P, class... Q>
   void launch(void (*kern)(P...), dim3 g, int threads, Q&&... args) const {
@@ -505,28 +463,51 @@ struct DavCtx {
     MB_CUDA(cudaLaunchKernelEx(&c, kern, P(args)...));
     note_launch();
   }
-  // out[0:ncol) = A^T v (columns of length n, leading dimension lda). Row
-  // blocks: all of the vector's for short vectors, about 4 blocks an SM over
-  // all chunks for long ones.
-  void multidot(const double* A, int64_t lda, int ncol, const double* v,
-                double* out) const {
+  // rep->row[0:ncol) = A^T v (columns of length n). Row blocks: all of the
+  // vector's for short vectors, about 4 blocks an SM over all chunks for long
+  // ones.
+  void multidot(const double* A, int ncol, const double* v) {
     const unsigned ch = unsigned(ncol + DV_CHUNK - 1) / DV_CHUNK;
     const unsigned want = std::max(1u, unsigned(num_sms()) * 4 / ch);
-    launch(multidot_k, dim3(std::min(nb, want), ch), DV_THREADS, A, lda, ncol,
-           v, n, partial, done, out);
+    launch(multidot_k, dim3(std::min(nb, want), ch), DV_THREADS, A, n, ncol, v,
+           n, partial, done, t0, rep, ++seq);
   }
-  unsigned rows_grid() const {
-    return std::min(nb, unsigned(num_sms()) * 4);
+  void step(StepArgs a, const RitzCoef& rc) {
+    a.n = n;
+    a.partial = partial;
+    a.done = done;
+    a.bar = bar;
+    a.bar0 = nbar;
+    a.rep = rep;
+    a.seq = a.ritz ? ++seq : seq;
+    if(a.ortho && step_blocks > 1) nbar += 3 * step_blocks;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(step_blocks);
+    c.blockDim = dim3(DV_THREADS);
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    MB_CUDA(cudaLaunchKernelEx(&c, dav_step_k, a, rc));
+    note_launch();
   }
-  // gram_schmidt (davidson.hpp:111-126): CGS2 against K columns, normalise
-  void cgs2(const double* Vb, int K, double* w) const {
-    for(int pass = 0; pass < 2; ++pass) {
-      multidot(Vb, n, K, w, dots);
-      launch(cgs_update_k, dim3(rows_grid()), DV_THREADS, Vb, n, K, dots, w, n,
-             partial, done, pass ? dots + 1024 : nullptr);
+  // Waits for the report numbered seq: polls for about the time that the
+  // vector work of a short iteration takes, then leaves the waiting to the
+  // runtime (long products).
+  void wait(const volatile unsigned& flag) const {
+    const auto t = std::chrono::steady_clock::now();
+    while(flag != seq) {
+      if(std::chrono::steady_clock::now() - t > std::chrono::microseconds(300)) {
+        MB_CUDA(cudaStreamSynchronize(s));
+        MB_REQUIRE(flag == seq, MACIS_B200_ETIMEOUT,
+                   "Davidson: a grid barrier timed out");
+      }
     }
-    launch(scale_k, dim3(grid_for(size_t(n), 256, size_t(num_sms()) * 8)), 256,
-           w, n, dots + 1024);
+    std::atomic_thread_fence(std::memory_order_acquire);
+    MB_REQUIRE(!rep->err, MACIS_B200_ETIMEOUT,
+               "Davidson: a grid barrier timed out");
   }
 };
 }  // namespace
@@ -539,6 +520,7 @@ int davidson_device(const macis_b200_csr* A, int64_t max_m, double tol,
   op.n = A->m;
   op.diag = A->diag;
   op.s = A->stream;
+  op.pinned = A->pinned;
   op.apply = [A](const double* x, double* y) {
     spmv_device_x64(A, 1.0, x, 0.0, y, A->stream);
   };
@@ -560,7 +542,6 @@ int davidson_op(const DavOperator& op, int64_t max_m, double tol,
   Arena Ar(s);
   const auto t_wall = std::chrono::steady_clock::now();
   macis_b200_davidson_stats st{};
-  PhaseMarks marks(s);
   max_m = std::min<int64_t>(max_m, N);
   if(restart_keep >= max_m) restart_keep = int(max_m) - 1;
   const double* D = op.diag;
@@ -571,77 +552,90 @@ int davidson_op(const DavOperator& op, int64_t max_m, double tol,
                     ? Ar.get<double>(size_t(N) * restart_keep)
                     : nullptr;
   const int ld = int(max_m + 1);
-  DavCtx ctx(s, N, ld, Ar);
-  // host-visible results: the Rayleigh row (ld), then |R|^2
-  HostResults res(size_t(ld) + 1, s);
+  DavCtx ctx(s, N, ld, Ar, op.pinned);
+  RitzCoef rc;
+  rc.dev = nullptr;
+  StepArgs sa{};
+  sa.V = V;
+  sa.AV = AV;
+  sa.D = D;
+  sa.X = X;
+  auto orthonormalise = [&](int k, double* w) {
+    StepArgs o = sa;
+    o.k = k;
+    o.ortho = 1;
+    o.W = w;
+    ctx.step(o, rc);
+  };
   MB_CUDA(cudaMemcpyAsync(V, X, N * 8, cudaMemcpyDeviceToDevice, s));
   op.apply(V, AV);
   MB_CUDA(cudaMemcpyAsync(V + N, AV, N * 8, cudaMemcpyDeviceToDevice, s));
-  ctx.cgs2(V, 1, V + N);
+  orthonormalise(1, V + N);
 
   std::vector<double> Cl(size_t(ld) * ld, 0.0), lower, W(ld), Vec;
   // first entry of the Rayleigh matrix, V_0 . AV_0
-  ctx.multidot(AV, N, 1, V, res.p);
-  MB_CUDA(cudaStreamSynchronize(s));
-  Cl[0] = res.p[0];
+  ctx.multidot(AV, 1, V);
+  ctx.wait(ctx.rep->row_seq);
+  Cl[0] = ctx.rep->row[0];
   double* d_c = Ar.get<double>(size_t(ld) * ld + 2);
+  auto ms = [](unsigned long long a, unsigned long long b) {
+    return b > a ? double(b - a) * 1e-6 : 0.0;
+  };
   bool converged = false;
   int64_t iter = 1;
   double lam0 = 0;
   int64_t i = 1;  // index of the newest basis vector (AV_i not yet formed)
   for(;; ++iter) {
     const int k = int(i + 1);
-    marks.cur = int(iter & 1);
-    marks.mark(0, &st.apply_ms);
     op.apply(V + i * N, AV + i * N);
     // new row of V^T AV: V_i . AV_c for c <= i (lower triangle)
-    marks.mark(1, &st.rayleigh_ms);
-    ctx.multidot(AV, N, k, V + i * N, res.p);
-    marks.mark(2, nullptr);
+    ctx.multidot(AV, k, V + i * N);
     st.vector_bytes += double(N) * (k + 1) * 8;
-    MB_CUDA(cudaStreamSynchronize(s));
-    marks.collect(marks.cur ^ 1);
-    for(int c = 0; c < k; ++c) Cl[i + size_t(c) * ld] = res.p[c];
+    ctx.wait(ctx.rep->row_seq);
+    // the step before has ended too: its last phase, the product behind it
+    // and the row
+    if(iter > 1) st.ortho_ms += ms(ctx.rep->t_res1, ctx.rep->t_end);
+    st.apply_ms += ms(ctx.rep->t_end, ctx.rep->t_row0);
+    st.rayleigh_ms += ms(ctx.rep->t_row0, ctx.rep->t_row1);
+    for(int c = 0; c < k; ++c) Cl[i + size_t(c) * ld] = ctx.rep->row[c];
     lower.assign(size_t(k) * k, 0.0);
     for(int c = 0; c < k; ++c)
       for(int r = c; r < k; ++r) lower[r + size_t(c) * k] = Cl[r + size_t(c) * ld];
     // the lowest pair; a restart of a full basis takes restart_keep of them
-    const int nwant = k >= max_m ? std::max(1, std::min(restart_keep, k)) : 1;
+    const bool full = k >= max_m;
+    const int nwant = full ? std::max(1, std::min(restart_keep, k)) : 1;
     Vec.assign(size_t(k) * nwant, 0.0);
     small_syev_lowest(k, lower.data(), nwant, W.data(), Vec.data());
     lam0 = W[0];
-    RitzCoef rc;
-    rc.dev = nullptr;
-    if(k <= DV_PARAM_COEF) {
+    if(k <= DV_PARAM_COEF)
       std::copy(Vec.begin(), Vec.begin() + k, rc.c);
-    } else {
+    else
       rc.dev = d_c;
-    }
     if(rc.dev || nwant > 1)
       MB_CUDA(cudaMemcpyAsync(d_c, Vec.data(), size_t(k) * nwant * 8,
                               cudaMemcpyHostToDevice, s));
     double* R = V + size_t(k) * N;
-    marks.mark(3, &st.residual_ms);
-    ctx.launch(ritz_residual_k, dim3(ctx.rows_grid()), DV_THREADS, V, AV, N, k,
-               rc, lam0, D, X, R, ctx.partial, ctx.done, res.p + ld);
-    marks.mark(4, &st.ortho_ms);
+    const bool last = max_iter > 0 && iter >= max_iter;
+    StepArgs a = sa;
+    a.k = k;
+    a.ritz = 1;
+    // the next direction is orthonormalised while the host looks at |R|^2
+    // (for nothing when that has converged)
+    a.ortho = !full && !last;
+    a.lam = lam0;
+    a.W = R;
+    ctx.step(a, rc);
     st.vector_bytes += double(N) * (2.0 * k + 3) * 8;
-    // the next direction is orthonormalised behind the residual while the
-    // host waits for its norm (not used when that has converged)
-    const bool full = k >= max_m;
-    if(!full && !(max_iter > 0 && iter >= max_iter)) {
-      ctx.cgs2(V, k, R);
-      st.vector_bytes += double(N) * (4.0 * k + 9) * 8;
-    }
-    marks.mark(5, nullptr);
-    marks.wait(4);
-    if(std::sqrt(res.p[ld]) < tol) {
+    if(a.ortho) st.vector_bytes += double(N) * (4.0 * k + 9) * 8;
+    ctx.wait(ctx.rep->res_seq);
+    st.residual_ms += ms(ctx.rep->t_res0, ctx.rep->t_res1);
+    if(std::sqrt(ctx.rep->rn2) < tol) {
       converged = true;
       break;
     }
     if(full) {
       // the reference stops here (davidson.hpp:161, 221)
-      if(!restart_keep || (max_iter > 0 && iter >= max_iter)) break;
+      if(!restart_keep || last) break;
       // thick restart: keep the lowest restart_keep Ritz vectors
       const int keep = restart_keep;
       const dim3 g(grid_for(size_t(N), 256, size_t(num_sms()) * 8));
@@ -659,18 +653,15 @@ int davidson_op(const DavOperator& op, int64_t max_m, double tol,
                               cudaMemcpyDeviceToDevice, s));
       std::fill(Cl.begin(), Cl.end(), 0.0);
       for(int c = 0; c < keep; ++c) Cl[c + size_t(c) * ld] = W[c];
-      ctx.cgs2(V, keep, V + size_t(keep) * N);
-      marks.mark(5, nullptr);
+      orthonormalise(keep, V + size_t(keep) * N);
       i = keep;
     } else {
-      if(max_iter > 0 && iter >= max_iter) break;
+      if(last) break;
       i = k;
     }
   }
   MB_CUDA(cudaGetLastError());
   MB_CUDA(cudaStreamSynchronize(s));
-  marks.collect(0);
-  marks.collect(1);
   st.iterations = iter;
   st.wall_ms = std::chrono::duration<double, std::milli>(
                    std::chrono::steady_clock::now() - t_wall)

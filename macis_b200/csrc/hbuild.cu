@@ -2076,6 +2076,7 @@ macis_b200_csr* build_csr_device(macis_b200_ham* h, const uint64_t* bra,
   out->idx_bytes = idx_bytes;
   out->val_bytes = val_bytes;
   out->device = h->device;
+  out->pinned = h->pinned;
   MB_CUDA(cudaStreamCreateWithFlags(&out->stream, cudaStreamNonBlocking));
   out->own_stream = true;
   cudaEvent_t e0, e1;
@@ -2128,6 +2129,7 @@ macis_b200_csr* build_csr_device(macis_b200_ham* h, const uint64_t* bra,
 // pointers: the generator must outlive every product, but destroying the
 // operator never touches it.
 struct macis_b200_hop {
+  std::shared_ptr<mb::PinnedPool> pinned;
   mb::Ints I{};
   int nbits = 64;
   cudaStream_t stream = nullptr;
@@ -2202,6 +2204,7 @@ macis_b200_hop* hop_create(macis_b200_ham* h, const uint64_t* dets, size_t n,
   const int sms = num_sms();
   const Ints I = h->ints();
   auto* op = new macis_b200_hop;
+  op->pinned = h->pinned;
   op->I = I;
   op->nbits = h->nbits;
   op->n = int64_t(n);
@@ -2280,6 +2283,9 @@ void hop_destroy(macis_b200_hop* op) {
 int64_t hop_size(const macis_b200_hop* op) { return op->n; }
 const double* hop_diag(const macis_b200_hop* op) { return op->diag; }
 cudaStream_t hop_stream(const macis_b200_hop* op) { return op->stream; }
+const std::shared_ptr<PinnedPool>& hop_pinned(const macis_b200_hop* op) {
+  return op->pinned;
+}
 
 }  // namespace mb
 

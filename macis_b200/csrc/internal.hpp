@@ -2,13 +2,68 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <functional>
-
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "common.cuh"
 
+namespace mb {
+// Page-locked blocks for the few numbers that kernels report to the host
+// while a solver runs. Allocating and freeing one takes longer than a small
+// solve's iterations, so up to KEEP blocks are kept for the next one. The
+// generators and the operators built from them share the pool, and it goes
+// with the last of them. Any thread may take and give blocks.
+class PinnedPool {
+ public:
+  static constexpr size_t BYTES = 16384;
+  static constexpr size_t KEEP = 4;
+  PinnedPool() = default;
+  PinnedPool(const PinnedPool&) = delete;
+  ~PinnedPool() {
+    for(void* p : free_) cudaFreeHost(p);
+  }
+  void* take() {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      if(!free_.empty()) {
+        void* p = free_.back();
+        free_.pop_back();
+        return p;
+      }
+    }
+    void* p = nullptr;
+    MB_CUDA(cudaHostAlloc(&p, BYTES, cudaHostAllocMapped | cudaHostAllocPortable));
+    return p;
+  }
+  void give(void* p) {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      if(free_.size() < KEEP) {
+        free_.push_back(p);
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+
+ private:
+  std::mutex mu_;
+  std::vector<void*> free_;
+};
+inline std::shared_ptr<PinnedPool> pinned_pool() {
+  static std::mutex mu;
+  static std::weak_ptr<PinnedPool> live;
+  std::lock_guard<std::mutex> lk(mu);
+  std::shared_ptr<PinnedPool> p = live.lock();
+  if(!p) live = p = std::make_shared<PinnedPool>();
+  return p;
+}
+}  // namespace mb
+
 struct macis_b200_ham {
+  std::shared_ptr<mb::PinnedPool> pinned = mb::pinned_pool();
   int nbits = 64;
   int norb = 0;
   int device = 0;
@@ -35,6 +90,7 @@ struct macis_b200_ham {
 };
 
 struct macis_b200_csr {
+  std::shared_ptr<mb::PinnedPool> pinned;
   int64_t m = 0, n = 0, nnz = 0;
   int idx_bytes = 4, val_bytes = 8;
   int device = 0;
@@ -130,6 +186,7 @@ struct DavOperator {
   int64_t n = 0;
   const double* diag = nullptr;
   cudaStream_t s = nullptr;
+  std::shared_ptr<PinnedPool> pinned;
   std::function<void(const double* x, double* y)> apply;
 };
 int davidson_op(const DavOperator& op, int64_t max_m, double tol,
@@ -151,6 +208,7 @@ void hop_destroy(macis_b200_hop* op);
 int64_t hop_size(const macis_b200_hop* op);
 const double* hop_diag(const macis_b200_hop* op);
 cudaStream_t hop_stream(const macis_b200_hop* op);
+const std::shared_ptr<PinnedPool>& hop_pinned(const macis_b200_hop* op);
 
 // Lowest nwant eigenpairs of a k x k symmetric matrix (lower triangle).
 void small_syev_lowest(int k, const double* lower, int nwant, double* W,

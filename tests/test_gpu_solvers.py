@@ -101,3 +101,31 @@ def test_guess_reuse_and_selected_space(ref):
     assert abs(E - Er) < 1e-8
     E2, X2 = mb.selected_ci_diag(sel, H, 1e-12, 300, 1e-9, C=X)
     assert abs(E2 - E) < 1e-8
+
+
+@pytest.mark.parametrize("n,na,nb", [(2, 1, 1), (4, 2, 1), (6, 3, 3), (7, 3, 4),
+                                     (8, 3, 4)])
+@pytest.mark.parametrize("max_m,keep", [(40, 8), (40, 12), (140, 10), (300, 0)])
+def test_davidson_against_dense(n, na, nb, max_m, keep):
+    """Lowest eigenpair against numpy's of the dense matrix: vectors from a
+    few rows to several blocks of rows, Ritz vectors above and below the
+    length that travels with the launch (128), restarts keeping more and
+    fewer columns than a thread holds. E to 1e-8 (residual 1e-9 over a gap
+    above 1e-2 squares to far less), the vector to 1e-6."""
+    T, V, d = fci(n, na, nb, 64, seed=3)
+    H = mb.HamiltonianGenerator(T, V, 64)
+    A = mb.make_csr_hamiltonian(d, H, np.finfo(float).eps)
+    rp, ci, nz = A.to_host()
+    M = np.zeros((A.m, A.m))
+    for i in range(A.m):
+        M[i, ci[rp[i]:rp[i + 1]]] = nz[rp[i]:rp[i + 1]]
+    w, U = np.linalg.eigh(M)
+    X = np.zeros(A.n)
+    keep = min(keep, max(min(max_m, A.n) - 1, 0))
+    it, E = mb.davidson(A.n, max_m, A, None, 1e-9, X, use_guess=False,
+                        restart_keep=keep, max_iter=3000)
+    assert abs(E - w[0]) < 1e-8
+    if len(w) == 1 or w[1] - w[0] > 1e-2:
+        assert abs(abs(U[:, 0] @ X) - 1.0) < 1e-6
+    st = mb.davidson_stats()
+    assert st["iterations"] == it and all(v >= 0 for v in st.values())
