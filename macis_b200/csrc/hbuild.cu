@@ -131,14 +131,6 @@ __global__ void dp_check_k(const uint64_t* dets, size_t n, size_t ub,
   }
 }
 
-template <int NW>
-__global__ void adjacent_dup_k(const uint64_t* keys, size_t n, int* dup) {
-  for(size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x + 1; i < n;
-      i += size_t(gridDim.x) * blockDim.x)
-    if(key_eq<NW>(load_key<NW>(keys, i), load_key<NW>(keys, i - 1)))
-      atomicOr(dup, 1);
-}
-
 template <int NBITS>
 __global__ void gather_block_spins_k(const uint64_t* dets, size_t ua,
                                      size_t ub, uint64_t* alphas,
@@ -152,45 +144,52 @@ __global__ void gather_block_spins_k(const uint64_t* dets, size_t ua,
 }
 
 // ----------------------------------------------------- spin connectivity
-// For every left string l, the right strings r (ascending) with
-// popcount(l ^ r) <= maxp, each with its packed excitation seen from bra=l,
-// ket=r and popcount in bits 29..31. Warp per left string; count pass when
-// col == nullptr.
+// What the direct-product plan needs to know before it can allocate.
+struct DPTotals {
+  int64_t na, n2, n4, nnz;      // entries of the lists, of the matrix
+  int dup;                      // some string occurs twice
+  int l2max, l4max;             // longest beta lists
+  unsigned long long dropped;   // elements below the threshold (fill)
+};
+
+// Per string l the connected strings of the same list: at popcount 0, 2 and
+// 4 (cls[3 l ..]), within 2 (cnt2) and within 4 (cnt4). Warp per string.
+// Strings that occur twice and the longest lists are noted on the way, which
+// a sort of the strings and a copy of all list offsets were needed for.
 template <int NSW>
-__global__ void spin_conn_k(const uint64_t* left, size_t nl,
-                            const uint64_t* right, size_t nr, int maxp,
-                            const int64_t* off, int64_t* cnt, int32_t* col,
-                            uint32_t* info) {
+__global__ void dp_conn_count_k(const uint64_t* strs, size_t ns, int32_t* cls,
+                                int64_t* cnt2, int64_t* cnt4, int beta,
+                                DPTotals* tot) {
   const int lane = threadIdx.x & 31;
   const size_t nwarp = size_t(gridDim.x) * (blockDim.x >> 5);
   for(size_t l = size_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-      l < nl; l += nwarp) {
-    const Spin<NSW> L = ld_spin<NSW>(left, l);
-    int64_t c = 0;
-    const int64_t base = off ? off[l] : 0;
-    for(size_t r0 = 0; r0 < nr; r0 += 32) {
-      const size_t r = r0 + lane;
-      Spin<NSW> R = sp_zero<NSW>();
-      int p = 99;
-      if(r < nr) {
-        R = ld_spin<NSW>(right, r);
-        p = sp_popc(L ^ R);
-      }
-      const bool hit = p <= maxp;
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      if(col && hit) {
-        const int64_t pos = base + c + __popc(m & lanemask_lt());
-        uint32_t e = 0;
-        if(p == 2)
-          e = single_ex(L, R);
-        else if(p == 4)
-          e = double_ex(L, R);
-        col[pos] = int32_t(r);
-        info[pos] = e | (uint32_t(p) << 29);
-      }
-      c += __popc(m);
+      l < ns; l += nwarp) {
+    const Spin<NSW> L = ld_spin<NSW>(strs, l);
+    int c0 = 0, c2 = 0, c4 = 0;
+    for(size_t r = lane; r < ns; r += 32) {
+      const int p = sp_popc(L ^ ld_spin<NSW>(strs, r));
+      c0 += p == 0;
+      c2 += p == 2;
+      c4 += p == 4;
     }
-    if(!col && lane == 0) cnt[l] = c;
+#pragma unroll
+    for(int o = 16; o; o >>= 1) {
+      c0 += __shfl_xor_sync(0xffffffffu, c0, o);
+      c2 += __shfl_xor_sync(0xffffffffu, c2, o);
+      c4 += __shfl_xor_sync(0xffffffffu, c4, o);
+    }
+    if(lane == 0) {
+      cls[3 * l] = c0;
+      cls[3 * l + 1] = c2;
+      cls[3 * l + 2] = c4;
+      cnt2[l] = c0 + c2;
+      cnt4[l] = c0 + c2 + c4;
+      if(c0 > 1) atomicOr(&tot->dup, 1);
+      if(beta) {
+        atomicMax(&tot->l2max, c0 + c2);
+        atomicMax(&tot->l4max, c0 + c2 + c4);
+      }
+    }
   }
 }
 
@@ -208,9 +207,8 @@ struct DPData {
   const int32_t* l4col;
   const uint32_t* l4info;
   // same-spin parts of the single-excitation elements (dp_pg_k)
-  const int64_t* pgaoff;   // UA+1
+  // at string x no nv (the electron counts of a product space are fixed)
   const double* pga;
-  const int64_t* pgboff;   // UB+1
   const double* pgb;
   // signed G value of every double of the alpha and beta L4 lists (0 for
   // the other entries): the fill reads it with the list entry instead of
@@ -240,19 +238,8 @@ __device__ __forceinline__ void spin_lists(const Spin<NSW>& s, int n, int lane,
   }
 }
 
-// Singles per spin string: popcount * (n - popcount).
-template <int NSW>
-__global__ void dp_pgcount_k(const uint64_t* strings, int64_t ns, int n,
-                             int64_t* cnt) {
-  for(int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < ns;
-      i += int64_t(gridDim.x) * blockDim.x) {
-    const int no = sp_popc(ld_spin<NSW>(strings, i));
-    cnt[i] = int64_t(no) * (n - no);
-  }
-}
-
 // Same-spin part of every single excitation of every spin string s:
-//   pg[off[s] + i nv + j] = T(v,o) + sum_{p in occ(s)} G_red(p,v,o)
+//   pg[s no nv + i nv + j] = T(v,o) + sum_{p in occ(s)} G_red(p,v,o)
 // with v the i-th occupied and o the j-th empty orbital of s, summed in the
 // order of matrix_element_2 (matrix_elements.hpp:86-104: T, then the
 // same-spin G_red terms by ascending p). The element of a determinant adds
@@ -260,7 +247,7 @@ __global__ void dp_pgcount_k(const uint64_t* strings, int64_t ns, int n,
 // split is bit-exact. One warp per string.
 template <int NSW>
 __global__ void dp_pg_k(Ints I, const uint64_t* strings, int64_t ns,
-                        const int64_t* off, double* pg) {
+                        double* pg) {
   __shared__ uint8_t lists[8][256];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int n = I.n, n2 = n * n;
@@ -273,7 +260,7 @@ __global__ void dp_pg_k(Ints I, const uint64_t* strings, int64_t ns,
     __syncwarp();
     spin_lists<NSW>(sp, n, lane, occ, vir);
     __syncwarp();
-    double* out = pg + off[st];
+    double* out = pg + st * no * nv;
     for(int u = lane; u < no * nv; u += 32) {
       const int v = occ[u / nv], o = vir[u % nv];
       double h = __ldg(I.T + v + o * n);
@@ -284,48 +271,13 @@ __global__ void dp_pg_k(Ints I, const uint64_t* strings, int64_t ns,
   }
 }
 
-// Signed G value of each double of an encoded connection list (0 for the
-// other entries).
-__global__ void dp_dval_k(const uint32_t* info, int64_t m, const double* G,
-                          double* val) {
-  for(int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m;
-      i += int64_t(gridDim.x) * blockDim.x) {
-    const uint32_t e = info[i];
-    double v = 0.0;
-    if(((e >> 29) & 3u) == 2u) {
-      const double g = G[e & 0x0FFFFFFFu];
-      v = (e >> 31) ? -g : g;
-    }
-    val[i] = v;
-  }
-}
-
-// Per alpha string: how many connected A' at popcount 0, 2, 4.
-__global__ void dp_acount_k(const int64_t* aoff, const uint32_t* ainfo,
-                            int64_t UA, int32_t* na) {
-  for(int64_t A = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; A < UA;
-      A += int64_t(gridDim.x) * blockDim.x) {
-    int c0 = 0, c2 = 0, c4 = 0;
-    for(int64_t j = aoff[A]; j < aoff[A + 1]; ++j) {
-      const int p = ainfo[j] >> 29;
-      c0 += p == 0;
-      c2 += p == 2;
-      c4 += p == 4;
-    }
-    na[3 * A] = c0;
-    na[3 * A + 1] = c2;
-    na[3 * A + 2] = c4;
-  }
-}
-
-__global__ void dp_rowcount_k(const int32_t* na, const int64_t* l2off,
-                              const int64_t* l4off, int64_t r0, int64_t nrows,
+__global__ void dp_rowcount_k(const int32_t* na, const int64_t* l2cnt,
+                              const int64_t* l4cnt, int64_t r0, int64_t nrows,
                               int64_t UB, int64_t* cnt) {
   for(int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nrows;
       i += int64_t(gridDim.x) * blockDim.x) {
     const int64_t A = (r0 + i) / UB, B = (r0 + i) % UB;
-    cnt[i] = int64_t(na[3 * A]) * (l4off[B + 1] - l4off[B]) +
-             int64_t(na[3 * A + 1]) * (l2off[B + 1] - l2off[B]) +
+    cnt[i] = int64_t(na[3 * A]) * l4cnt[B] + int64_t(na[3 * A + 1]) * l2cnt[B] +
              int64_t(na[3 * A + 2]);
   }
 }
@@ -406,28 +358,79 @@ __host__ __device__ inline DPShared dp_shared_layout(int n, int64_t l2max,
 //   beta L2:     single -> pair index b = v1 + o1 n (column b of VT)
 //   beta L4:     single -> singles-table index n^2 + v1 n + o1
 //                double -> G offset
-__global__ void dp_encode_k(uint32_t* info, int64_t m, int n, int which) {
+__device__ __forceinline__ uint32_t dp_encode(uint32_t e, int p, int n,
+                                              int which) {
   const uint32_t n2 = uint32_t(n) * n;
-  for(int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m;
-      i += int64_t(gridDim.x) * blockDim.x) {
-    const uint32_t e = info[i];
-    const int p = int(e >> 29);
-    const uint32_t sg = (e >> 28) & 1u;
-    uint32_t off = 0, cls = 0;
-    const uint32_t o1 = ex_o1(e), v1 = ex_v1(e), o2 = ex_o2(e), v2 = ex_v2(e);
-    if(p == 2) {
-      cls = 1;
-      if(which == 0)  // pair index (row of VT) | singles-table index << 14
-        off = (v1 + o1 * n) | ((v1 * n + o1) << 14);
-      else if(which == 1)
-        off = v1 + o1 * n;  // pair index: column of VT
-      else
-        off = n2 + v1 * n + o1;
-    } else if(p == 4) {
-      cls = 2;
-      off = v1 + n * (o1 + n * (v2 + n * o2));
+  const uint32_t sg = (e >> 28) & 1u;
+  uint32_t off = 0, cls = 0;
+  const uint32_t o1 = ex_o1(e), v1 = ex_v1(e), o2 = ex_o2(e), v2 = ex_v2(e);
+  if(p == 2) {
+    cls = 1;
+    if(which == 0)  // pair index (row of VT) | singles-table index << 14
+      off = (v1 + o1 * n) | ((v1 * n + o1) << 14);
+    else if(which == 1)
+      off = v1 + o1 * n;  // pair index: column of VT
+    else
+      off = n2 + v1 * n + o1;
+  } else if(p == 4) {
+    cls = 2;
+    off = v1 + n * (o1 + n * (v2 + n * o2));
+  }
+  return off | (cls << 29) | (sg << 31);
+}
+
+// The lists of dp_conn_count_k, encoded: for every string the strings within
+// 4 (ascending; encoding `which`, and the signed G value of the doubles, 0
+// for the others) and, when col2 is given, those within 2 (encoding 1). The
+// excitation is seen from bra = the string. Warp per string.
+template <int NSW>
+__global__ void dp_conn_fill_k(const uint64_t* strs, size_t ns, int n,
+                               int which, const double* G, const int64_t* off4,
+                               int32_t* col4, uint32_t* info4, double* val4,
+                               const int64_t* off2, int32_t* col2,
+                               uint32_t* info2) {
+  const int lane = threadIdx.x & 31;
+  const size_t nwarp = size_t(gridDim.x) * (blockDim.x >> 5);
+  for(size_t l = size_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+      l < ns; l += nwarp) {
+    const Spin<NSW> L = ld_spin<NSW>(strs, l);
+    int64_t p4 = off4[l], p2 = col2 ? off2[l] : 0;
+    for(size_t r0 = 0; r0 < ns; r0 += 32) {
+      const size_t r = r0 + lane;
+      Spin<NSW> R = sp_zero<NSW>();
+      int p = 99;
+      if(r < ns) {
+        R = ld_spin<NSW>(strs, r);
+        p = sp_popc(L ^ R);
+      }
+      const unsigned m4 = __ballot_sync(0xffffffffu, p <= 4);
+      if(!m4) continue;
+      const unsigned m2 = __ballot_sync(0xffffffffu, p <= 2);
+      if(p <= 4) {
+        uint32_t e = 0;
+        if(p == 2)
+          e = single_ex(L, R);
+        else if(p == 4)
+          e = double_ex(L, R);
+        const int64_t x = p4 + __popc(m4 & lanemask_lt());
+        const uint32_t w = dp_encode(e, p, n, which);
+        double v = 0.0;
+        if(p == 4) {
+          v = __ldg(G + (w & 0x0FFFFFFFu));
+          if(w >> 31) v = -v;
+        }
+        col4[x] = int32_t(r);
+        info4[x] = w;
+        val4[x] = v;
+        if(col2 && p <= 2) {
+          const int64_t y = p2 + __popc(m2 & lanemask_lt());
+          col2[y] = int32_t(r);
+          info2[y] = dp_encode(e, p, n, 1);
+        }
+      }
+      p4 += __popc(m4);
+      p2 += __popc(m2);
     }
-    info[i] = off | (cls << 29) | (sg << 31);
   }
 }
 
@@ -462,7 +465,7 @@ __global__ void __launch_bounds__(DP_THREADS, DP_CTAS)
               const int64_t* __restrict__ rowptr, CI* __restrict__ colind,
               VT* __restrict__ nzval, double* __restrict__ diag,
               int64_t* __restrict__ rowcnt, double thresh, int64_t r0,
-              int64_t nrows) {
+              int64_t nrows, unsigned long long* __restrict__ ndropped) {
   constexpr int NSW = DetTraits<NBITS>::NSW;
   extern __shared__ __align__(16) unsigned char dsm[];
   // alpha-single segments of the current chunk: (row position, column
@@ -522,8 +525,8 @@ __global__ void __launch_bounds__(DP_THREADS, DP_CTAS)
     // in the bra. The bracket is the per-string partial sum of dp_pg_k.
     {
       const int nsa = no[0] * nv[0], nsb = no[1] * nv[1];
-      const double* __restrict__ pga = d.pga + d.pgaoff[A];
-      const double* __restrict__ pgb = d.pgb + d.pgboff[B];
+      const double* __restrict__ pga = d.pga + A * nsa;
+      const double* __restrict__ pgb = d.pgb + int64_t(B) * nsb;
       // i = u / nv by a float product: (u + 0.5) / nv stays >= 0.5 / nv
       // away from an integer, far above the rounding error for u < 2^14
       const float rva = 1.0f / float(nv[0] > 0 ? nv[0] : 1);
@@ -749,8 +752,20 @@ __global__ void __launch_bounds__(DP_THREADS, DP_CTAS)
 #pragma unroll
     for(int o = 16; o > 0; o >>= 1)
       dropped += __shfl_xor_sync(0xffffffffu, dropped, o);
-    if(lane == 0) rowcnt[row] = int64_t(pos) - dropped;
+    if(lane == 0) {
+      rowcnt[row] = int64_t(pos) - dropped;
+      if(dropped) atomicAdd(ndropped, (unsigned long long)dropped);
+    }
   }
+}
+
+__global__ void dp_totals_k(const int64_t* aoff, size_t ua, const int64_t* l2off,
+                            const int64_t* l4off, size_t ub,
+                            const int64_t* rowptr, size_t nbra, DPTotals* t) {
+  t->na = aoff[ua];
+  t->n2 = l2off[ub];
+  t->n4 = l4off[ub];
+  t->nnz = rowptr[nbra];
 }
 
 // Removes the entries marked with column -1 while packing rows to their
@@ -1773,31 +1788,19 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     UB = f == big ? nket : size_t(f);
     if(UB > 0 && nket % UB == 0) {
       UA = nket / UB;
-      int* bad = A.get<int>(2);
-      MB_CUDA(cudaMemsetAsync(bad, 0, 8, s));
+      int* bad = A.get<int>(1);
+      MB_CUDA(cudaMemsetAsync(bad, 0, 4, s));
       dp_check_k<NBITS><<<grid_for(nket, 256, 8 * sms), 256, 0, s>>>(
           ket, nket, UB, bad), note_launch();
       ua = A.get<uint64_t>(UA * NSW);
       ub = A.get<uint64_t>(UB * NSW);
       gather_block_spins_k<NBITS><<<grid_for(std::max(UA, UB), 256, 8 * sms),
                                     256, 0, s>>>(ket, UA, UB, ua, ub), note_launch();
-      // uniqueness of block alphas and of the betas of block 0
-      uint64_t* sa = A.get<uint64_t>(UA * NSW);
-      uint64_t* sb = A.get<uint64_t>(UB * NSW);
-      uint64_t* tmp = A.get<uint64_t>(std::max(UA, UB) * NSW);
-      MB_CUDA(cudaMemcpyAsync(sa, ua, UA * NSW * 8, cudaMemcpyDeviceToDevice, s));
-      MB_CUDA(cudaMemcpyAsync(sb, ub, UB * NSW * 8, cudaMemcpyDeviceToDevice, s));
-      radix_sort<NSW, uint32_t>(sa, nullptr, tmp, nullptr, UA, A);
-      radix_sort<NSW, uint32_t>(sb, nullptr, tmp, nullptr, UB, A);
-      adjacent_dup_k<NSW><<<grid_for(UA, 256, 4 * sms), 256, 0, s>>>(sa, UA, bad + 1), note_launch();
-      adjacent_dup_k<NSW><<<grid_for(UB, 256, 4 * sms), 256, 0, s>>>(sb, UB, bad + 1), note_launch();
-      int hb[2];
-      MB_CUDA(cudaMemcpyAsync(hb, bad, 8, cudaMemcpyDeviceToHost, s));
-      MB_CUDA(cudaStreamSynchronize(s));
+      const int hb = to_host(bad, s);
       // the fill keeps a singles table of 2 norb^2 doubles per warp in
       // shared memory: spaces whose orbitals make it too large (norb above
       // ~33) take the general path even when they have the product layout
-      direct = hb[0] == 0 && hb[1] == 0 && UA < (size_t(1) << 31) &&
+      direct = hb == 0 && UA < (size_t(1) << 31) &&
                UB < (size_t(1) << 31) && h->norb <= 127 &&
                dp_shared_layout(int(h->norb), 512, 1024).bytes <= 220 * 1024;
     }
@@ -1806,95 +1809,73 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
   int64_t nnz_ub = 0;
   CI* colind = nullptr;
   VT* nzval = nullptr;
+  // direct product: connectivity counts and row sizes, read back together
+  DPTotals tot{};
+  DPTotals* d_tot = nullptr;
+  int64_t *aoff = nullptr, *l2off = nullptr, *l4off = nullptr;
+  if(direct) {
+    d_tot = A.get<DPTotals>(1);
+    MB_CUDA(cudaMemsetAsync(d_tot, 0, sizeof(DPTotals), s));
+    int32_t* cls_a = A.get<int32_t>(3 * UA);
+    int32_t* cls_b = A.get<int32_t>(3 * UB);
+    int64_t* cnt = A.get<int64_t>(2 * (UA + UB));
+    int64_t *ca2 = cnt, *ca4 = ca2 + UA, *cb2 = ca4 + UA, *cb4 = cb2 + UB;
+    dp_conn_count_k<NSW><<<grid_for(UA * 32, 256, 16 * sms), 256, 0, s>>>(
+        ua, UA, cls_a, ca2, ca4, 0, d_tot), note_launch();
+    dp_conn_count_k<NSW><<<grid_for(UB * 32, 256, 16 * sms), 256, 0, s>>>(
+        ub, UB, cls_b, cb2, cb4, 1, d_tot), note_launch();
+    aoff = A.get<int64_t>(UA + 1);
+    l2off = A.get<int64_t>(UB + 1);
+    l4off = A.get<int64_t>(UB + 1);
+    exclusive_scan<int64_t, int64_t>(ca4, aoff, UA, aoff + UA, A);
+    exclusive_scan<int64_t, int64_t>(cb2, l2off, UB, l2off + UB, A);
+    exclusive_scan<int64_t, int64_t>(cb4, l4off, UB, l4off + UB, A);
+    dp_rowcount_k<<<grid_for(nbra, 256, 8 * sms), 256, 0, s>>>(
+        cls_a, cb2, cb4, r0, int64_t(nbra), int64_t(UB), rowcnt), note_launch();
+    exclusive_scan<int64_t, int64_t>(rowcnt, rowptr64, nbra, rowptr64 + nbra, A);
+    dp_totals_k<<<1, 1, 0, s>>>(aoff, UA, l2off, l4off, UB, rowptr64, nbra,
+                                d_tot), note_launch();
+    tot = to_host(d_tot, s);
+    direct = !tot.dup;  // a string twice: not a product space after all
+  }
   if(direct) {
     out->direct_product = true;
-    // spin connectivity lists
-    auto conn = [&](const uint64_t* L, size_t nl, int maxp, int64_t*& off,
-                    int32_t*& col, uint32_t*& info) {
-      int64_t* cnt = A.get<int64_t>(nl + 1);
-      off = A.get<int64_t>(nl + 1);
-      const unsigned g = grid_for(nl * 32, 256, 16 * sms);
-      spin_conn_k<NSW><<<g, 256, 0, s>>>(L, nl, L, nl, maxp, nullptr, cnt,
-                                         nullptr, nullptr), note_launch();
-      exclusive_scan<int64_t, int64_t>(cnt, off, nl, off + nl, A);
-      const int64_t tot = to_host(off + nl, s);
-      col = A.get<int32_t>(tot + 1);
-      info = A.get<uint32_t>(tot + 1);
-      spin_conn_k<NSW><<<g, 256, 0, s>>>(L, nl, L, nl, maxp, off, cnt, col,
-                                         info), note_launch();
-    };
-    int64_t *aoff, *l2off, *l4off;
-    int32_t *acol, *l2col, *l4col;
-    uint32_t *ainfo, *l2info, *l4info;
-    conn(ua, UA, 4, aoff, acol, ainfo);
-    conn(ub, UB, 2, l2off, l2col, l2info);
-    conn(ub, UB, 4, l4off, l4col, l4info);
-    int32_t* na = A.get<int32_t>(3 * UA);
-    dp_acount_k<<<grid_for(UA, 256, 4 * sms), 256, 0, s>>>(aoff, ainfo,
-                                                          int64_t(UA), na), note_launch();
-    dp_rowcount_k<<<grid_for(nbra, 256, 8 * sms), 256, 0, s>>>(
-        na, l2off, l4off, r0, int64_t(nbra), int64_t(UB), rowcnt), note_launch();
-    exclusive_scan<int64_t, int64_t>(rowcnt, rowptr64, nbra, rowptr64 + nbra, A);
-    nnz_ub = to_host(rowptr64 + nbra, s);
+    nnz_ub = tot.nnz;
     out->nnz_candidates = nnz_ub;
     MB_CUDA(dev_malloc_async(&colind, std::max<int64_t>(nnz_ub, 1) * sizeof(CI), s));
     MB_CUDA(dev_malloc_async(&nzval, std::max<int64_t>(nnz_ub, 1) * sizeof(VT), s));
-    {
-      const int nn0 = h->norb;
-      const int64_t na_ = to_host(aoff + UA, s), n2_ = to_host(l2off + UB, s),
-                    n4_ = to_host(l4off + UB, s);
-      dp_encode_k<<<grid_for(size_t(na_), 256, 8 * sms), 256, 0, s>>>(ainfo, na_, nn0, 0), note_launch();
-      dp_encode_k<<<grid_for(size_t(n2_), 256, 8 * sms), 256, 0, s>>>(l2info, n2_, nn0, 1), note_launch();
-      dp_encode_k<<<grid_for(size_t(n4_), 256, 8 * sms), 256, 0, s>>>(l4info, n4_, nn0, 2), note_launch();
-    }
     // orbital lists of the kernels below hold 128 entries per spin
     MB_REQUIRE(nket < (size_t(1) << 31) && h->norb <= 127,
                MACIS_B200_ECAPACITY,
                "direct-product fill needs < 2^31 determinants, norb < 128");
-    // same-spin partial sums of the singles, per alpha and per beta string
-    auto pg_table = [&](const uint64_t* strs, size_t ns, int64_t*& off,
-                        double*& pg) {
-      int64_t* cnt = A.get<int64_t>(ns + 1);
-      off = A.get<int64_t>(ns + 1);
-      dp_pgcount_k<NSW><<<grid_for(ns, 256, 4 * sms), 256, 0, s>>>(
-          strs, int64_t(ns), h->norb, cnt), note_launch();
-      exclusive_scan<int64_t, int64_t>(cnt, off, ns, off + ns, A);
-      const int64_t tot = to_host(off + ns, s);
-      pg = A.get<double>(size_t(std::max<int64_t>(tot, 1)));
-      dp_pg_k<NSW><<<grid_for(ns * 32, 256, 8 * sms), 256, 0, s>>>(
-          I, strs, int64_t(ns), off, pg), note_launch();
-    };
-    int64_t *pgaoff, *pgboff;
-    double *pga, *pgb;
-    pg_table(ua, UA, pgaoff, pga);
-    pg_table(ub, UB, pgboff, pgb);
-    // signed values of the alpha doubles and of the beta L4 doubles
-    double *aval, *l4val;
-    {
-      const int64_t na_ = to_host(aoff + UA, s), n4_ = to_host(l4off + UB, s);
-      aval = A.get<double>(size_t(std::max<int64_t>(na_, 1)));
-      l4val = A.get<double>(size_t(std::max<int64_t>(n4_, 1)));
-      dp_dval_k<<<grid_for(size_t(na_), 256, 8 * sms), 256, 0, s>>>(
-          ainfo, na_, I.G, aval), note_launch();
-      dp_dval_k<<<grid_for(size_t(n4_), 256, 8 * sms), 256, 0, s>>>(
-          l4info, n4_, I.G, l4val), note_launch();
-    }
+    int32_t* acol = A.get<int32_t>(tot.na + 1);
+    uint32_t* ainfo = A.get<uint32_t>(tot.na + 1);
+    double* aval = A.get<double>(tot.na + 1);
+    int32_t* l2col = A.get<int32_t>(tot.n2 + 1);
+    uint32_t* l2info = A.get<uint32_t>(tot.n2 + 1);
+    int32_t* l4col = A.get<int32_t>(tot.n4 + 1);
+    uint32_t* l4info = A.get<uint32_t>(tot.n4 + 1);
+    double* l4val = A.get<double>(tot.n4 + 1);
+    dp_conn_fill_k<NSW><<<grid_for(UA * 32, 256, 16 * sms), 256, 0, s>>>(
+        ua, UA, h->norb, 0, I.G, aoff, acol, ainfo, aval, nullptr, nullptr,
+        nullptr), note_launch();
+    dp_conn_fill_k<NSW><<<grid_for(UB * 32, 256, 16 * sms), 256, 0, s>>>(
+        ub, UB, h->norb, 2, I.G, l4off, l4col, l4info, l4val, l2off, l2col,
+        l2info), note_launch();
+    // same-spin partial sums of the singles, per alpha and per beta string:
+    // at most norb^2 / 4 singles per string
+    const size_t nsing = size_t(h->norb) * h->norb / 4 + 1;
+    double* pga = A.get<double>(UA * nsing);
+    double* pgb = A.get<double>(UB * nsing);
+    dp_pg_k<NSW><<<grid_for(UA * 32, 256, 8 * sms), 256, 0, s>>>(
+        I, ua, int64_t(UA), pga), note_launch();
+    dp_pg_k<NSW><<<grid_for(UB * 32, 256, 8 * sms), 256, 0, s>>>(
+        I, ub, int64_t(UB), pgb), note_launch();
     DPData d{int64_t(UA), int64_t(UB), ua, ub, aoff, acol, ainfo,
              l2off, l2col, l2info, l4off, l4col, l4info,
-             pgaoff, pga, pgboff, pgb, aval, l4val};
-    // shared-memory plan: integrals for the singles if they fit, the longest
-    // beta lists, per-warp singles tables
-    int64_t l2max = 0, l4max = 0;
-    {
-      std::vector<int64_t> h2(UB + 1), h4(UB + 1);
-      MB_CUDA(cudaMemcpyAsync(h2.data(), l2off, (UB + 1) * 8, cudaMemcpyDeviceToHost, s));
-      MB_CUDA(cudaMemcpyAsync(h4.data(), l4off, (UB + 1) * 8, cudaMemcpyDeviceToHost, s));
-      MB_CUDA(cudaStreamSynchronize(s));
-      for(size_t b = 0; b < UB; ++b) {
-        l2max = std::max(l2max, h2[b + 1] - h2[b]);
-        l4max = std::max(l4max, h4[b + 1] - h4[b]);
-      }
-    }
+             pga, pgb, aval, l4val};
+    // shared-memory plan: the longest beta lists, per-warp singles tables
+    int64_t l2max = tot.l2max, l4max = tot.l4max;
     const int nn = h->norb;
     // The integrals of the singles are read through L1 rather than staged in
     // shared memory: per-CTA copies would take the L1 capacity that the
@@ -1938,7 +1919,7 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     cudaEventRecord(ev[0], s);
     dp_fill_k<NBITS, CI, VT><<<g, DP_THREADS, Ls.bytes, s>>>(
         I, h->VT, d, Ls, hdiag, rowptr64, colind, nzval, out->diag, rowcnt, thresh,
-        r0, int64_t(nbra)), note_launch();
+        r0, int64_t(nbra), &d_tot->dropped), note_launch();
     cudaEventRecord(ev[1], s);
     MB_CUDA(cudaGetLastError());
   } else {
@@ -2031,9 +2012,14 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
   }
 
   // ------------------------------------------- exact row pointer + compaction
-  int64_t* newptr = A.get<int64_t>(nbra + 1);
-  exclusive_scan<int64_t, int64_t>(rowcnt, newptr, nbra, newptr + nbra, A);
-  const int64_t nnz = to_host(newptr + nbra, s);
+  int64_t* newptr = rowptr64;
+  int64_t nnz = nnz_ub;
+  // (a direct product that dropped nothing keeps its row pointer)
+  if(!direct || to_host(&d_tot->dropped, s) != 0) {
+    newptr = A.get<int64_t>(nbra + 1);
+    exclusive_scan<int64_t, int64_t>(rowcnt, newptr, nbra, newptr + nbra, A);
+    nnz = to_host(newptr + nbra, s);
+  }
   out->nnz = nnz;
   if(sizeof(CI) == 4)
     MB_REQUIRE(nnz <= int32_index_limit(), MACIS_B200_ECAPACITY,
