@@ -769,7 +769,7 @@ __global__ void dp_totals_k(const int64_t* aoff, size_t ua, const int64_t* l2off
 }
 
 // Removes the entries marked with column -1 while packing rows to their
-// final offsets (direct-product path with dropped elements).
+// final offsets (builds with dropped elements).
 template <typename CI, typename VT>
 __global__ void compact_marked_k(const int64_t* oldptr, const int64_t* newptr,
                                  size_t m, const CI* ci, const VT* nz, CI* ci2,
@@ -878,18 +878,20 @@ __global__ void gen_group_flags_k(const uint64_t* keys, size_t n,
   }
 }
 
-// Group tables: goff[g] (first sorted position), galpha[g]; sorted betas;
+// Group tables: goff[g] (first sorted position), galpha[g]; sorted strings;
 // per original index its group (or -1 for zero determinants).
 template <int NBITS>
 __global__ void gen_groups_k(const uint64_t* keys, const uint32_t* idx,
                              const uint32_t* flags, const uint32_t* gid_excl,
                              size_t n, int64_t* goff, uint64_t* galpha,
-                             uint64_t* sbeta, int32_t* rowgroup) {
+                             uint64_t* salpha, uint64_t* sbeta,
+                             int32_t* rowgroup) {
   constexpr int NSW = DetTraits<NBITS>::NSW;
   for(size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
       i += size_t(gridDim.x) * blockDim.x) {
     Spin<NSW> a, b;
     key_spins<NBITS>(keys, i, a, b);
+    st_spin<NSW>(salpha, i, a);
     st_spin<NSW>(sbeta, i, b);
     const bool zero = sp_popc(a) + sp_popc(b) == 0;
     const uint32_t g = gid_excl[i] + flags[i] - 1;
@@ -1054,7 +1056,7 @@ struct GenData {
   const int32_t* acol;      // ket group
   const uint8_t* apa;
   const int64_t* goff;      // ket group -> sorted range
-  const uint64_t* kalpha;   // ket group alpha
+  const uint64_t* salpha;   // sorted ket alphas
   const uint64_t* sbeta;    // sorted ket betas
   const uint32_t* sidx;     // sorted ket -> original index
   // beta hash tables of the large ket groups (gen_hsize_k / gen_hinsert_k)
@@ -1125,33 +1127,41 @@ __global__ void gen_hsize_k(const int64_t* goff, uint32_t ng,
 
 // Inserts the first sorted position of every distinct beta of a ket group
 // into its table (linear probing; the table has at least twice as many
-// slots as entries, so every insertion finds a free slot).
+// slots as entries, so every insertion finds a free slot). One thread per
+// member: a warp per group left the largest groups (1e4 members) to one warp.
 template <int NSW>
-__global__ void gen_hinsert_k(const int64_t* goff, uint32_t ng,
-                              const uint64_t* sbeta, const int64_t* hoff,
-                              int32_t* htab) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nw = int64_t(gridDim.x) * (blockDim.x >> 5);
-  for(int64_t gi = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-      gi < int64_t(ng); gi += nw) {
+__global__ void gen_hinsert_k(const int64_t* goff, const int32_t* mgroup,
+                              size_t n, const uint64_t* sbeta,
+                              const int64_t* hoff, int32_t* htab) {
+  for(size_t m = size_t(blockIdx.x) * blockDim.x + threadIdx.x; m < n;
+      m += size_t(gridDim.x) * blockDim.x) {
+    const int32_t gi = mgroup[m];
+    if(gi < 0) continue;
     const int64_t h0 = hoff[gi], hs = hoff[gi + 1] - h0;
     if(hs == 0) continue;
     const uint64_t mask = uint64_t(hs) - 1;
-    const int64_t m0 = goff[gi], m1 = goff[gi + 1];
-    for(int64_t m = m0 + lane; m < m1; m += 32) {
-      const Spin<NSW> b = ld_spin<NSW>(sbeta, m);
-      if(m > m0 && ld_spin<NSW>(sbeta, m - 1) == b) continue;  // duplicate
-      uint64_t slot = spin_hash<NSW>(b) & mask;
-      for(int64_t t = 0; t < hs; ++t) {
-        if(atomicCAS(htab + h0 + slot, -1, int32_t(m - m0)) == -1) break;
-        slot = (slot + 1) & mask;
-      }
+    const int64_t m0 = goff[gi];
+    const Spin<NSW> b = ld_spin<NSW>(sbeta, m);
+    if(int64_t(m) > m0 && ld_spin<NSW>(sbeta, m - 1) == b) continue;  // duplicate
+    uint64_t slot = spin_hash<NSW>(b) & mask;
+    for(int64_t t = 0; t < hs; ++t) {
+      if(atomicCAS(htab + h0 + slot, -1, int32_t(int64_t(m) - m0)) == -1) break;
+      slot = (slot + 1) & mask;
     }
   }
 }
 
+// Next row of a kernel whose warps take rows from a counter: rows differ by
+// orders of magnitude in work (the members of the largest alpha groups test
+// 1e4 kets more than others), so a fixed assignment leaves a long tail.
+__device__ __forceinline__ int64_t next_row(unsigned* ctr) {
+  unsigned r = 0;
+  if((threadIdx.x & 31) == 0) r = atomicAdd(ctr, 1u);
+  return int64_t(__shfl_sync(0xffffffffu, r, 0));
+}
+
 // Enumerates the candidate kets of one bra row warp-synchronously; calls
-// emit(active, sorted_pos, ket_group, pa, pb) for chunks of <= 32.
+// emit(active, sorted_pos, pa, pb) for chunks of <= 32.
 template <int NSW, class F>
 __device__ __forceinline__ void gen_enumerate(const GenData& g, int32_t rg,
                                               Spin<NSW> ba, Spin<NSW> bb,
@@ -1166,19 +1176,19 @@ __device__ __forceinline__ void gen_enumerate(const GenData& g, int32_t rg,
   spin_lists<NSW>(bb, g.n, lane, ov, ov + 128);
   __syncwarp();
   // the kets with beta bb (beta-major range [b0, b1))
-  int64_t b0 = 0, b1 = 0;
+  int b0 = 0, b1 = 0;
   {
-    int64_t lo = 0, hi = g.nbgb;
+    int lo = 0, hi = int(g.nbgb);
     while(lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
+      const int mid = (lo + hi) >> 1;
       if(sp_cmp(ld_spin<NSW>(g.bgbeta, mid), bb) < 0)
         lo = mid + 1;
       else
         hi = mid;
     }
-    if(lo < g.nbgb && ld_spin<NSW>(g.bgbeta, lo) == bb) {
-      b0 = g.bgoff[lo];
-      b1 = g.bgoff[lo + 1];
+    if(lo < int(g.nbgb) && ld_spin<NSW>(g.bgbeta, lo) == bb) {
+      b0 = int(g.bgoff[lo]);
+      b1 = int(g.bgoff[lo + 1]);
     }
   }
   const int64_t c1 = g.aoff[rg + 1];
@@ -1188,43 +1198,47 @@ __device__ __forceinline__ void gen_enumerate(const GenData& g, int32_t rg,
   const bool by_beta = b1 - b0 < c1 - c4;
   const int64_t cend = by_beta ? c4 : c1;
   if(by_beta) {
-    for(int64_t p0 = b0; p0 < b1; p0 += 32) {
-      const int64_t p = p0 + lane;
-      bool act = false;
+    for(int p0 = b0; p0 < b1; p0 += 32) {
+      const int p = p0 + lane;
+      const bool act = p < b1 && sp_popc(ld_spin<NSW>(g.bm_alpha, p) ^ ba) == 4;
       int64_t m = 0;
-      int32_t kg = 0;
-      if(p < b1) {
-        m = g.bm_m[p];
-        kg = g.mgroup[m];
-        act = kg >= 0 && sp_popc(ld_spin<NSW>(g.bm_alpha, p) ^ ba) == 4;
-      }
-      emit(act, m, kg, 4, 0);
+      if(act) m = g.bm_m[p];
+      emit(act && g.mgroup[m] >= 0, m, 4, 0);
     }
   }
   for(int64_t c = g.aoff[rg]; c < cend; c += 32) {
     const int64_t j = c + lane;
     const bool valid = j < cend;
-    int32_t kg = 0;
     int pa = 99;
+    int m0 = 0, m1 = 0;  // this lane's group
+    int64_t h0 = 0, hs = 0;
+    bool probe = false;
     if(valid) {
-      kg = g.acol[j];
+      const int32_t kg = g.acol[j];
       pa = g.apa[j];
+      m0 = int(g.goff[kg]);
+      m1 = int(g.goff[kg + 1]);
+      if(pa == 2) {
+        h0 = g.hoff[kg];
+        hs = g.hoff[kg + 1] - h0;
+        probe = hs > 0 && g.gbpop[kg] == nob && m1 - m0 > 8 * nenum;
+      }
     }
     // alpha doubles (pa == 4): only the identical beta can connect
-    int64_t lo = 0, hi = 0;
+    int lo = 0, hi = 0;
     if(valid && pa == 4) {
-      int64_t a = g.goff[kg], b = g.goff[kg + 1];
+      int a = m0, b = m1;
       while(a < b) {  // lower bound
-        const int64_t mid = (a + b) >> 1;
+        const int mid = (a + b) >> 1;
         if(sp_cmp(ld_spin<NSW>(g.sbeta, mid), bb) < 0)
           a = mid + 1;
         else
           b = mid;
       }
       lo = a;
-      b = g.goff[kg + 1];
+      b = m1;
       while(a < b) {  // upper bound
-        const int64_t mid = (a + b) >> 1;
+        const int mid = (a + b) >> 1;
         if(sp_cmp(ld_spin<NSW>(g.sbeta, mid), bb) <= 0)
           a = mid + 1;
         else
@@ -1232,74 +1246,87 @@ __device__ __forceinline__ void gen_enumerate(const GenData& g, int32_t rg,
       }
       hi = a;
     }
-    int rem = int(hi - lo);
-    int maxrem = rem;
+    const int rem = hi - lo;
+    const int maxrem = __reduce_max_sync(0xffffffffu, rem);
+    for(int r = 0; r < maxrem; ++r) emit(r < rem, lo + r, 4, 0);
+    // pa <= 3: the members of small groups, taken together
+    const bool scan = valid && pa <= 3;
+    const int small = scan && m1 - m0 <= 32 ? m1 - m0 : 0;
+    int incl = warp_incl_scan(small);
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const int mbase = m0 - (incl - small);  // member e of the run is mbase + e
+    for(int e0 = 0; e0 < total; e0 += 32) {
+      const int e = e0 + lane;
+      int L = 0;  // lanes whose members end at or before e
 #pragma unroll
-    for(int o = 16; o; o >>= 1)
-      maxrem = max(maxrem, __shfl_xor_sync(0xffffffffu, maxrem, o));
-    for(int r = 0; r < maxrem; ++r) emit(r < rem, lo + r, kg, 4, 0);
-    // pa <= 3: scan the group members
-    unsigned scan = __ballot_sync(0xffffffffu, valid && pa <= 3);
-    while(scan) {
-      const int L = __ffs(scan) - 1;
-      scan &= scan - 1;
-      const int32_t gg = __shfl_sync(0xffffffffu, kg, L);
+      for(int st = 16; st; st >>= 1)
+        if(__shfl_sync(0xffffffffu, incl, L + st - 1) <= e) L += st;
+      const int src = L < 32 ? L : 31;
+      const int64_t m = __shfl_sync(0xffffffffu, mbase, src) + e;
+      const int ppa = __shfl_sync(0xffffffffu, pa, src);
+      int pb = 99;
+      if(e < total) pb = sp_popc(ld_spin<NSW>(g.sbeta, m) ^ bb);
+      emit(pb <= 4 - ppa, m, ppa, pb);
+    }
+    // the larger groups, one at a time
+    unsigned big = __ballot_sync(0xffffffffu, scan && m1 - m0 > 32);
+    while(big) {
+      const int L = __ffs(big) - 1;
+      big &= big - 1;
       const int ppa = __shfl_sync(0xffffffffu, pa, L);
       const int limit = 4 - ppa;
-      const int64_t m0 = g.goff[gg], m1 = g.goff[gg + 1];
-      const int64_t h0 = g.hoff[gg], hs = g.hoff[gg + 1] - h0;
-      if(ppa == 2 && hs > 0 && g.gbpop[gg] == nob &&
-         m1 - m0 > 8 * int64_t(nenum)) {
+      const int gm0 = __shfl_sync(0xffffffffu, m0, L);
+      const int gm1 = __shfl_sync(0xffffffffu, m1, L);
+      if(__shfl_sync(0xffffffffu, int(probe), L)) {
         // alpha single into a large group: only betas within one
         // excitation of bb connect, and all of them have bb's popcount
-        const uint64_t mask = uint64_t(hs) - 1;
+        const int64_t gh0 = __shfl_sync(0xffffffffu, h0, L);
+        const int64_t ghs = __shfl_sync(0xffffffffu, hs, L);
+        const uint64_t mask = uint64_t(ghs) - 1;
         for(int u0 = 0; u0 < nenum; u0 += 32) {
           const int u = u0 + lane;
-          int64_t lo = 0, hi = 0;
+          int plo = 0, phi = 0;
           int pbv = 0;
           if(u < nenum) {
             Spin<NSW> q = bb;
             if(u > 0) {
               const int i = int((float(u - 1) + 0.5f) * rnv);
-              const int j = (u - 1) - i * nvb;
-              q = sp_flip(sp_flip(q, ov[i]), ov[128 + j]);
+              const int jv = (u - 1) - i * nvb;
+              q = sp_flip(sp_flip(q, ov[i]), ov[128 + jv]);
               pbv = 2;
             }
             uint64_t slot = spin_hash<NSW>(q) & mask;
-            for(int64_t t = 0; t < hs; ++t) {
-              const int32_t r = g.htab[h0 + slot];
+            for(int64_t t = 0; t < ghs; ++t) {
+              const int32_t r = g.htab[gh0 + slot];
               if(r < 0) break;
-              if(ld_spin<NSW>(g.sbeta, m0 + r) == q) {
-                lo = m0 + r;
-                hi = lo + 1;
-                while(hi < m1 && ld_spin<NSW>(g.sbeta, hi) == q) ++hi;
+              if(ld_spin<NSW>(g.sbeta, gm0 + r) == q) {
+                plo = gm0 + r;
+                phi = plo + 1;
+                while(phi < gm1 && ld_spin<NSW>(g.sbeta, phi) == q) ++phi;
                 break;
               }
               slot = (slot + 1) & mask;
             }
           }
-          const int rem = int(hi - lo);
-          int mr = rem;
-#pragma unroll
-          for(int o = 16; o; o >>= 1)
-            mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, o));
-          for(int r = 0; r < mr; ++r) emit(r < rem, lo + r, gg, 2, pbv);
+          const int prem = phi - plo;
+          const int mr = __reduce_max_sync(0xffffffffu, prem);
+          for(int r = 0; r < mr; ++r) emit(r < prem, plo + r, 2, pbv);
         }
         continue;
       }
       // four loads in flight: groups are a few hundred members, and the loop
       // waits for each load
-      for(int64_t base = m0; base < m1; base += 128) {
+      for(int mb = gm0; mb < gm1; mb += 128) {
         int pb[4];
 #pragma unroll
         for(int u = 0; u < 4; ++u) {
-          const int64_t m = base + 32 * u + lane;
-          pb[u] = m < m1 ? sp_popc(ld_spin<NSW>(g.sbeta, m) ^ bb) : 99;
+          const int m = mb + 32 * u + lane;
+          pb[u] = m < gm1 ? sp_popc(ld_spin<NSW>(g.sbeta, m) ^ bb) : 99;
         }
 #pragma unroll
         for(int u = 0; u < 4; ++u)
-          if(base + 32 * u < m1)
-            emit(pb[u] <= limit, base + 32 * u + lane, gg, ppa, pb[u]);
+          if(mb + 32 * u < gm1)
+            emit(pb[u] <= limit, mb + 32 * u + lane, ppa, pb[u]);
       }
     }
   }
@@ -1307,39 +1334,32 @@ __device__ __forceinline__ void gen_enumerate(const GenData& g, int32_t rg,
 
 // The connected kets of a row are a few of the members that gen_enumerate
 // tests (1.5 % on an n = 48 list of 1.5e5 determinants), so its chunks of 32
-// hold one or two each. gen_pairs queues them and calls eval(on, m, ket
-// group, is_double) with 32 at a time, doubles and the rest (singles, the
-// diagonal, lists of mixed electron counts) apart: an element then costs a
-// lane's share of the warp's instructions and not all of them. q: 128
-// entries of shared memory per warp.
+// hold one or two each. gen_pairs queues them and calls eval(on, m,
+// is_double) with 32 at a time, doubles and the rest (singles, the diagonal,
+// lists of mixed electron counts) apart: an element then costs a lane's share
+// of the warp's instructions and not all of them. q: 128 entries of shared
+// memory per warp.
 template <int NSW, class F>
 __device__ __forceinline__ void gen_pairs(const GenData& g, int32_t rg,
                                           Spin<NSW> ba, Spin<NSW> bb,
-                                          uint8_t* ov, uint64_t* q, F&& eval) {
+                                          uint8_t* ov, uint32_t* q, F&& eval) {
   const int lane = threadIdx.x & 31;
   int n[2] = {0, 0};  // queued: others, doubles
-  auto run = [&](int c, int cnt) {
-    const bool on = lane < cnt;
-    const uint64_t e = on ? q[64 * c + lane] : 0;
-    eval(on, int64_t(e & 0xffffffffu), int32_t(e >> 32), c == 1);
-  };
   gen_enumerate<NSW>(g, rg, ba, bb, ov,
-                     [&](bool act, int64_t m, int32_t kg, int pa, int pb) {
+                     [&](bool act, int64_t m, int pa, int pb) {
     if(!__any_sync(0xffffffffu, act)) return;
     const bool dbl = pa + pb == 4 && !(pa & 1);
 #pragma unroll
     for(int c = 0; c < 2; ++c) {
       const bool mine = act && dbl == (c == 1);
       const unsigned msk = __ballot_sync(0xffffffffu, mine);
-      if(mine)
-        q[64 * c + n[c] + __popc(msk & lanemask_lt())] =
-            (uint64_t(uint32_t(kg)) << 32) | uint32_t(m);
+      if(mine) q[64 * c + n[c] + __popc(msk & lanemask_lt())] = uint32_t(m);
       n[c] += __popc(msk);
       if(n[c] >= 32) {
         __syncwarp();
-        run(c, 32);
+        eval(true, int64_t(q[64 * c + lane]), c == 1);
         n[c] -= 32;
-        const uint64_t t = lane < n[c] ? q[64 * c + 32 + lane] : 0;
+        const uint32_t t = lane < n[c] ? q[64 * c + 32 + lane] : 0;
         __syncwarp();
         if(lane < n[c]) q[64 * c + lane] = t;
       }
@@ -1348,169 +1368,222 @@ __device__ __forceinline__ void gen_pairs(const GenData& g, int32_t rg,
   __syncwarp();
 #pragma unroll
   for(int c = 0; c < 2; ++c)
-    if(n[c]) run(c, n[c]);
+    if(n[c]) eval(lane < n[c], int64_t(lane < n[c] ? q[64 * c + lane] : 0), c == 1);
   __syncwarp();
 }
-constexpr int GEN_SCRATCH = 256 + 128 * 8;  // bytes per warp: ov, q
+constexpr int GEN_SCRATCH = 256 + 128 * 4;  // bytes per warp: ov, q
 
+// H(bra, ket) of a connected pair, evaluated by class.
+template <int NSW>
+__device__ __forceinline__ double gen_element(const Ints& I, bool dbl,
+                                              Spin<NSW> ba, Spin<NSW> bb,
+                                              Spin<NSW> ka, Spin<NSW> kb,
+                                              double hd) {
+  if(dbl) return me_double(I, ba, bb, ka, kb);
+  if(ka == ba && kb == bb) return hd;
+  return me_generic(I, ba, bb, ka, kb);
+}
+
+// Candidates per row, and the rows' candidates themselves (sorted positions)
+// as far as `list` holds them: a row of at most GEN_CAP takes its run of the
+// list when it is done (list_off: its start, -1 when it found no room or is
+// longer), so the fill need not enumerate again.
 template <int NBITS>
 __global__ void __launch_bounds__(HB_THREADS)
-    gen_count_k(GenData g, const uint64_t* bra, size_t nbra, int64_t* cnt) {
+    gen_list_k(GenData g, const uint64_t* bra, int64_t nbra, int64_t* cnt,
+               uint32_t* list, unsigned long long cap,
+               unsigned long long* used, int64_t* list_off, unsigned* ctr) {
   using D = DetTraits<NBITS>;
   __shared__ uint8_t s_ov[HB_WARPS][256];
-  const int64_t nwarp = int64_t(gridDim.x) * HB_WARPS;
-  for(int64_t row = int64_t(blockIdx.x) * HB_WARPS + (threadIdx.x >> 5);
-      row < int64_t(nbra); row += nwarp) {
+  __shared__ uint32_t s_m[HB_WARPS][GEN_CAP];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t* sm = s_m[wid];
+  for(int64_t row; (row = next_row(ctr)) < nbra;) {
     const int32_t rg = g.rowgroup[row];
-    int64_t c = 0;
+    int c = 0;
     if(rg >= 0) {
       const auto ba = D::alpha(bra + row * D::NW);
       const auto bb = D::beta(bra + row * D::NW);
-      gen_enumerate<D::NSW>(g, rg, ba, bb, s_ov[threadIdx.x >> 5],
-                            [&](bool act, int64_t, int32_t, int, int) {
-        c += __popc(__ballot_sync(0xffffffffu, act));
+      gen_enumerate<D::NSW>(g, rg, ba, bb, s_ov[wid],
+                            [&](bool act, int64_t m, int, int) {
+        const unsigned msk = __ballot_sync(0xffffffffu, act);
+        if(act) {
+          const int pos = c + __popc(msk & lanemask_lt());
+          if(pos < GEN_CAP) sm[pos] = uint32_t(m);
+        }
+        c += __popc(msk);
       });
     }
-    if((threadIdx.x & 31) == 0) cnt[row] = c;
+    __syncwarp();
+    unsigned long long off = 0;
+    if(lane == 0) {
+      cnt[row] = c;
+      off = c && c <= GEN_CAP ? atomicAdd(used, (unsigned long long)c) : cap;
+      list_off[row] = off + c <= cap ? int64_t(off) : -1;
+    }
+    off = __shfl_sync(0xffffffffu, off, 0);
+    if(off + c <= cap)
+      for(int i = lane; i < c; i += 32) list[off + i] = sm[i];
+    __syncwarp();
   }
 }
 
-// Fill: candidates go to a per-warp shared buffer (col, value), are sorted
-// by column with a bitonic network and written with threshold compaction.
-// Rows with more than GEN_CAP candidates are written unsorted to the
-// long-row scratch (lcol/lval at loff[row]) and finished by the radix sort.
+// Fill: a row's candidates go to a per-warp shared buffer as (column, sorted
+// position), are sorted by column with a bitonic network, evaluated in that
+// order with every lane busy and written in place; singles (sums over the
+// occupied orbitals) are put off and evaluated together. Elements at or below
+// the threshold are marked with column -1. Rows with more than GEN_CAP
+// candidates are written unsorted to the long-row scratch (lkey/lval at
+// loff[row]) and finished by the radix sort.
 template <int NBITS, typename CI, typename VT>
 __global__ void __launch_bounds__(HB_THREADS)
     gen_fill_k(Ints I, GenData g, const uint64_t* bra, int64_t row_a,
                int64_t row_b, const double* __restrict__ hdiag,
                const int64_t* __restrict__ rowptr,
+               const uint32_t* __restrict__ list,
+               const int64_t* __restrict__ list_off,
                const int64_t* __restrict__ loff, int64_t lbase0,
                const uint32_t* __restrict__ lidx, uint64_t* lkey,
                double* lval, CI* __restrict__ colind, VT* __restrict__ nzval,
                double* __restrict__ diag, int64_t* __restrict__ rowcnt,
-               double thresh) {
+               double thresh, unsigned* ctr, unsigned long long* ndropped) {
   using D = DetTraits<NBITS>;
   constexpr int NSW = D::NSW;
-  __shared__ uint32_t s_col[HB_WARPS][GEN_CAP];
-  __shared__ double s_val[HB_WARPS][GEN_CAP];
-  // orbital lists of the bra beta and the pair queues: dynamic, since the
-  // candidate buffers take the whole static allowance
-  extern __shared__ __align__(16) uint8_t gen_ov[];
+  __shared__ uint64_t s_key[HB_WARPS][GEN_CAP];
+  __shared__ __align__(16) uint8_t s_scr[HB_WARPS][GEN_SCRATCH];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t* bc = s_col[wid];
-  double* bv = s_val[wid];
-  const int64_t nwarp = int64_t(gridDim.x) * HB_WARPS;
-  for(int64_t row = row_a + int64_t(blockIdx.x) * HB_WARPS + wid; row < row_b;
-      row += nwarp) {
+  uint64_t* bk = s_key[wid];
+  uint8_t* ov = s_scr[wid];
+  uint32_t* q = reinterpret_cast<uint32_t*>(ov + 256);
+  for(int64_t row; (row = row_a + next_row(ctr)) < row_b;) {
     const int32_t rg = g.rowgroup[row];
     const int64_t ncand = rowptr[row + 1] - rowptr[row];
     if(rg < 0 || ncand == 0) {
       if(lane == 0) rowcnt[row] = 0;
       continue;
     }
-    const bool lng = ncand > GEN_CAP;
-    // long rows: (long-row index, column) sort keys and values into this
-    // chunk's scratch
-    const int64_t lbase = lng ? loff[row] - lbase0 : 0;
-    const uint64_t lhi = lng ? uint64_t(lidx[row]) << 32 : 0;
     const uint64_t* bd = bra + row * D::NW;
     const Spin<NSW> ba = D::alpha(bd), bb = D::beta(bd);
     const double hd = hdiag[row];
-    int64_t c = 0;
-    gen_pairs<NSW>(g, rg, ba, bb, gen_ov + wid * GEN_SCRATCH,
-                   reinterpret_cast<uint64_t*>(gen_ov + wid * GEN_SCRATCH + 256),
-                   [&](bool act, int64_t m, int32_t kg, bool dbl) {
-      double h = 0;
-      uint32_t col = 0;
-      if(act) {
-        const Spin<NSW> ka = ld_spin<NSW>(g.kalpha, kg);
-        const Spin<NSW> kb = ld_spin<NSW>(g.sbeta, m);
-        if(dbl)
-          h = me_double(I, ba, bb, ka, kb);
-        else if(ka == ba && kb == bb)
-          h = hd;
-        else
-          h = me_generic(I, ba, bb, ka, kb);
-        col = g.sidx[m];
-      }
-      const unsigned msk = __ballot_sync(0xffffffffu, act);
-      if(act) {
-        const int64_t pos = c + __popc(msk & lanemask_lt());
-        if(lng) {
-          lkey[lbase + pos] = lhi | col;
-          lval[lbase + pos] = h;
-        } else {
-          bc[pos] = col;
-          bv[pos] = h;
+    if(ncand > GEN_CAP) {
+      // long rows: (long-row index, column) sort keys and values into this
+      // chunk's scratch; rowcnt comes from the long-row pass
+      const int64_t lbase = loff[row] - lbase0;
+      const uint64_t lhi = uint64_t(lidx[row]) << 32;
+      int64_t c = 0;
+      gen_pairs<NSW>(g, rg, ba, bb, ov, q, [&](bool act, int64_t m, bool dbl) {
+        const unsigned msk = __ballot_sync(0xffffffffu, act);
+        if(act) {
+          const int64_t pos = lbase + c + __popc(msk & lanemask_lt());
+          lkey[pos] = lhi | g.sidx[m];
+          lval[pos] = gen_element<NSW>(I, dbl, ba, bb, ld_spin<NSW>(g.salpha, m),
+                                       ld_spin<NSW>(g.sbeta, m), hd);
         }
-      }
-      c += __popc(msk);
-    });
-    if(lng) {
-      if(lane == 0) rowcnt[row] = -1;  // finished by the long-row pass
+        c += __popc(msk);
+      });
       continue;
     }
-    __syncwarp();
-    // bitonic sort of the c entries by column
+    const int c = int(ncand);
+    const int64_t lo = list_off[row];
+    if(lo >= 0) {
+      for(int i = lane; i < c; i += 32) {
+        const uint32_t m = list[lo + i];
+        bk[i] = (uint64_t(g.sidx[m]) << 32) | m;
+      }
+    } else {
+      int n = 0;
+      gen_enumerate<NSW>(g, rg, ba, bb, ov, [&](bool act, int64_t m, int, int) {
+        const unsigned msk = __ballot_sync(0xffffffffu, act);
+        if(act)
+          bk[n + __popc(msk & lanemask_lt())] =
+              (uint64_t(g.sidx[m]) << 32) | uint32_t(m);
+        n += __popc(msk);
+      });
+    }
     int P = 1;
     while(P < c) P <<= 1;
-    for(int i = int(c) + lane; i < P; i += 32) bc[i] = 0xffffffffu;
+    for(int i = c + lane; i < P; i += 32) bk[i] = ~0ull;
     __syncwarp();
     for(int k = 2; k <= P; k <<= 1)
       for(int jj = k >> 1; jj > 0; jj >>= 1) {
-        for(int i = lane; i < P; i += 32) {
-          const int ixj = i ^ jj;
-          if(ixj > i) {
-            const bool up = (i & k) == 0;
-            const uint32_t a = bc[i], b = bc[ixj];
-            if((a > b) == up) {
-              bc[i] = b;
-              bc[ixj] = a;
-              const double t = bv[i];
-              bv[i] = bv[ixj];
-              bv[ixj] = t;
-            }
+        for(int t = lane; t < (P >> 1); t += 32) {
+          const int i = 2 * t - (t & (jj - 1));  // the pair (i, i + jj)
+          const uint64_t x = bk[i], y = bk[i + jj];
+          if((x > y) == ((i & k) == 0)) {
+            bk[i] = y;
+            bk[i + jj] = x;
           }
         }
         __syncwarp();
       }
-    // threshold compaction into the row
     const int64_t out0 = rowptr[row];
-    int64_t kept = 0;
-    for(int64_t base = 0; base < c; base += 32) {
-      const int64_t i = base + lane;
-      bool keep = false;
-      uint32_t col = 0;
-      double h = 0;
+    CI* __restrict__ rc = colind + out0;
+    VT* __restrict__ rv = nzval + out0;
+    int dropped = 0, nq = 0;
+    auto put = [&](int i, uint32_t col, double h) {
+      const bool keep = fabs(h) > thresh;
+      const bool isd = keep && int64_t(col) == row;
+      dropped += !keep;
+      rc[i] = keep ? CI(col) : CI(-1);
+      rv[i] = store_val<VT>(h, isd);
+      if(isd) diag[row] = h;
+    };
+    auto others = [&](int cnt) {  // queued positions of singles / diagonal
+      if(lane < cnt) {
+        const int i = int(q[lane]);
+        const uint64_t key = bk[i];
+        const uint32_t m = uint32_t(key);
+        put(i, uint32_t(key >> 32),
+            gen_element<NSW>(I, false, ba, bb, ld_spin<NSW>(g.salpha, m),
+                             ld_spin<NSW>(g.sbeta, m), hd));
+      }
+    };
+    for(int i0 = 0; i0 < c; i0 += 32) {
+      const int i = i0 + lane;
+      bool put_off = false;
       if(i < c) {
-        col = bc[i];
-        h = bv[i];
-        keep = fabs(h) > thresh;
+        const uint64_t key = bk[i];
+        const uint32_t m = uint32_t(key);
+        const Spin<NSW> ka = ld_spin<NSW>(g.salpha, m);
+        const Spin<NSW> kb = ld_spin<NSW>(g.sbeta, m);
+        const int ca = sp_popc(ba ^ ka), cb = sp_popc(bb ^ kb);
+        if(ca + cb == 4 && !(ca & 1))
+          put(i, uint32_t(key >> 32), me_double(I, ba, bb, ka, kb));
+        else
+          put_off = true;
       }
-      const unsigned msk = __ballot_sync(0xffffffffu, keep);
-      if(keep) {
-        const int64_t pos = out0 + kept + __popc(msk & lanemask_lt());
-        const bool isd = int64_t(col) == row;
-        colind[pos] = CI(col);
-        nzval[pos] = store_val<VT>(h, isd);
-        if(isd) diag[row] = h;
+      const unsigned msk = __ballot_sync(0xffffffffu, put_off);
+      if(put_off) q[nq + __popc(msk & lanemask_lt())] = uint32_t(i);
+      nq += __popc(msk);
+      if(nq >= 32) {
+        __syncwarp();
+        others(32);
+        nq -= 32;
+        const uint32_t t = lane < nq ? q[32 + lane] : 0;
+        __syncwarp();
+        if(lane < nq) q[lane] = t;
       }
-      kept += __popc(msk);
     }
-    if(lane == 0) rowcnt[row] = kept;
+    __syncwarp();
+    others(nq);
+    dropped = __reduce_add_sync(0xffffffffu, dropped);
+    if(lane == 0) {
+      rowcnt[row] = ncand - dropped;
+      if(dropped) atomicAdd(ndropped, (unsigned long long)dropped);
+    }
     __syncwarp();
   }
 }
 
 // Long rows: the keys (row_rank << 32 | col) were radix-sorted with their
-// FP64 values; write them back with threshold compaction.
+// FP64 values; write them back, marking what the threshold drops.
 template <typename CI, typename VT>
 __global__ void long_rows_write_k(const int64_t* lrows, int64_t nl,
                                   const int64_t* loff_sorted, int64_t base0,
                                   const uint64_t* keys, const double* vals,
                                   const int64_t* rowptr, CI* colind,
                                   VT* nzval, double* diag, int64_t* rowcnt,
-                                  double thresh) {
+                                  double thresh, unsigned long long* ndropped) {
   const int lane = threadIdx.x & 31;
   const int64_t nwarp = int64_t(gridDim.x) * (blockDim.x >> 5);
   for(int64_t r = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1518,28 +1591,22 @@ __global__ void long_rows_write_k(const int64_t* lrows, int64_t nl,
     const int64_t row = lrows[r];
     const int64_t b = loff_sorted[r] - base0, e = loff_sorted[r + 1] - base0;
     const int64_t out0 = rowptr[row];
-    int64_t kept = 0;
-    for(int64_t base = b; base < e; base += 32) {
-      const int64_t i = base + lane;
-      bool keep = false;
-      uint32_t col = 0;
-      double h = 0;
-      if(i < e) {
-        col = uint32_t(keys[i] & 0xffffffffull);
-        h = vals[i];
-        keep = fabs(h) > thresh;
-      }
-      const unsigned msk = __ballot_sync(0xffffffffu, keep);
-      if(keep) {
-        const int64_t pos = out0 + kept + __popc(msk & lanemask_lt());
-        const bool isd = int64_t(col) == row;
-        colind[pos] = CI(col);
-        nzval[pos] = store_val<VT>(h, isd);
-        if(isd) diag[row] = h;
-      }
-      kept += __popc(msk);
+    int dropped = 0;
+    for(int64_t i = b + lane; i < e; i += 32) {
+      const uint32_t col = uint32_t(keys[i] & 0xffffffffull);
+      const double h = vals[i];
+      const bool keep = fabs(h) > thresh;
+      const bool isd = keep && int64_t(col) == row;
+      dropped += !keep;
+      colind[out0 + i - b] = keep ? CI(col) : CI(-1);
+      nzval[out0 + i - b] = store_val<VT>(h, isd);
+      if(isd) diag[row] = h;
     }
-    if(lane == 0) rowcnt[row] = kept;
+    dropped = __reduce_add_sync(0xffffffffu, dropped);
+    if(lane == 0) {
+      rowcnt[row] = e - b - dropped;
+      if(dropped) atomicAdd(ndropped, (unsigned long long)dropped);
+    }
   }
 }
 
@@ -1567,23 +1634,6 @@ __global__ void long_rowoff_k(const int64_t* lrows, const int64_t* loff,
     loff_row[lrows[r]] = loff[r];
 }
 
-// --------------------------------------------------------- compaction
-template <typename CI, typename VT>
-__global__ void compact_rows_k(const int64_t* oldptr, const int64_t* newptr,
-                               size_t m, const CI* ci, const VT* nz, CI* ci2,
-                               VT* nz2) {
-  const int lane = threadIdx.x & 31;
-  const size_t nwarp = size_t(gridDim.x) * (blockDim.x >> 5);
-  for(size_t r = size_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-      r < m; r += nwarp) {
-    const int64_t s = oldptr[r], d = newptr[r], n = newptr[r + 1] - d;
-    for(int64_t i = lane; i < n; i += 32) {
-      ci2[d + i] = ci[s + i];
-      nz2[d + i] = nz[s + i];
-    }
-  }
-}
-
 template <typename CI>
 __global__ void rowptr_cast_k(const int64_t* in, size_t n, CI* out) {
   for(size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -1609,7 +1659,8 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
   constexpr int KW = GenKey<NBITS>::KW;
   auto sort_side = [&](const uint64_t* dets, size_t n, uint64_t*& keys,
                        uint32_t*& idx, int64_t*& goff, uint64_t*& galpha,
-                       uint64_t*& sbeta, int32_t* rowgroup, uint32_t& ng) {
+                       uint64_t*& salpha, uint64_t*& sbeta, int32_t* rowgroup,
+                       uint32_t& ng) {
     keys = A.get<uint64_t>(n * KW);
     idx = A.get<uint32_t>(n);
     uint64_t* k2 = A.get<uint64_t>(n * KW);
@@ -1629,25 +1680,33 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     ng = to_host(gx + n, s);
     goff = A.get<int64_t>(ng + 1);
     galpha = A.get<uint64_t>((ng + 1) * NSW);
+    salpha = A.get<uint64_t>(n * NSW);
     sbeta = A.get<uint64_t>(n * NSW);
     gen_groups_k<NBITS><<<grid_for(n, 256, 8 * sms), 256, 0, s>>>(
-        keys, idx, flags, gx, n, goff, galpha, sbeta, rowgroup), note_launch();
+        keys, idx, flags, gx, n, goff, galpha, salpha, sbeta, rowgroup),
+        note_launch();
+    A.release(keys);
+    A.release(flags);
+    A.release(gx);
     gen_group_end_k<<<1, 1, 0, s>>>(goff, ng, int64_t(n)), note_launch();
   };
-  uint64_t *kkeys, *kalpha, *ksbeta;
+  uint64_t *kkeys, *kalpha, *ksalpha, *ksbeta;
   uint32_t *kidx, nkg = 0;
   int64_t* kgoff;
   int32_t* rowgroup = A.get<int32_t>(sub ? nket : nbra);
-  sort_side(ket, nket, kkeys, kidx, kgoff, kalpha, ksbeta,
+  sort_side(ket, nket, kkeys, kidx, kgoff, kalpha, ksalpha, ksbeta,
             sub ? rowgroup : nullptr, nkg);
   if(sub) rowgroup += r0;
   const uint64_t* balpha = kalpha;
   uint32_t nbg = nkg;
   if(!sub) {
-    uint64_t *bkeys, *bsbeta, *bal;
+    uint64_t *bkeys, *bsalpha, *bsbeta, *bal;
     uint32_t* bidx;
     int64_t* bgoff;
-    sort_side(bra, nbra, bkeys, bidx, bgoff, bal, bsbeta, rowgroup, nbg);
+    sort_side(bra, nbra, bkeys, bidx, bgoff, bal, bsalpha, bsbeta, rowgroup,
+              nbg);
+    A.release(bsalpha);
+    A.release(bsbeta);
     balpha = bal;
   }
   // alpha connectivity bra groups -> ket groups
@@ -1663,6 +1722,10 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
   uint8_t* apa = A.get<uint8_t>(natot + 1);
   gen_aconn_k<NSW><<<ga, 256, 0, s>>>(balpha, nbg, kalpha, nkg, aoff, acnt,
                                       acnt4, acol, apa), note_launch();
+  int32_t* mgroup = A.get<int32_t>(nket);
+  MB_CUDA(cudaMemsetAsync(mgroup, 0xFF, nket * 4, s));
+  gen_mgroup_k<<<grid_for(size_t(nkg) * 32, 256, 16 * sms), 256, 0, s>>>(
+      kgoff, nkg, mgroup), note_launch();
   // beta hash tables of the large ket groups
   int64_t* hoff = A.get<int64_t>(nkg + 1);
   int32_t* gbpop = A.get<int32_t>(nkg + 1);
@@ -1677,12 +1740,12 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     htab = A.get<int32_t>(size_t(std::max<int64_t>(htot, 1)));
     MB_CUDA(cudaMemsetAsync(htab, 0xFF, size_t(std::max<int64_t>(htot, 1)) * 4, s));
     if(htot > 0)
-      gen_hinsert_k<NSW><<<gh, 256, 0, s>>>(kgoff, nkg, ksbeta, hoff, htab), note_launch();
+      gen_hinsert_k<NSW><<<grid_for(nket, 256, 16 * sms), 256, 0, s>>>(
+          kgoff, mgroup, nket, ksbeta, hoff, htab), note_launch();
   }
   // beta-major view of the kets
   uint64_t *bm_alpha, *bgbeta;
   uint32_t* bm_m;
-  int32_t* mgroup;
   int64_t* bgoff;
   int64_t nbgb = 0;
   {
@@ -1698,10 +1761,6 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     uint32_t* amaj = A.get<uint32_t>(nket);
     gen_invert_k<<<grid_for(nket, 256, 8 * sms), 256, 0, s>>>(kidx, nket,
                                                              amaj), note_launch();
-    mgroup = A.get<int32_t>(nket);
-    MB_CUDA(cudaMemsetAsync(mgroup, 0xFF, nket * 4, s));
-    gen_mgroup_k<<<grid_for(size_t(nkg) * 32, 256, 16 * sms), 256, 0, s>>>(
-        kgoff, nkg, mgroup), note_launch();
     bm_alpha = A.get<uint64_t>(nket * NSW);
     bm_m = A.get<uint32_t>(nket);
     uint32_t* bfl = A.get<uint32_t>(nket);
@@ -1721,7 +1780,7 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     A.release(bfl);
     A.release(bgx);
   }
-  GenData gd{rowgroup, aoff, acol, apa, kgoff, kalpha, ksbeta, kidx,
+  GenData gd{rowgroup, aoff, acol, apa, kgoff, ksalpha, ksbeta, kidx,
              hoff, htab, gbpop, h->norb, acnt4,
              bgbeta, bgoff, nbgb, bm_alpha, bm_m, mgroup};
   return gd;
@@ -1811,11 +1870,10 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
   VT* nzval = nullptr;
   // direct product: connectivity counts and row sizes, read back together
   DPTotals tot{};
-  DPTotals* d_tot = nullptr;
+  DPTotals* d_tot = A.get<DPTotals>(1);
+  MB_CUDA(cudaMemsetAsync(d_tot, 0, sizeof(DPTotals), s));
   int64_t *aoff = nullptr, *l2off = nullptr, *l4off = nullptr;
   if(direct) {
-    d_tot = A.get<DPTotals>(1);
-    MB_CUDA(cudaMemsetAsync(d_tot, 0, sizeof(DPTotals), s));
     int32_t* cls_a = A.get<int32_t>(3 * UA);
     int32_t* cls_b = A.get<int32_t>(3 * UB);
     int64_t* cnt = A.get<int64_t>(2 * (UA + UB));
@@ -1926,9 +1984,27 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     // ------------------------------------------------ general path
     GenData gd = gen_plan<NBITS>(h, bra, nbra, ket, nket, sub, r0, A);
     const unsigned gr = grid_for(nbra, HB_WARPS, size_t(sms) * 16);
-    gen_count_k<NBITS><<<gr, HB_THREADS, 0, s>>>(gd, bra, nbra, rowcnt), note_launch();
+    // candidate lists of the rows, as far as a tenth of the memory holds
+    // them (4 B per candidate, at most GEN_CAP per row)
+    unsigned* ctr = A.get<unsigned>(1);
+    auto* used = A.get<unsigned long long>(1);
+    int64_t* list_off = A.get<int64_t>(nbra);
+    const uint64_t cap = std::min<uint64_t>(uint64_t(nbra) * GEN_CAP,
+                                            uint64_t(device_bytes_available() / 40));
+    uint32_t* list = A.get<uint32_t>(cap);
+    MB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), s));
+    MB_CUDA(cudaMemsetAsync(used, 0, 8, s));
+    gen_list_k<NBITS><<<gr, HB_THREADS, 0, s>>>(
+        gd, bra, int64_t(nbra), rowcnt, list, cap, used, list_off, ctr),
+        note_launch();
     exclusive_scan<int64_t, int64_t>(rowcnt, rowptr64, nbra, rowptr64 + nbra, A);
     nnz_ub = to_host(rowptr64 + nbra, s);
+    // a matrix that needs their memory goes without the lists
+    if(1.05 * double(nnz_ub) * (sizeof(CI) + sizeof(VT)) + 1073741824.0 >
+       double(device_bytes_available())) {
+      A.release(list);
+      MB_CUDA(cudaMemsetAsync(list_off, 0xFF, nbra * 8, s));
+    }
     out->nnz_candidates = nnz_ub;
     MB_CUDA(dev_malloc_async(&colind, std::max<int64_t>(nnz_ub, 1) * sizeof(CI), s));
     MB_CUDA(dev_malloc_async(&nzval, std::max<int64_t>(nnz_ub, 1) * sizeof(VT), s));
@@ -1967,10 +2043,6 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     // what is free; short rows of the chunk are written by the same launch.
     int64_t lchunk = int64_t(0.7 * double(device_bytes_available()) / 32.0);
     lchunk = std::max<int64_t>(lchunk, int64_t(1) << 20);
-    constexpr int gen_dyn = HB_WARPS * GEN_SCRATCH;
-    MB_CUDA(cudaFuncSetAttribute(gen_fill_k<NBITS, CI, VT>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 gen_dyn));
     float fill_ms_tot = 0.f;
     int64_t la = 0;  // next long row (list index)
     int64_t row_a = 0;
@@ -1985,9 +2057,11 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
       uint64_t* lkey = C.get<uint64_t>(centries + 1);
       double* lval = C.get<double>(centries + 1);
       cudaEventRecord(ev[0], s);
-      gen_fill_k<NBITS, CI, VT><<<gr, HB_THREADS, gen_dyn, s>>>(
-          I, gd, bra, row_a, row_b, hdiag, rowptr64, loff_row, cbase, lpos,
-          lkey, lval, colind, nzval, out->diag, rowcnt, thresh), note_launch();
+      MB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), s));
+      gen_fill_k<NBITS, CI, VT><<<gr, HB_THREADS, 0, s>>>(
+          I, gd, bra, row_a, row_b, hdiag, rowptr64, list, list_off, loff_row,
+          cbase, lpos, lkey, lval, colind, nzval, out->diag, rowcnt, thresh,
+          ctr, &d_tot->dropped), note_launch();
       cudaEventRecord(ev[1], s);
       MB_CUDA(cudaGetLastError());
       MB_CUDA(cudaEventSynchronize(ev[1]));
@@ -2001,7 +2075,8 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
         long_rows_write_k<CI, VT><<<grid_for(size_t(lb - la) * 32, 256, 8 * sms),
                                     256, 0, s>>>(
             lrows + la, lb - la, loff + la, cbase, lkey, lval, rowptr64,
-            colind, nzval, out->diag, rowcnt, thresh), note_launch();
+            colind, nzval, out->diag, rowcnt, thresh, &d_tot->dropped),
+            note_launch();
         MB_CUDA(cudaGetLastError());
       }
       la = lb;
@@ -2014,8 +2089,8 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
   // ------------------------------------------- exact row pointer + compaction
   int64_t* newptr = rowptr64;
   int64_t nnz = nnz_ub;
-  // (a direct product that dropped nothing keeps its row pointer)
-  if(!direct || to_host(&d_tot->dropped, s) != 0) {
+  // (when nothing was dropped the candidate row pointer stands)
+  if(to_host(&d_tot->dropped, s) != 0) {
     newptr = A.get<int64_t>(nbra + 1);
     exclusive_scan<int64_t, int64_t>(rowcnt, newptr, nbra, newptr + nbra, A);
     nnz = to_host(newptr + nbra, s);
@@ -2029,12 +2104,8 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     VT* nz2 = nullptr;
     MB_CUDA(dev_malloc_async(&ci2, std::max<int64_t>(nnz, 1) * sizeof(CI), s));
     MB_CUDA(dev_malloc_async(&nz2, std::max<int64_t>(nnz, 1) * sizeof(VT), s));
-    if(direct)
-      compact_marked_k<CI, VT><<<grid_for(nbra * 32, 256, 16 * sms), 256, 0, s>>>(
-          rowptr64, newptr, nbra, colind, nzval, ci2, nz2), note_launch();
-    else
-      compact_rows_k<CI, VT><<<grid_for(nbra * 32, 256, 16 * sms), 256, 0, s>>>(
-          rowptr64, newptr, nbra, colind, nzval, ci2, nz2), note_launch();
+    compact_marked_k<CI, VT><<<grid_for(nbra * 32, 256, 16 * sms), 256, 0, s>>>(
+        rowptr64, newptr, nbra, colind, nzval, ci2, nz2), note_launch();
     cudaFreeAsync(colind, s);
     cudaFreeAsync(nzval, s);
     colind = ci2;
@@ -2125,6 +2196,7 @@ struct macis_b200_hop {
   uint64_t* dets = nullptr;  // device copy of the determinant list
   double* diag = nullptr;    // H_ii
   mb::Arena* A = nullptr;    // owns dets, diag and the enumeration tables
+  unsigned* ctr = nullptr;   // row counter of a product
   mb::GenData g{};
 };
 
@@ -2139,34 +2211,25 @@ __global__ void __launch_bounds__(HB_THREADS)
     gen_apply_k(Ints I, GenData g, const uint64_t* dets, int64_t n,
                 const double* __restrict__ hdiag, double thresh, int mixed,
                 double alpha, const double* __restrict__ x, double beta,
-                double* __restrict__ y) {
+                double* __restrict__ y, unsigned* ctr) {
   using D = DetTraits<NBITS>;
   constexpr int NSW = D::NSW;
-  extern __shared__ __align__(16) uint8_t gen_ov[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t nwarp = int64_t(gridDim.x) * HB_WARPS;
-  for(int64_t row = int64_t(blockIdx.x) * HB_WARPS + wid; row < n;
-      row += nwarp) {
+  __shared__ __align__(16) uint8_t s_scr[HB_WARPS][GEN_SCRATCH];
+  const int lane = threadIdx.x & 31;
+  uint8_t* ov = s_scr[threadIdx.x >> 5];
+  for(int64_t row; (row = next_row(ctr)) < n;) {
     const int32_t rg = g.rowgroup[row];
     double acc = 0.0;
     if(rg >= 0) {
       const uint64_t* bd = dets + row * D::NW;
       const Spin<NSW> ba = D::alpha(bd), bb = D::beta(bd);
       const double hd = hdiag[row];
-      gen_pairs<NSW>(g, rg, ba, bb, gen_ov + wid * GEN_SCRATCH,
-                     reinterpret_cast<uint64_t*>(gen_ov + wid * GEN_SCRATCH + 256),
-                     [&](bool act, int64_t m, int32_t kg, bool dbl) {
+      gen_pairs<NSW>(g, rg, ba, bb, ov, reinterpret_cast<uint32_t*>(ov + 256),
+                     [&](bool act, int64_t m, bool dbl) {
         if(act) {
           const uint32_t col = g.sidx[m];
-          const Spin<NSW> ka = ld_spin<NSW>(g.kalpha, kg);
-          const Spin<NSW> kb = ld_spin<NSW>(g.sbeta, m);
-          double h;
-          if(dbl)
-            h = me_double(I, ba, bb, ka, kb);
-          else if(ka == ba && kb == bb)
-            h = hd;
-          else
-            h = me_generic(I, ba, bb, ka, kb);
+          double h = gen_element<NSW>(I, dbl, ba, bb, ld_spin<NSW>(g.salpha, m),
+                                      ld_spin<NSW>(g.sbeta, m), hd);
           if(fabs(h) > thresh) {
             if(mixed && int64_t(col) != row) h = double(float(h));
             acc += h * x[col];
@@ -2209,6 +2272,7 @@ macis_b200_hop* hop_create(macis_b200_ham* h, const uint64_t* dets, size_t n,
                             device_ptrs ? cudaMemcpyDeviceToDevice
                                         : cudaMemcpyHostToDevice, s));
     op->diag = op->A->get<double>(n);
+    op->ctr = op->A->get<unsigned>(1);
 #define MB_HOP_PLAN(NB)                                                     \
   hdiag_k<NB><<<grid_for(n, 256, 8 * sms), 256, 0, s>>>(I, op->dets, n,     \
                                                         op->diag),          \
@@ -2238,13 +2302,13 @@ void hop_apply(const macis_b200_hop* op, double alpha, const double* x,
                double beta, double* y) {
   cudaStream_t s = op->stream;
   const unsigned gr = grid_for(size_t(op->n), HB_WARPS, size_t(num_sms()) * 16);
-  constexpr int dyn = HB_WARPS * GEN_SCRATCH;
   const Ints I = op->I;
+  MB_CUDA(cudaMemsetAsync(op->ctr, 0, sizeof(unsigned), s));
 #define MB_HOP_APPLY(NB)                                                     \
-  gen_apply_k<NB><<<gr, HB_THREADS, dyn, s>>>(I, op->g, op->dets, op->n,     \
-                                              op->diag, op->thresh,          \
-                                              op->mixed ? 1 : 0, alpha, x,   \
-                                              beta, y),                      \
+  gen_apply_k<NB><<<gr, HB_THREADS, 0, s>>>(I, op->g, op->dets, op->n,       \
+                                            op->diag, op->thresh,            \
+                                            op->mixed ? 1 : 0, alpha, x,     \
+                                            beta, y, op->ctr),               \
       note_launch();
   if(op->nbits == 64) {
     MB_HOP_APPLY(64)
@@ -2349,27 +2413,24 @@ __device__ __forceinline__ bool rdm_pair(Spin<NSW> ba, Spin<NSW> bb,
 template <int NBITS>
 __global__ void __launch_bounds__(HB_THREADS)
     rdm_k(GenData g, const uint64_t* dets, int64_t n, const double* C,
-          int norb, double* ordm, int two, RdmSums S) {
+          int norb, double* ordm, int two, RdmSums S, unsigned* ctr) {
   using D = DetTraits<NBITS>;
   constexpr int NSW = D::NSW;
-  extern __shared__ __align__(16) uint8_t gen_ov[];
-  const int wid = threadIdx.x >> 5;
-  const int64_t nwarp = int64_t(gridDim.x) * HB_WARPS;
-  for(int64_t row = int64_t(blockIdx.x) * HB_WARPS + wid; row < n;
-      row += nwarp) {
+  __shared__ __align__(16) uint8_t s_scr[HB_WARPS][GEN_SCRATCH];
+  uint8_t* ov = s_scr[threadIdx.x >> 5];
+  for(int64_t row; (row = next_row(ctr)) < n;) {
     const int32_t rg = g.rowgroup[row];
     double dsum = 0.0;
     if(rg >= 0) {
       const uint64_t* bd = dets + row * D::NW;
       const Spin<NSW> ba = D::alpha(bd), bb = D::beta(bd);
       const double ci = C[row];
-      gen_pairs<NSW>(g, rg, ba, bb, gen_ov + wid * GEN_SCRATCH,
-                     reinterpret_cast<uint64_t*>(gen_ov + wid * GEN_SCRATCH + 256),
-                     [&](bool act, int64_t m, int32_t kg, bool) {
+      gen_pairs<NSW>(g, rg, ba, bb, ov, reinterpret_cast<uint32_t*>(ov + 256),
+                     [&](bool act, int64_t m, bool) {
         if(!act) return;
         const double val = ci * C[g.sidx[m]];
         if(!(fabs(val) > 1e-16)) return;
-        if(rdm_pair<NSW>(ba, bb, ld_spin<NSW>(g.kalpha, kg),
+        if(rdm_pair<NSW>(ba, bb, ld_spin<NSW>(g.salpha, m),
                          ld_spin<NSW>(g.sbeta, m), val, norb, ordm, two != 0, S))
           dsum += val;
       });
@@ -2453,7 +2514,8 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
   cudaStream_t s = h->stream;
   Arena A(s);
   const unsigned gr = grid_for(n, HB_WARPS, size_t(num_sms()) * 16);
-  constexpr int dyn = HB_WARPS * GEN_SCRATCH;
+  unsigned* ctr = A.get<unsigned>(1);
+  MB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), s));
   const size_t n1 = size_t(h->norb), n3 = n1 * n1 * n1, n4 = n3 * n1;
   RdmSums S{};
   S.diag = A.get<double>(n);
@@ -2473,8 +2535,8 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
 #define MB_RDM(NB)                                                          \
   {                                                                         \
     const GenData g = gen_plan<NB>(h, dets, n, dets, n, true, 0, A);        \
-    rdm_k<NB><<<gr, HB_THREADS, dyn, s>>>(g, dets, int64_t(n), C, h->norb,  \
-                                         ordm, two, S),                     \
+    rdm_k<NB><<<gr, HB_THREADS, 0, s>>>(g, dets, int64_t(n), C, h->norb,    \
+                                       ordm, two, S, ctr),                  \
         note_launch();                                                      \
     rdm_diag_k<NB><<<gd, 256, 0, s>>>(dets, int64_t(n), S.diag, h->norb,    \
                                       ordm, two, S),                        \
