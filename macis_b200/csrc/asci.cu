@@ -972,10 +972,12 @@ __device__ __forceinline__ uint32_t bf16_bits(float x) {
   return __bfloat16_as_ushort(__float2bfloat16_rn(x));
 }
 
-// put(k, v): 16-byte piece k (columns [8k, 8k+8)) of the unit's row.
+// put(k, v): 16-byte piece k (columns [8k, 8k+8)) of the unit's row. part: -1
+// all pieces; 0 the occupation bits, 1 the scalar features, 2 and 3 the halves
+// of the eps-weighted occupations.
 template <int NBITS, class Put>
 __device__ void unit_features(const CoreData& cd, double E0, int64_t u,
-                              Put&& put) {
+                              int part, Put&& put) {
   using D = DetTraits<NBITS>;
   constexpr int NSW = D::NSW;
   const size_t c = unit_owner(cd, u);
@@ -987,66 +989,73 @@ __device__ void unit_features(const CoreData& cd, double E0, int64_t u,
   const uint64_t* det = cd.dets + c * D::NW;
   Spin<NSW> sp[2] = {D::alpha(det), D::beta(det)};
   const double* eps[2] = {cd.eps + (c * 2) * n, cd.eps + (c * 2 + 1) * n};
-  int S = 0, hole = -1, part = -1;
+  int S = 0, hole = -1, ptcl = -1;
   if(ud.kind >= 2) {
     S = ud.kind == 3 ? 1 : 0;
     hole = cd.occ[(c * 2 + S) * MAXORB + ud.ii];
-    part = cd.vir[(c * 2 + S) * MAXORB + ud.aa];
-    sp[S] = sp_flip(sp_flip(sp[S], hole), part);
+    ptcl = cd.vir[(c * 2 + S) * MAXORB + ud.aa];
+    sp[S] = sp_flip(sp_flip(sp[S], hole), ptcl);
   }
   // occupation bits, one byte per piece
+  if(part <= 0) {
 #pragma unroll
-  for(int s = 0; s < 2; ++s)
+    for(int s = 0; s < 2; ++s)
 #pragma unroll
-    for(int b = 0; b < NSW * 8; ++b) {
-      const uint32_t byte = uint32_t(sp[s].w[b >> 3] >> ((b & 7) * 8)) & 0xFFu;
-      uint32_t w[4];
+      for(int b = 0; b < NSW * 8; ++b) {
+        const uint32_t byte = uint32_t(sp[s].w[b >> 3] >> ((b & 7) * 8)) & 0xFFu;
+        uint32_t w[4];
 #pragma unroll
-      for(int q = 0; q < 4; ++q)
-        w[q] = (((byte >> (2 * q)) & 1u) ? 0x3F80u : 0u) |
-               (((byte >> (2 * q + 1)) & 1u) ? 0x3F800000u : 0u);
-      put(s * NSW * 8 + b, make_uint4(w[0], w[1], w[2], w[3]));
-    }
-  // scalar features
-  const double eh = hole >= 0 ? eps[S][hole] : 0.0;
-  const double ep = part >= 0 ? eps[S][part] : 0.0;
-  float f[16];
-  f[0] = 1.f;
-  f[1] = float(log(fabs(cd.C[c]) + 1e-300) / 10.0);
-#pragma unroll
-  for(int k = 0; k < 5; ++k) f[2 + k] = ud.kind == k ? 1.f : 0.f;
-  f[7] = float(eh);
-  f[8] = float(ep);
-  f[9] = float(ep - eh);
-  f[10] = float(E0 - cd.hd[c]);
-  f[11] = float(log(1.0 + double(ud.ninner)) / 10.0);
-  f[12] = hole >= 0 ? float(hole + 1) / float(n) : 0.f;
-  f[13] = part >= 0 ? float(part + 1) / float(n) : 0.f;
-  // outer-pair integral bound and a crude log-score estimate
-  const double lnc = log(fabs(cd.C[c]) + 1e-300);
-  if(ud.kind >= 2) {
-    const size_t pr = size_t(part) + size_t(hole) * n;
-    const double bound =
-        cd.pairmax[(ud.kind == 4 ? size_t(n) * n : 0) + pr];
-    const double lb = log(bound + 1e-300);
-    f[14] = float(lb / 10.0);
-    f[15] = float((lnc + lb - log(fabs(E0 - cd.hd[c] - (ep - eh)) + 1e-3)) /
-                  10.0);
-  } else {
-    f[14] = 0.f;
-    f[15] = float((lnc - log(fabs(E0 - cd.hd[c]) + 1e-3)) / 10.0);
+        for(int q = 0; q < 4; ++q)
+          w[q] = (((byte >> (2 * q)) & 1u) ? 0x3F80u : 0u) |
+                 (((byte >> (2 * q + 1)) & 1u) ? 0x3F800000u : 0u);
+        put(s * NSW * 8 + b, make_uint4(w[0], w[1], w[2], w[3]));
+      }
   }
   const int base = 2 * NSW * 8;
+  if(part < 0 || part == 1) {
+    // scalar features
+    const double eh = hole >= 0 ? eps[S][hole] : 0.0;
+    const double ep = ptcl >= 0 ? eps[S][ptcl] : 0.0;
+    float f[16];
+    f[0] = 1.f;
+    f[1] = float(log(fabs(cd.C[c]) + 1e-300) / 10.0);
 #pragma unroll
-  for(int q = 0; q < 2; ++q) {
-    uint32_t w[4];
+    for(int k = 0; k < 5; ++k) f[2 + k] = ud.kind == k ? 1.f : 0.f;
+    f[7] = float(eh);
+    f[8] = float(ep);
+    f[9] = float(ep - eh);
+    f[10] = float(E0 - cd.hd[c]);
+    f[11] = float(log(1.0 + double(ud.ninner)) / 10.0);
+    f[12] = hole >= 0 ? float(hole + 1) / float(n) : 0.f;
+    f[13] = ptcl >= 0 ? float(ptcl + 1) / float(n) : 0.f;
+    // outer-pair integral bound and a crude log-score estimate
+    const double lnc = log(fabs(cd.C[c]) + 1e-300);
+    if(ud.kind >= 2) {
+      const size_t pr = size_t(ptcl) + size_t(hole) * n;
+      const double bound =
+          cd.pairmax[(ud.kind == 4 ? size_t(n) * n : 0) + pr];
+      const double lb = log(bound + 1e-300);
+      f[14] = float(lb / 10.0);
+      f[15] = float((lnc + lb - log(fabs(E0 - cd.hd[c] - (ep - eh)) + 1e-3)) /
+                    10.0);
+    } else {
+      f[14] = 0.f;
+      f[15] = float((lnc - log(fabs(E0 - cd.hd[c]) + 1e-3)) / 10.0);
+    }
 #pragma unroll
-    for(int k = 0; k < 4; ++k)
-      w[k] = bf16_bits(f[8 * q + 2 * k]) | (bf16_bits(f[8 * q + 2 * k + 1]) << 16);
-    put(base + q, make_uint4(w[0], w[1], w[2], w[3]));
+    for(int q = 0; q < 2; ++q) {
+      uint32_t w[4];
+#pragma unroll
+      for(int k = 0; k < 4; ++k)
+        w[k] = bf16_bits(f[8 * q + 2 * k]) | (bf16_bits(f[8 * q + 2 * k + 1]) << 16);
+      put(base + q, make_uint4(w[0], w[1], w[2], w[3]));
+    }
   }
   // eps-weighted occupations
-  for(int q = 0; q < UNIT_EPS_ORBS / 8; ++q) {
+  constexpr int NQ = UNIT_EPS_ORBS / 8;
+  const int q0 = part < 0 || part == 2 ? 0 : part == 3 ? NQ / 2 : NQ;
+  const int q1 = part == 2 ? NQ / 2 : NQ;
+  for(int q = q0; q < q1; ++q) {
     uint32_t w[4];
 #pragma unroll
     for(int k = 0; k < 4; ++k) {
@@ -1073,13 +1082,15 @@ struct UnitRows {
   CoreData cd;
   double E0;
   __device__ void fill(int64_t row0, int nvalid, uint8_t* xs, int tid) const {
-    uint8_t* base = xs + tid * 16;
-    if(tid < nvalid) {
-      unit_features<NBITS>(cd, E0, row0 + tid, [&](int k, uint4 v) {
+    const int r = tid % MLP_TM, part = tid / MLP_TM;  // 4 threads per row
+    static_assert(MLP_GROUPS == 4, "unit_features has four parts");
+    uint8_t* base = xs + r * 16;
+    if(r < nvalid) {
+      unit_features<NBITS>(cd, E0, row0 + r, part, [&](int k, uint4 v) {
         *reinterpret_cast<uint4*>(base + size_t(k) * (MLP_TM * 16)) = v;
       });
     } else {
-      for(int k = 0; k < unit_din<NBITS>() / 8; ++k)
+      for(int k = part; k < unit_din<NBITS>() / 8; k += MLP_GROUPS)
         *reinterpret_cast<uint4*>(base + size_t(k) * (MLP_TM * 16)) =
             make_uint4(0, 0, 0, 0);
     }
@@ -1097,7 +1108,8 @@ __global__ void unit_rows_k(CoreData cd, double E0, const int64_t* units,
       i += size_t(gridDim.x) * blockDim.x) {
     const int64_t u = units ? units[i] : first + int64_t(i);
     uint4* row = reinterpret_cast<uint4*>(X + i * DIN);
-    unit_features<NBITS>(cd, E0, u, [&](int k, uint4 v) { row[k] = v; });
+    unit_features<NBITS>(cd, E0, u, -1,
+                         [&](int k, uint4 v) { row[k] = v; });
     if(t) t[i] = (logf(fmaxf(umax[u], 1e-12f)) + 20.f) / 5.f;
   }
 }
@@ -1619,7 +1631,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
     MB_CUDA(cudaEventCreate(&ev[0]));
     MB_CUDA(cudaEventCreate(&ev[1]));
     MB_CUDA(cudaEventRecord(ev[0], s));
-    kern<<<unsigned(std::min<int64_t>(tiles, sms)), MLP_TM, smem, s>>>(
+    kern<<<unsigned(std::min<int64_t>(tiles, sms)), MLP_THREADS, smem, s>>>(
         mlp_weights(net), UnitRows<NBITS>{cd, E0}, U, pred, MlpTaps{},
         net->err, wait_limit_ns()), note_launch();
     MB_CUDA(cudaGetLastError());

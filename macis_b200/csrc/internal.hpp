@@ -122,6 +122,8 @@ struct macis_b200_mlp {
   // training scratch for batches of B rows
   int64_t B = 0;
   std::vector<void*> scratch;
+  cudaStream_t side = nullptr;  // the second branch of a training step
+  cudaEvent_t fork = nullptr, join = nullptr;
   uint16_t *xb = nullptr, *xbt = nullptr, *h1t = nullptr, *dz2t_b = nullptr,
            *dz2_b = nullptr, *dz1t_b = nullptr;
   float *tb = nullptr, *yb = nullptr, *z1t = nullptr, *z2t = nullptr,

@@ -4,7 +4,7 @@
 //   gather minibatch -> forward (mlp_fwd_k, taps) -> loss / dZ2 -> bias and
 //   head gradients (row sums) -> dW2 = dZ2^T H1 (tcgen05) -> dZ1 = (dZ2 W2)
 //   * GELU'(Z1) (tcgen05, fused epilogue) -> dW1 = dZ1^T X (tcgen05) -> Adam
-//   -> repack BF16 operands.
+//   with the new BF16 operand copies.
 //
 // The network has no counterpart in MACIS; the ASCI search uses it to rank
 // its work units before exact scoring.
@@ -23,12 +23,22 @@ namespace mb {
 
 namespace {
 
-constexpr int GT_M = 128;  // backward GEMM tile
-constexpr int GT_N = 64;
-constexpr int GT_K = 64;
+constexpr int GT_M = 128;  // backward GEMM tile rows
+constexpr int GT_K = 64;   // K columns per chunk
+// chunks in flight: the GEMMs of a training batch (256 x 256 x 1024) are
+// bound by the latency of their loads
+constexpr int GT_S = 4;
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   tc::smem_addr(dst)), "l"(src) : "memory");
+}
 
 // C = A B^T for row-major BF16 A [M][K] (lda) and B [N][K] (ldb); M % 128,
-// N % 64, K % 64 == 0. MODE 0 stores C (FP32 row-major, ldc). MODE 1 is the
+// N % GN, K % 64 == 0. A CTA takes a 128 x GN tile: narrow tiles put a batch's
+// GEMMs on 24 to 64 CTAs instead of 6 to 32 and leave the sums of each element
+// in K order. Chunks of K arrive by asynchronous copies, GT_S - 1 ahead.
+// MODE 0 stores C (FP32 row-major, ldc). MODE 1 is the
 // dZ1 epilogue: v = C[m][n] * GELU'(z1t[n][m]); writes v to of32t[n][m] and
 // BF16(v) to obf16t[n][m] (both leading dimension ldo), 0 for m >= mvalid.
 struct GemmOut {
@@ -41,67 +51,65 @@ struct GemmOut {
   int64_t mvalid = 0;
 };
 
-template <int MODE>
+template <int MODE, int GN>
 __global__ void __launch_bounds__(128)
     gemm_tc_k(const __nv_bfloat16* A, int64_t lda, const __nv_bfloat16* B,
               int64_t ldb, int64_t K, GemmOut o, int* err, uint64_t limit_ns) {
   constexpr int ABYTES = GT_M * GT_K * 2;  // 16 KB
-  constexpr int BBYTES = GT_N * GT_K * 2;  // 8 KB
-  constexpr uint32_t A_LBO = GT_M * 16, B_LBO = GT_N * 16;
-  constexpr uint32_t IDESC = tc::idesc_bf16(GT_M, GT_N);
+  constexpr int BBYTES = GN * GT_K * 2;
+  constexpr int TCOLS = GN < 32 ? 32 : GN;
+  constexpr uint32_t A_LBO = GT_M * 16, B_LBO = GN * 16;
+  constexpr uint32_t IDESC = tc::idesc_bf16(GT_M, GN);
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ uint64_t bar[2];
+  __shared__ uint64_t bar[GT_S];
   __shared__ uint64_t drain;  // used once, by the timeout path only
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t m0 = int64_t(blockIdx.y) * GT_M, n0 = int64_t(blockIdx.x) * GT_N;
+  const int64_t m0 = int64_t(blockIdx.y) * GT_M, n0 = int64_t(blockIdx.x) * GN;
   if(tid == 0) {
-    tc::mbar_init(&bar[0], 1);
-    tc::mbar_init(&bar[1], 1);
+    for(int i = 0; i < GT_S; ++i) tc::mbar_init(&bar[i], 1);
     tc::mbar_init(&drain, 1);
     tc::mbar_init_fence();
   }
-  if(warp == 0) tc::tmem_alloc(&tslot, GT_N);
+  if(warp == 0) tc::tmem_alloc(&tslot, TCOLS);
+  // a warp copies 4 rows x 128 contiguous bytes at a time
+  const int slab = tid & 7, row8 = tid >> 3;
+  auto load = [&](int64_t c) {
+    uint8_t* as = smem + int(c % GT_S) * (ABYTES + BBYTES);
+    uint8_t* bs = as + ABYTES;
+    const int64_t k0 = c * GT_K + slab * 8;
+#pragma unroll
+    for(int r = 0; r < GT_M; r += 16)
+      cp_async16(as + slab * A_LBO + (r + row8) * 16,
+                 A + (m0 + r + row8) * lda + k0);
+#pragma unroll
+    for(int r = 0; r < GN; r += 16)
+      cp_async16(bs + slab * B_LBO + (r + row8) * 16,
+                 B + (n0 + r + row8) * ldb + k0);
+  };
+  const int64_t nk = K / GT_K;
+  for(int64_t c = 0; c < GT_S - 1; ++c) {
+    if(c < nk) load(c);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tslot;
-  const int64_t nk = K / GT_K;
   bool fail = false, abort = false;
   for(int64_t c = 0; c < nk; ++c) {
-    const int s = int(c & 1);
-    uint8_t* as = smem + s * (ABYTES + BBYTES);
-    uint8_t* bs = as + ABYTES;
-    // the MMAs of chunk c-2 read this stage
-    if(c >= 2 &&
-       !tc::mbar_wait(&bar[s], uint32_t(((c - 2) >> 1) & 1), limit_ns))
-      fail = true;
+    const int s = int(c % GT_S);
+    // chunk c has arrived in this thread's copies
+    asm volatile("cp.async.wait_group %0;" ::"n"(GT_S - 2) : "memory");
+    tc::fence_async_smem();
     if(__syncthreads_or(fail)) {
       abort = true;
       break;
     }
-    const int64_t k0 = c * GT_K;
-    {
-      const uint4* src =
-          reinterpret_cast<const uint4*>(A + (m0 + tid) * lda + k0);
-#pragma unroll
-      for(int i = 0; i < GT_K / 8; ++i)
-        *reinterpret_cast<uint4*>(as + i * A_LBO + tid * 16) = __ldg(src + i);
-      const int br = tid & (GT_N - 1), half = tid / GT_N;
-      const uint4* bsrc =
-          reinterpret_cast<const uint4*>(B + (n0 + br) * ldb + k0);
-#pragma unroll
-      for(int i = 0; i < GT_K / 16; ++i) {
-        const int slab = half * (GT_K / 16) + i;
-        *reinterpret_cast<uint4*>(bs + slab * B_LBO + br * 16) =
-            __ldg(bsrc + slab);
-      }
-    }
-    tc::fence_async_smem();
-    __syncthreads();
     if(tid == 0) {
       tc::fence_after_sync();
-      const uint32_t aa = tc::smem_addr(as), ba = tc::smem_addr(bs);
+      const uint32_t aa = tc::smem_addr(smem + s * (ABYTES + BBYTES));
+      const uint32_t ba = aa + ABYTES;
 #pragma unroll
       for(int ks = 0; ks < GT_K / 16; ++ks)
         tc::mma_bf16(tmem, tc::sdesc(aa + 2 * ks * A_LBO, A_LBO, 128),
@@ -109,11 +117,23 @@ __global__ void __launch_bounds__(128)
                      (c | ks) ? 1u : 0u);
       tc::mma_commit(&bar[s]);
     }
+    __syncwarp();
+    // refill the stage of chunk c - 1 once its MMAs have read it
+    const int64_t cn = c + GT_S - 1;
+    if(cn < nk) {
+      if(c >= 1 &&
+         !tc::mbar_wait(&bar[(c - 1) % GT_S],
+                        uint32_t(((c - 1) / GT_S) & 1), limit_ns))
+        fail = true;
+      if(!fail) load(cn);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   // the last commit covers every MMA of this tile
   if(!abort && nk > 0) {
     const int64_t c = nk - 1;
-    if(!tc::mbar_wait(&bar[c & 1], uint32_t((c >> 1) & 1), limit_ns))
+    if(!tc::mbar_wait(&bar[c % GT_S], uint32_t((c / GT_S) & 1), limit_ns))
       fail = true;
   }
   if(__syncthreads_or(fail)) abort = true;
@@ -122,7 +142,7 @@ __global__ void __launch_bounds__(128)
     const int r = warp * 32 + lane;
     const int64_t m = m0 + r;
     const uint32_t trow = tmem + (uint32_t(warp * 32) << 16);
-    for(int c0 = 0; c0 < GT_N; c0 += 16) {
+    for(int c0 = 0; c0 < GN; c0 += 16) {
       uint32_t v[16];
       tc::tmem_ld16(trow + uint32_t(c0), v);
       tc::tmem_wait_ld();
@@ -161,21 +181,20 @@ __global__ void __launch_bounds__(128)
   __syncthreads();
   if(warp == 0) {
     tc::fence_after_sync();
-    tc::tmem_dealloc(tmem, GT_N);
+    tc::tmem_dealloc(tmem, TCOLS);
   }
 }
 
 // Loss L = sum_m (y_m - t_m)^2 / (2 nvalid) and its first backward step.
-// Thread (j, m), m fastest.
+// Block row j, threads over m.
 __global__ void mlp_loss_k(const float* y, const float* t, int64_t nvalid,
                            int64_t B, const float* z2t, const float* w3,
                            float* dy, float* dz2t, __nv_bfloat16* dz2t_b,
                            __nv_bfloat16* dz2_b, float* p3t, double* loss) {
-  const int64_t total = int64_t(MLP_H) * B;
-  for(int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-      idx += int64_t(gridDim.x) * blockDim.x) {
-    const int j = int(idx / B);
-    const int64_t m = idx % B;
+  const int j = blockIdx.y;
+  for(int64_t m = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; m < B;
+      m += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t idx = int64_t(j) * B + m;
     float g = 0.f, p = 0.f, d = 0.f;
     if(m < nvalid) {
       const float e = y[m] - t[m];
@@ -232,26 +251,64 @@ __global__ void rowsum_k(const float* in, int64_t ld, int64_t n, float* out) {
   if(threadIdx.x == 0) out[blockIdx.x] = sh[0];
 }
 
-// Minibatch rows idx[0..nvalid) of X [S][din]: xb [B][din], xbt [din][B].
-__global__ void mlp_gather_k(const uint16_t* X, const float* t,
-                             const int64_t* idx, int64_t nvalid, int64_t B,
-                             int din, uint16_t* xb, uint16_t* xbt, float* tb) {
-  const int64_t total = int64_t(din) * B;
-  for(int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < total;
-      q += int64_t(gridDim.x) * blockDim.x) {
-    const int k = int(q / B);
-    const int64_t m = q % B;
-    uint16_t v = 0;
-    if(m < nvalid) v = X[idx[m] * din + k];
-    xbt[q] = v;
-    xb[m * din + k] = v;
-    if(k == 0) tb[m] = m < nvalid ? t[idx[m]] : 0.f;
+// Minibatch rows idx[0..nvalid) of X [S][din]: xb [B][din], xbt [din][B]. A
+// block takes 32 rows x 64 columns through shared memory, so that both copies
+// and the rows themselves are read and written in runs.
+constexpr int GATHER_ROWS = 32, GATHER_COLS = 64;
+__global__ void __launch_bounds__(256)
+    mlp_gather_k(const uint16_t* X, const float* t, const int64_t* idx,
+                 int64_t nvalid, int64_t B, int din, uint16_t* xb,
+                 uint16_t* xbt, float* tb) {
+  constexpr int W = GATHER_COLS / 2;  // pairs of columns
+  __shared__ uint32_t grow[GATHER_ROWS][W + 1];
+  const int64_t m0 = int64_t(blockIdx.x) * GATHER_ROWS;
+  const int c0 = blockIdx.y * W;
+  for(int q = threadIdx.x; q < GATHER_ROWS * W; q += blockDim.x) {
+    const int r = q / W, c = q % W;
+    const int64_t m = m0 + r;
+    uint32_t v = 0;
+    if(m < nvalid) v = reinterpret_cast<const uint32_t*>(X + idx[m] * din)[c0 + c];
+    reinterpret_cast<uint32_t*>(xb + m * din)[c0 + c] = v;
+    grow[r][c] = v;
+  }
+  if(blockIdx.y == 0 && threadIdx.x < GATHER_ROWS) {
+    const int64_t m = m0 + threadIdx.x;
+    tb[m] = m < nvalid ? t[idx[m]] : 0.f;
+  }
+  __syncthreads();
+  const int r = threadIdx.x & (GATHER_ROWS - 1);
+  for(int c = threadIdx.x / GATHER_ROWS; c < W; c += blockDim.x / GATHER_ROWS) {
+    const uint32_t v = grow[r][c];
+    xbt[int64_t(2 * (c0 + c)) * B + m0 + r] = uint16_t(v & 0xFFFF);
+    xbt[int64_t(2 * (c0 + c) + 1) * B + m0 + r] = uint16_t(v >> 16);
   }
 }
 
+// BF16 operand copies of W1 [256][din] and W2 [256][256], which lead the
+// parameters (W2 at off_w2): the forward's slab layout and the row-major
+// transpose W2^T used by the backward.
+struct PackedWeights {
+  int din, off_w2;
+  uint16_t *w1t, *w2t, *w2T;
+};
+__device__ __forceinline__ void pack_weight(const PackedWeights& w, int i,
+                                            float p) {
+  const uint16_t b = __bfloat16_as_ushort(__float2bfloat16_rn(p));
+  if(i < w.din * MLP_H) {
+    const int n = i / w.din, k = i % w.din;
+    w.w1t[((k / 8) * MLP_H + n) * 8 + (k & 7)] = b;
+  } else if(i >= w.off_w2 && i < w.off_w2 + MLP_H * MLP_H) {
+    const int j = i - w.off_w2;
+    const int n = j / MLP_H, k = j % MLP_H;
+    w.w2t[((k / 8) * MLP_H + n) * 8 + (k & 7)] = b;
+    w.w2T[k * MLP_H + n] = b;
+  }
+}
+
+// One Adam step; the new weights go to their operand copies as well.
 __global__ void adam_k(float* P, const float* G, float* Mo, float* Ve,
                        int64_t n, float lr, float b1, float b2, float eps,
-                       float bc1, float bc2) {
+                       float bc1, float bc2, PackedWeights w) {
   for(int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
       i += int64_t(gridDim.x) * blockDim.x) {
     const float g = G[i];
@@ -260,28 +317,14 @@ __global__ void adam_k(float* P, const float* G, float* Mo, float* Ve,
     Mo[i] = m;
     Ve[i] = v;
     P[i] -= lr * (m / bc1) / (sqrtf(v / bc2) + eps);
+    pack_weight(w, int(i), P[i]);
   }
 }
 
-// BF16 operand copies of W1 [256][din] and W2 [256][256]: the forward's
-// slab layout and the row-major transpose W2^T used by the backward.
-__global__ void mlp_pack_k(const float* W1, const float* W2, int din,
-                           uint16_t* w1t, uint16_t* w2t, uint16_t* w2T) {
-  const int64_t n1 = int64_t(MLP_H) * din, n2 = int64_t(MLP_H) * MLP_H;
-  for(int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n1 + n2;
-      i += int64_t(gridDim.x) * blockDim.x) {
-    if(i < n1) {
-      const int n = int(i / din), k = int(i % din);
-      w1t[(int64_t(k / 8) * MLP_H + n) * 8 + (k & 7)] =
-          __bfloat16_as_ushort(__float2bfloat16_rn(W1[i]));
-    } else {
-      const int64_t j = i - n1;
-      const int n = int(j / MLP_H), k = int(j % MLP_H);
-      const uint16_t b = __bfloat16_as_ushort(__float2bfloat16_rn(W2[j]));
-      w2t[(int64_t(k / 8) * MLP_H + n) * 8 + (k & 7)] = b;
-      w2T[int64_t(k) * MLP_H + n] = b;
-    }
-  }
+__global__ void mlp_pack_k(const float* P, int64_t n, PackedWeights w) {
+  for(int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+      i += int64_t(gridDim.x) * blockDim.x)
+    pack_weight(w, int(i), P[i]);
 }
 
 uint64_t splitmix(uint64_t& s) {
@@ -312,10 +355,13 @@ void check_err(macis_b200_mlp* m) {
              "screening network kernel timed out waiting on a barrier");
 }
 
+PackedWeights packed(const macis_b200_mlp* m) {
+  return PackedWeights{m->din, int(m->off_w2), m->w1t, m->w2t, m->w2T};
+}
+
 void repack(macis_b200_mlp* m, cudaStream_t s) {
-  mlp_pack_k<<<grid_for(size_t(MLP_H) * (m->din + MLP_H), 256, 4 * num_sms()),
-               256, 0, s>>>(m->P + m->off_w1, m->P + m->off_w2, m->din,
-                            m->w1t, m->w2t, m->w2T), note_launch();
+  mlp_pack_k<<<grid_for(m->nparams, 256, 4 * num_sms()), 256, 0, s>>>(
+      m->P, int64_t(m->nparams), packed(m)), note_launch();
   MB_CUDA(cudaGetLastError());
 }
 
@@ -370,23 +416,23 @@ void launch_fwd(const macis_b200_mlp* m, const Src& src, int64_t nrows,
                                int(smem)));
   const int64_t tiles = (nrows + MLP_TM - 1) / MLP_TM;
   const unsigned grid = unsigned(std::min<int64_t>(tiles, num_sms()));
-  kern<<<grid, MLP_TM, smem, s>>>(weights_of(m), src, nrows, y, taps, m->err,
+  kern<<<grid, MLP_THREADS, smem, s>>>(weights_of(m), src, nrows, y, taps, m->err,
                                   wait_limit_ns()),
       note_launch();
   MB_CUDA(cudaGetLastError());
 }
 
-template <int MODE>
+template <int MODE, int GN>
 void gemm(const macis_b200_mlp* m, const uint16_t* A, int64_t lda,
           const uint16_t* B, int64_t ldb, int64_t M, int64_t N, int64_t K,
           const GemmOut& o, cudaStream_t s) {
-  MB_REQUIRE(M % GT_M == 0 && N % GT_N == 0 && K % GT_K == 0,
+  MB_REQUIRE(M % GT_M == 0 && N % GN == 0 && K % GT_K == 0,
              MACIS_B200_EINVAL, "network GEMM shape not tile aligned");
-  const int smem = 2 * (GT_M + GT_N) * GT_K * 2;
-  auto kern = gemm_tc_k<MODE>;
+  const int smem = GT_S * (GT_M + GN) * GT_K * 2;
+  auto kern = gemm_tc_k<MODE, GN>;
   MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                smem));
-  dim3 grid(unsigned(N / GT_N), unsigned(M / GT_M));
+  dim3 grid(unsigned(N / GN), unsigned(M / GT_M));
   kern<<<grid, 128, smem, s>>>(reinterpret_cast<const __nv_bfloat16*>(A), lda,
                                reinterpret_cast<const __nv_bfloat16*>(B), ldb,
                                K, o, m->err, wait_limit_ns()), note_launch();
@@ -398,8 +444,8 @@ void fwd_bwd(macis_b200_mlp* m, const uint16_t* X, const float* t,
              const int64_t* idx, int64_t nvalid, int64_t B, double* loss_acc,
              cudaStream_t s) {
   const int din = m->din;
-  const int sms = num_sms();
-  mlp_gather_k<<<grid_for(size_t(din) * B, 256, 8 * sms), 256, 0, s>>>(
+  mlp_gather_k<<<dim3(unsigned(B / GATHER_ROWS), unsigned(din / GATHER_COLS)),
+                 256, 0, s>>>(
       X, t, idx, nvalid, B, din, m->xb, m->xbt, m->tb), note_launch();
   MlpTaps taps;
   taps.z1t = m->z1t;
@@ -409,20 +455,25 @@ void fwd_bwd(macis_b200_mlp* m, const uint16_t* X, const float* t,
   launch_fwd<DenseRows, true>(
       m, DenseRows{reinterpret_cast<const uint4*>(m->xb), din}, nvalid, m->yb,
       taps, s);
-  mlp_loss_k<<<grid_for(size_t(MLP_H) * B, 256, 8 * sms), 256, 0, s>>>(
+  mlp_loss_k<<<dim3(grid_for(size_t(B), 256, 64), MLP_H), 256, 0, s>>>(
       m->yb, m->tb, nvalid, B, m->z2t, m->P + m->off_w3, m->dy, m->dz2t,
       reinterpret_cast<__nv_bfloat16*>(m->dz2t_b),
       reinterpret_cast<__nv_bfloat16*>(m->dz2_b), m->p3t, loss_acc), note_launch();
   float* G = m->G;
+  // dW2 and the sums of its inputs run beside dZ1 and dW1: each of these
+  // GEMMs keeps 24 to 64 SMs busy
+  MB_CUDA(cudaEventRecord(m->fork, s));
+  MB_CUDA(cudaStreamWaitEvent(m->side, m->fork, 0));
   RowSums rs{{m->dz2t, m->p3t, m->dy},
              {G + m->off_b2, G + m->off_w3, G + m->off_b3},
              {MLP_H, MLP_H, 1}};
-  rowsums_k<<<2 * MLP_H + 1, 256, 0, s>>>(rs, B, B), note_launch();
+  rowsums_k<<<2 * MLP_H + 1, 256, 0, m->side>>>(rs, B, B), note_launch();
   // dW2[o][i] = sum_m dZ2[m][o] H1[m][i]
   GemmOut o2;
   o2.c = G + m->off_w2;
   o2.ldc = MLP_H;
-  gemm<0>(m, m->dz2t_b, B, m->h1t, B, MLP_H, MLP_H, B, o2, s);
+  gemm<0, 16>(m, m->dz2t_b, B, m->h1t, B, MLP_H, MLP_H, B, o2, m->side);
+  MB_CUDA(cudaEventRecord(m->join, m->side));
   // dZ1[m][i] = (sum_o dZ2[m][o] W2[o][i]) GELU'(Z1[m][i]), stored transposed
   GemmOut o1;
   o1.z1t = m->z1t;
@@ -430,13 +481,14 @@ void fwd_bwd(macis_b200_mlp* m, const uint16_t* X, const float* t,
   o1.obf16t = reinterpret_cast<__nv_bfloat16*>(m->dz1t_b);
   o1.ldo = B;
   o1.mvalid = nvalid;
-  gemm<1>(m, m->dz2_b, MLP_H, m->w2T, MLP_H, B, MLP_H, MLP_H, o1, s);
+  gemm<1, 32>(m, m->dz2_b, MLP_H, m->w2T, MLP_H, B, MLP_H, MLP_H, o1, s);
   rowsum_k<<<MLP_H, 256, 0, s>>>(m->dz1t, B, B, G + m->off_b1), note_launch();
   // dW1[o][k] = sum_m dZ1[m][o] X[m][k]
   GemmOut o3;
   o3.c = G + m->off_w1;
   o3.ldc = din;
-  gemm<0>(m, m->dz1t_b, B, m->xbt, B, MLP_H, din, B, o3, s);
+  gemm<0, 16>(m, m->dz1t_b, B, m->xbt, B, MLP_H, din, B, o3, s);
+  MB_CUDA(cudaStreamWaitEvent(s, m->join, 0));
 }
 
 }  // namespace
@@ -450,6 +502,9 @@ macis_b200_mlp* mlp_create(int din, uint64_t seed) {
     m->din = din;
     MB_CUDA(cudaGetDevice(&m->device));
     MB_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
+    MB_CUDA(cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking));
+    MB_CUDA(cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming));
+    MB_CUDA(cudaEventCreateWithFlags(&m->join, cudaEventDisableTiming));
     m->off_w1 = 0;
     m->off_b1 = m->off_w1 + size_t(MLP_H) * din;
     m->off_w2 = m->off_b1 + MLP_H;
@@ -486,6 +541,7 @@ macis_b200_mlp* mlp_create(int din, uint64_t seed) {
 
 void mlp_destroy(macis_b200_mlp* m) {
   if(!m) return;
+  if(m->side) cudaStreamSynchronize(m->side);
   if(m->stream) cudaStreamSynchronize(m->stream);
   for(void* p : {static_cast<void*>(m->P), static_cast<void*>(m->G),
                  static_cast<void*>(m->Mo), static_cast<void*>(m->Ve),
@@ -494,6 +550,9 @@ void mlp_destroy(macis_b200_mlp* m) {
                  static_cast<void*>(m->xs), static_cast<void*>(m->ts)})
     if(p) cudaFree(p);
   for(void* p : m->scratch) cudaFree(p);
+  if(m->fork) cudaEventDestroy(m->fork);
+  if(m->join) cudaEventDestroy(m->join);
+  if(m->side) cudaStreamDestroy(m->side);
   if(m->stream) cudaStreamDestroy(m->stream);
   delete m;
 }
@@ -578,8 +637,7 @@ double mlp_train_device(macis_b200_mlp* m, const uint16_t* X, const float* t,
       const float bc2 = float(1.0 - std::pow(double(b2), double(m->step)));
       adam_k<<<grid_for(m->nparams, 256, 4 * num_sms()), 256, 0, s>>>(
           m->P, m->G, m->Mo, m->Ve, int64_t(m->nparams), float(lr), b1, b2, eps,
-          bc1, bc2), note_launch();
-      repack(m, s);
+          bc1, bc2, packed(m)), note_launch();
     }
     MB_CUDA(cudaMemcpyAsync(&last, dl, 8, cudaMemcpyDeviceToHost, s));
     MB_CUDA(cudaStreamSynchronize(s));

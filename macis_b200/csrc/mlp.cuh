@@ -9,11 +9,12 @@
 //   2. one thread issues the layer-1 MMAs (M = 128, N = 256, K = 16 each)
 //      while the weights stream through a 3-stage ring of 32 KB chunks
 //      (64 K-columns x 256 rows) loaded with untiled bulk copies;
-//   3. the 128 threads read the accumulator rows from TMEM, add the bias,
-//      apply GELU and write H1 back into the input tile's shared memory in
-//      the MMA operand layout;
+//   3. the threads read the accumulator from TMEM (a warp its 32 rows, 64 of
+//      the columns), add the bias, apply GELU and write H1 back into the
+//      input tile's shared memory in the MMA operand layout;
 //   4. layer 2 runs the same way on H1 with W2, and the epilogue applies bias
-//      + GELU and the FP32 dot product with the head.
+//      + GELU and the FP32 dot product with the head (in column order: the
+//      column groups of a row pass the partial sum on).
 // The weights are kept in HBM already in the operand layout (tc.cuh), so a
 // chunk is one contiguous 32 KB copy.
 #pragma once
@@ -25,6 +26,12 @@ namespace mb {
 
 constexpr int MLP_H = 256;                     // hidden width
 constexpr int MLP_TM = 128;                    // rows per tile (MMA M)
+// Threads of the forward: four warps per 32 accumulator rows. The epilogues
+// (256 erf evaluations per row and layer) and the row source are bound by
+// latency with one warp per 32 rows, so one per scheduler: 8.2 ms against 6.6
+// for the 6.5e6 rows of a search's prediction.
+constexpr int MLP_THREADS = 512;
+constexpr int MLP_GROUPS = MLP_THREADS / MLP_TM;  // threads per tile row
 constexpr int MLP_KC = 64;                     // K columns per weight chunk
 constexpr int MLP_WCHUNK = MLP_H * MLP_KC * 2;  // 32 KB
 constexpr int MLP_STAGES = 3;
@@ -63,7 +70,7 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
 inline size_t mlp_fwd_smem_bytes(int din) {
   const int kx = din > MLP_H ? din : MLP_H;
   return size_t(kx) * MLP_TM * 2 + size_t(MLP_STAGES) * MLP_WCHUNK +
-         (2 * MLP_STAGES + 2) * 8 + 3 * MLP_H * 4 + 16;
+         (2 * MLP_STAGES + 2) * 8 + 3 * MLP_H * 4 + MLP_TM * 4 + 16;
 }
 
 // Dense row source: X row-major [nrows][din] BF16.
@@ -72,7 +79,7 @@ struct DenseRows {
   int din;
   __device__ void fill(int64_t row0, int nvalid, uint8_t* xs, int tid) const {
     const int nkc = din / 8;
-    for(int q = tid; q < MLP_TM * nkc; q += MLP_TM) {
+    for(int q = tid; q < MLP_TM * nkc; q += MLP_THREADS) {
       const int kc = q / MLP_TM, r = q % MLP_TM;
       uint4 v = make_uint4(0, 0, 0, 0);
       if(r < nvalid) v = __ldg(x + (row0 + r) * nkc + kc);
@@ -86,7 +93,7 @@ struct DenseRows {
 // (device) is set, the CTA waits (at most 100 ms each) for its bulk copies
 // and MMAs still in flight, frees its TMEM and returns.
 template <class Src, bool TRAIN>
-__global__ void __launch_bounds__(MLP_TM, 1)
+__global__ void __launch_bounds__(MLP_THREADS, 1)
     mlp_fwd_k(MlpWeights W, Src src, int64_t nrows, float* y, MlpTaps tap,
               int* err, uint64_t limit_ns) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -105,12 +112,13 @@ __global__ void __launch_bounds__(MLP_TM, 1)
   float* sb1 = reinterpret_cast<float*>(drain + 1);
   float* sb2 = sb1 + MLP_H;
   float* sw3 = sb2 + MLP_H;
+  float* sacc = sw3 + MLP_H;  // partial dot product of each row
 
   const int64_t ntiles = (nrows + MLP_TM - 1) / MLP_TM;
   if(int64_t(blockIdx.x) >= ntiles) return;  // uniform; before any TMEM use
   const int64_t my_tiles = (ntiles - 1 - blockIdx.x) / gridDim.x + 1;
 
-  for(int i = tid; i < MLP_H; i += MLP_TM) {
+  for(int i = tid; i < MLP_H; i += MLP_THREADS) {
     sb1[i] = W.b1[i];
     sb2[i] = W.b2[i];
     sw3[i] = W.w3[i];
@@ -151,8 +159,12 @@ __global__ void __launch_bounds__(MLP_TM, 1)
   uint32_t acc_n = 0;                      // accumulator commits so far
   bool fail = false;                       // this thread saw a timeout
   bool abort = false;                      // some thread did (uniform)
-  const int r = warp * 32 + lane;          // tile row of this thread
-  const uint32_t trow = tmem + (uint32_t(warp * 32) << 16);
+  // tile row of this thread (a warp reads the TMEM lanes of its rank mod 4)
+  // and its column group
+  const int r = (warp & 3) * 32 + lane, grp = warp >> 2;
+  constexpr int GC = MLP_H / MLP_GROUPS;
+  const int gc0 = grp * GC;
+  const uint32_t trow = tmem + (uint32_t((warp & 3) * 32) << 16);
 
   for(int64_t lt = 0; lt < my_tiles; ++lt) {
     const int64_t row0 = (int64_t(blockIdx.x) + lt * gridDim.x) * MLP_TM;
@@ -210,7 +222,7 @@ __global__ void __launch_bounds__(MLP_TM, 1)
       tc::fence_after_sync();
       const int64_t row = row0 + r;
       if(layer == 0) {
-        for(int c0 = 0; c0 < MLP_H; c0 += 16) {
+        for(int c0 = gc0; c0 < gc0 + GC; c0 += 16) {
           uint32_t v[16];
           tc::tmem_ld16(trow + uint32_t(c0), v);
           tc::tmem_wait_ld();
@@ -238,19 +250,30 @@ __global__ void __launch_bounds__(MLP_TM, 1)
         tc::fence_before_sync();
         tc::fence_async_smem();
       } else {
-        float acc = 0.f;
-        for(int c0 = 0; c0 < MLP_H; c0 += 16) {
+        float h2[GC];
+#pragma unroll
+        for(int c = 0; c < GC; c += 16) {
           uint32_t v[16];
-          tc::tmem_ld16(trow + uint32_t(c0), v);
+          tc::tmem_ld16(trow + uint32_t(gc0 + c), v);
           tc::tmem_wait_ld();
 #pragma unroll
           for(int q = 0; q < 16; ++q) {
-            const float z = __uint_as_float(v[q]) + sb2[c0 + q];
-            acc = fmaf(gelu_f(z), sw3[c0 + q], acc);
-            if(TRAIN && r < nvalid) tap.z2t[size_t(c0 + q) * tap.ld + row] = z;
+            const float z = __uint_as_float(v[q]) + sb2[gc0 + c + q];
+            h2[c + q] = gelu_f(z);
+            if(TRAIN && r < nvalid) tap.z2t[size_t(gc0 + c + q) * tap.ld + row] = z;
           }
         }
-        if(r < nvalid) y[row] = acc + b3;
+        // the dot product in column order: one group after another
+        for(int g = 0; g < MLP_GROUPS; ++g) {
+          if(grp == g) {
+            float acc = g ? sacc[r] : 0.f;
+#pragma unroll
+            for(int c = 0; c < GC; ++c) acc = fmaf(h2[c], sw3[gc0 + c], acc);
+            sacc[r] = acc;
+            if(g == MLP_GROUPS - 1 && r < nvalid) y[row] = acc + b3;
+          }
+          __syncthreads();
+        }
         tc::fence_before_sync();
       }
       if(__syncthreads_or(fail)) {
