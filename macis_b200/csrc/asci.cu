@@ -255,14 +255,16 @@ struct AlphaLists {
   int g = -1;                      // group of the range, -1: not used
 };
 
-// String ranks. The candidate determinants of a search are the core dets'
+// String numbers. The candidate determinants of a search are the core dets'
 // alpha strings, their singles and doubles, combined with beta strings of
-// the same kinds. With every distinct candidate string of a spin replaced
-// by its rank in the sorted list of those strings, a candidate determinant
-// is one 64-bit key, (beta rank << bits_a) | alpha rank, that sorts in the
-// same order as the determinant's bitset: the digit passes of the candidate
-// sort cover bits_a + bits_b bits instead of the 2 x norb varying bits of
-// the determinant, over 16-byte instead of 24- or 40-byte records. Per
+// the same kinds. With the distinct candidate strings of a spin numbered, a
+// candidate determinant is one 64-bit key, (beta number << bits_a) | alpha
+// number: 16-byte instead of 24- or 40-byte records. Where the accumulated
+// list itself is the result the numbers are ranks in the sorted list of the
+// strings, so that the key sorts in the same order as the determinant's
+// bitset; a search only groups equal keys, and its numbers come from a hash
+// table (a sort of the 7e7 candidates of the 122 strings of an n = 100 core
+// set cost 18 digit passes a spin). Per
 // distinct core string u of a spin the table R holds the ranks of its
 // M = 1 + N1 + N2 candidates: u itself, its N1 singles (index ii * nv + aa,
 // occupied ii -> virtual aa) and its N2 doubles (row ii * nv + aa, then the
@@ -324,7 +326,63 @@ __global__ void cand_strings_k(const uint64_t* words, const uint8_t* occ,
     }
 #pragma unroll
     for(int j = 0; j < NSW; ++j) cand[e * NSW + j] = st.w[j];
-    idx[e] = uint32_t(e);
+    if(idx) idx[e] = uint32_t(e);
+  }
+}
+// first[e] = the candidate that stands for candidate e's string (itself, or
+// the equal one whose index is in the table): open addressing with linear
+// probing over a power-of-two table of candidate indices, -1 empty. The table
+// has at least 1.5 slots per candidate, so every search ends.
+template <int NSW>
+__global__ void string_insert_k(const uint64_t* cand, size_t n, uint32_t* table,
+                                uint64_t mask, uint32_t* first) {
+  for(size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
+      e += size_t(gridDim.x) * blockDim.x) {
+    Spin<NSW> st;
+    uint64_t h = 0;
+#pragma unroll
+    for(int j = 0; j < NSW; ++j) {
+      st.w[j] = cand[e * NSW + j];
+      h = (h ^ st.w[j]) * 0x9E3779B97F4A7C15ull;
+      h ^= h >> 31;
+    }
+    h *= 0xD6E8FEB86659FD93ull;
+    uint64_t slot = (h ^ (h >> 32)) & mask;
+    uint32_t found = uint32_t(e);
+    for(uint64_t t = 0; t <= mask; ++t) {
+      uint32_t o = __ldcg(table + slot);
+      if(o == 0xFFFFFFFFu) o = atomicCAS(table + slot, 0xFFFFFFFFu, uint32_t(e));
+      if(o == 0xFFFFFFFFu) break;  // the string's first
+      bool eq = true;
+#pragma unroll
+      for(int j = 0; j < NSW; ++j) eq &= cand[size_t(o) * NSW + j] == st.w[j];
+      if(eq) {
+        found = o;
+        break;
+      }
+      slot = (slot + 1) & mask;
+    }
+    first[e] = found;
+  }
+}
+__global__ void string_first_k(const uint32_t* first, size_t n, uint32_t* f) {
+  for(size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
+      e += size_t(gridDim.x) * blockDim.x)
+    f[e] = first[e] == uint32_t(e) ? 1u : 0u;
+}
+// R[e] = the number of candidate e's string (R may hold `first`), and the
+// strings by number.
+template <int NSW>
+__global__ void string_number_k(const uint64_t* cand, const uint32_t* fx,
+                                size_t n, uint32_t* R, uint64_t* L) {
+  for(size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
+      e += size_t(gridDim.x) * blockDim.x) {
+    const uint32_t o = R[e], x = fx[o];
+    R[e] = x;
+    if(o == uint32_t(e)) {
+#pragma unroll
+      for(int j = 0; j < NSW; ++j) L[size_t(x) * NSW + j] = cand[e * NSW + j];
+    }
   }
 }
 // Rank of every candidate (sorted position p holds candidate idx[p]) and
@@ -1450,13 +1508,13 @@ static int64_t spin_candidates(int ne, int nv) {
          int64_t(ne) * (ne - 1) / 2 * (int64_t(nv) * (nv - 1) / 2);
 }
 
-// Rank table of one spin (SpinRanks) and its distinct candidate strings in
-// rank order (*L, NSW words each); returns their number. The candidates are
-// generated with their index, radix-sorted, and equal neighbours share a
-// rank.
+// Number table of one spin (SpinRanks) and its distinct candidate strings by
+// number (*L, NSW words each); returns how many they are. ordered: the
+// numbers are ranks (the candidates are radix-sorted with their index, and
+// equal neighbours share a rank); else they are those of a hash table.
 template <int NBITS>
-static size_t build_spin_ranks(const SpinPlan& sp, Arena& A, cudaStream_t s,
-                               SpinRanks& out, uint64_t** L) {
+static size_t build_spin_ranks(const SpinPlan& sp, bool ordered, Arena& A,
+                               cudaStream_t s, SpinRanks& out, uint64_t** L) {
   constexpr int NSW = DetTraits<NBITS>::NSW;
   const int ne = sp.ne, nv = sp.nv, nrows = ne * nv;
   const int64_t M = spin_candidates(ne, nv);
@@ -1481,33 +1539,45 @@ static size_t build_spin_ranks(const SpinPlan& sp, Arena& A, cudaStream_t s,
   MB_CUDA(cudaMemcpyAsync(dbase, db.data(), db.size() * 8,
                           cudaMemcpyHostToDevice, s));
   uint64_t* cand = A.get<uint64_t>(tot * NSW + NSW);
-  uint32_t* idx = A.get<uint32_t>(tot + 1);
-  cand_strings_k<NSW><<<grid_for(tot, 256, 16 * sms), 256, 0, s>>>(
-      words, occ, vir, sp.nu, ne, nv, M, int64_t(nrows), dbase, nrows, cand,
-      idx), note_launch();
+  uint32_t* idx = ordered ? A.get<uint32_t>(tot + 1) : nullptr;
+  const unsigned g = grid_for(tot, 256, 16 * sms);
+  cand_strings_k<NSW><<<g, 256, 0, s>>>(words, occ, vir, sp.nu, ne, nv, M,
+                                        int64_t(nrows), dbase, nrows, cand,
+                                        idx), note_launch();
   MB_CUDA(cudaGetLastError());
-  {
+  uint32_t* f = A.get<uint32_t>(tot + 1);
+  uint32_t* fx = A.get<uint32_t>(tot + 1);
+  if(ordered) {
     uint64_t* cand2 = A.get<uint64_t>(tot * NSW + NSW);
     uint32_t* idx2 = A.get<uint32_t>(tot + 1);
     radix_sort<NSW, uint32_t>(cand, idx, cand2, idx2, tot, A);
     A.release(cand2);
     A.release(idx2);
+    seg_flags_k<NSW><<<g, 256, 0, s>>>(cand, tot, f), note_launch();
+  } else {
+    size_t slots = 1024;
+    while(slots < tot + tot / 2) slots <<= 1;
+    uint32_t* table = A.get<uint32_t>(slots);
+    MB_CUDA(cudaMemsetAsync(table, 0xFF, slots * 4, s));
+    string_insert_k<NSW><<<g, 256, 0, s>>>(cand, tot, table,
+                                           uint64_t(slots) - 1, R), note_launch();
+    A.release(table);
+    string_first_k<<<g, 256, 0, s>>>(R, tot, f), note_launch();
   }
-  uint32_t* f = A.get<uint32_t>(tot + 1);
-  uint32_t* fx = A.get<uint32_t>(tot + 1);
-  seg_flags_k<NSW><<<grid_for(tot, 256, 16 * sms), 256, 0, s>>>(cand, tot, f),
-      note_launch();
   exclusive_scan<uint32_t, uint32_t>(f, fx, tot, fx + tot, A);
   const size_t NL = to_host(fx + tot, s);
   uint64_t* Ls = A.get<uint64_t>(NL * NSW + NSW);
-  rank_scatter_k<NSW><<<grid_for(tot, 256, 16 * sms), 256, 0, s>>>(
-      cand, idx, f, fx, tot, R, Ls), note_launch();
+  if(ordered)
+    rank_scatter_k<NSW><<<g, 256, 0, s>>>(cand, idx, f, fx, tot, R, Ls),
+        note_launch();
+  else
+    string_number_k<NSW><<<g, 256, 0, s>>>(cand, fx, tot, R, Ls), note_launch();
   MB_CUDA(cudaGetLastError());
   for(void* q : {static_cast<void*>(cand), static_cast<void*>(idx),
                  static_cast<void*>(f), static_cast<void*>(fx),
                  static_cast<void*>(words), static_cast<void*>(occ),
                  static_cast<void*>(vir), static_cast<void*>(dbase)})
-    A.release(q);
+    if(q) A.release(q);
   out.R = R;
   out.M = M;
   out.N1 = int64_t(nrows);
@@ -1525,7 +1595,8 @@ static int bits_for(size_t n) {
 // bits_a + bits_b <= 64. Returns the key width in bits, 0 when not built.
 template <int NBITS>
 static int build_ranks(const SpinPlan& pa, const SpinPlan& pb, size_t ncdets,
-                       Arena& A, cudaStream_t s, RankTables& rt) {
+                       bool ordered, Arena& A, cudaStream_t s,
+                       RankTables& rt) {
   constexpr int NSW = DetTraits<NBITS>::NSW;
   const size_t ta = pa.nu * size_t(spin_candidates(pa.ne, pa.nv));
   const size_t tb = pb.nu * size_t(spin_candidates(pb.ne, pb.nv));
@@ -1539,8 +1610,8 @@ static int build_ranks(const SpinPlan& pa, const SpinPlan& pb, size_t ncdets,
   if(tables > 0.1 * avail || tables + trans > 0.5 * avail) return 0;
   uint64_t *La = nullptr, *Lb = nullptr;
   SpinRanks ra, rb;
-  const size_t na = build_spin_ranks<NBITS>(pa, A, s, ra, &La);
-  const size_t nb = build_spin_ranks<NBITS>(pb, A, s, rb, &Lb);
+  const size_t na = build_spin_ranks<NBITS>(pa, ordered, A, s, ra, &La);
+  const size_t nb = build_spin_ranks<NBITS>(pb, ordered, A, s, rb, &Lb);
   const int ba = bits_for(na), bb = bits_for(nb);
   const double strings = 8.0 * NSW * (double(na) + double(nb));
   if(ba + bb > 64 || tables + strings > 0.15 * avail) {
@@ -1739,7 +1810,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
       const SpinPlan& a = alpha_plan();
       const SpinPlan b = plan_spin<NBITS>(host_dets(), ncdets, h->norb, 1);
       if(a.nu && b.nu) {
-        const int bits = build_ranks<NBITS>(a, b, ncdets, A, s, rt);
+        const int bits = build_ranks<NBITS>(a, b, ncdets, pairs_only, A, s, rt);
         ranked = bits > 0;
         stats.key_bits = uint64_t(bits);
       }
