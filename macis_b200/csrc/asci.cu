@@ -630,21 +630,41 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
     // virtual a (the aa-th): a - aa occupied lie below a
     par0 = (a - aa) ^ ii ^ int(a > i);
   }
-  for(int64_t q0 = 0; q0 < nloop; q0 += 32) {
-    const int64_t qi = q0 + lane;
-    bool keep = false;
-    double r = 0;
-    uint64_t ex[D::NW];
-    uint64_t rkey = 0;
-    if(qi < nloop) {
-      const int q = qlist ? int(qlist[qi]) : int(qi);
-      const int qd = small_div(q, rspan);
-      const int jj = jj0 + qd, bb = bb0 + (q - qd * span);
-      const int j = occI[jj], b = virI[bb];
-      if(kind <= 1) {
-        // append_singles_asci_contributions (determinant_contributions.hpp:25-66)
-        const int nS = S ? nB : nA, nO = S ? nA : nB;
-        const uint8_t* occO = S ? occA : occB;
+  // writes the kept contributions of the warp's 32 (flip: the determinant's
+  // excitation) in lane order
+  auto emit = [&](bool keep, double r, uint64_t rkey, auto&& flip) {
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if(MODE >= 1 && keep) {
+      const int64_t pos = out0 + done + __popc(m & lanemask_lt());
+      if constexpr(MODE == 1) {
+        uint64_t ex[D::NW];
+#pragma unroll
+        for(int w = 0; w < D::NW; ++w) ex[w] = det[w];
+        flip(ex);
+#pragma unroll
+        for(int w = 0; w < D::NW; ++w) keys[pos * D::NW + w] = ex[w];
+      } else {
+        keys[pos] = rkey;
+      }
+      rv[pos] = r;
+      if(umax) mx = fmaxf(mx, float(fabs(r)));
+    }
+    done += __popc(m);
+  };
+  if(kind <= 1) {
+    // append_singles_asci_contributions (determinant_contributions.hpp:25-66)
+    const int nS = S ? nB : nA, nO = S ? nA : nB;
+    const uint8_t* occO = S ? occA : occB;
+    for(int q0 = 0; q0 < int(nloop); q0 += 32) {
+      const int q = q0 + lane;
+      bool keep = false;
+      double r = 0;
+      uint64_t rkey = 0;
+      int j = 0, b = 0;
+      if(q < int(nloop)) {
+        const int qd = small_div(q, rspan);
+        j = occI[qd];
+        b = virI[q - qd * span];
         uint32_t cbin = 0;
         if(S == 0 && (chk || hist))
           cbin = alpha_bin<NSW>(sp_flip(sp_flip(sA, j), b));
@@ -666,92 +686,105 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
           const double hd = hii + epsI[b] - epsI[j] - G2R(b, j) - G2R(j, b);
           h /= (E0 - hd);
           r = coeff * h;
-          if constexpr(MODE == 1) {
-#pragma unroll
-            for(int w = 0; w < D::NW; ++w) ex[w] = det[w];
-            det_flip<NBITS>(ex, S, j);
-            det_flip<NBITS>(ex, S, b);
-          }
-        }
-      } else if(kind <= 3) {
-        // append_ss_doubles_asci_contributions (determinant_contributions.hpp:68-120)
-        uint32_t cbin = 0;
-        if(S == 0 && (chk || hist))
-          cbin = alpha_bin<NSW>(
-              sp_flip(sp_flip(sp_flip(sp_flip(sA, i), j), a), b));
-        bool inr = !chk || (cbin >= blo && cbin < bhi);
-        if(chkb)  // S == 1
-          inr = beta_sub<NSW>(
-                    sp_flip(sp_flip(sp_flip(sp_flip(sB, i), j), a), b), nsub) ==
-                sub;
-        const double Gv = inr ? __ldg(row4 + b + j * n) : 0.0;
-        keep = inr && !(fabs(Gv) < tol);
-        if(MODE == 0 && hist && S == 0 && keep) atomicAdd(hist + cbin, 1ull);
-        if(MODE >= 1 && keep) {
-          // double_ex's sign (i < j, a < b): i <-> a in the string without
-          // j and with b, then j <-> b in the string itself
-          const int par = par0 ^ (b - bb) ^ jj ^ int(b > j) ^
-                          int(a > i ? j < a : b < i);
-          const double2 gji = __ldg(GGi + j), gba = __ldg(GGa + b),
-                        gbi = __ldg(GGi + b), gja = __ldg(GGa + j),
-                        gbj = __ldg(cd.GG + b + j * n);
-          double h = (par & 1) ? -Gv : Gv;
-          const double hd = hia + epsI[b] - eI - epsI[j] + gji.y + gji.x +
-                            gba.y + gba.x - gai - gia - gbi.x - gbi.y -
-                            gja.y - gja.x - gbj.x - gbj.y;
-          h /= (E0 - hd);
-          r = coeff * h;
-          if constexpr(MODE == 1) {
-#pragma unroll
-            for(int w = 0; w < D::NW; ++w) ex[w] = det[w];
-            det_flip<NBITS>(ex, S, i);
-            det_flip<NBITS>(ex, S, j);
-            det_flip<NBITS>(ex, S, a);
-            det_flip<NBITS>(ex, S, b);
-          }
-        }
-      } else {
-        // append_os_doubles_asci_contributions (determinant_contributions.hpp:122-160)
-        const bool inr =
-            !chkb || beta_sub<NSW>(sp_flip(sp_flip(sB, j), b), nsub) == sub;
-        // V(a,i,b,j) from row (a,i) of the pair-swapped copy
-        const double Vv = inr ? __ldg(row4 + b + j * n) : 0.0;
-        keep = inr && !(fabs(Vv) < tol);
-        if(MODE >= 1 && keep) {
-          const int par = par0 ^ (b - bb) ^ jj ^ int(b > j);
-          const double2 gbj = __ldg(cd.GG + b + j * n);
-          double h = (par & 1) ? -Vv : Vv;
-          const double hd = hia + epsI[b] - eI - epsI[j] + __ldg(Vi + j) +
-                            __ldg(Va + b) - gai - gia - gbj.x - gbj.y -
-                            __ldg(Va + j) - __ldg(Vi + b);
-          h /= (E0 - hd);
-          r = coeff * h;
-          if constexpr(MODE == 1) {
-#pragma unroll
-            for(int w = 0; w < D::NW; ++w) ex[w] = det[w];
-            det_flip<NBITS>(ex, 0, a);
-            det_flip<NBITS>(ex, 0, i);
-            det_flip<NBITS>(ex, 1, j);
-            det_flip<NBITS>(ex, 1, b);
-          }
+          if(MODE == 2) rkey = rfix | (uint64_t(__ldg(rvar + q)) << rshift);
         }
       }
-      if constexpr(MODE == 2)
-        if(keep) rkey = rfix | (uint64_t(__ldg(rvar + q)) << rshift);
+      emit(keep, r, rkey, [&](uint64_t* ex) {
+        det_flip<NBITS>(ex, S, j);
+        det_flip<NBITS>(ex, S, b);
+      });
     }
-    const unsigned m = __ballot_sync(0xffffffffu, keep);
-    if(MODE >= 1 && keep) {
-      const int64_t pos = out0 + done + __popc(m & lanemask_lt());
-      if constexpr(MODE == 1) {
-#pragma unroll
-        for(int w = 0; w < D::NW; ++w) keys[pos * D::NW + w] = ex[w];
-      } else {
-        keys[pos] = rkey;
+  } else {
+    // append_ss_doubles_asci_contributions (determinant_contributions.hpp:
+    // 68-120) and append_os_doubles_asci_contributions (:122-160). The element
+    // and the string number of the next 32 are loaded while these are formed:
+    // both come from L2 (a pair's row of V or G, a string's table row), the
+    // rest from L1.
+    struct Item {
+      double v;
+      uint32_t num;
+      int b, j, bb, jj;
+      bool on;
+    };
+    auto fetch = [&](int qi) {
+      Item t{};
+      t.on = qi < int(nloop);
+      if(t.on) {
+        const int q = qlist ? int(qlist[qi]) : qi;
+        const int qd = small_div(q, rspan);
+        t.jj = jj0 + qd;
+        t.bb = bb0 + (q - qd * span);
+        t.j = occI[t.jj];
+        t.b = virI[t.bb];
+        t.v = __ldg(row4 + t.b + t.j * n);
+        if(MODE == 2) t.num = __ldg(rvar + q);
       }
-      rv[pos] = r;
-      mx = fmaxf(mx, float(fabs(r)));
-    }
-    done += __popc(m);
+      return t;
+    };
+    auto loop = [&](auto os_) {
+      constexpr bool OS = decltype(os_)::value;
+      Item nx = fetch(lane);
+      for(int q0 = 0; q0 < int(nloop); q0 += 32) {
+        const Item t = nx;
+        if(q0 + 32 < int(nloop)) nx = fetch(q0 + 32 + lane);
+        const int b = t.b, j = t.j;
+        bool keep = false;
+        double r = 0;
+        uint64_t rkey = 0;
+        if(t.on) {
+          uint32_t cbin = 0;
+          bool inr = true;
+          if constexpr(!OS) {
+            if(S == 0 && (chk || hist))
+              cbin = alpha_bin<NSW>(
+                  sp_flip(sp_flip(sp_flip(sp_flip(sA, i), j), a), b));
+            inr = !chk || (cbin >= blo && cbin < bhi);
+            if(chkb)  // S == 1
+              inr = beta_sub<NSW>(
+                        sp_flip(sp_flip(sp_flip(sp_flip(sB, i), j), a), b),
+                        nsub) == sub;
+          } else {
+            if(chkb) inr = beta_sub<NSW>(sp_flip(sp_flip(sB, j), b), nsub) == sub;
+          }
+          keep = inr && !(fabs(t.v) < tol);
+          if(!OS && MODE == 0 && hist && S == 0 && keep)
+            atomicAdd(hist + cbin, 1ull);
+          if(MODE >= 1 && keep) {
+            // sign of the inner excitation; for one spin, double_ex's (i < j,
+            // a < b): i <-> a in the string without j and with b, then j <-> b
+            // in the string itself
+            int par = par0 ^ (b - t.bb) ^ t.jj ^ int(b > j);
+            const double2 gbj = __ldg(cd.GG + b + j * n);
+            double hd;
+            if constexpr(OS) {
+              hd = hia + epsI[b] - eI - epsI[j] + __ldg(Vi + j) + __ldg(Va + b) -
+                   gai - gia - gbj.x - gbj.y - __ldg(Va + j) - __ldg(Vi + b);
+            } else {
+              par ^= int(a > i ? j < a : b < i);
+              const double2 gji = __ldg(GGi + j), gba = __ldg(GGa + b),
+                            gbi = __ldg(GGi + b), gja = __ldg(GGa + j);
+              hd = hia + epsI[b] - eI - epsI[j] + gji.y + gji.x + gba.y +
+                   gba.x - gai - gia - gbi.x - gbi.y - gja.y - gja.x - gbj.x -
+                   gbj.y;
+            }
+            double h = (par & 1) ? -t.v : t.v;
+            h /= (E0 - hd);
+            r = coeff * h;
+            if(MODE == 2) rkey = rfix | (uint64_t(t.num) << rshift);
+          }
+        }
+        emit(keep, r, rkey, [&](uint64_t* ex) {
+          det_flip<NBITS>(ex, S, i);
+          det_flip<NBITS>(ex, SI, j);
+          det_flip<NBITS>(ex, S, a);
+          det_flip<NBITS>(ex, SI, b);
+        });
+      }
+    };
+    if(kind == 4)
+      loop(std::true_type{});
+    else
+      loop(std::false_type{});
   }
   if(MODE == 0 && lane == 0) {
     *count_out = done;
@@ -771,8 +804,11 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
 // output offsets at once, and the warp runs the units with work one after
 // another (a fill pass skips the units without contributions in its range:
 // output positions come from the offsets, not from the order).
+// (256 bits: 3 resident blocks; the generation of 1.13e9 contributions takes
+// 13.4 ms so and 40 ms before, mostly from the prefetch in unit_run. At 128
+// bits the bound spills and is no faster: 37 ms of 2.7e9.)
 template <int NBITS, int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, NBITS == 256 && MODE == 2 ? 3 : 1)
     units_k(Ints I, CoreData cd, int64_t u0, int64_t u1, size_t c0, size_t c1,
             double E0, double tol, int64_t* counts, const int64_t* outoff,
             uint64_t* keys, double* rv, const uint8_t* umask, float* umax,
