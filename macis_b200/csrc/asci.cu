@@ -804,11 +804,12 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
 // output offsets at once, and the warp runs the units with work one after
 // another (a fill pass skips the units without contributions in its range:
 // output positions come from the offsets, not from the order).
-// (256 bits: 3 resident blocks; the generation of 1.13e9 contributions takes
-// 13.4 ms so and 40 ms before, mostly from the prefetch in unit_run. At 128
-// bits the bound spills and is no faster: 37 ms of 2.7e9.)
+// Three resident blocks for the generation with number keys: with the
+// prefetch of unit_run it takes 13.4 ms of 1.13e9 contributions at 256 bits
+// (40 before) and 37 ms of 2.7e9 at 128 bits, where the compiler's own choice
+// of registers (two blocks) takes 59.
 template <int NBITS, int MODE>
-__global__ void __launch_bounds__(256, NBITS == 256 && MODE == 2 ? 3 : 1)
+__global__ void __launch_bounds__(256, MODE == 2 ? 3 : 1)
     units_k(Ints I, CoreData cd, int64_t u0, int64_t u1, size_t c0, size_t c1,
             double E0, double tol, int64_t* counts, const int64_t* outoff,
             uint64_t* keys, double* rv, const uint8_t* umask, float* umax,
