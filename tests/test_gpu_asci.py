@@ -386,3 +386,30 @@ def test_grouped_candidates_match_accumulated_list(monkeypatch, nbits, n, k,
                 assert np.array_equal(got, np.concatenate([sel, core]))
                 if stat["batches"] == 1:
                     assert stat["kept_pairs"] == len(st)
+
+
+@pytest.mark.parametrize("nbits,n,k,ncore", [(64, 8, 4, 300), (128, 8, 4, 200)])
+def test_search_with_many_contributions_per_determinant(nbits, n, k, ncore):
+    """Dense cores, where determinants get more contributions than a warp has
+    lanes, and cuts at the ends of the range (no determinant beyond the core
+    ones, one, all but one), against the fully sorted accumulated list. The
+    sums are formed in the same order on both sides, so the determinants are
+    equal."""
+    from cases import core_set
+    T, V = mb.synthetic_integrals(n, 3)
+    cd, C = core_set(n, k, ncore, nbits, nalpha=40)
+    H = mb.HamiltonianGenerator(T, V, nbits)
+    E0 = float(H.matrix_element(cd[:1], cd[:1])) - 0.5
+    st, rv = mb.asci_pairs(_settings(), cd, E0, C, H)
+    W = nbits // 64
+    core = {tuple(d) for d in cd.tolist()}
+    ok = (rv != 0) & np.array([tuple(d) not in core for d in st.tolist()])
+    st, rv = st[ok], np.abs(rv[ok])
+    order = np.lexsort(tuple(st[:, w] for w in range(W)) + (-rv,))
+    for top in (0, 1, len(st) // 2, len(st) - 1):
+        got = mb.asci_search(_settings(), top + ncore, cd, E0, C, n, H)
+        stat = mb.last_search_stats(H)
+        assert stat["raw_pairs"] > 10 * len(st)
+        sel = st[order[:top]]
+        sel = sel[np.lexsort(tuple(sel[:, w] for w in range(W)))]
+        assert np.array_equal(got, np.concatenate([sel, cd]))
