@@ -311,6 +311,7 @@ struct RankTables {
   int bits_a = 0;
   const uint64_t* La = nullptr;  // distinct candidate alpha strings (NSW words)
   const uint64_t* Lb = nullptr;
+  bool mixed = false;  // records hold mix_key of the number keys
 };
 // First double of row ii * nv + aa among the doubles of a string with ne
 // electrons and nv virtuals (rows before it hold (ne-1-ii')(nv-1-aa') each).
@@ -454,7 +455,7 @@ __global__ void unrank_k(const uint64_t* rk, size_t n, RankTables rt,
   const uint64_t ma = (uint64_t(1) << rt.bits_a) - 1;
   for(size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
       i += size_t(gridDim.x) * blockDim.x) {
-    const uint64_t k = rk[i];
+    const uint64_t k = rt.mixed ? unmix_key(rk[i]) : rk[i];
     const size_t ra = size_t(k & ma), rb = size_t(k >> rt.bits_a);
     Spin<NSW> a, b;
 #pragma unroll
@@ -676,7 +677,7 @@ __device__ void unit_run(const Ints& I, const CoreData& cd, size_t c, int64_t t,
 #pragma unroll
         for(int w = 0; w < D::NW; ++w) keys[pos * D::NW + w] = ex[w];
       } else {
-        keys[pos] = rkey;
+        keys[pos] = rt.mixed ? mix_key(rkey) : rkey;
       }
       rv[pos] = r;
       if(umax) mx = fmaxf(mx, float(fabs(r)));
@@ -1926,6 +1927,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
       if(a.nu && b.nu) {
         const int bits = build_ranks<NBITS>(a, b, ncdets, pairs_only, A, s, rt);
         ranked = bits > 0;
+        rt.mixed = !pairs_only;
         stats.key_bits = uint64_t(bits);
       }
       stats.rank_ms = ms_since(t_rk);
@@ -1956,7 +1958,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
     cap = int64_t((0.8 * double(device_bytes_available()) - keep_reserve) /
                   per_pair);
     cap = std::min<int64_t>(std::max<int64_t>(cap, int64_t(1) << 20),
-                            int64_t(1) << 31);
+                            (int64_t(1) << 32) - 1);
   }
   // ranges: consecutive alpha-string bins packed up to the cap from the
   // measured bin loads (a single bin above the cap is a range of its own)
@@ -2271,8 +2273,10 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
     uint64_t nuniq = 0, nscored = 0, npruned = 0;
     uint64_t* k2 = nullptr;
     double* r2 = nullptr;
-    auto accumulate = [&](auto kw) {  // KW key words per record
+    // KW key words per record; MIXED: the keys are mixed number keys
+    auto accumulate = [&](auto kw, auto mixed_) {
       constexpr int KW = decltype(kw)::value;
+      constexpr bool MIXED = decltype(mixed_)::value;
       k2 = B.get<uint64_t>(size_t(P) * KW + KW);
       r2 = B.get<double>(size_t(P) + 1);
       const size_t n = size_t(P);
@@ -2300,7 +2304,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
         {
           DigitPasses<KW, double> passes(n, B);
           for(int p = 0; p < np; ++p) {
-            passes.run(keys, rv, k2, r2, HashDigit<KW>{sh + 8 * p});
+            passes.run(keys, rv, k2, r2, HashDigit<KW, MIXED>{sh + 8 * p});
             std::swap(keys, k2);
             std::swap(rv, r2);
           }
@@ -2310,8 +2314,10 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
         auto* gc = B.get<GroupCounts>(1);
         auto run = [&](size_t n1, uint64_t tout) {
           MB_CUDA(cudaMemsetAsync(gc, 0, sizeof(GroupCounts), s));
-          group_sum_k<KW><<<grid_for(n1, GS_TILE, 8 * sms), GS_THREADS, 0, s>>>(
-              keys, rv, n, 0, n1, sh, tcut, tout, st.rv_prune_tol, k2, r2, gc),
+          group_sum_k<KW, MIXED>
+              <<<grid_for(n1, GroupTile<KW>::N * GS_WARPS, 16 * sms), GS_THREADS,
+                 0, s>>>(
+              keys, rv, n, n1, sh, tcut, tout, st.rv_prune_tol, k2, r2, gc),
               note_launch();
           MB_CUDA(cudaGetLastError());
         };
@@ -2337,7 +2343,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
         nuniq = hc.unique;
         if(ncdets) {
           MB_CUDA(cudaMemsetAsync(gc, 0, sizeof(GroupCounts), s));
-          group_core_k<KW><<<grid_for(ncdets, 128, 16 * sms), 128, 0, s>>>(
+          group_core_k<KW, MIXED><<<grid_for(ncdets, 128, 16 * sms), 128, 0, s>>>(
               keys, rv, n, sh, tcut, st.rv_prune_tol, core_key, ncdets, gc),
               note_launch();
           const GroupCounts cc = to_host(gc, s);
@@ -2353,7 +2359,10 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
     };
     if(P) {
       if(ranked) {
-        accumulate(std::integral_constant<int, 1>{});
+        if(rt.mixed)
+          accumulate(std::integral_constant<int, 1>{}, std::true_type{});
+        else
+          accumulate(std::integral_constant<int, 1>{}, std::false_type{});
         // ranked keys back to determinants
         uint64_t* kd = B.get<uint64_t>(uq.n * NW + NW);
         if(uq.n)
@@ -2362,7 +2371,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
         B.release(k2);
         k2 = kd;
       } else {
-        accumulate(std::integral_constant<int, NW>{});
+        accumulate(std::integral_constant<int, NW>{}, std::false_type{});
       }
       uq.keys = k2;
       uq.rv = r2;

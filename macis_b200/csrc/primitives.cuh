@@ -286,21 +286,43 @@ __device__ __forceinline__ unsigned digit_of(const Key<NW>& k, int shift) {
   return unsigned(w >> (shift & 63)) & 255u;
 }
 
+// Digit counts of every tile, counts[digit * ntiles + tile]. A block takes
+// RS_HT consecutive tiles, so that it writes whole sectors of counts, and
+// loads 8 keys a thread at a time; ntiles is a multiple of RS_HT (tiles past
+// the end count nothing). 2.7e9 keys: 3.4 ms (6.4 TB/s); 6.9 ms with a tile
+// per block and a lone 4-byte count per digit and block.
+constexpr int RS_HT = 8;
 template <int NW, class Digit>
-__global__ void __launch_bounds__(RS_THREADS)
+__global__ void __launch_bounds__(256)
     radix_hist_k(const uint64_t* keys, size_t n, Digit digit, uint32_t* counts,
-                 unsigned nblocks) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
+                 unsigned ntiles) {
+  __shared__ uint32_t h[RS_HT][256];
+#pragma unroll
+  for(int t = 0; t < RS_HT; ++t) h[t][threadIdx.x] = 0;
   __syncthreads();
-  const size_t base = size_t(blockIdx.x) * RS_TILE;
-#pragma unroll 4
-  for(int r = 0; r < RS_IPT; ++r) {
-    size_t i = base + size_t(r) * RS_THREADS + threadIdx.x;
-    if(i < n) atomicAdd(&h[digit(load_key<NW>(keys, i))], 1u);
+  const unsigned tile0 = blockIdx.x * RS_HT;
+  for(int t = 0; t < RS_HT; ++t) {
+    const size_t base = size_t(tile0 + t) * RS_TILE;
+    if(base >= n) break;
+    for(int r0 = 0; r0 < RS_TILE / 256; r0 += 8) {
+      unsigned d[8];
+#pragma unroll
+      for(int u = 0; u < 8; ++u) {
+        const size_t i = base + size_t(r0 + u) * 256 + threadIdx.x;
+        d[u] = i < n ? digit(load_key<NW>(keys, i)) : 256u;
+      }
+#pragma unroll
+      for(int u = 0; u < 8; ++u)
+        if(d[u] < 256u) atomicAdd(&h[t][d[u]], 1u);
+    }
   }
   __syncthreads();
-  counts[size_t(threadIdx.x) * nblocks + blockIdx.x] = h[threadIdx.x];
+  uint32_t* out = counts + size_t(threadIdx.x) * ntiles + tile0;
+#pragma unroll
+  for(int t = 0; t < RS_HT; t += 4)
+    *reinterpret_cast<uint4*>(out + t) =
+        make_uint4(h[t][threadIdx.x], h[t + 1][threadIdx.x],
+                   h[t + 2][threadIdx.x], h[t + 3][threadIdx.x]);
 }
 
 // Bytes of shared memory the scatter stages a tile in.
@@ -338,7 +360,6 @@ __device__ __forceinline__ void rs_tile_pass(const uint64_t* keys,
   uint64_t* skeys = reinterpret_cast<uint64_t*>(rs_smem);
   P* svals = reinterpret_cast<P*>(skeys + size_t(RS_TILE) * NW);
   __shared__ uint32_t wcount[RS_WARPS][256];
-  __shared__ uint32_t bstart[256];
   __shared__ uint64_t boff[256];
   __shared__ uint32_t scan_sh[RS_WARPS + 1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -369,25 +390,28 @@ __device__ __forceinline__ void rs_tile_pass(const uint64_t* keys,
   }
   __syncthreads();
   {
-    // per digit: exclusive prefix over warps, then over digits (bucket
-    // starts inside the tile), and the digit's output position
+    // per digit: exclusive prefix over warps and digits (the position in the
+    // tile's bucket-ordered copy), and the digit's output position less that
     const int d = threadIdx.x;
     uint32_t acc = 0;
+#pragma unroll
+    for(int w = 0; w < RS_WARPS; ++w) acc += wcount[w][d];
+    const uint32_t start = block_excl_scan<uint32_t>(acc, scan_sh, nullptr);
+    boff[d] = resolve(d, acc) - start;
+    acc = start;
 #pragma unroll
     for(int w = 0; w < RS_WARPS; ++w) {
       const uint32_t c = wcount[w][d];
       wcount[w][d] = acc;
       acc += c;
     }
-    bstart[d] = block_excl_scan<uint32_t>(acc, scan_sh, nullptr);
-    boff[d] = resolve(d, acc);
   }
   __syncthreads();
 #pragma unroll
   for(int r = 0; r < RS_IPT; ++r) {
     if(dig[r] < 256u) {
       const size_t i = wbase + size_t(r) * 32 + lane;
-      const uint32_t pos = bstart[dig[r]] + wcount[wid][dig[r]] + rank[r];
+      const uint32_t pos = wcount[wid][dig[r]] + rank[r];
       store_key<NW>(skeys, pos, load_key<NW>(keys, i));
       if(vals) svals[pos] = vals[i];
     }
@@ -396,22 +420,21 @@ __device__ __forceinline__ void rs_tile_pass(const uint64_t* keys,
   const int cnt = int(n - tile0 < size_t(RS_TILE) ? n - tile0 : size_t(RS_TILE));
   for(int j = threadIdx.x; j < cnt; j += RS_THREADS) {
     const Key<NW> kk = load_key<NW>(skeys, j);
-    const unsigned d = digit(kk);
-    const size_t dst = boff[d] + uint32_t(j - bstart[d]);
+    const size_t dst = boff[digit(kk)] + uint32_t(j);
     store_key<NW>(keys_out, dst, kk);
     if(vals) vals_out[dst] = svals[j];
   }
 }
 
 // One digit pass with per-block bucket offsets from radix_hist_k + scan.
-template <int NW, typename P, class Digit>
+template <int NW, typename P, class Digit, typename OT>
 __global__ void __launch_bounds__(RS_THREADS, 4)
     radix_scatter_k(const uint64_t* keys, const P* vals, size_t n, Digit digit,
-                    const uint64_t* offsets, unsigned nblocks,
-                    uint64_t* keys_out, P* vals_out) {
+                    const OT* offsets, unsigned ntiles, uint64_t* keys_out,
+                    P* vals_out) {
   // issued before the ranking: its latency hides behind the tile loads
   const uint64_t my_off =
-      offsets[size_t(threadIdx.x) * nblocks + blockIdx.x];
+      offsets[size_t(threadIdx.x) * ntiles + blockIdx.x];
   rs_tile_pass<NW, P>(keys, vals, n, digit, size_t(blockIdx.x) * RS_TILE,
                       keys_out, vals_out, [&](int, uint32_t) { return my_off; });
 }
@@ -505,34 +528,25 @@ __global__ void __launch_bounds__(RS_THREADS, 4)
       });
 }
 
-// Classic digit passes (per-block histogram, scan, scatter) over n records,
-// with their scratch.
+// Classic digit passes (per-tile histogram, scan, scatter) over n records,
+// with their scratch. Output positions are 32-bit below 2^32 records.
 template <int NW, typename P>
 struct DigitPasses {
   size_t n;
   Arena& A;
-  unsigned nblocks;
+  unsigned nblocks, ntiles;  // tiles, and padded to RS_HT
   uint32_t* counts = nullptr;
-  uint64_t* offs = nullptr;
+  void* offs = nullptr;
   DigitPasses(size_t n_, Arena& A_)
-      : n(n_), A(A_), nblocks(unsigned((n_ + RS_TILE - 1) / RS_TILE)) {}
+      : n(n_), A(A_), nblocks(unsigned((n_ + RS_TILE - 1) / RS_TILE)),
+        ntiles((nblocks + RS_HT - 1) / RS_HT * RS_HT) {}
   template <class Digit>
   void run(const uint64_t* kin, const P* vin, uint64_t* kout, P* vout,
            Digit digit) {
-    constexpr size_t stage = rs_stage_bytes<NW, P>();
-    if(!counts) {
-      MB_CUDA(cudaFuncSetAttribute(radix_scatter_k<NW, P, Digit>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   int(stage)));
-      counts = A.get<uint32_t>(size_t(256) * nblocks);
-      offs = A.get<uint64_t>(size_t(256) * nblocks);
-    }
-    radix_hist_k<NW><<<nblocks, RS_THREADS, 0, A.s>>>(kin, n, digit, counts,
-                                                      nblocks), note_launch();
-    exclusive_scan<uint32_t, uint64_t>(counts, offs, size_t(256) * nblocks,
-                                       nullptr, A);
-    radix_scatter_k<NW, P><<<nblocks, RS_THREADS, stage, A.s>>>(
-        kin, vin, n, digit, offs, nblocks, kout, vout), note_launch();
+    if(n >> 32)
+      run_as<uint64_t>(kin, vin, kout, vout, digit);
+    else
+      run_as<uint32_t>(kin, vin, kout, vout, digit);
   }
   void release() {
     if(counts) {
@@ -541,6 +555,26 @@ struct DigitPasses {
     }
     counts = nullptr;
     offs = nullptr;
+  }
+
+ private:
+  template <typename OT, class Digit>
+  void run_as(const uint64_t* kin, const P* vin, uint64_t* kout, P* vout,
+              Digit digit) {
+    constexpr size_t stage = rs_stage_bytes<NW, P>();
+    if(!counts) {
+      MB_CUDA(cudaFuncSetAttribute(radix_scatter_k<NW, P, Digit, OT>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(stage)));
+      counts = A.get<uint32_t>(size_t(256) * ntiles);
+      offs = A.get<OT>(size_t(256) * ntiles);
+    }
+    OT* off = static_cast<OT*>(offs);
+    radix_hist_k<NW><<<ntiles / RS_HT, 256, 0, A.s>>>(kin, n, digit, counts,
+                                                      ntiles), note_launch();
+    exclusive_scan<uint32_t, OT>(counts, off, size_t(256) * ntiles, nullptr, A);
+    radix_scatter_k<NW, P><<<nblocks, RS_THREADS, stage, A.s>>>(
+        kin, vin, n, digit, off, ntiles, kout, vout), note_launch();
   }
 };
 
