@@ -66,7 +66,7 @@ typedef struct {
 /* Diagnostics of the last asci_search call on a handle. */
 typedef struct {
   uint64_t raw_pairs;     /* contributions generated (after h_el_tol) */
-  uint64_t unique_pairs;  /* after sort + accumulate */
+  uint64_t unique_pairs;  /* distinct determinants of the contributions */
   uint64_t kept_pairs;    /* after dropping core dets, zero scores and, in
                              ranges after the running top-k first filled,
                              scores below its k-th score */
@@ -77,17 +77,17 @@ typedef struct {
   uint64_t samples;       /* training samples recorded into the network */
   double screen_ms;       /* prediction + selection + recording */
   double predict_ms;      /* network forward over all units (device time) */
-  uint64_t sort_pass_items; /* sum over the sorted candidate ranges of
+  uint64_t sort_pass_items; /* sum over the candidate ranges of
                                (radix digit passes x records): each pass
                                reads and writes every record once */
   uint64_t alpha_strings;   /* alpha strings of the core dets whose alpha
                                doubles the candidate ranges read from
                                per-range lists (those shared by the most
                                core dets), else 0 */
-  uint64_t key_bits;        /* bits of the ranked candidate keys (alpha and
-                               beta string ranks) the candidates were sorted
-                               by, 0 when sorted by the determinant bitset */
-  double rank_ms;           /* building the string rank tables */
+  uint64_t key_bits;        /* bits of the candidate keys made of alpha and
+                               beta string numbers, 0 when the candidates
+                               were keyed by the determinant bitset */
+  double rank_ms;           /* building the string number tables */
 } macis_b200_asci_stats;
 
 /* Learned screening (no MACIS counterpart). A "unit" of the ASCI search is

@@ -21,12 +21,12 @@
 namespace mb {
 
 // 32 consecutive rows per block and up to 64 blocks per SM: neighbouring rows
-// share many columns and find x in L1 while they advance together; gathers
-// that go to L2 bound the product. CAS(12,12), 853,776 rows and 1.55e9 FP64
-// elements, build and one product: 10.45 -> 9.78 ms against blocks of 8 rows
-// with a grid-stride loop; CAS(10,10) mixed, 80 products: 19.6 -> 19.2 ms. 2
-// blocks an SM with a loop: 10.35 ms; 16 rows a block: 9.97 to the 9.62 of 32
-// on the same box. Loads that leave the matrix out of L1: no change.
+// share many columns and find x in L1 while they advance together, where
+// blocks of 8 rows with a grid-stride loop were bound by gathers of x from L2.
+// CAS(12,12), 853,776 rows and 1.55e9 elements: FP64 3.46 -> 2.88 ms (6.5
+// TB/s), FP32 values 2.6 -> 2.30 ms. 2 blocks per SM with a loop, or 16 rows a
+// block, gained a fifth of that at most; loads that leave the matrix out of L1
+// changed nothing.
 constexpr int SPMV_THREADS = 1024;
 
 // X32: the off-diagonal products use the FP32 copy x32 (the operator of
