@@ -1315,18 +1315,20 @@ __device__ __forceinline__ void gen_enumerate(const GenData& g, int32_t rg,
         continue;
       }
       // four loads in flight: groups are a few hundred members, and the loop
-      // waits for each load
+      // waits for each load (one copy of emit, see gen_pairs)
       for(int mb = gm0; mb < gm1; mb += 128) {
-        int pb[4];
+        uint32_t pbs = 0;  // their four distances, a byte each
 #pragma unroll
         for(int u = 0; u < 4; ++u) {
           const int m = mb + 32 * u + lane;
-          pb[u] = m < gm1 ? sp_popc(ld_spin<NSW>(g.sbeta, m) ^ bb) : 99;
+          const int pb = m < gm1 ? sp_popc(ld_spin<NSW>(g.sbeta, m) ^ bb) : 255;
+          pbs |= uint32_t(pb) << (8 * u);
         }
-#pragma unroll
-        for(int u = 0; u < 4; ++u)
-          if(mb + 32 * u < gm1)
-            emit(pb[u] <= limit, mb + 32 * u + lane, ppa, pb[u]);
+#pragma unroll 1
+        for(int m = mb; m < gm1 && m < mb + 128; m += 32, pbs >>= 8) {
+          const int pb = int(pbs & 255u);
+          emit(pb <= limit, m + lane, ppa, pb);
+        }
       }
     }
   }
@@ -1337,38 +1339,53 @@ __device__ __forceinline__ void gen_enumerate(const GenData& g, int32_t rg,
 // hold one or two each. gen_pairs queues them and calls eval(on, m,
 // is_double) with 32 at a time, doubles and the rest (singles, the diagonal,
 // lists of mixed electron counts) apart: an element then costs a lane's share
-// of the warp's instructions and not all of them. q: 128 entries of shared
-// memory per warp.
+// of the warp's instructions and not all of them. eval is expanded once in the
+// queueing, which stands at five places of the enumeration, and once at the
+// end: with a copy per kind of pair and unrolled chunk (18 in all) a warp
+// waited half of its time for instructions, and the matrix-free product on an
+// n = 64 list took 3.93 and not 2.46 ms (2.97 with eval as a call), form_rdms on
+// CAS(9,9) 0.94 and not 0.89. q: 128 entries of shared memory per warp.
 template <int NSW, class F>
 __device__ __forceinline__ void gen_pairs(const GenData& g, int32_t rg,
                                           Spin<NSW> ba, Spin<NSW> bb,
                                           uint8_t* ov, uint32_t* q, F&& eval) {
   const int lane = threadIdx.x & 31;
-  int n[2] = {0, 0};  // queued: others, doubles
+  int n0 = 0, n1 = 0;  // queued: others, doubles
   gen_enumerate<NSW>(g, rg, ba, bb, ov,
                      [&](bool act, int64_t m, int pa, int pb) {
-    if(!__any_sync(0xffffffffu, act)) return;
+    const unsigned any = __ballot_sync(0xffffffffu, act);
+    if(!any) return;
     const bool dbl = pa + pb == 4 && !(pa & 1);
-#pragma unroll
-    for(int c = 0; c < 2; ++c) {
-      const bool mine = act && dbl == (c == 1);
-      const unsigned msk = __ballot_sync(0xffffffffu, mine);
-      if(mine) q[64 * c + n[c] + __popc(msk & lanemask_lt())] = uint32_t(m);
-      n[c] += __popc(msk);
-      if(n[c] >= 32) {
-        __syncwarp();
-        eval(true, int64_t(q[64 * c + lane]), c == 1);
-        n[c] -= 32;
-        const uint32_t t = lane < n[c] ? q[64 * c + 32 + lane] : 0;
-        __syncwarp();
-        if(lane < n[c]) q[64 * c + lane] = t;
-      }
+    const unsigned md = __ballot_sync(0xffffffffu, act && dbl), mo = any & ~md;
+    if(act) {
+      const int at = dbl ? 64 + n1 + __popc(md & lanemask_lt())
+                         : n0 + __popc(mo & lanemask_lt());
+      q[at] = uint32_t(m);
+    }
+    n0 += __popc(mo);
+    n1 += __popc(md);
+#pragma unroll 1
+    while(n0 >= 32 || n1 >= 32) {
+      const bool d = n0 < 32;
+      uint32_t* qc = d ? q + 64 : q;
+      __syncwarp();
+      eval(true, int64_t(qc[lane]), d);
+      const int left = (d ? n1 : n0) - 32;
+      const uint32_t t = lane < left ? qc[32 + lane] : 0;
+      __syncwarp();
+      if(lane < left) qc[lane] = t;
+      if(d)
+        n1 = left;
+      else
+        n0 = left;
     }
   });
   __syncwarp();
-#pragma unroll
-  for(int c = 0; c < 2; ++c)
-    if(n[c]) eval(lane < n[c], int64_t(lane < n[c] ? q[64 * c + lane] : 0), c == 1);
+#pragma unroll 1
+  for(int c = 0; c < 2; ++c) {
+    const int nc = c ? n1 : n0;
+    if(nc) eval(lane < nc, int64_t(lane < nc ? q[64 * c + lane] : 0), c == 1);
+  }
   __syncwarp();
 }
 constexpr int GEN_SCRATCH = 256 + 128 * 4;  // bytes per warp: ov, q
