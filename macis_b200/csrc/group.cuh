@@ -63,8 +63,8 @@ struct HashDigit {  // the byte of the key's hash at bit `shift`
 };
 
 // Hash digits for n records: 20 per bucket at most, of which a window of 32
-// still ends a whole bucket. A digit pass moves every record once (11.7 ms of
-// 1e9); for 2.9e8 records a fourth pass takes 3.4 ms and their sums 4.0 in
+// still ends a whole bucket. A digit pass moves every record once (10.6 ms of
+// 1e9); for 2.9e8 records a fourth pass takes 3.1 ms and their sums 4.0 in
 // place of 6.5 ms, and fuller buckets are read one key after another.
 inline int group_digits(size_t n) {
   int np = 1;
@@ -96,7 +96,7 @@ struct GroupCounts {
 // and, with a threshold, next to no writes: with a full sort, the flag, scan,
 // start and sum passes over it, and the core filter, compaction and selection
 // over the 1.6e9 sums they left, the sort and merge phases of the n = 48 search
-// of 2.7e9 contributions took 311 + 90 ms; with this 176 + 1 ms.
+// of 2.7e9 contributions took 311 + 90 ms; with this 163 + 1 ms.
 //
 // A warp stages a tile and goes through it 32 records at a time, each time
 // from the start of a bucket to the end of the last whole one in the window:
