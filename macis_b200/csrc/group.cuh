@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(GS_THREADS)
   const uint64_t tmin = tcut > tout ? tcut : tout;
   uint32_t nuniq = 0, nscored = 0, npruned = 0;
   auto bucket = [&](const Key<NW>& k) { return rec_hash<NW, MIXED>(k) >> sh; };
-  auto judge = [&](double a) {  // a finished sum: is it to be written?
+  auto accept = [&](double a) {  // a finished sum: is it to be written?
     ++nuniq;
     const double m = fabs(a);
     const uint64_t bits = uint64_t(__double_as_longlong(m));
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(GS_THREADS)
               }
               if(mb != ALL) break;
             }
-            if(lane == src && judge(a)) {
+            if(lane == src && accept(a)) {
               const size_t o = size_t(atomicAdd(&cnt->out, 1ull));
               store_key<NW>(okeys, o, q);
               osum[o] = a;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(GS_THREADS)
           rest &= rest - 1;
         }
       }
-      const bool take = first && judge(a);
+      const bool take = first && accept(a);
       const unsigned tm = __ballot_sync(ALL, take);
       if(tm) {
         __syncwarp();  // the window has been read
