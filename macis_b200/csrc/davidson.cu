@@ -1,7 +1,7 @@
 // Single-vector Davidson on the GPU, replacing macis::davidson
 // (include/macis/solvers/davidson.hpp:129-225) and diagonal_guess (:62-68).
 //
-// Basis V and A*V live in HBM (N x (max_m+1) FP64 each). Per iteration:
+// Basis V and A*V live in HBM (N x (max(max_m, 2) + 1) FP64 each). Per iteration:
 //   AV_i = H V_i                                  (spmv.cu)
 //   row i of the Rayleigh matrix V^T AV           (multidot_k, FP64)
 //   k x k symmetric eigenproblem on the host      (eig.cpp, lowest pair)
@@ -52,7 +52,7 @@ struct DavReport {
   volatile double rn2;
   // phase boundaries, ns: the row's kernel, the step's residual, its end
   volatile unsigned long long t_row0, t_row1, t_res0, t_res1, t_end;
-  volatile double row[1];      // max_m + 1 entries
+  volatile double row[1];      // an entry per basis column
 };
 
 // Sum of acc[c] over the warp for 8 values at once: each step halves the
@@ -545,13 +545,29 @@ int davidson_op(const DavOperator& op, int64_t max_m, double tol,
   max_m = std::min<int64_t>(max_m, N);
   if(restart_keep >= max_m) restart_keep = int(max_m) - 1;
   const double* D = op.diag;
-  if(!use_guess) unit_guess_k<<<1, 1024, 0, s>>>(D, N, X), note_launch();
-  double* V = Ar.get<double>(size_t(N) * (max_m + 1));
-  double* AV = Ar.get<double>(size_t(N) * (max_m + 1));
+  if(!use_guess || N == 1) unit_guess_k<<<1, 1024, 0, s>>>(D, N, X), note_launch();
+  auto wall_ms = [&] {
+    return std::chrono::duration<double, std::milli>(
+               std::chrono::steady_clock::now() - t_wall)
+        .count();
+  };
+  if(N == 1) {  // no second basis vector: the product of the unit vector
+    double* y = Ar.get<double>(1);
+    op.apply(X, y);
+    *E = to_host(y, s);
+    *niter = st.iterations = 1;
+    st.wall_ms = wall_ms();
+    g_dav_stats = st;
+    return std::isfinite(*E) ? 0 : MACIS_B200_ENOCONV;
+  }
+  // the first step has two basis vectors, whatever max_m, and writes a third
+  const int64_t cols = std::max<int64_t>(max_m, 2) + 1;
+  double* V = Ar.get<double>(size_t(N) * cols);
+  double* AV = Ar.get<double>(size_t(N) * cols);
   double* tmp = restart_keep > DV_CHUNK
                     ? Ar.get<double>(size_t(N) * restart_keep)
                     : nullptr;
-  const int ld = int(max_m + 1);
+  const int ld = int(cols);
   DavCtx ctx(s, N, ld, Ar, op.pinned);
   RitzCoef rc;
   rc.dev = nullptr;
@@ -663,9 +679,7 @@ int davidson_op(const DavOperator& op, int64_t max_m, double tol,
   MB_CUDA(cudaGetLastError());
   MB_CUDA(cudaStreamSynchronize(s));
   st.iterations = iter;
-  st.wall_ms = std::chrono::duration<double, std::milli>(
-                   std::chrono::steady_clock::now() - t_wall)
-                   .count();
+  st.wall_ms = wall_ms();
   g_dav_stats = st;
   *E = lam0;
   *niter = iter;

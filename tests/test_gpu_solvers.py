@@ -129,3 +129,39 @@ def test_davidson_against_dense(n, na, nb, max_m, keep):
         assert abs(abs(U[:, 0] @ X) - 1.0) < 1e-6
     st = mb.davidson_stats()
     assert st["iterations"] == it and all(v >= 0 for v in st.values())
+
+
+@pytest.mark.parametrize("stored", [True, False])
+@pytest.mark.parametrize("n,na,nb,max_m", [(1, 1, 0, 1), (2, 2, 2, 40),
+                                           (2, 1, 1, 1), (2, 1, 1, 2),
+                                           (6, 3, 3, 1), (6, 3, 3, 2)])
+def test_davidson_smallest_subspaces(n, na, nb, max_m, stored):
+    """A single determinant (E is its diagonal element, the vector the unit
+    vector) and the smallest subspaces, where the solver stops after one step
+    with the basis (x0, H x0): the lowest pair of numpy's 2 x 2 projection.
+    Entries of order 10 in sums of 400 at most: 1e-9."""
+    from macis_b200 import _lib
+    T, V, d = fci(n, na, nb, 64, seed=3)
+    H = mb.HamiltonianGenerator(T, V, 64)
+    A = mb.make_csr_hamiltonian(d, H, 0.0)
+    rp, ci, nz = A.to_host()
+    M = np.zeros((A.m, A.m))
+    for i in range(A.m):
+        M[i, ci[rp[i]:rp[i + 1]]] = nz[rp[i]:rp[i + 1]]
+    op = A if stored else mb.MatrixFreeHamiltonian(d, H, 0.0)
+    solve = (_lib.LIB.macis_b200_davidson_ex if stored
+             else _lib.LIB.macis_b200_hop_davidson)
+    import ctypes as C
+    X, E, it = np.zeros(A.m), C.c_double(), C.c_int64()
+    o = _lib.DavidsonOptsC(max_m, 1e-13, 0, 0, 0)
+    rc = solve(op.handle, C.byref(o), X.ctypes.data, C.byref(E), C.byref(it), 0)
+    assert it.value == 1
+    if A.m == 1:
+        assert rc == 0 and E.value == M[0, 0] and X[0] == 1.0
+        return
+    assert rc == _lib.ENOCONV
+    Q = np.linalg.qr(np.stack([np.eye(A.m)[np.argmin(np.diag(M))],
+                               M[:, np.argmin(np.diag(M))]], axis=1))[0]
+    w, U = np.linalg.eigh(Q.T @ M @ Q)
+    assert abs(E.value - w[0]) < 1e-9
+    assert abs(abs(X @ Q @ U[:, 0]) - 1.0) < 1e-9
