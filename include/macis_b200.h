@@ -403,7 +403,7 @@ int macis_b200_mlp_num_params(const macis_b200_mlp* m, size_t* n);
 int macis_b200_mlp_get_params(const macis_b200_mlp* m, float* P);
 /* Sets the master weights and resets the Adam state. */
 int macis_b200_mlp_set_params(macis_b200_mlp* m, const float* P);
-/* y[i] = network(X[i]) for X [n][din]. */
+/* y[i] = network(X[i]) for X [n][din] (16-byte aligned in device memory). */
 int macis_b200_mlp_forward(macis_b200_mlp* m, const uint16_t* X, size_t n,
                            float* y, unsigned flags);
 /* Gradient of L = sum_i (y_i - t_i)^2 / (2 n) over all n rows (host grad,

@@ -502,6 +502,10 @@ int macis_b200_mlp_forward(macis_b200_mlp* m, const uint16_t* X, size_t n,
                            float* y, unsigned flags) {
   return guarded([&] {
     MB_REQUIRE(m && (n == 0 || (X && y)), MACIS_B200_EINVAL, "null argument");
+    MB_REQUIRE(!(flags & MACIS_B200_DEVICE_PTRS) ||
+                   (reinterpret_cast<uintptr_t>(X) & 15) == 0,
+               MACIS_B200_EINVAL,
+               "device network inputs must be 16-byte aligned");
     const size_t din = size_t(m->din);
     DevBuf<uint16_t> xd(X, n * din, flags, m->stream);
     DevBuf<float> yd(nullptr, (flags & MACIS_B200_DEVICE_PTRS) ? 0 : n, 0,

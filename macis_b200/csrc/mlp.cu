@@ -253,7 +253,9 @@ __global__ void rowsum_k(const float* in, int64_t ld, int64_t n, float* out) {
 
 // Minibatch rows idx[0..nvalid) of X [S][din]: xb [B][din], xbt [din][B]. A
 // block takes 32 rows x 64 columns through shared memory, so that both copies
-// and the rows themselves are read and written in runs.
+// and the rows themselves are read and written in runs. X may lie at any even
+// address: its elements are read in pairs where it is 4-byte aligned (a row is
+// a whole number of pairs).
 constexpr int GATHER_ROWS = 32, GATHER_COLS = 64;
 __global__ void __launch_bounds__(256)
     mlp_gather_k(const uint16_t* X, const float* t, const int64_t* idx,
@@ -263,11 +265,16 @@ __global__ void __launch_bounds__(256)
   __shared__ uint32_t grow[GATHER_ROWS][W + 1];
   const int64_t m0 = int64_t(blockIdx.x) * GATHER_ROWS;
   const int c0 = blockIdx.y * W;
+  const bool pairs = (reinterpret_cast<uintptr_t>(X) & 3) == 0;
   for(int q = threadIdx.x; q < GATHER_ROWS * W; q += blockDim.x) {
     const int r = q / W, c = q % W;
     const int64_t m = m0 + r;
     uint32_t v = 0;
-    if(m < nvalid) v = reinterpret_cast<const uint32_t*>(X + idx[m] * din)[c0 + c];
+    if(m < nvalid) {
+      const uint16_t* x = X + idx[m] * din + 2 * (c0 + c);
+      v = pairs ? *reinterpret_cast<const uint32_t*>(x)
+                : x[0] | uint32_t(x[1]) << 16;
+    }
     reinterpret_cast<uint32_t*>(xb + m * din)[c0 + c] = v;
     grow[r][c] = v;
   }

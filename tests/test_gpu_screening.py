@@ -276,3 +276,42 @@ def test_recall_check_keeps_exact_selections():
     # the selection is still the exact search's
     E4, d4, _ = mb.asci_iter(s, m2, 6000, E1, d1, X1, H, norb, None)
     assert np.array_equal(d3, d4) and abs(E3 - E4) < 1e-9
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 3, 7])
+def test_training_inputs_at_any_even_address(shift):
+    """Gradients and training from device inputs whose first element lies
+    `shift` elements after an aligned address: bit-equal to host inputs, which
+    are staged aligned. The forward reads 16 bytes at a time and refuses
+    other addresses."""
+    import torch
+    from macis_b200 import _lib
+    din, n = 192, 300
+    rng = np.random.default_rng(5)
+    Xb = _rand_inputs(rng, n, din, 128)
+    t = rng.normal(0, 1, n).astype(np.float32)
+    net = mb.ScreeningNetwork(din=din, seed=4)
+    P = net.params.copy()
+    g0, _ = net.gradients(Xb, t)
+    net.train(Xb, t, epochs=2, batch=128, lr=1e-3, seed=3)
+    P0 = net.params
+    buf = torch.zeros(n * din + 16, dtype=torch.int16, device="cuda")
+    x = buf[shift:shift + n * din]
+    x.copy_(torch.from_numpy(Xb.view(np.int16).reshape(-1)))
+    td = torch.from_numpy(t).cuda()
+    g = torch.zeros(len(P), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    net.params = P
+    check = _lib.check
+    check(_lib.LIB.macis_b200_mlp_gradients(
+        net.handle, x.data_ptr(), td.data_ptr(), n, g.data_ptr(), None,
+        _lib.DEVICE_PTRS))
+    assert np.array_equal(g.cpu().numpy(), g0)
+    check(_lib.LIB.macis_b200_mlp_train(
+        net.handle, x.data_ptr(), td.data_ptr(), n, 2, 128, 1e-3, 3, None,
+        _lib.DEVICE_PTRS))
+    assert np.array_equal(net.params, P0)
+    y = torch.zeros(n, dtype=torch.float32, device="cuda")
+    rc = _lib.LIB.macis_b200_mlp_forward(net.handle, x.data_ptr(), n,
+                                         y.data_ptr(), _lib.DEVICE_PTRS)
+    assert rc == (_lib.EINVAL if shift else _lib.OK)
