@@ -256,7 +256,8 @@ __device__ __forceinline__ double me_os_double(const Ints& I, uint32_t ea,
 }
 // The element of a double excitation of any class (same-spin alpha or beta,
 // opposite-spin): the same instructions for all three, so that a warp whose
-// lanes hold different classes does not run them one after another.
+// lanes hold different classes does not run them one after another. The
+// electron counts of each spin have to be equal.
 template <int NSW>
 __device__ __forceinline__ double me_double(const Ints& I, Spin<NSW> ba,
                                             Spin<NSW> bb, Spin<NSW> ka,
@@ -322,12 +323,23 @@ __device__ double me_diag(const Ints& I, Spin<NSW> a, Spin<NSW> b) {
   return h;
 }
 
-// Full matrix_element(bra, ket) dispatch (matrix_elements.hpp:22-53).
+// Whether two strings that differ in an even number of orbitals hold unequal
+// numbers of electrons: such a pair is no excitation, and the hole or particle
+// that the element functions look up does not exist.
+template <int NSW>
+__device__ __forceinline__ bool unbalanced(Spin<NSW> bra, Spin<NSW> ket) {
+  const int d = sp_popc(bra) - sp_popc(ket);
+  return d != 0 && !(d & 1);
+}
+// Full matrix_element(bra, ket) dispatch (matrix_elements.hpp:22-53). Pairs
+// whose electron counts of a spin differ by 2 or 4 have no element (the
+// reference indexes orbital -1 for them); by an odd number, the reference's
+// dispatch is kept.
 template <int NSW>
 __device__ double me_generic(const Ints& I, Spin<NSW> ba, Spin<NSW> bb,
                              Spin<NSW> ka, Spin<NSW> kb) {
   const int ca = sp_popc(ba ^ ka), cb = sp_popc(bb ^ kb);
-  if(ca + cb > 4) return 0.;
+  if(ca + cb > 4 || unbalanced(ba, ka) || unbalanced(bb, kb)) return 0.;
   if(ca == 4) return me_ss_double(I, double_ex(ba, ka));
   if(cb == 4) return me_ss_double(I, double_ex(bb, kb));
   if(ca == 2 && cb == 2) return me_os_double(I, single_ex(ba, ka), single_ex(bb, kb));

@@ -849,33 +849,44 @@ __device__ __forceinline__ void key_spins(const uint64_t* keys, size_t i,
   }
 }
 
+// What the host reads back of a sorted list.
+struct GenInfo {
+  uint32_t groups;  // alpha groups
+  uint32_t mixed;   // the nonzero determinants' electron counts differ
+  uint32_t counts;  // of the last determinant: alpha + 256 beta
+};
+
 // flags[i] = 1 at the first nonzero key of each alpha group; zero keys
-// (zero determinants, which the reference skips) get 0 and are counted.
+// (zero determinants, which the reference skips, first in the order) get 0.
+// Electron counts are compared with the last key's.
 template <int NBITS>
 __global__ void gen_group_flags_k(const uint64_t* keys, size_t n,
-                                  uint32_t* flags,
-                                  unsigned long long* nzero) {
+                                  uint32_t* flags, GenInfo* info) {
   constexpr int NSW = DetTraits<NBITS>::NSW;
-  constexpr int KW = GenKey<NBITS>::KW;
+  Spin<NSW> la, lb;
+  key_spins<NBITS>(keys, n - 1, la, lb);
+  const int na = sp_popc(la), nb = sp_popc(lb);
+  if(blockIdx.x == 0 && threadIdx.x == 0) info->counts = uint32_t(na + 256 * nb);
+  bool mixed = false;
   for(size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
       i += size_t(gridDim.x) * blockDim.x) {
     Spin<NSW> a, b;
     key_spins<NBITS>(keys, i, a, b);
-    const bool zero = sp_popc(a) + sp_popc(b) == 0;
+    const int ca = sp_popc(a), cb = sp_popc(b);
     uint32_t f = 0;
-    if(zero)
-      atomicAdd(nzero, 1ull);
-    else if(i == 0)
+    if(ca + cb != 0) {
+      mixed |= ca != na || cb != nb;
       f = 1;
-    else {
-      Spin<NSW> pa, pb;
-      key_spins<NBITS>(keys, i - 1, pa, pb);
-      const bool pzero = sp_popc(pa) + sp_popc(pb) == 0;
-      f = (pzero || !(pa == a)) ? 1 : 0;
+      if(i > 0) {
+        Spin<NSW> pa, pb;
+        key_spins<NBITS>(keys, i - 1, pa, pb);
+        const bool pzero = sp_popc(pa) + sp_popc(pb) == 0;
+        f = (pzero || !(pa == a)) ? 1 : 0;
+      }
     }
     flags[i] = f;
-    (void)KW;
   }
+  if(mixed) info->mixed = 1;
 }
 
 // Group tables: goff[g] (first sorted position), galpha[g]; sorted strings;
@@ -1072,6 +1083,7 @@ struct GenData {
   const uint64_t* bm_alpha; // per beta-major position: alpha string
   const uint32_t* bm_m;     // per beta-major position: alpha-major position
   const int32_t* mgroup;    // alpha-major position -> ket group (-1: none)
+  bool mixed;               // electron counts differ in the lists
 };
 
 // Ket groups of at least GEN_HASH_MIN members get a hash table of their
@@ -1355,7 +1367,7 @@ __device__ __forceinline__ void gen_pairs(const GenData& g, int32_t rg,
                      [&](bool act, int64_t m, int pa, int pb) {
     const unsigned any = __ballot_sync(0xffffffffu, act);
     if(!any) return;
-    const bool dbl = pa + pb == 4 && !(pa & 1);
+    const bool dbl = pa + pb == 4 && !(pa & 1) && !g.mixed;
     const unsigned md = __ballot_sync(0xffffffffu, act && dbl), mo = any & ~md;
     if(act) {
       const int at = dbl ? 64 + n1 + __popc(md & lanemask_lt())
@@ -1390,7 +1402,8 @@ __device__ __forceinline__ void gen_pairs(const GenData& g, int32_t rg,
 }
 constexpr int GEN_SCRATCH = 256 + 128 * 4;  // bytes per warp: ov, q
 
-// H(bra, ket) of a connected pair, evaluated by class.
+// H(bra, ket) of a connected pair, evaluated by class; dbl only where the
+// lists hold one electron count per spin.
 template <int NSW>
 __device__ __forceinline__ double gen_element(const Ints& I, bool dbl,
                                               Spin<NSW> ba, Spin<NSW> bb,
@@ -1564,7 +1577,7 @@ __global__ void __launch_bounds__(HB_THREADS)
         const Spin<NSW> ka = ld_spin<NSW>(g.salpha, m);
         const Spin<NSW> kb = ld_spin<NSW>(g.sbeta, m);
         const int ca = sp_popc(ba ^ ka), cb = sp_popc(bb ^ kb);
-        if(ca + cb == 4 && !(ca & 1))
+        if(ca + cb == 4 && !(ca & 1) && !g.mixed)
           put(i, uint32_t(key >> 32), me_double(I, ba, bb, ka, kb));
         else
           put_off = true;
@@ -1676,8 +1689,7 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
   constexpr int KW = GenKey<NBITS>::KW;
   auto sort_side = [&](const uint64_t* dets, size_t n, uint64_t*& keys,
                        uint32_t*& idx, int64_t*& goff, uint64_t*& galpha,
-                       uint64_t*& salpha, uint64_t*& sbeta, int32_t* rowgroup,
-                       uint32_t& ng) {
+                       uint64_t*& salpha, uint64_t*& sbeta, int32_t* rowgroup) {
     keys = A.get<uint64_t>(n * KW);
     idx = A.get<uint32_t>(n);
     uint64_t* k2 = A.get<uint64_t>(n * KW);
@@ -1688,13 +1700,14 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     A.release(k2);
     A.release(i2);
     uint32_t* flags = A.get<uint32_t>(n);
-    uint32_t* gx = A.get<uint32_t>(n + 1);
-    auto* nz = A.get<unsigned long long>(1);
-    MB_CUDA(cudaMemsetAsync(nz, 0, 8, s));
+    uint32_t* gx = A.get<uint32_t>(n);
+    auto* d_info = A.get<GenInfo>(1);
+    MB_CUDA(cudaMemsetAsync(d_info, 0, sizeof(GenInfo), s));
     gen_group_flags_k<NBITS><<<grid_for(n, 256, 8 * sms), 256, 0, s>>>(
-        keys, n, flags, nz), note_launch();
-    exclusive_scan<uint32_t, uint32_t>(flags, gx, n, gx + n, A);
-    ng = to_host(gx + n, s);
+        keys, n, flags, d_info), note_launch();
+    exclusive_scan<uint32_t, uint32_t>(flags, gx, n, &d_info->groups, A);
+    const GenInfo info = to_host(d_info, s);
+    const uint32_t ng = info.groups;
     goff = A.get<int64_t>(ng + 1);
     galpha = A.get<uint64_t>((ng + 1) * NSW);
     salpha = A.get<uint64_t>(n * NSW);
@@ -1706,13 +1719,16 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     A.release(flags);
     A.release(gx);
     gen_group_end_k<<<1, 1, 0, s>>>(goff, ng, int64_t(n)), note_launch();
+    return info;
   };
   uint64_t *kkeys, *kalpha, *ksalpha, *ksbeta;
-  uint32_t *kidx, nkg = 0;
+  uint32_t* kidx;
   int64_t* kgoff;
   int32_t* rowgroup = A.get<int32_t>(sub ? nket : nbra);
-  sort_side(ket, nket, kkeys, kidx, kgoff, kalpha, ksalpha, ksbeta,
-            sub ? rowgroup : nullptr, nkg);
+  const GenInfo ki = sort_side(ket, nket, kkeys, kidx, kgoff, kalpha, ksalpha,
+                               ksbeta, sub ? rowgroup : nullptr);
+  const uint32_t nkg = ki.groups;
+  bool mixed = ki.mixed;
   if(sub) rowgroup += r0;
   const uint64_t* balpha = kalpha;
   uint32_t nbg = nkg;
@@ -1720,8 +1736,10 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     uint64_t *bkeys, *bsalpha, *bsbeta, *bal;
     uint32_t* bidx;
     int64_t* bgoff;
-    sort_side(bra, nbra, bkeys, bidx, bgoff, bal, bsalpha, bsbeta, rowgroup,
-              nbg);
+    const GenInfo bi = sort_side(bra, nbra, bkeys, bidx, bgoff, bal, bsalpha,
+                                 bsbeta, rowgroup);
+    nbg = bi.groups;
+    mixed = mixed || bi.mixed || bi.counts != ki.counts;
     A.release(bsalpha);
     A.release(bsbeta);
     balpha = bal;
@@ -1799,7 +1817,7 @@ static GenData gen_plan(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
   }
   GenData gd{rowgroup, aoff, acol, apa, kgoff, ksalpha, ksbeta, kidx,
              hoff, htab, gbpop, h->norb, acnt4,
-             bgbeta, bgoff, nbgb, bm_alpha, bm_m, mgroup};
+             bgbeta, bgoff, nbgb, bm_alpha, bm_m, mgroup, mixed};
   return gd;
 }
 
@@ -2379,15 +2397,18 @@ struct RdmSums {
   double* dos;    // n^2: p occupied in alpha, q in beta
 };
 
-// One pair with at least two determinants apart by an even count, in the
-// reference's dispatch (:15-66); pairs of the diagonal branch return true.
+// One pair in the reference's dispatch (:15-66); pairs of the diagonal branch
+// return true. mixed: the list holds several electron counts; pairs that
+// differ by 2 or 4 electrons of a spin contribute nothing.
 template <int NSW>
 __device__ __forceinline__ bool rdm_pair(Spin<NSW> ba, Spin<NSW> bb,
                                          Spin<NSW> ka, Spin<NSW> kb,
-                                         double val, int n, double* ordm,
-                                         bool two, const RdmSums& S) {
+                                         bool mixed, double val, int n,
+                                         double* ordm, bool two,
+                                         const RdmSums& S) {
   const int ca = sp_popc(ba ^ ka), cb = sp_popc(bb ^ kb);
   if(ca + cb > 4) return false;
+  if(mixed && (unbalanced(ba, ka) || unbalanced(bb, kb))) return false;
   auto at = [n](int p, int q, int r) { return size_t(p) + size_t(n) * (q + size_t(n) * r); };
   if((ca == 4 || cb == 4) && two) {  // rdm_contributions_4, :15-25
     const uint32_t e = ca == 4 ? double_ex(ba, ka) : double_ex(bb, kb);
@@ -2448,7 +2469,8 @@ __global__ void __launch_bounds__(HB_THREADS)
         const double val = ci * C[g.sidx[m]];
         if(!(fabs(val) > 1e-16)) return;
         if(rdm_pair<NSW>(ba, bb, ld_spin<NSW>(g.salpha, m),
-                         ld_spin<NSW>(g.sbeta, m), val, norb, ordm, two != 0, S))
+                         ld_spin<NSW>(g.sbeta, m), g.mixed, val, norb, ordm,
+                         two != 0, S))
           dsum += val;
       });
 #pragma unroll

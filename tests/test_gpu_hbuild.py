@@ -244,3 +244,52 @@ def test_product_layout_with_many_orbitals_takes_general_path(ref):
     assert_csr_equal(A.to_host(), ref.build_csr(ref.ham(128, n, T, V), dets,
                                                 dets, np.finfo(float).eps,
                                                 nthreads=8))
+
+
+@pytest.mark.parametrize("nbits", [64, 128, 256])
+@pytest.mark.parametrize("da,db", [(2, 0), (0, 2), (2, -2), (4, 0)])
+def test_lists_of_two_electron_counts(nbits, da, db):
+    """Determinants whose counts of a spin differ by 2 or 4 do not interact
+    (no hole or no particle to look up): H of a list of two such counts is the
+    two pure lists' H side by side, stored, matrix-free and by element, and
+    its density matrices are their sums. Products of at most 500 terms of
+    order 1: 1e-11; elements exactly."""
+    rng = np.random.default_rng(7)
+    n = 6
+    T, V, d0 = fci(n, 1, 3, nbits, seed=6)
+    d1 = fci(n, 1 + da, 3 + db, nbits, seed=6)[2]
+    H = mb.HamiltonianGenerator(T, V, nbits)
+    both = np.concatenate([d0, d1])
+    N, n0 = len(both), len(d0)
+    M = np.zeros((N, N))
+    for d, o in ((d0, 0), (d1, n0)):
+        rp, ci, nz = mb.make_csr_hamiltonian(d, H, 0.0).to_host()
+        for i in range(len(d)):
+            M[o + i, o + ci[rp[i]:rp[i + 1]]] = nz[rp[i]:rp[i + 1]]
+    p = rng.permutation(N)
+    d, M = both[p], M[np.ix_(p, p)]
+    A = mb.make_csr_hamiltonian(d, H, 0.0)
+    assert A.build_stats()["direct_product"] == 0
+
+    def dense(A):
+        rp, ci, nz = A.to_host()
+        D = np.zeros((A.m, A.n))
+        for i in range(A.m):
+            D[i, ci[rp[i]:rp[i + 1]]] = nz[rp[i]:rp[i + 1]]
+        return D
+    assert np.array_equal(dense(A), M)
+    # rows of the one count, columns of the other
+    assert mb.make_csr_hamiltonian_block(d0, d1, H, 0.0).nnz == 0
+    k = rng.integers(0, N, (2, 2000))
+    assert np.array_equal(H.matrix_element(d[k[0]], d[k[1]]), M[k[0], k[1]])
+    x = rng.standard_normal(N)
+    np.testing.assert_allclose(mb.MatrixFreeHamiltonian(d, H, 0.0).spmv(x),
+                               M @ x, rtol=0, atol=1e-11)
+    c = rng.standard_normal(N) / np.sqrt(N)
+    q = np.argsort(p)                       # positions of d0, d1 in d
+    for two in (True, False):
+        got = H.form_rdms(d, c, two=two)
+        a, b = (H.form_rdms(dd, c[q[s]], two=two) for dd, s in
+                ((d0, slice(0, n0)), (d1, slice(n0, N))))
+        for g, u, v in list(zip(got, a, b))[:2 if two else 1]:
+            np.testing.assert_allclose(g, u + v, rtol=0, atol=1e-11)
