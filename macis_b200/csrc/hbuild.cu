@@ -2231,7 +2231,7 @@ struct macis_b200_hop {
   uint64_t* dets = nullptr;  // device copy of the determinant list
   double* diag = nullptr;    // H_ii
   mb::Arena* A = nullptr;    // owns dets, diag and the enumeration tables
-  unsigned* ctr = nullptr;   // row counter of a product
+  unsigned* ctr = nullptr;   // next row and finished blocks of a product
   mb::GenData g{};
 };
 
@@ -2241,6 +2241,9 @@ namespace mb {
 // build's enumeration (gen_enumerate), each element evaluated, thresholded
 // as in the build and accumulated into the row sum (no storage). mixed:
 // off-diagonal elements rounded to FP32 first, as in an FP32-valued CSR.
+// ctr: {next row, finished blocks}, both 0 before and after: the last block
+// clears them, so that a product is one stream operation and two that are
+// enqueued at once by several host threads follow one another.
 template <int NBITS>
 __global__ void __launch_bounds__(HB_THREADS)
     gen_apply_k(Ints I, GenData g, const uint64_t* dets, int64_t n,
@@ -2277,6 +2280,11 @@ __global__ void __launch_bounds__(HB_THREADS)
     }
     if(lane == 0) y[row] = alpha * acc + (beta != 0.0 ? beta * y[row] : 0.0);
   }
+  __syncthreads();  // this block takes no more rows
+  if(threadIdx.x == 0 && atomicAdd(ctr + 1, 1u) == gridDim.x - 1) {
+    ctr[0] = 0;
+    ctr[1] = 0;
+  }
 }
 
 macis_b200_hop* hop_create(macis_b200_ham* h, const uint64_t* dets, size_t n,
@@ -2307,7 +2315,8 @@ macis_b200_hop* hop_create(macis_b200_ham* h, const uint64_t* dets, size_t n,
                             device_ptrs ? cudaMemcpyDeviceToDevice
                                         : cudaMemcpyHostToDevice, s));
     op->diag = op->A->get<double>(n);
-    op->ctr = op->A->get<unsigned>(1);
+    op->ctr = op->A->get<unsigned>(2);
+    MB_CUDA(cudaMemsetAsync(op->ctr, 0, 2 * sizeof(unsigned), s));
 #define MB_HOP_PLAN(NB)                                                     \
   hdiag_k<NB><<<grid_for(n, 256, 8 * sms), 256, 0, s>>>(I, op->dets, n,     \
                                                         op->diag),          \
@@ -2338,7 +2347,6 @@ void hop_apply(const macis_b200_hop* op, double alpha, const double* x,
   cudaStream_t s = op->stream;
   const unsigned gr = grid_for(size_t(op->n), HB_WARPS, size_t(num_sms()) * 16);
   const Ints I = op->I;
-  MB_CUDA(cudaMemsetAsync(op->ctr, 0, sizeof(unsigned), s));
 #define MB_HOP_APPLY(NB)                                                     \
   gen_apply_k<NB><<<gr, HB_THREADS, 0, s>>>(I, op->g, op->dets, op->n,       \
                                             op->diag, op->thresh,            \

@@ -124,3 +124,38 @@ def test_selected_ci_diag_matrix_free_and_fallback(monkeypatch):
     assert abs(E2 - E0) < 1e-9 and t["nnz"] is None
     with pytest.raises(_lib.MacisError):
         mb.selected_ci_diag(sel, H, EPS, 80, 1e-8, matrix_free=False)
+
+
+def test_products_from_several_threads():
+    """One operator applied by four host threads at once: every product is
+    whole. The output is filled before each call, so that one which does
+    nothing shows. Sums of 1,500 terms of order 1 in a varying order: 1e-11."""
+    import threading
+    import torch
+    from macis_b200 import _lib
+    T, V, sel = _selected(64, seed=8)
+    H = mb.HamiltonianGenerator(T, V, 64)
+    Hm = mb.MatrixFreeHamiltonian(sel, H, EPS)
+    n, bad, go = Hm.m, [], threading.Barrier(4)
+    x = [torch.randn(n, dtype=torch.float64, device="cuda") for _ in range(4)]
+    ref = [torch.from_numpy(Hm.spmv(v.cpu().numpy())).cuda() for v in x]
+    ys = [torch.full((200, n), 1e3, dtype=torch.float64, device="cuda")
+          for _ in range(4)]
+    torch.cuda.synchronize()
+
+    def work(t):
+        go.wait()
+        for k in range(200):
+            rc = _lib.LIB.macis_b200_hop_apply(
+                Hm.handle, 1, 1.0, x[t].data_ptr(), n, 0.0,
+                ys[t][k].data_ptr(), n, _lib.DEVICE_PTRS)
+            if rc:
+                bad.append(rc)
+    th = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not bad
+    for t in range(4):
+        assert float((ys[t] - ref[t]).abs().max()) < 1e-11
