@@ -391,6 +391,13 @@ int macis_b200_asci_pairs(macis_b200_ham* h, const macis_b200_asci_settings* s,
                           size_t* npairs);
 int macis_b200_asci_last_stats(const macis_b200_ham* h,
                                macis_b200_asci_stats* out);
+/* Contributions that one candidate range of a search may hold when
+ * avail_bytes of device memory can be had: nbits of the determinants, whether
+ * the records carry number keys, the search's raw contributions, the wanted
+ * and the core determinants. Host-only arithmetic; needs no GPU. */
+int64_t macis_b200_asci_range_records(double avail_bytes, int nbits,
+                                      int numbered, uint64_t raw_pairs,
+                                      uint64_t ndets_max, uint64_t ncdets);
 
 /* --- Learned screening network (no MACIS counterpart) ---------------------
  * din -> 256 -> 256 -> 1 with GELU, BF16 tcgen05 GEMMs with FP32

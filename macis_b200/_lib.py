@@ -133,6 +133,8 @@ _SIGS = {
     "macis_b200_mlp_samples": (C.c_int, [_vp, C.POINTER(_sz), _vp, _vp]),
     "macis_b200_mlp_clamp_samples": (C.c_int, [_vp, C.c_double,
                                                C.POINTER(C.c_float)]),
+    "macis_b200_asci_range_records": (C.c_int64, [
+        C.c_double, C.c_int, C.c_int, C.c_uint64, C.c_uint64, C.c_uint64]),
     "macis_b200_asci_unit_width": (C.c_int, [C.c_int]),
     "macis_b200_asci_search_screened": (C.c_int, [
         _vp, C.POINTER(AsciSettingsC), C.POINTER(AsciScreenC), _sz, _vp, _sz,

@@ -1480,6 +1480,38 @@ __global__ void iota_k(uint32_t* x, size_t n) {
 // ----------------------------------------------------------------- driver
 // A range's score threshold is sampled from one part in GROUP_SAMPLE of it.
 constexpr size_t GROUP_SAMPLE = 32;
+// Records of a range: their positions are 32-bit.
+constexpr int64_t ASCI_MAX_RECORDS = (int64_t(1) << 32) - 1;
+
+// Bytes per contribution of a range while it is grouped: the record (its
+// determinant or number key, and the score), its copy and the digit counts of
+// the partition.
+static double asci_record_bytes(int nbits, bool numbered) {
+  return 2.0 * (numbered ? 16.0 : nbits / 8 + 8.0) + 2.0;
+}
+
+// Contributions that a range may hold: the largest n with
+//   n records + c candidates + the running top-k with its copies
+// inside 0.8 of the available memory. The candidates are what a range leaves
+// above its sampled threshold, as determinants with their flags and kept
+// copy: about GROUP_SAMPLE times the wanted ones (counted twice), but never
+// more than the range's records, so a search for very many determinants gets
+// smaller ranges and not ranges of the least size (a reserve of 128 GB for
+// the candidates of the whole search, at 3.4e7 wanted determinants, left
+// ranges of 2^20 contributions).
+int64_t asci_range_records(double avail, int nbits, bool numbered,
+                           uint64_t raw, size_t ndets_max, size_t ncdets) {
+  const double cand = nbits / 8 + 8.0;  // a candidate: determinant and score
+  const double per_pair = asci_record_bytes(nbits, numbered);
+  const double per_cand = 2.0 * cand + 16.0;
+  const size_t topk = ndets_max - ncdets;
+  const double most = 2.0 * GROUP_SAMPLE * (double(topk) + double(ncdets));
+  const double left =
+      0.8 * avail - 6.0 * cand * double(std::min<uint64_t>(topk, raw));
+  double n = left / (per_pair + per_cand);
+  if(n > most) n = (left - per_cand * most) / per_pair;
+  return int64_t(std::min(std::max(n, 1048576.0), double(ASCI_MAX_RECORDS)));
+}
 
 namespace {
 struct Pairs {
@@ -1933,33 +1965,18 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
       stats.rank_ms = ms_since(t_rk);
     }
   }
-  // bytes of a record, and of a candidate with its determinant
-  const double rs = ranked ? 16.0 : double(NW * 8 + 8);
-  const double rf = double(NW * 8 + 8);
-  // per raw contribution while a range is processed: the record, its copy
-  // and the digit counts of the partition
-  const double per_pair = 2.0 * rs + 2.0;
   const size_t topk = ndets_max - ncdets;   // size_t arithmetic (:547)
-  // the running top-k with its copies, and the candidates a range leaves
-  // above its sampled threshold (about GROUP_SAMPLE times the wanted ones)
-  // as determinants with their flags and kept copy
-  const double keep_reserve =
-      6.0 * rf * double(std::min<uint64_t>(topk, uint64_t(Ptot))) +
-      (2.0 * rf + 16.0) *
-          std::min(2.0 * GROUP_SAMPLE * (double(topk) + double(ncdets)),
-                   double(Ptot));
+  const double avail = double(device_bytes_available());
+  auto plan_cap = [&](double bytes) {
+    return asci_range_records(bytes, NBITS, ranked, uint64_t(Ptot), ndets_max,
+                              ncdets);
+  };
   // MACIS_B200_ASCI_BATCH_PAIRS caps the raw pairs per range (exercises the
   // partitioned path on small problems).
-  int64_t cap = 0;
   const char* cap_env = getenv("MACIS_B200_ASCI_BATCH_PAIRS");
-  if(const char* e = cap_env) {
-    cap = std::max<int64_t>(1, atoll(e));
-  } else {
-    cap = int64_t((0.8 * double(device_bytes_available()) - keep_reserve) /
-                  per_pair);
-    cap = std::min<int64_t>(std::max<int64_t>(cap, int64_t(1) << 20),
-                            (int64_t(1) << 32) - 1);
-  }
+  int64_t cap = cap_env ? std::min(std::max<int64_t>(1, atoll(cap_env)),
+                                   ASCI_MAX_RECORDS)
+                        : plan_cap(avail);
   // ranges: consecutive alpha-string bins packed up to the cap from the
   // measured bin loads (a single bin above the cap is a range of its own)
   // (a bin above the cap is split into beta-hash classes)
@@ -2035,8 +2052,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
         nlist = std::min<size_t>(ap.nu, size_t(budget / per_list));
         if(al_max > 0) nlist = std::min<size_t>(nlist, size_t(al_max));
         const double bytes = fixed + double(nlist) * per_list;
-        if(!cap_env)
-          cap = std::max<int64_t>(cap - int64_t(bytes / per_pair), int64_t(1) << 20);
+        if(!cap_env) cap = plan_cap(avail - bytes / 0.8);
       }
     }
   }

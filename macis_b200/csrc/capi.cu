@@ -442,6 +442,13 @@ int macis_b200_asci_last_stats(const macis_b200_ham* h,
   });
 }
 
+int64_t macis_b200_asci_range_records(double avail_bytes, int nbits,
+                                      int numbered, uint64_t raw_pairs,
+                                      uint64_t ndets_max, uint64_t ncdets) {
+  return asci_range_records(avail_bytes, nbits, numbered != 0, raw_pairs,
+                            ndets_max, ncdets);
+}
+
 int macis_b200_asci_unit_width(int nbits) { return asci_unit_din(nbits); }
 
 int macis_b200_asci_unit_features(macis_b200_ham* h, const uint64_t* cdets,

@@ -239,6 +239,9 @@ int64_t asci_unit_features_device(macis_b200_ham* h, const uint64_t* cdets,
                                   size_t ncdets, double E0, const double* C,
                                   size_t first, size_t n, uint16_t* X);
 int asci_unit_din(int nbits);
+// Contributions that one candidate range of a search may hold (host only).
+int64_t asci_range_records(double avail, int nbits, bool numbered,
+                           uint64_t raw, size_t ndets_max, size_t ncdets);
 
 void set_error(const std::string& s);
 

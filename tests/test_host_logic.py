@@ -275,3 +275,32 @@ def test_merge_asci_parts_topk_rules():
         merge_asci_parts(parts, 1, core, 64)    # 1 - 2 wraps: nothing cut
     empty = [(np.zeros((0, 1), dtype=np.uint64), np.zeros(0))]
     assert merge_asci_parts(empty, 1, core, 64)[:, 0].tolist() == [200, 100]
+
+
+@pytest.mark.parametrize("nbits,numbered", [(64, 0), (128, 0), (128, 1),
+                                            (256, 0), (256, 1)])
+def test_search_range_plan(nbits, numbered):
+    """Candidate ranges are the largest whose records, candidates and running
+    top-k fit 0.8 of the memory, whatever number of determinants is wanted:
+    a range leaves no more candidates than it has records, so a search for
+    very many determinants does not fall back to ranges of the least size."""
+    plan = _lib.LIB.macis_b200_asci_range_records
+    cand = nbits // 8 + 8
+    rec = 2 * (16 if numbered else cand) + 2
+    for avail in (8e9, 170e9):
+        for raw in (10 ** 6, 2 * 10 ** 9, 27 * 10 ** 9):
+            for ncore in (100, 10 ** 5):
+                for top in (10 ** 4, 10 ** 6, 3 * 10 ** 7, 10 ** 8):
+                    n = plan(avail, nbits, numbered, raw, ncore + top, ncore)
+                    left = 0.8 * avail - 6 * cand * min(top, raw)
+                    need = lambda m: m * rec + (2 * cand + 16) * min(
+                        64 * (top + ncore), m)
+                    assert 1 << 20 <= n < 1 << 32
+                    if n > 1 << 20:
+                        assert need(n) <= left
+                    if n < (1 << 32) - 1:
+                        assert need(n + 2) > left
+    # a grow of 3.4e7 determinants from 1e5 core determinants
+    assert plan(170e9, 128, 1, 27 * 10 ** 9, 34 * 10 ** 6, 10 ** 5) > 10 ** 9
+    # no wanted determinants (the accumulated list): a plan all the same
+    assert plan(170e9, nbits, numbered, 10 ** 6, 0, 10) >= 1 << 20
