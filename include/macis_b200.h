@@ -131,11 +131,15 @@ int macis_b200_set_wait_limit_ns(uint64_t ns);
  * allocations by the library, the next one reports out-of-memory
  * (MACIS_B200_ENOMEM), once. MACIS_B200_FAULT_INT32_LIMIT: CSR builds with
  * int32 indices reject more than `arg` nonzeros (MACIS_B200_ECAPACITY).
- * MACIS_B200_FAULT_NONE clears both. Process-wide; nothing fails on the
+ * MACIS_B200_FAULT_LIST_LIMIT: CSR builds of selected lists keep at most
+ * `arg` listed candidates and enumerate the rows beyond them again (what they
+ * do when memory is short; the matrix is the same).
+ * MACIS_B200_FAULT_NONE clears all. Process-wide; nothing fails on the
  * device. */
 #define MACIS_B200_FAULT_NONE 0
 #define MACIS_B200_FAULT_ALLOC 1
 #define MACIS_B200_FAULT_INT32_LIMIT 2
+#define MACIS_B200_FAULT_LIST_LIMIT 3
 int macis_b200_inject_fault(int kind, int64_t arg);
 
 /* --- Hamiltonian generator ------------------------------------------------

@@ -173,6 +173,7 @@ int macis_b200_inject_fault(int kind, int64_t arg) {
       case MACIS_B200_FAULT_NONE:
         faults().alloc_countdown.store(-1);
         faults().int32_limit.store(INT32_MAX);
+        faults().list_limit.store(INT64_MAX);
         break;
       case MACIS_B200_FAULT_ALLOC:
         MB_REQUIRE(arg >= 0, MACIS_B200_EINVAL, "allocation count must be >= 0");
@@ -182,6 +183,10 @@ int macis_b200_inject_fault(int kind, int64_t arg) {
         MB_REQUIRE(arg >= 0 && arg <= INT32_MAX, MACIS_B200_EINVAL,
                    "int32 limit must be in [0, 2^31 - 1]");
         faults().int32_limit.store(arg);
+        break;
+      case MACIS_B200_FAULT_LIST_LIMIT:
+        MB_REQUIRE(arg >= 0, MACIS_B200_EINVAL, "list limit must be >= 0");
+        faults().list_limit.store(arg);
         break;
       default:
         MB_REQUIRE(false, MACIS_B200_EINVAL, "unknown fault kind");

@@ -2024,8 +2024,9 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     unsigned* ctr = A.get<unsigned>(1);
     auto* used = A.get<unsigned long long>(1);
     int64_t* list_off = A.get<int64_t>(nbra);
-    const uint64_t cap = std::min<uint64_t>(uint64_t(nbra) * GEN_CAP,
-                                            uint64_t(device_bytes_available() / 40));
+    const uint64_t cap = std::min<uint64_t>(
+        {uint64_t(nbra) * GEN_CAP, uint64_t(device_bytes_available() / 40),
+         candidate_list_limit()});
     uint32_t* list = A.get<uint32_t>(cap);
     MB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), s));
     MB_CUDA(cudaMemsetAsync(used, 0, 8, s));
@@ -2038,6 +2039,7 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     if(1.05 * double(nnz_ub) * (sizeof(CI) + sizeof(VT)) + 1073741824.0 >
        double(device_bytes_available())) {
       A.release(list);
+      list = nullptr;
       MB_CUDA(cudaMemsetAsync(list_off, 0xFF, nbra * 8, s));
     }
     out->nnz_candidates = nnz_ub;
@@ -2119,6 +2121,9 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     } while(row_a < int64_t(nbra));
     out->fill_ms = fill_ms_tot;
     general_fill_timed = true;
+    // the compaction below takes a second copy of the matrix: nothing of the
+    // candidates is held beside it
+    if(list) A.release(list);
   }
 
   // ------------------------------------------- exact row pointer + compaction

@@ -293,3 +293,67 @@ def test_lists_of_two_electron_counts(nbits, da, db):
                 ((d0, slice(0, n0)), (d1, slice(n0, N))))
         for g, u, v in list(zip(got, a, b))[:2 if two else 1]:
             np.testing.assert_allclose(g, u + v, rtol=0, atol=1e-11)
+
+
+def _peak_pool_bytes(f):
+    """Most device memory that the library's pool held while f() ran, beyond
+    what it held before."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    attr = rt.cudaMemPoolAttr
+    _, pool = rt.cudaDeviceGetDefaultMemPool(0)
+
+    def get(a):
+        err, v = rt.cudaMemPoolGetAttribute(pool, a)
+        assert int(err) == 0
+        return int(v)
+    base = get(attr.cudaMemPoolAttrUsedMemCurrent)
+    from cuda.bindings import driver
+    (err,) = rt.cudaMemPoolSetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh,
+                                        driver.cuuint64_t(0))
+    assert int(err) == 0
+    f()
+    return get(attr.cudaMemPoolAttrUsedMemHigh) - base
+
+
+def test_compaction_does_not_hold_the_candidate_lists():
+    """A build that drops elements takes a second copy of the matrix to close
+    the gaps. The rows' candidate lists (4 KB a row: the larger part here) are
+    given back by then, so that the build needs no more memory than one that
+    drops nothing. 2 MB for what the pool rounds up."""
+    T, V, d = fci(10, 5, 5, 64, seed=2)
+    sel = shuffled(d, seed=6, frac=0.3)
+    H = mb.HamiltonianGenerator(T, V, 64)
+    vals = np.abs(mb.make_csr_hamiltonian(sel, H, 0.0).to_host()[2])
+    A = []
+    whole = _peak_pool_bytes(
+        lambda: A.append(mb.make_csr_hamiltonian(sel, H, -1.0)))
+    nnz = A.pop().nnz
+    thr = float(np.sort(vals)[len(vals) // 100])
+    cut = _peak_pool_bytes(
+        lambda: A.append(mb.make_csr_hamiltonian(sel, H, thr)))
+    assert 0.9 * nnz < A.pop().nnz < nnz
+    assert 12 * nnz < 4096 * len(sel) and cut <= whole + (2 << 20)
+
+
+@pytest.mark.parametrize("limit", [0, 5000, 200000])
+def test_rows_without_candidate_lists(limit):
+    """Rows whose candidates are not listed (memory too short for the lists)
+    are enumerated again by the fill: the same matrix, with elements dropped
+    and not, with duplicates and long rows."""
+    from macis_b200 import _lib
+    T, V, d = fci(8, 4, 4, 64, seed=11)
+    sel = shuffled(d, seed=3, frac=0.4)
+    sel = np.concatenate([sel, sel[:300]])
+    H = mb.HamiltonianGenerator(T, V, 64)
+    lists = (sel, shuffled(np.concatenate([d, d, d]), seed=3))
+    want = [mb.make_csr_hamiltonian(s, H, t).to_host() for s in lists
+            for t in (0.0, 1e-3)]
+    try:
+        _lib.check(_lib.LIB.macis_b200_inject_fault(_lib.FAULT_LIST_LIMIT,
+                                                    limit))
+        got = [mb.make_csr_hamiltonian(s, H, t).to_host() for s in lists
+               for t in (0.0, 1e-3)]
+    finally:
+        _lib.check(_lib.LIB.macis_b200_inject_fault(_lib.FAULT_NONE, 0))
+    for g, w in zip(got, want):
+        assert_csr_equal(g, w)
