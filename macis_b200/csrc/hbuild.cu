@@ -1901,6 +1901,7 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
   }
 
   int64_t nnz_ub = 0;
+  // the matrix is the arena's until the build has succeeded
   CI* colind = nullptr;
   VT* nzval = nullptr;
   // direct product: connectivity counts and row sizes, read back together
@@ -1935,8 +1936,8 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     out->direct_product = true;
     nnz_ub = tot.nnz;
     out->nnz_candidates = nnz_ub;
-    MB_CUDA(dev_malloc_async(&colind, std::max<int64_t>(nnz_ub, 1) * sizeof(CI), s));
-    MB_CUDA(dev_malloc_async(&nzval, std::max<int64_t>(nnz_ub, 1) * sizeof(VT), s));
+    colind = A.get<CI>(size_t(nnz_ub));
+    nzval = A.get<VT>(size_t(nnz_ub));
     // orbital lists of the kernels below hold 128 entries per spin
     MB_REQUIRE(nket < (size_t(1) << 31) && h->norb <= 127,
                MACIS_B200_ECAPACITY,
@@ -2043,8 +2044,8 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
       MB_CUDA(cudaMemsetAsync(list_off, 0xFF, nbra * 8, s));
     }
     out->nnz_candidates = nnz_ub;
-    MB_CUDA(dev_malloc_async(&colind, std::max<int64_t>(nnz_ub, 1) * sizeof(CI), s));
-    MB_CUDA(dev_malloc_async(&nzval, std::max<int64_t>(nnz_ub, 1) * sizeof(VT), s));
+    colind = A.get<CI>(size_t(nnz_ub));
+    nzval = A.get<VT>(size_t(nnz_ub));
     // long rows
     uint32_t* lf = A.get<uint32_t>(nbra + 1);
     uint32_t* lpos = A.get<uint32_t>(nbra + 1);
@@ -2140,20 +2141,20 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     MB_REQUIRE(nnz <= int32_index_limit(), MACIS_B200_ECAPACITY,
                "nnz exceeds the int32 index range; use 64-bit indices");
   if(nnz != nnz_ub) {
-    CI* ci2 = nullptr;
-    VT* nz2 = nullptr;
-    MB_CUDA(dev_malloc_async(&ci2, std::max<int64_t>(nnz, 1) * sizeof(CI), s));
-    MB_CUDA(dev_malloc_async(&nz2, std::max<int64_t>(nnz, 1) * sizeof(VT), s));
+    CI* ci2 = A.get<CI>(size_t(nnz));
+    VT* nz2 = A.get<VT>(size_t(nnz));
     compact_marked_k<CI, VT><<<grid_for(nbra * 32, 256, 16 * sms), 256, 0, s>>>(
         rowptr64, newptr, nbra, colind, nzval, ci2, nz2), note_launch();
-    cudaFreeAsync(colind, s);
-    cudaFreeAsync(nzval, s);
+    A.release(colind);
+    A.release(nzval);
     colind = ci2;
     nzval = nz2;
   }
   MB_CUDA(dev_malloc_async(&out->rowptr, (nbra + 1) * sizeof(CI), s));
   rowptr_cast_k<CI><<<grid_for(nbra + 1, 256, 8 * sms), 256, 0, s>>>(
       newptr, nbra + 1, static_cast<CI*>(out->rowptr)), note_launch();
+  A.keep(colind);
+  A.keep(nzval);
   out->colind = colind;
   out->nzval = nzval;
   MB_CUDA(cudaGetLastError());

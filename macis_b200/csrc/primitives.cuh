@@ -53,6 +53,11 @@ struct Arena {
         q = nullptr;
       }
   }
+  // p outlives the arena (freed by its new owner).
+  void keep(void* p) {
+    for(auto& q : ptrs)
+      if(q == p) q = nullptr;
+  }
   ~Arena() {
     for(void* p : ptrs)
       if(p) cudaFreeAsync(p, s);

@@ -153,3 +153,34 @@ def test_injected_int32_capacity(faults):
                                 **dav)
     assert abs(E1 - E0) < 1e-9 and t["nnz"] == A.nnz
     assert H._int64_from_ndets == len(d)
+
+
+@pytest.mark.parametrize("product", [True, False])
+def test_failed_builds_give_their_memory_back(faults, product):
+    """A build that ends with ECAPACITY or, at any of its allocations, with
+    ENOMEM holds nothing afterwards: the matrix part that it had is there for
+    the 64-bit build or the matrix-free operator that follows."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    _, pool = rt.cudaDeviceGetDefaultMemPool(0)
+    used = lambda: int(rt.cudaMemPoolGetAttribute(
+        pool, rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent)[1])
+    T, V, d = fci(8, 4, 4, 64, seed=5)
+    if not product:
+        d = shuffled(d, seed=2, frac=0.6).copy()
+    H = mb.HamiltonianGenerator(T, V, 64)
+    nnz = mb.make_csr_hamiltonian(d, H, 1e-3).nnz   # elements are dropped
+    base = used()
+    faults(_lib.FAULT_INT32_LIMIT, nnz - 1)
+    with pytest.raises(mb.MacisError) as e:
+        mb.make_csr_hamiltonian(d, H, 1e-3)
+    assert e.value.code == _lib.ECAPACITY and used() == base
+    faults(_lib.FAULT_NONE)
+    for k in range(400):
+        faults(_lib.FAULT_ALLOC, k)
+        try:
+            A = mb.make_csr_hamiltonian(d, H, 1e-3)
+        except mb.MacisError as e:
+            assert e.code == _lib.ENOMEM and used() == base, k
+        else:
+            break
+    assert 10 < k < 399 and A.nnz == nnz
