@@ -134,12 +134,16 @@ int macis_b200_set_wait_limit_ns(uint64_t ns);
  * MACIS_B200_FAULT_LIST_LIMIT: CSR builds of selected lists keep at most
  * `arg` listed candidates and enumerate the rows beyond them again (what they
  * do when memory is short; the matrix is the same).
+ * MACIS_B200_FAULT_RECORD_LIMIT: candidate ranges and accumulated lists of
+ * the search hold at most `arg` contributions (2^32 - 1 by default; a longer
+ * list is MACIS_B200_ECAPACITY, a longer search takes more ranges).
  * MACIS_B200_FAULT_NONE clears all. Process-wide; nothing fails on the
  * device. */
 #define MACIS_B200_FAULT_NONE 0
 #define MACIS_B200_FAULT_ALLOC 1
 #define MACIS_B200_FAULT_INT32_LIMIT 2
 #define MACIS_B200_FAULT_LIST_LIMIT 3
+#define MACIS_B200_FAULT_RECORD_LIMIT 4
 int macis_b200_inject_fault(int kind, int64_t arg);
 
 /* --- Hamiltonian generator ------------------------------------------------

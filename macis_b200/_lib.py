@@ -12,7 +12,8 @@ LIB_PATH = os.path.join(HERE, "libmacis_b200.so")
 
 OK, EINVAL, ENOMEM, ECAPACITY, ETIMEOUT, ENOCONV, ECUDA, ENOGROW = range(8)
 DEVICE_PTRS = 1
-FAULT_NONE, FAULT_ALLOC, FAULT_INT32_LIMIT, FAULT_LIST_LIMIT = range(4)
+(FAULT_NONE, FAULT_ALLOC, FAULT_INT32_LIMIT, FAULT_LIST_LIMIT,
+ FAULT_RECORD_LIMIT) = range(5)
 HOP_FP32 = 2  # matrix-free H: off-diagonal elements rounded to FP32
 FP64, MIXED = 0, 1
 

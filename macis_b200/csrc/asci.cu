@@ -1480,9 +1480,6 @@ __global__ void iota_k(uint32_t* x, size_t n) {
 // ----------------------------------------------------------------- driver
 // A range's score threshold is sampled from one part in GROUP_SAMPLE of it.
 constexpr size_t GROUP_SAMPLE = 32;
-// Records of a range: their positions are 32-bit.
-constexpr int64_t ASCI_MAX_RECORDS = (int64_t(1) << 32) - 1;
-
 // Bytes per contribution of a range while it is grouped: the record (its
 // determinant or number key, and the score), its copy and the digit counts of
 // the partition.
@@ -1510,7 +1507,7 @@ int64_t asci_range_records(double avail, int nbits, bool numbered,
       0.8 * avail - 6.0 * cand * double(std::min<uint64_t>(topk, raw));
   double n = left / (per_pair + per_cand);
   if(n > most) n = (left - per_cand * most) / per_pair;
-  return int64_t(std::min(std::max(n, 1048576.0), double(ASCI_MAX_RECORDS)));
+  return int64_t(std::min(std::max(n, 1048576.0), double(RS_MAX_RECORDS)));
 }
 
 namespace {
@@ -1974,9 +1971,11 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
   // MACIS_B200_ASCI_BATCH_PAIRS caps the raw pairs per range (exercises the
   // partitioned path on small problems).
   const char* cap_env = getenv("MACIS_B200_ASCI_BATCH_PAIRS");
-  int64_t cap = cap_env ? std::min(std::max<int64_t>(1, atoll(cap_env)),
-                                   ASCI_MAX_RECORDS)
-                        : plan_cap(avail);
+  // ranges and accumulated lists number their records with 32 bits
+  const int64_t max_records = int64_t(record_limit());
+  int64_t cap = std::min(
+      cap_env ? std::max<int64_t>(1, atoll(cap_env)) : plan_cap(avail),
+      max_records);
   // ranges: consecutive alpha-string bins packed up to the cap from the
   // measured bin loads (a single bin above the cap is a range of its own)
   // (a bin above the cap is split into beta-hash classes)
@@ -2052,7 +2051,8 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
         nlist = std::min<size_t>(ap.nu, size_t(budget / per_list));
         if(al_max > 0) nlist = std::min<size_t>(nlist, size_t(al_max));
         const double bytes = fixed + double(nlist) * per_list;
-        if(!cap_env) cap = plan_cap(avail - bytes / 0.8);
+        if(!cap_env)
+          cap = std::min(plan_cap(avail - bytes / 0.8), max_records);
       }
     }
   }
@@ -2258,6 +2258,11 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
       exclusive_scan<int64_t, int64_t>(rc, off, size_t(U), off + U, B);
       P = to_host(off + U, s);
     }
+    MB_REQUIRE(P <= max_records, MACIS_B200_ECAPACITY,
+               pairs_only ? "the accumulated list has more than 2^32 - 1 "
+                            "contributions"
+                          : "a candidate range has more than 2^32 - 1 "
+                            "contributions");
     const size_t KWr = ranked ? 1 : NW;  // words per record key
     uint64_t* keys = B.get<uint64_t>(size_t(P) * KWr + KWr);
     double* rv = B.get<double>(size_t(P) + 1);

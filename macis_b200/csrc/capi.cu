@@ -174,6 +174,7 @@ int macis_b200_inject_fault(int kind, int64_t arg) {
         faults().alloc_countdown.store(-1);
         faults().int32_limit.store(INT32_MAX);
         faults().list_limit.store(INT64_MAX);
+        faults().record_limit.store(UINT32_MAX);
         break;
       case MACIS_B200_FAULT_ALLOC:
         MB_REQUIRE(arg >= 0, MACIS_B200_EINVAL, "allocation count must be >= 0");
@@ -187,6 +188,11 @@ int macis_b200_inject_fault(int kind, int64_t arg) {
       case MACIS_B200_FAULT_LIST_LIMIT:
         MB_REQUIRE(arg >= 0, MACIS_B200_EINVAL, "list limit must be >= 0");
         faults().list_limit.store(arg);
+        break;
+      case MACIS_B200_FAULT_RECORD_LIMIT:
+        MB_REQUIRE(arg >= 1 && arg <= int64_t(UINT32_MAX), MACIS_B200_EINVAL,
+                   "record limit must be in [1, 2^32 - 1]");
+        faults().record_limit.store(arg);
         break;
       default:
         MB_REQUIRE(false, MACIS_B200_EINVAL, "unknown fault kind");

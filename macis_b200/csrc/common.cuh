@@ -369,12 +369,13 @@ struct NvtxRange {
 // Host-side failures for the tests of the error paths
 // (macis_b200_inject_fault): the (k+1)-th next device allocation made by the
 // library reports out-of-memory (once), CSR builds with int32 indices
-// accept fewer nonzeros, or general CSR builds list fewer candidates. Nothing
-// is made to fail on the device.
+// accept fewer nonzeros, general CSR builds list fewer candidates, or searches
+// take fewer records at a time. Nothing is made to fail on the device.
 struct FaultInjection {
   std::atomic<int64_t> alloc_countdown{-1};  // -1: off
   std::atomic<int64_t> int32_limit{INT32_MAX};
   std::atomic<int64_t> list_limit{INT64_MAX};
+  std::atomic<int64_t> record_limit{UINT32_MAX};
 };
 inline FaultInjection& faults() {
   static FaultInjection f;
@@ -400,6 +401,9 @@ inline cudaError_t dev_malloc(T** p, size_t bytes) {
 }
 inline int64_t int32_index_limit() {
   return faults().int32_limit.load(std::memory_order_relaxed);
+}
+inline uint64_t record_limit() {
+  return uint64_t(faults().record_limit.load(std::memory_order_relaxed));
 }
 inline uint64_t candidate_list_limit() {
   return uint64_t(faults().list_limit.load(std::memory_order_relaxed));

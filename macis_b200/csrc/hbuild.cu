@@ -2080,7 +2080,8 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     // (key + value, and the sort's second copy: 32 B per entry) fits in
     // what is free; short rows of the chunk are written by the same launch.
     int64_t lchunk = int64_t(0.7 * double(device_bytes_available()) / 32.0);
-    lchunk = std::max<int64_t>(lchunk, int64_t(1) << 20);
+    lchunk = std::min<int64_t>(std::max<int64_t>(lchunk, int64_t(1) << 20),
+                               int64_t(RS_MAX_RECORDS));
     float fill_ms_tot = 0.f;
     int64_t la = 0;  // next long row (list index)
     int64_t row_a = 0;

@@ -446,10 +446,10 @@ __device__ __forceinline__ void rs_tile_pass(const uint64_t* keys,
 }
 
 // One digit pass with per-block bucket offsets from radix_hist_k + scan.
-template <int NW, typename P, class Digit, typename OT>
+template <int NW, typename P, class Digit>
 __global__ void __launch_bounds__(RS_THREADS, 4)
     radix_scatter_k(const uint64_t* keys, const P* vals, size_t n, Digit digit,
-                    const OT* offsets, unsigned ntiles, uint64_t* keys_out,
+                    const uint32_t* offsets, unsigned ntiles, uint64_t* keys_out,
                     P* vals_out) {
   // issued before the ranking: its latency hides behind the tile loads
   const uint64_t my_off =
@@ -547,53 +547,47 @@ __global__ void __launch_bounds__(RS_THREADS, 4)
       });
 }
 
+// Records of a sort or a partition: their positions are 32-bit.
+constexpr size_t RS_MAX_RECORDS = (size_t(1) << 32) - 1;
+
 // Classic digit passes (per-tile histogram, scan, scatter) over n records,
-// with their scratch. Output positions are 32-bit below 2^32 records.
+// with their scratch.
 template <int NW, typename P>
 struct DigitPasses {
   size_t n;
   Arena& A;
   unsigned nblocks, ntiles;  // tiles, and padded to RS_HT
-  uint32_t* counts = nullptr;
-  void* offs = nullptr;
+  uint32_t *counts = nullptr, *offs = nullptr;
   DigitPasses(size_t n_, Arena& A_)
       : n(n_), A(A_), nblocks(unsigned((n_ + RS_TILE - 1) / RS_TILE)),
-        ntiles((nblocks + RS_HT - 1) / RS_HT * RS_HT) {}
+        ntiles((nblocks + RS_HT - 1) / RS_HT * RS_HT) {
+    MB_REQUIRE(n <= RS_MAX_RECORDS, MACIS_B200_ECAPACITY,
+               "more than 2^32 - 1 records in a sort");
+  }
   template <class Digit>
   void run(const uint64_t* kin, const P* vin, uint64_t* kout, P* vout,
            Digit digit) {
-    if(n >> 32)
-      run_as<uint64_t>(kin, vin, kout, vout, digit);
-    else
-      run_as<uint32_t>(kin, vin, kout, vout, digit);
+    constexpr size_t stage = rs_stage_bytes<NW, P>();
+    if(!counts) {
+      MB_CUDA(cudaFuncSetAttribute(radix_scatter_k<NW, P, Digit>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(stage)));
+      counts = A.get<uint32_t>(size_t(256) * ntiles);
+      offs = A.get<uint32_t>(size_t(256) * ntiles);
+    }
+    radix_hist_k<NW><<<ntiles / RS_HT, 256, 0, A.s>>>(kin, n, digit, counts,
+                                                      ntiles), note_launch();
+    exclusive_scan<uint32_t, uint32_t>(counts, offs, size_t(256) * ntiles,
+                                       nullptr, A);
+    radix_scatter_k<NW, P><<<nblocks, RS_THREADS, stage, A.s>>>(
+        kin, vin, n, digit, offs, ntiles, kout, vout), note_launch();
   }
   void release() {
     if(counts) {
       A.release(counts);
       A.release(offs);
     }
-    counts = nullptr;
-    offs = nullptr;
-  }
-
- private:
-  template <typename OT, class Digit>
-  void run_as(const uint64_t* kin, const P* vin, uint64_t* kout, P* vout,
-              Digit digit) {
-    constexpr size_t stage = rs_stage_bytes<NW, P>();
-    if(!counts) {
-      MB_CUDA(cudaFuncSetAttribute(radix_scatter_k<NW, P, Digit, OT>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   int(stage)));
-      counts = A.get<uint32_t>(size_t(256) * ntiles);
-      offs = A.get<OT>(size_t(256) * ntiles);
-    }
-    OT* off = static_cast<OT*>(offs);
-    radix_hist_k<NW><<<ntiles / RS_HT, 256, 0, A.s>>>(kin, n, digit, counts,
-                                                      ntiles), note_launch();
-    exclusive_scan<uint32_t, OT>(counts, off, size_t(256) * ntiles, nullptr, A);
-    radix_scatter_k<NW, P><<<nblocks, RS_THREADS, stage, A.s>>>(
-        kin, vin, n, digit, off, ntiles, kout, vout), note_launch();
+    counts = offs = nullptr;
   }
 };
 

@@ -413,3 +413,37 @@ def test_search_with_many_contributions_per_determinant(nbits, n, k, ncore):
         sel = st[order[:top]]
         sel = sel[np.lexsort(tuple(sel[:, w] for w in range(W)))]
         assert np.array_equal(got, np.concatenate([sel, cd]))
+
+
+def test_more_contributions_than_positions_count():
+    """Records are numbered with 32 bits (the limit lowered here): an
+    accumulated list beyond them is refused, a search takes more ranges and
+    selects the same, also where a larger range was asked for."""
+    from cases import core_set
+    from macis_b200 import _lib
+    n, k, nbits = 48, 12, 128
+    T, V = mb.synthetic_integrals(n, 3)
+    cd, C = core_set(n, k, 12, nbits)
+    H = mb.HamiltonianGenerator(T, V, nbits)
+    E0 = float(H.matrix_element(cd[:1], cd[:1])) - 0.5
+    whole = mb.asci_search(_settings(), 5000, cd, E0, C, n, H)
+    raw = mb.last_search_stats(H)["raw_pairs"]
+    inject = lambda kind, arg=0: _lib.check(
+        _lib.LIB.macis_b200_inject_fault(kind, arg))
+    try:
+        inject(_lib.FAULT_RECORD_LIMIT, raw)
+        mb.asci_pairs(_settings(), cd, E0, C, H)
+        inject(_lib.FAULT_RECORD_LIMIT, raw - 1)
+        with pytest.raises(mb.MacisError) as e:
+            mb.asci_pairs(_settings(), cd, E0, C, H)
+        assert e.value.code == _lib.ECAPACITY
+        inject(_lib.FAULT_RECORD_LIMIT, 3 * raw // 4)
+        for cap in (None, str(2 * raw)):
+            with pytest.MonkeyPatch.context() as m:
+                if cap:
+                    m.setenv("MACIS_B200_ASCI_BATCH_PAIRS", cap)
+                got = mb.asci_search(_settings(), 5000, cd, E0, C, n, H)
+            assert mb.last_search_stats(H)["batches"] >= 2
+            assert np.array_equal(got, whole)
+    finally:
+        inject(_lib.FAULT_NONE)
