@@ -2401,8 +2401,11 @@ __device__ __forceinline__ void rdm_add(double* a, size_t i, double v) {
 // costs 1 atomic instead of 2 (opposite-spin doubles), 1 instead of 4 (same
 // spin), and a single 1 per occupied orbital instead of 4 or 2; rdm_expand_k
 // then forms every element of the 2-RDM from the entries that reach it.
-// Indices as the 2-RDM's, (p,q,r,s) at p + n (q + n (r + n s)).
+// Indices as the 2-RDM's, (p,q,r,s) at p + n (q + n (r + n s)). The sums take
+// twice the 2-RDM's memory and two passes over it; DIRECT kernels add every
+// pair to the 2-RDM itself and need neither (form_rdms_device chooses).
 struct RdmSums {
+  double* trdm;   // the 2-RDM (DIRECT)
   double* os;     // n^4: (v1, o1, v2, o2), alpha and beta excitation
   double* ss;     // n^4: (v1, o1, v2, o2) of double_ex, both spins
   double* ss1;    // n^3: (v1, o1, p), p occupied in the excited spin
@@ -2415,7 +2418,7 @@ struct RdmSums {
 // One pair in the reference's dispatch (:15-66); pairs of the diagonal branch
 // return true. mixed: the list holds several electron counts; pairs that
 // differ by 2 or 4 electrons of a spin contribute nothing.
-template <int NSW>
+template <bool DIRECT, int NSW>
 __device__ __forceinline__ bool rdm_pair(Spin<NSW> ba, Spin<NSW> bb,
                                          Spin<NSW> ka, Spin<NSW> kb,
                                          bool mixed, double val, int n,
@@ -2425,14 +2428,31 @@ __device__ __forceinline__ bool rdm_pair(Spin<NSW> ba, Spin<NSW> bb,
   if(ca + cb > 4) return false;
   if(mixed && (unbalanced(ba, ka) || unbalanced(bb, kb))) return false;
   auto at = [n](int p, int q, int r) { return size_t(p) + size_t(n) * (q + size_t(n) * r); };
+  auto t4 = [&](int p, int q, int r, int s, double v) {
+    rdm_add(S.trdm, idx4(p, q, r, s, n), v);
+  };
   if((ca == 4 || cb == 4) && two) {  // rdm_contributions_4, :15-25
     const uint32_t e = ca == 4 ? double_ex(ba, ka) : double_ex(bb, kb);
-    rdm_add(S.ss, at(ex_v1(e), ex_o1(e), ex_v2(e)) + size_t(n) * n * n * ex_o2(e),
-            val * ex_sgn(e));
+    const int o1 = ex_o1(e), v1 = ex_v1(e), o2 = ex_o2(e), v2 = ex_v2(e);
+    if constexpr(DIRECT) {
+      const double v = val * (ex_sgn(e) * 0.5);
+      t4(v1, o1, v2, o2, v);
+      t4(v2, o1, v1, o2, -v);
+      t4(v1, o2, v2, o1, -v);
+      t4(v2, o2, v1, o1, v);
+    } else {
+      rdm_add(S.ss, idx4(v1, o1, v2, o2, n), val * ex_sgn(e));
+    }
   } else if(ca == 2 && cb == 2 && two) {  // rdm_contributions_22, :27-41
     const uint32_t ea = single_ex(ba, ka), eb = single_ex(bb, kb);
-    rdm_add(S.os, at(ex_v1(ea), ex_o1(ea), ex_v1(eb)) + size_t(n) * n * n * ex_o1(eb),
-            val * (ex_sgn(ea) * ex_sgn(eb)));
+    const int o1 = ex_o1(ea), v1 = ex_v1(ea), o2 = ex_o1(eb), v2 = ex_v1(eb);
+    const double sg = ex_sgn(ea) * ex_sgn(eb);
+    if constexpr(DIRECT) {
+      t4(v1, o1, v2, o2, val * (sg * 0.5));
+      t4(v2, o2, v1, o1, val * (sg * 0.5));
+    } else {
+      rdm_add(S.os, idx4(v1, o1, v2, o2, n), val * sg);
+    }
   } else if(ca == 2 || cb == 2) {  // rdm_contributions_2, :43-66
     const bool a = ca == 2;
     const uint32_t e = a ? single_ex(ba, ka) : single_ex(bb, kb);
@@ -2443,12 +2463,24 @@ __device__ __forceinline__ bool rdm_pair(Spin<NSW> ba, Spin<NSW> bb,
       for(Spin<NSW> s = a ? ba : bb; sp_popc(s);) {
         const int p = sp_lowest(s);
         s = sp_flip(s, p);
-        rdm_add(S.ss1, at(v1, o1, p), v);
+        if constexpr(DIRECT) {
+          t4(v1, o1, p, p, 0.5 * v);
+          t4(p, p, v1, o1, 0.5 * v);
+          t4(v1, p, p, o1, -0.5 * v);
+          t4(p, o1, v1, p, -0.5 * v);
+        } else {
+          rdm_add(S.ss1, at(v1, o1, p), v);
+        }
       }
       for(Spin<NSW> s = a ? bb : ba; sp_popc(s);) {
         const int p = sp_lowest(s);
         s = sp_flip(s, p);
-        rdm_add(S.os1, at(v1, o1, p), v);
+        if constexpr(DIRECT) {
+          t4(v1, o1, p, p, 0.5 * v);
+          t4(p, p, v1, o1, 0.5 * v);
+        } else {
+          rdm_add(S.os1, at(v1, o1, p), v);
+        }
       }
     }
   } else {
@@ -2463,7 +2495,7 @@ __device__ __forceinline__ bool rdm_pair(Spin<NSW> ba, Spin<NSW> bb,
 // the general build's enumeration; sums are atomic (order not fixed). The
 // contributions of the diagonal branch depend on the bra alone: their sum
 // per row goes to S.diag.
-template <int NBITS>
+template <int NBITS, bool DIRECT>
 __global__ void __launch_bounds__(HB_THREADS)
     rdm_k(GenData g, const uint64_t* dets, int64_t n, const double* C,
           int norb, double* ordm, int two, RdmSums S, unsigned* ctr) {
@@ -2483,9 +2515,9 @@ __global__ void __launch_bounds__(HB_THREADS)
         if(!act) return;
         const double val = ci * C[g.sidx[m]];
         if(!(fabs(val) > 1e-16)) return;
-        if(rdm_pair<NSW>(ba, bb, ld_spin<NSW>(g.salpha, m),
-                         ld_spin<NSW>(g.sbeta, m), g.mixed, val, norb, ordm,
-                         two != 0, S))
+        if(rdm_pair<DIRECT>(ba, bb, ld_spin<NSW>(g.salpha, m),
+                            ld_spin<NSW>(g.sbeta, m), g.mixed, val, norb, ordm,
+                            two != 0, S))
           dsum += val;
       });
 #pragma unroll
@@ -2501,7 +2533,7 @@ __global__ void __launch_bounds__(HB_THREADS)
 // one partial sum per pair: atomics per orbital pair and block, not per row
 // (every row adds to the pairs of the deepest orbitals).
 constexpr int DG_ROWS = 128;
-template <int NBITS>
+template <int NBITS, bool DIRECT>
 __global__ void rdm_diag_k(const uint64_t* dets, int64_t n, const double* w,
                            int norb, double* ordm, int two, RdmSums S) {
   using D = DetTraits<NBITS>;
@@ -2528,7 +2560,13 @@ __global__ void rdm_diag_k(const uint64_t* dets, int64_t n, const double* w,
       if(ap & bq) os += v;
     }
     if(p == q && one != 0.0) rdm_add(ordm, size_t(p) * (norb + 1), one);
-    if(two) {
+    if(DIRECT && two) {
+      const double same = 0.5 * ss, opp = 0.5 * os;
+      if(ss != 0.0) rdm_add(S.trdm, idx4(p, q, p, q, norb), -same);
+      if(ss != 0.0 || os != 0.0)
+        rdm_add(S.trdm, idx4(p, p, q, q, norb), same + opp);
+      if(os != 0.0) rdm_add(S.trdm, idx4(q, q, p, p, norb), opp);
+    } else if(two) {
       if(ss != 0.0) rdm_add(S.dss, size_t(x), ss);
       if(os != 0.0) rdm_add(S.dos, size_t(x), os);
     }
@@ -2572,29 +2610,50 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
   MB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), s));
   const size_t n1 = size_t(h->norb), n3 = n1 * n1 * n1, n4 = n3 * n1;
   RdmSums S{};
+  S.trdm = trdm;
   S.diag = A.get<double>(n);
-  if(trdm) {
+  const int two = trdm ? 1 : 0;
+  const unsigned gd = grid_for(n, DG_ROWS);
+  // The sums are taken last, so that without the memory for them the pairs go
+  // straight to the 2-RDM; so do those of short lists, where the passes over
+  // the sums cost more than the additions that they save. Selected lists of
+  // norb^2 / 20, 4 norb^2 and 16 norb^2 determinants, sums / straight: n = 24
+  // 0.37 / 0.34, 0.41 / 0.40, 0.57 / 0.58 ms; n = 48 0.50 / 0.39, 0.81 / 0.72,
+  // 1.55 / 1.76; n = 100 3.39 / 1.19, 7.9 / 6.0, 24.6 / 25.2. CAS spaces (more
+  // pairs a determinant) lie above the line: CAS(9,8) 0.87 / 1.32 ms.
+  auto sums = [&] {
     const size_t tot = 2 * n4 + 2 * n3 + 2 * n1 * n1;
-    double* z = A.get<double>(tot);
-    MB_CUDA(cudaMemsetAsync(z, 0, tot * 8, s));
-    S.os = z;
+    if(!trdm || n <= 4 * n1 * n1) return false;
+    try {
+      S.os = A.get<double>(tot);
+    } catch(const Error& e) {
+      if(e.code != MACIS_B200_ENOMEM) throw;
+      cudaGetLastError();  // the allocation's
+      return false;
+    }
+    MB_CUDA(cudaMemsetAsync(S.os, 0, tot * 8, s));
     S.ss = S.os + n4;
     S.ss1 = S.ss + n4;
     S.os1 = S.ss1 + n3;
     S.dss = S.os1 + n3;
     S.dos = S.dss + n1 * n1;
-  }
-  const int two = trdm ? 1 : 0;
-  const unsigned gd = grid_for(n, DG_ROWS);
-#define MB_RDM(NB)                                                          \
-  {                                                                         \
-    const GenData g = gen_plan<NB>(h, dets, n, dets, n, true, 0, A);        \
-    rdm_k<NB><<<gr, HB_THREADS, 0, s>>>(g, dets, int64_t(n), C, h->norb,    \
-                                       ordm, two, S, ctr),                  \
-        note_launch();                                                      \
-    rdm_diag_k<NB><<<gd, 256, 0, s>>>(dets, int64_t(n), S.diag, h->norb,    \
-                                      ordm, two, S),                        \
-        note_launch();                                                      \
+    return true;
+  };
+#define MB_RDM_RUN(NB, DIRECT)                                               \
+  rdm_k<NB, DIRECT><<<gr, HB_THREADS, 0, s>>>(g, dets, int64_t(n), C,        \
+                                              h->norb, ordm, two, S, ctr),   \
+      note_launch();                                                         \
+  rdm_diag_k<NB, DIRECT><<<gd, 256, 0, s>>>(dets, int64_t(n), S.diag,        \
+                                            h->norb, ordm, two, S),          \
+      note_launch();
+#define MB_RDM(NB)                                                           \
+  {                                                                          \
+    const GenData g = gen_plan<NB>(h, dets, n, dets, n, true, 0, A);         \
+    if(sums() || !trdm) {                                                    \
+      MB_RDM_RUN(NB, false)                                                  \
+    } else {                                                                 \
+      MB_RDM_RUN(NB, true)                                                   \
+    }                                                                        \
   }
   if(h->nbits == 64) {
     MB_RDM(64)
@@ -2603,9 +2662,10 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
   } else {
     MB_RDM(256)
   }
-  if(trdm)
+  if(S.os)
     rdm_expand_k<<<grid_for(n4, 256, 16 * num_sms()), 256, 0, s>>>(
         S, h->norb, trdm), note_launch();
+#undef MB_RDM_RUN
 #undef MB_RDM
   MB_CUDA(cudaGetLastError());
   MB_CUDA(cudaStreamSynchronize(s));

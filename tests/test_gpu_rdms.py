@@ -141,3 +141,54 @@ def test_rdms_match_pair_sums(nbits, n, na, nb, frac):
         np.testing.assert_allclose(o, ro, rtol=0, atol=1e-12)
         if two:
             np.testing.assert_allclose(t, rt, rtol=0, atol=1e-12)
+
+
+@pytest.mark.parametrize("n,na,nb,ndets", [(3, 1, 2, 9), (5, 2, 2, 100),
+                                           (6, 3, 2, 144), (6, 3, 2, 145),
+                                           (7, 2, 3, 196), (7, 2, 3, 197)])
+def test_rdms_of_short_lists_and_without_scratch(n, na, nb, ndets):
+    """Lists at and one above the length up to which the pairs go straight to
+    the 2-RDM (4 n^2), and longer ones without the memory for the sums: an
+    allocation that fails is an ENOMEM or, for the sums (the last one), that
+    path. Against the pair sums in plain Python: 1e-12 as above."""
+    from macis_b200 import _lib
+    T, V, d = fci(n, na, nb, 64, seed=1)
+    d = shuffled(d, seed=5)[:ndets].copy()
+    d[3] = 0
+    d[5] = d[6]
+    C = np.random.default_rng(2).standard_normal(len(d))
+    C /= np.linalg.norm(C)
+    H = mb.HamiltonianGenerator(T, V, 64)
+    ro, rt = _rdms_by_pairs(d, C, n, True)
+    good = 0
+    try:
+        for k in range(200):
+            _lib.check(_lib.LIB.macis_b200_inject_fault(_lib.FAULT_ALLOC, k))
+            try:
+                o, t = H.form_rdms(d, C)
+            except mb.MacisError as e:
+                assert e.code == _lib.ENOMEM and good == 0
+                continue
+            np.testing.assert_allclose(o, ro, rtol=0, atol=1e-12)
+            np.testing.assert_allclose(t, rt, rtol=0, atol=1e-12)
+            good += 1
+            if good == 2:      # without the sums, and with everything
+                break
+    finally:
+        _lib.check(_lib.LIB.macis_b200_inject_fault(_lib.FAULT_NONE, 0))
+    assert good == 2
+
+
+def test_rdm_scratch_of_a_short_list():
+    """Ten determinants of 64 orbitals need no multiple of their 2-RDM (134
+    MB) beside it: a tenth of it for the tables and what the pool rounds up."""
+    from test_gpu_hbuild import _peak_pool_bytes
+    n, k = 64, 4
+    T, V = mb.synthetic_integrals(n, 1)
+    hf = (1 << k) - 1
+    a = [hf] + [hf ^ 1 ^ (1 << v) for v in range(k, k + 9)]
+    d = mb.sd.make_dets(a, [hf] * 10, 128)
+    H = mb.HamiltonianGenerator(T, V, 128)
+    C = np.full(10, 10 ** -0.5)
+    H.form_rdms(d, C)
+    assert _peak_pool_bytes(lambda: H.form_rdms(d, C)) < 1.1 * 8 * n ** 4
