@@ -334,12 +334,14 @@ __device__ __forceinline__ bool unbalanced(Spin<NSW> bra, Spin<NSW> ket) {
 // Full matrix_element(bra, ket) dispatch (matrix_elements.hpp:22-53). Pairs
 // whose electron counts of a spin differ by 2 or 4 have no element (the
 // reference indexes orbital -1 for them); by an odd number, the reference's
-// dispatch is kept.
-template <int NSW>
+// dispatch is kept. CHECK false: lists of one electron count, which hold no
+// such pair.
+template <bool CHECK = true, int NSW>
 __device__ double me_generic(const Ints& I, Spin<NSW> ba, Spin<NSW> bb,
                              Spin<NSW> ka, Spin<NSW> kb) {
   const int ca = sp_popc(ba ^ ka), cb = sp_popc(bb ^ kb);
-  if(ca + cb > 4 || unbalanced(ba, ka) || unbalanced(bb, kb)) return 0.;
+  if(ca + cb > 4) return 0.;
+  if(CHECK && (unbalanced(ba, ka) || unbalanced(bb, kb))) return 0.;
   if(ca == 4) return me_ss_double(I, double_ex(ba, ka));
   if(cb == 4) return me_ss_double(I, double_ex(bb, kb));
   if(ca == 2 && cb == 2) return me_os_double(I, single_ex(ba, ka), single_ex(bb, kb));

@@ -1357,7 +1357,7 @@ __device__ __forceinline__ void gen_enumerate(const GenData& g, int32_t rg,
 // waited half of its time for instructions, and the matrix-free product on an
 // n = 64 list took 3.93 and not 2.46 ms (2.97 with eval as a call), form_rdms on
 // CAS(9,9) 0.94 and not 0.89. q: 128 entries of shared memory per warp.
-template <int NSW, class F>
+template <bool MIXED, int NSW, class F>
 __device__ __forceinline__ void gen_pairs(const GenData& g, int32_t rg,
                                           Spin<NSW> ba, Spin<NSW> bb,
                                           uint8_t* ov, uint32_t* q, F&& eval) {
@@ -1367,7 +1367,7 @@ __device__ __forceinline__ void gen_pairs(const GenData& g, int32_t rg,
                      [&](bool act, int64_t m, int pa, int pb) {
     const unsigned any = __ballot_sync(0xffffffffu, act);
     if(!any) return;
-    const bool dbl = pa + pb == 4 && !(pa & 1) && !g.mixed;
+    const bool dbl = !MIXED && pa + pb == 4 && !(pa & 1);
     const unsigned md = __ballot_sync(0xffffffffu, act && dbl), mo = any & ~md;
     if(act) {
       const int at = dbl ? 64 + n1 + __popc(md & lanemask_lt())
@@ -1402,16 +1402,18 @@ __device__ __forceinline__ void gen_pairs(const GenData& g, int32_t rg,
 }
 constexpr int GEN_SCRATCH = 256 + 128 * 4;  // bytes per warp: ov, q
 
-// H(bra, ket) of a connected pair, evaluated by class; dbl only where the
-// lists hold one electron count per spin.
-template <int NSW>
+// H(bra, ket) of a connected pair, evaluated by class. MIXED: the lists hold
+// several electron counts, and every pair takes the general element; in
+// instantiations of their own, for the test of each pair made the matrix-free
+// product of the usual lists 3 % slower.
+template <bool MIXED, int NSW>
 __device__ __forceinline__ double gen_element(const Ints& I, bool dbl,
                                               Spin<NSW> ba, Spin<NSW> bb,
                                               Spin<NSW> ka, Spin<NSW> kb,
                                               double hd) {
-  if(dbl) return me_double(I, ba, bb, ka, kb);
+  if(!MIXED && dbl) return me_double(I, ba, bb, ka, kb);
   if(ka == ba && kb == bb) return hd;
-  return me_generic(I, ba, bb, ka, kb);
+  return me_generic<MIXED>(I, ba, bb, ka, kb);
 }
 
 // Candidates per row, and the rows' candidates themselves (sorted positions)
@@ -1465,7 +1467,7 @@ __global__ void __launch_bounds__(HB_THREADS)
 // the threshold are marked with column -1. Rows with more than GEN_CAP
 // candidates are written unsorted to the long-row scratch (lkey/lval at
 // loff[row]) and finished by the radix sort.
-template <int NBITS, typename CI, typename VT>
+template <int NBITS, bool MIXED, typename CI, typename VT>
 __global__ void __launch_bounds__(HB_THREADS)
     gen_fill_k(Ints I, GenData g, const uint64_t* bra, int64_t row_a,
                int64_t row_b, const double* __restrict__ hdiag,
@@ -1501,12 +1503,12 @@ __global__ void __launch_bounds__(HB_THREADS)
       const int64_t lbase = loff[row] - lbase0;
       const uint64_t lhi = uint64_t(lidx[row]) << 32;
       int64_t c = 0;
-      gen_pairs<NSW>(g, rg, ba, bb, ov, q, [&](bool act, int64_t m, bool dbl) {
+      gen_pairs<MIXED>(g, rg, ba, bb, ov, q, [&](bool act, int64_t m, bool dbl) {
         const unsigned msk = __ballot_sync(0xffffffffu, act);
         if(act) {
           const int64_t pos = lbase + c + __popc(msk & lanemask_lt());
           lkey[pos] = lhi | g.sidx[m];
-          lval[pos] = gen_element<NSW>(I, dbl, ba, bb, ld_spin<NSW>(g.salpha, m),
+          lval[pos] = gen_element<MIXED>(I, dbl, ba, bb, ld_spin<NSW>(g.salpha, m),
                                        ld_spin<NSW>(g.sbeta, m), hd);
         }
         c += __popc(msk);
@@ -1564,7 +1566,7 @@ __global__ void __launch_bounds__(HB_THREADS)
         const uint64_t key = bk[i];
         const uint32_t m = uint32_t(key);
         put(i, uint32_t(key >> 32),
-            gen_element<NSW>(I, false, ba, bb, ld_spin<NSW>(g.salpha, m),
+            gen_element<MIXED>(I, false, ba, bb, ld_spin<NSW>(g.salpha, m),
                              ld_spin<NSW>(g.sbeta, m), hd));
       }
     };
@@ -1577,7 +1579,7 @@ __global__ void __launch_bounds__(HB_THREADS)
         const Spin<NSW> ka = ld_spin<NSW>(g.salpha, m);
         const Spin<NSW> kb = ld_spin<NSW>(g.sbeta, m);
         const int ca = sp_popc(ba ^ ka), cb = sp_popc(bb ^ kb);
-        if(ca + cb == 4 && !(ca & 1) && !g.mixed)
+        if(!MIXED && ca + cb == 4 && !(ca & 1))
           put(i, uint32_t(key >> 32), me_double(I, ba, bb, ka, kb));
         else
           put_off = true;
@@ -2097,7 +2099,9 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
       double* lval = C.get<double>(centries + 1);
       cudaEventRecord(ev[0], s);
       MB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), s));
-      gen_fill_k<NBITS, CI, VT><<<gr, HB_THREADS, 0, s>>>(
+      auto fill = gd.mixed ? gen_fill_k<NBITS, true, CI, VT>
+                           : gen_fill_k<NBITS, false, CI, VT>;
+      fill<<<gr, HB_THREADS, 0, s>>>(
           I, gd, bra, row_a, row_b, hdiag, rowptr64, list, list_off, loff_row,
           cbase, lpos, lkey, lval, colind, nzval, out->diag, rowcnt, thresh,
           ctr, &d_tot->dropped), note_launch();
@@ -2251,7 +2255,7 @@ namespace mb {
 // ctr: {next row, finished blocks}, both 0 before and after: the last block
 // clears them, so that a product is one stream operation and two that are
 // enqueued at once by several host threads follow one another.
-template <int NBITS>
+template <int NBITS, bool MIXED>
 __global__ void __launch_bounds__(HB_THREADS)
     gen_apply_k(Ints I, GenData g, const uint64_t* dets, int64_t n,
                 const double* __restrict__ hdiag, double thresh, int mixed,
@@ -2269,11 +2273,11 @@ __global__ void __launch_bounds__(HB_THREADS)
       const uint64_t* bd = dets + row * D::NW;
       const Spin<NSW> ba = D::alpha(bd), bb = D::beta(bd);
       const double hd = hdiag[row];
-      gen_pairs<NSW>(g, rg, ba, bb, ov, reinterpret_cast<uint32_t*>(ov + 256),
+      gen_pairs<MIXED>(g, rg, ba, bb, ov, reinterpret_cast<uint32_t*>(ov + 256),
                      [&](bool act, int64_t m, bool dbl) {
         if(act) {
           const uint32_t col = g.sidx[m];
-          double h = gen_element<NSW>(I, dbl, ba, bb, ld_spin<NSW>(g.salpha, m),
+          double h = gen_element<MIXED>(I, dbl, ba, bb, ld_spin<NSW>(g.salpha, m),
                                       ld_spin<NSW>(g.sbeta, m), hd);
           if(fabs(h) > thresh) {
             if(mixed && int64_t(col) != row) h = double(float(h));
@@ -2355,10 +2359,10 @@ void hop_apply(const macis_b200_hop* op, double alpha, const double* x,
   const unsigned gr = grid_for(size_t(op->n), HB_WARPS, size_t(num_sms()) * 16);
   const Ints I = op->I;
 #define MB_HOP_APPLY(NB)                                                     \
-  gen_apply_k<NB><<<gr, HB_THREADS, 0, s>>>(I, op->g, op->dets, op->n,       \
-                                            op->diag, op->thresh,            \
-                                            op->mixed ? 1 : 0, alpha, x,     \
-                                            beta, y, op->ctr),               \
+  (op->g.mixed ? gen_apply_k<NB, true> : gen_apply_k<NB, false>)             \
+      <<<gr, HB_THREADS, 0, s>>>(I, op->g, op->dets, op->n, op->diag,        \
+                                 op->thresh, op->mixed ? 1 : 0, alpha, x,    \
+                                 beta, y, op->ctr),                          \
       note_launch();
   if(op->nbits == 64) {
     MB_HOP_APPLY(64)
@@ -2416,17 +2420,16 @@ struct RdmSums {
 };
 
 // One pair in the reference's dispatch (:15-66); pairs of the diagonal branch
-// return true. mixed: the list holds several electron counts; pairs that
+// return true. MIXED: the list holds several electron counts; pairs that
 // differ by 2 or 4 electrons of a spin contribute nothing.
-template <bool DIRECT, int NSW>
+template <bool DIRECT, bool MIXED, int NSW>
 __device__ __forceinline__ bool rdm_pair(Spin<NSW> ba, Spin<NSW> bb,
                                          Spin<NSW> ka, Spin<NSW> kb,
-                                         bool mixed, double val, int n,
-                                         double* ordm, bool two,
-                                         const RdmSums& S) {
+                                         double val, int n, double* ordm,
+                                         bool two, const RdmSums& S) {
   const int ca = sp_popc(ba ^ ka), cb = sp_popc(bb ^ kb);
   if(ca + cb > 4) return false;
-  if(mixed && (unbalanced(ba, ka) || unbalanced(bb, kb))) return false;
+  if(MIXED && (unbalanced(ba, ka) || unbalanced(bb, kb))) return false;
   auto at = [n](int p, int q, int r) { return size_t(p) + size_t(n) * (q + size_t(n) * r); };
   auto t4 = [&](int p, int q, int r, int s, double v) {
     rdm_add(S.trdm, idx4(p, q, r, s, n), v);
@@ -2495,7 +2498,7 @@ __device__ __forceinline__ bool rdm_pair(Spin<NSW> ba, Spin<NSW> bb,
 // the general build's enumeration; sums are atomic (order not fixed). The
 // contributions of the diagonal branch depend on the bra alone: their sum
 // per row goes to S.diag.
-template <int NBITS, bool DIRECT>
+template <int NBITS, bool DIRECT, bool MIXED>
 __global__ void __launch_bounds__(HB_THREADS)
     rdm_k(GenData g, const uint64_t* dets, int64_t n, const double* C,
           int norb, double* ordm, int two, RdmSums S, unsigned* ctr) {
@@ -2510,14 +2513,14 @@ __global__ void __launch_bounds__(HB_THREADS)
       const uint64_t* bd = dets + row * D::NW;
       const Spin<NSW> ba = D::alpha(bd), bb = D::beta(bd);
       const double ci = C[row];
-      gen_pairs<NSW>(g, rg, ba, bb, ov, reinterpret_cast<uint32_t*>(ov + 256),
+      gen_pairs<MIXED>(g, rg, ba, bb, ov, reinterpret_cast<uint32_t*>(ov + 256),
                      [&](bool act, int64_t m, bool) {
         if(!act) return;
         const double val = ci * C[g.sidx[m]];
         if(!(fabs(val) > 1e-16)) return;
-        if(rdm_pair<DIRECT>(ba, bb, ld_spin<NSW>(g.salpha, m),
-                            ld_spin<NSW>(g.sbeta, m), g.mixed, val, norb, ordm,
-                            two != 0, S))
+        if(rdm_pair<DIRECT, MIXED>(ba, bb, ld_spin<NSW>(g.salpha, m),
+                                   ld_spin<NSW>(g.sbeta, m), val, norb, ordm,
+                                   two != 0, S))
           dsum += val;
       });
 #pragma unroll
@@ -2640,8 +2643,9 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
     return true;
   };
 #define MB_RDM_RUN(NB, DIRECT)                                               \
-  rdm_k<NB, DIRECT><<<gr, HB_THREADS, 0, s>>>(g, dets, int64_t(n), C,        \
-                                              h->norb, ordm, two, S, ctr),   \
+  (g.mixed ? rdm_k<NB, DIRECT, true> : rdm_k<NB, DIRECT, false>)             \
+      <<<gr, HB_THREADS, 0, s>>>(g, dets, int64_t(n), C, h->norb, ordm, two, \
+                                 S, ctr),                                    \
       note_launch();                                                         \
   rdm_diag_k<NB, DIRECT><<<gd, 256, 0, s>>>(dets, int64_t(n), S.diag,        \
                                             h->norb, ordm, two, S),          \
