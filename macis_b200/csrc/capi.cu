@@ -694,8 +694,8 @@ int macis_b200_hop_davidson(const macis_b200_hop* op,
     dop.diag = hop_diag(op);
     dop.s = s;
     dop.pinned = hop_pinned(op);
-    dop.apply = [op](const double* xin, double* y) {
-      hop_apply(op, 1.0, xin, 0.0, y);
+    dop.apply = [op](const double* xin, double* y, unsigned long long* t0) {
+      hop_apply(op, 1.0, xin, 0.0, y, t0);
     };
     rc = davidson_op(dop, o->max_m, o->tol, o->use_guess != 0, x.d, E, niter,
                      o->restart_keep, o->max_iter);

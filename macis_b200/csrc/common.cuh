@@ -443,6 +443,17 @@ inline unsigned grid_for(size_t work, int block, size_t max_blocks = 0) {
   return unsigned(g);
 }
 
+__device__ __forceinline__ unsigned long long gpu_time_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Notes the start of a kernel at *t0 (may be null).
+__device__ __forceinline__ void note_start(unsigned long long* t0) {
+  if(t0 && blockIdx.x == 0 && threadIdx.x == 0) *t0 = gpu_time_ns();
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -38,11 +38,6 @@ constexpr int DV_CHUNK = 8;  // columns held by one multi-dot block
 __device__ __forceinline__ void dav_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-__device__ __forceinline__ unsigned long long gpu_time_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 
 // What the kernels report to the host, in page-locked host memory.
 struct DavReport {
@@ -50,8 +45,9 @@ struct DavReport {
   volatile unsigned res_seq;   // |R|^2 of this number is there
   volatile unsigned err;       // a grid barrier gave up
   volatile double rn2;
-  // phase boundaries, ns: the row's kernel, the step's residual, its end
-  volatile unsigned long long t_row0, t_row1, t_res0, t_res1, t_end;
+  // phase boundaries, ns: the product's start, the row's kernel, the step's
+  // residual, its end
+  volatile unsigned long long t_app0, t_row0, t_row1, t_res0, t_res1, t_end;
   volatile double row[1];      // an entry per basis column
 };
 
@@ -115,7 +111,9 @@ __device__ __forceinline__ double warp_sum_partials(const double* p, int nb,
 // gridDim.x, ... (in units of DV_THREADS) of the DV_CHUNK columns from
 // DV_CHUNK y, the last block of a chunk adds the chunk's partial sums in a
 // fixed order, and the last chunk reports. HBM-bound for long vectors.
-// done: one counter per chunk, one for the chunks; t0: scratch.
+// done: one counter per chunk, one for the chunks; t0: scratch, and the start
+// of the product before it, which is reported with the row (a product that
+// wrote it to host memory itself ended about 2 us later).
 __global__ void __launch_bounds__(DV_THREADS)
     multidot_k(const double* __restrict__ A, int64_t lda, int ncol,
                const double* __restrict__ v, int64_t n, double* partial,
@@ -156,6 +154,7 @@ __global__ void __launch_bounds__(DV_THREADS)
   __threadfence_system();  // before the report of the last chunk
   if(last_block(done + gridDim.y, gridDim.y) && threadIdx.x == 0) {
     rep->t_row0 = *static_cast<volatile unsigned long long*>(t0);
+    rep->t_app0 = *static_cast<volatile unsigned long long*>(t0 + 1);
     rep->t_row1 = gpu_time_ns();
     __threadfence_system();
     rep->row_seq = seq;
@@ -418,7 +417,7 @@ struct DavCtx {
   double* partial;
   unsigned* done;         // arrival counters: per column chunk, of the chunks
   unsigned* bar;
-  unsigned long long* t0;
+  unsigned long long* t0;  // starts of the row's kernel and of the product
   unsigned nbar = 0;      // barrier arrivals so far
   unsigned seq = 0;
   DavReport* rep = nullptr;
@@ -437,7 +436,7 @@ struct DavCtx {
     done = A.get<unsigned>(chunks + 3);
     bar = done + chunks + 2;
     MB_CUDA(cudaMemsetAsync(done, 0, (chunks + 3) * sizeof(unsigned), st));
-    t0 = A.get<unsigned long long>(1);
+    t0 = A.get<unsigned long long>(2);
     const size_t bytes = sizeof(DavReport) + size_t(ncol) * 8;
     MB_REQUIRE(bytes <= PinnedPool::BYTES, MACIS_B200_EINVAL,
                "Davidson: subspace too large");
@@ -521,8 +520,8 @@ int davidson_device(const macis_b200_csr* A, int64_t max_m, double tol,
   op.diag = A->diag;
   op.s = A->stream;
   op.pinned = A->pinned;
-  op.apply = [A](const double* x, double* y) {
-    spmv_device_x64(A, 1.0, x, 0.0, y, A->stream);
+  op.apply = [A](const double* x, double* y, unsigned long long* t0) {
+    spmv_device_x64(A, 1.0, x, 0.0, y, A->stream, t0);
   };
   return davidson_op(op, max_m, tol, use_guess, X, E, niter, restart_keep,
                      max_iter);
@@ -553,7 +552,7 @@ int davidson_op(const DavOperator& op, int64_t max_m, double tol,
   };
   if(N == 1) {  // no second basis vector: the product of the unit vector
     double* y = Ar.get<double>(1);
-    op.apply(X, y);
+    op.apply(X, y, nullptr);
     *E = to_host(y, s);
     *niter = st.iterations = 1;
     st.wall_ms = wall_ms();
@@ -584,7 +583,7 @@ int davidson_op(const DavOperator& op, int64_t max_m, double tol,
     ctx.step(o, rc);
   };
   MB_CUDA(cudaMemcpyAsync(V, X, N * 8, cudaMemcpyDeviceToDevice, s));
-  op.apply(V, AV);
+  op.apply(V, AV, nullptr);
   MB_CUDA(cudaMemcpyAsync(V + N, AV, N * 8, cudaMemcpyDeviceToDevice, s));
   orthonormalise(1, V + N);
 
@@ -603,15 +602,16 @@ int davidson_op(const DavOperator& op, int64_t max_m, double tol,
   int64_t i = 1;  // index of the newest basis vector (AV_i not yet formed)
   for(;; ++iter) {
     const int k = int(i + 1);
-    op.apply(V + i * N, AV + i * N);
+    op.apply(V + i * N, AV + i * N, ctx.t0 + 1);
     // new row of V^T AV: V_i . AV_c for c <= i (lower triangle)
     ctx.multidot(AV, k, V + i * N);
     st.vector_bytes += double(N) * (k + 1) * 8;
     ctx.wait(ctx.rep->row_seq);
-    // the step before has ended too: its last phase, the product behind it
-    // and the row
+    // the step before has ended too: its last phase; then the product, timed
+    // from its own start (the GPU may have waited for the host before it), and
+    // the row
     if(iter > 1) st.ortho_ms += ms(ctx.rep->t_res1, ctx.rep->t_end);
-    st.apply_ms += ms(ctx.rep->t_end, ctx.rep->t_row0);
+    st.apply_ms += ms(ctx.rep->t_app0, ctx.rep->t_row0);
     st.rayleigh_ms += ms(ctx.rep->t_row0, ctx.rep->t_row1);
     for(int c = 0; c < k; ++c) Cl[i + size_t(c) * ld] = ctx.rep->row[c];
     lower.assign(size_t(k) * k, 0.0);

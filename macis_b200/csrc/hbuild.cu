@@ -2260,10 +2260,12 @@ __global__ void __launch_bounds__(HB_THREADS)
     gen_apply_k(Ints I, GenData g, const uint64_t* dets, int64_t n,
                 const double* __restrict__ hdiag, double thresh, int mixed,
                 double alpha, const double* __restrict__ x, double beta,
-                double* __restrict__ y, unsigned* ctr) {
+                double* __restrict__ y, unsigned* ctr,
+                unsigned long long* t0) {
   using D = DetTraits<NBITS>;
   constexpr int NSW = D::NSW;
   __shared__ __align__(16) uint8_t s_scr[HB_WARPS][GEN_SCRATCH];
+  note_start(t0);
   const int lane = threadIdx.x & 31;
   uint8_t* ov = s_scr[threadIdx.x >> 5];
   for(int64_t row; (row = next_row(ctr)) < n;) {
@@ -2354,7 +2356,7 @@ macis_b200_hop* hop_create(macis_b200_ham* h, const uint64_t* dets, size_t n,
 }
 
 void hop_apply(const macis_b200_hop* op, double alpha, const double* x,
-               double beta, double* y) {
+               double beta, double* y, unsigned long long* t0) {
   cudaStream_t s = op->stream;
   const unsigned gr = grid_for(size_t(op->n), HB_WARPS, size_t(num_sms()) * 16);
   const Ints I = op->I;
@@ -2362,7 +2364,7 @@ void hop_apply(const macis_b200_hop* op, double alpha, const double* x,
   (op->g.mixed ? gen_apply_k<NB, true> : gen_apply_k<NB, false>)             \
       <<<gr, HB_THREADS, 0, s>>>(I, op->g, op->dets, op->n, op->diag,        \
                                  op->thresh, op->mixed ? 1 : 0, alpha, x,    \
-                                 beta, y, op->ctr),                          \
+                                 beta, y, op->ctr, t0),                      \
       note_launch();
   if(op->nbits == 64) {
     MB_HOP_APPLY(64)

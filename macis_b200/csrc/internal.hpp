@@ -171,10 +171,13 @@ void matrix_elements_device(macis_b200_ham* h, const uint64_t* bra,
 // y = alpha*A*x + beta*y on device vectors (one column).
 // Davidson's product: on a mixed matrix, FP32 values times the FP64 x with
 // FP64 sums (one fixed linear operator); FP64 matrices as spmv_device.
+// t0: where the product's kernel notes its start, ns (may be null).
 void spmv_device_x64(const macis_b200_csr* A, double alpha, const double* x,
-                     double beta, double* y, cudaStream_t s);
+                     double beta, double* y, cudaStream_t s,
+                     unsigned long long* t0 = nullptr);
 void spmv_device(const macis_b200_csr* A, double alpha, const double* x,
-                 double beta, double* y, cudaStream_t s);
+                 double beta, double* y, cudaStream_t s,
+                 unsigned long long* t0 = nullptr);
 
 // Davidson on device-resident matrix; X is a device vector.
 int davidson_device(const macis_b200_csr* A, int64_t max_m, double tol,
@@ -184,12 +187,14 @@ int davidson_device(const macis_b200_csr* A, int64_t max_m, double tol,
 // The operator Davidson works with: y = H x on device vectors of length n,
 // diag(H) in device memory, everything on stream s (the reference's
 // davidson takes any functor with operator_action, davidson.hpp:47-58, 129).
+// The product notes its start at t0 (device-visible, may be null), for the
+// solver's phase times.
 struct DavOperator {
   int64_t n = 0;
   const double* diag = nullptr;
   cudaStream_t s = nullptr;
   std::shared_ptr<PinnedPool> pinned;
-  std::function<void(const double* x, double* y)> apply;
+  std::function<void(const double* x, double* y, unsigned long long* t0)> apply;
 };
 int davidson_op(const DavOperator& op, int64_t max_m, double tol,
                 bool use_guess, double* X, double* E, int64_t* niter,
@@ -205,7 +210,7 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
 macis_b200_hop* hop_create(macis_b200_ham* h, const uint64_t* dets, size_t n,
                            double thresh, bool mixed, bool device_ptrs);
 void hop_apply(const macis_b200_hop* op, double alpha, const double* x,
-               double beta, double* y);
+               double beta, double* y, unsigned long long* t0 = nullptr);
 void hop_destroy(macis_b200_hop* op);
 int64_t hop_size(const macis_b200_hop* op);
 const double* hop_diag(const macis_b200_hop* op);

@@ -39,7 +39,8 @@ __global__ void __launch_bounds__(SPMV_THREADS, 2)
            const CI* __restrict__ colind, const VT* __restrict__ nzval,
            const double* __restrict__ diag, const double* __restrict__ x,
            const float* __restrict__ x32, double alpha, double beta,
-           double* __restrict__ y) {
+           double* __restrict__ y, unsigned long long* t0) {
+  note_start(t0);
   const int lane = threadIdx.x & 31;
   const int64_t nwarp = int64_t(gridDim.x) * (SPMV_THREADS / 32);
   for(int64_t row = int64_t(blockIdx.x) * (SPMV_THREADS / 32) + (threadIdx.x >> 5);
@@ -88,7 +89,8 @@ static unsigned spmv_grid(int64_t m) {
 }
 
 void spmv_device(const macis_b200_csr* A, double alpha, const double* x,
-                 double beta, double* y, cudaStream_t s) {
+                 double beta, double* y, cudaStream_t s,
+                 unsigned long long* t0) {
   const int64_t m = A->m;
   if(m == 0) return;
   const unsigned g = spmv_grid(m);
@@ -96,11 +98,11 @@ void spmv_device(const macis_b200_csr* A, double alpha, const double* x,
     if(A->idx_bytes == 4)
       spmv_k<int32_t, double, false><<<g, SPMV_THREADS, 0, s>>>(
           m, A->n, (const int32_t*)A->rowptr, (const int32_t*)A->colind,
-          (const double*)A->nzval, A->diag, x, nullptr, alpha, beta, y), note_launch();
+          (const double*)A->nzval, A->diag, x, nullptr, alpha, beta, y, t0), note_launch();
     else
       spmv_k<int64_t, double, false><<<g, SPMV_THREADS, 0, s>>>(
           m, A->n, (const int64_t*)A->rowptr, (const int64_t*)A->colind,
-          (const double*)A->nzval, A->diag, x, nullptr, alpha, beta, y), note_launch();
+          (const double*)A->nzval, A->diag, x, nullptr, alpha, beta, y, t0), note_launch();
   } else {
     Arena W(s);
     float* x32 = W.get<float>(size_t(A->n));
@@ -109,29 +111,30 @@ void spmv_device(const macis_b200_csr* A, double alpha, const double* x,
     if(A->idx_bytes == 4)
       spmv_k<int32_t, float, true><<<g, SPMV_THREADS, 0, s>>>(
           m, A->n, (const int32_t*)A->rowptr, (const int32_t*)A->colind,
-          (const float*)A->nzval, A->diag, x, x32, alpha, beta, y), note_launch();
+          (const float*)A->nzval, A->diag, x, x32, alpha, beta, y, t0), note_launch();
     else
       spmv_k<int64_t, float, true><<<g, SPMV_THREADS, 0, s>>>(
           m, A->n, (const int64_t*)A->rowptr, (const int64_t*)A->colind,
-          (const float*)A->nzval, A->diag, x, x32, alpha, beta, y), note_launch();
+          (const float*)A->nzval, A->diag, x, x32, alpha, beta, y, t0), note_launch();
   }
   MB_CUDA(cudaGetLastError());
 }
 
 void spmv_device_x64(const macis_b200_csr* A, double alpha, const double* x,
-                     double beta, double* y, cudaStream_t s) {
-  if(A->val_bytes == 8) return spmv_device(A, alpha, x, beta, y, s);
+                     double beta, double* y, cudaStream_t s,
+                     unsigned long long* t0) {
+  if(A->val_bytes == 8) return spmv_device(A, alpha, x, beta, y, s, t0);
   const int64_t m = A->m;
   if(m == 0) return;
   const unsigned g = spmv_grid(m);
   if(A->idx_bytes == 4)
     spmv_k<int32_t, float, true, false><<<g, SPMV_THREADS, 0, s>>>(
         m, A->n, (const int32_t*)A->rowptr, (const int32_t*)A->colind,
-        (const float*)A->nzval, A->diag, x, nullptr, alpha, beta, y), note_launch();
+        (const float*)A->nzval, A->diag, x, nullptr, alpha, beta, y, t0), note_launch();
   else
     spmv_k<int64_t, float, true, false><<<g, SPMV_THREADS, 0, s>>>(
         m, A->n, (const int64_t*)A->rowptr, (const int64_t*)A->colind,
-        (const float*)A->nzval, A->diag, x, nullptr, alpha, beta, y), note_launch();
+        (const float*)A->nzval, A->diag, x, nullptr, alpha, beta, y, t0), note_launch();
   MB_CUDA(cudaGetLastError());
 }
 
@@ -226,12 +229,12 @@ extern "C" int macis_b200_spmv_mixed_noalloc(const macis_b200_csr* A,
       if(A->idx_bytes == 4)
         mb::spmv_k<int32_t, float, true><<<g, mb::SPMV_THREADS, 0, s>>>(
             m, A->n, (const int32_t*)A->rowptr, (const int32_t*)A->colind,
-            (const float*)A->nzval, A->diag, x, x32, alpha, beta, y),
+            (const float*)A->nzval, A->diag, x, x32, alpha, beta, y, nullptr),
             mb::note_launch();
       else
         mb::spmv_k<int64_t, float, true><<<g, mb::SPMV_THREADS, 0, s>>>(
             m, A->n, (const int64_t*)A->rowptr, (const int64_t*)A->colind,
-            (const float*)A->nzval, A->diag, x, x32, alpha, beta, y),
+            (const float*)A->nzval, A->diag, x, x32, alpha, beta, y, nullptr),
             mb::note_launch();
       MB_CUDA(cudaGetLastError());
     }
