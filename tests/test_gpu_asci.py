@@ -447,3 +447,31 @@ def test_more_contributions_than_positions_count():
             assert np.array_equal(got, whole)
     finally:
         inject(_lib.FAULT_NONE)
+
+
+def test_four_hash_digits_match_three(monkeypatch):
+    """A range of more than 20 * 2^24 contributions is partitioned by four
+    hash digits, smaller ranges by three: equal selections and counts from one
+    range and from several, with number keys and with determinants."""
+    from cases import core_set
+    n, k, nbits = 48, 12, 128
+    T, V = mb.synthetic_integrals(n, 0)
+    cd, C = core_set(n, k, 1350, nbits, nalpha=80, top=40)
+    H = mb.HamiltonianGenerator(T, V, nbits)
+    E0 = float(H.matrix_element(cd[:1], cd[:1])) - 0.5
+    got = []
+    for ranks, cap, digits in (("1", None, 4), ("1", "150000000", 3),
+                               ("0", None, 4)):
+        monkeypatch.setenv("MACIS_B200_ASCI_RANKS", ranks)
+        if cap:
+            monkeypatch.setenv("MACIS_B200_ASCI_BATCH_PAIRS", cap)
+        else:
+            monkeypatch.delenv("MACIS_B200_ASCI_BATCH_PAIRS", raising=False)
+        sel = mb.asci_search(_settings(), 60000, cd, E0, C, n, H)
+        st = mb.last_search_stats(H)
+        assert st["raw_pairs"] > 20 << 24
+        assert st["sort_pass_items"] == digits * st["raw_pairs"]
+        assert (st["batches"] == 1) == (cap is None)
+        got.append((sel, st["unique_pairs"]))
+    for sel, uniq in got[1:]:
+        assert np.array_equal(sel, got[0][0]) and uniq == got[0][1]
