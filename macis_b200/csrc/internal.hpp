@@ -22,26 +22,23 @@ class PinnedPool {
   PinnedPool() = default;
   PinnedPool(const PinnedPool&) = delete;
   ~PinnedPool() {
-    for(void* p : free_) cudaFreeHost(p);
+    for(size_t i = 0; i < nfree_; ++i) cudaFreeHost(free_[i]);
   }
   void* take() {
     {
       std::lock_guard<std::mutex> lk(mu_);
-      if(!free_.empty()) {
-        void* p = free_.back();
-        free_.pop_back();
-        return p;
-      }
+      if(nfree_) return free_[--nfree_];
     }
     void* p = nullptr;
     MB_CUDA(cudaHostAlloc(&p, BYTES, cudaHostAllocMapped | cudaHostAllocPortable));
     return p;
   }
-  void give(void* p) {
+  // Called while a solver unwinds: allocates nothing.
+  void give(void* p) noexcept {
     {
       std::lock_guard<std::mutex> lk(mu_);
-      if(free_.size() < KEEP) {
-        free_.push_back(p);
+      if(nfree_ < KEEP) {
+        free_[nfree_++] = p;
         return;
       }
     }
@@ -50,7 +47,8 @@ class PinnedPool {
 
  private:
   std::mutex mu_;
-  std::vector<void*> free_;
+  void* free_[KEEP] = {};
+  size_t nfree_ = 0;
 };
 inline std::shared_ptr<PinnedPool> pinned_pool() {
   static std::mutex mu;
