@@ -26,15 +26,19 @@ namespace mb {
 // CAS(12,12), 853,776 rows and 1.55e9 elements: FP64 3.46 -> 2.88 ms (6.5
 // TB/s), FP32 values 2.6 -> 2.30 ms. 2 blocks per SM with a loop, or 16 rows a
 // block, gained a fifth of that at most; loads that leave the matrix out of L1
-// changed nothing.
-constexpr int SPMV_THREADS = 1024;
+// changed nothing. Short matrices keep 8 rows a block, for 32 leave SMs empty
+// (4,900 rows: 153 blocks on 148 SMs): us a product with 8 / 32 rows, FP64,
+// 400 rows 2.5 / 2.7, 4,900 5.1 / 6.3, 15,876 19.1 / 20.1, 63,504 114 / 112.
+// (The stride of a block is a constant of the kernel: with blockDim the FP64
+// product of 63,504 rows took 136.)
+constexpr int64_t SPMV_SHORT = 32768;  // rows
 
 // X32: the off-diagonal products use the FP32 copy x32 (the operator of
 // macis_b200_spmv on a mixed matrix); otherwise FP32 values multiply the
 // FP64 x, so that the product is one fixed linear operator of x (what the
 // Davidson residual needs to converge below FP32 resolution).
-template <typename CI, typename VT, bool MIXED, bool X32 = MIXED>
-__global__ void __launch_bounds__(SPMV_THREADS, 2)
+template <typename CI, typename VT, bool MIXED, bool X32, int THREADS>
+__global__ void __launch_bounds__(THREADS, 2048 / THREADS)
     spmv_k(int64_t m, int64_t n, const CI* __restrict__ rowptr,
            const CI* __restrict__ colind, const VT* __restrict__ nzval,
            const double* __restrict__ diag, const double* __restrict__ x,
@@ -42,8 +46,8 @@ __global__ void __launch_bounds__(SPMV_THREADS, 2)
            double* __restrict__ y, unsigned long long* t0) {
   note_start(t0);
   const int lane = threadIdx.x & 31;
-  const int64_t nwarp = int64_t(gridDim.x) * (SPMV_THREADS / 32);
-  for(int64_t row = int64_t(blockIdx.x) * (SPMV_THREADS / 32) + (threadIdx.x >> 5);
+  const int64_t nwarp = int64_t(gridDim.x) * (THREADS / 32);
+  for(int64_t row = int64_t(blockIdx.x) * (THREADS / 32) + (threadIdx.x >> 5);
       row < m; row += nwarp) {
     const int64_t b = int64_t(rowptr[row]), e = int64_t(rowptr[row + 1]);
     double acc0 = 0, acc1 = 0;
@@ -84,58 +88,56 @@ __global__ void to_f32_k(const double* x, float* y, int64_t n) {
     y[i] = float(x[i]);
 }
 
-static unsigned spmv_grid(int64_t m) {
-  return grid_for(size_t(m), SPMV_THREADS / 32, size_t(num_sms()) * 64);
+template <typename CI, typename VT, bool MIXED, bool X32, int THREADS>
+static void spmv_launch_as(const macis_b200_csr* A, double alpha,
+                           const double* x, const float* x32, double beta,
+                           double* y, cudaStream_t s, unsigned long long* t0) {
+  spmv_k<CI, VT, MIXED, X32, THREADS>
+      <<<grid_for(size_t(A->m), THREADS / 32, size_t(num_sms()) * 64), THREADS,
+         0, s>>>(A->m, A->n, static_cast<const CI*>(A->rowptr),
+                 static_cast<const CI*>(A->colind),
+                 static_cast<const VT*>(A->nzval), A->diag, x, x32, alpha, beta,
+                 y, t0),
+      note_launch();
+}
+// The products with an FP32 copy of x have one shape, so that any of them
+// loads the code that the allocation-free call runs (a kernel is loaded at its
+// first use, which can allocate).
+template <typename VT, bool MIXED, bool X32>
+static void spmv_launch(const macis_b200_csr* A, double alpha, const double* x,
+                        const float* x32, double beta, double* y,
+                        cudaStream_t s, unsigned long long* t0 = nullptr) {
+  constexpr int FEW = X32 ? 1024 : 256;
+  const bool i4 = A->idx_bytes == 4, few = A->m < SPMV_SHORT;
+  const auto f =
+      i4 ? (few ? spmv_launch_as<int32_t, VT, MIXED, X32, FEW>
+                : spmv_launch_as<int32_t, VT, MIXED, X32, 1024>)
+         : (few ? spmv_launch_as<int64_t, VT, MIXED, X32, FEW>
+                : spmv_launch_as<int64_t, VT, MIXED, X32, 1024>);
+  f(A, alpha, x, x32, beta, y, s, t0);
+  MB_CUDA(cudaGetLastError());
 }
 
 void spmv_device(const macis_b200_csr* A, double alpha, const double* x,
                  double beta, double* y, cudaStream_t s,
                  unsigned long long* t0) {
-  const int64_t m = A->m;
-  if(m == 0) return;
-  const unsigned g = spmv_grid(m);
-  if(A->val_bytes == 8) {
-    if(A->idx_bytes == 4)
-      spmv_k<int32_t, double, false><<<g, SPMV_THREADS, 0, s>>>(
-          m, A->n, (const int32_t*)A->rowptr, (const int32_t*)A->colind,
-          (const double*)A->nzval, A->diag, x, nullptr, alpha, beta, y, t0), note_launch();
-    else
-      spmv_k<int64_t, double, false><<<g, SPMV_THREADS, 0, s>>>(
-          m, A->n, (const int64_t*)A->rowptr, (const int64_t*)A->colind,
-          (const double*)A->nzval, A->diag, x, nullptr, alpha, beta, y, t0), note_launch();
-  } else {
-    Arena W(s);
-    float* x32 = W.get<float>(size_t(A->n));
-    to_f32_k<<<grid_for(size_t(A->n), 256, 8 * num_sms()), 256, 0, s>>>(
-        x, x32, A->n), note_launch();
-    if(A->idx_bytes == 4)
-      spmv_k<int32_t, float, true><<<g, SPMV_THREADS, 0, s>>>(
-          m, A->n, (const int32_t*)A->rowptr, (const int32_t*)A->colind,
-          (const float*)A->nzval, A->diag, x, x32, alpha, beta, y, t0), note_launch();
-    else
-      spmv_k<int64_t, float, true><<<g, SPMV_THREADS, 0, s>>>(
-          m, A->n, (const int64_t*)A->rowptr, (const int64_t*)A->colind,
-          (const float*)A->nzval, A->diag, x, x32, alpha, beta, y, t0), note_launch();
-  }
-  MB_CUDA(cudaGetLastError());
+  if(A->m == 0) return;
+  if(A->val_bytes == 8)
+    return spmv_launch<double, false, false>(A, alpha, x, nullptr, beta, y, s,
+                                             t0);
+  Arena W(s);
+  float* x32 = W.get<float>(size_t(A->n));
+  to_f32_k<<<grid_for(size_t(A->n), 256, 8 * num_sms()), 256, 0, s>>>(
+      x, x32, A->n), note_launch();
+  spmv_launch<float, true, true>(A, alpha, x, x32, beta, y, s, t0);
 }
 
 void spmv_device_x64(const macis_b200_csr* A, double alpha, const double* x,
                      double beta, double* y, cudaStream_t s,
                      unsigned long long* t0) {
   if(A->val_bytes == 8) return spmv_device(A, alpha, x, beta, y, s, t0);
-  const int64_t m = A->m;
-  if(m == 0) return;
-  const unsigned g = spmv_grid(m);
-  if(A->idx_bytes == 4)
-    spmv_k<int32_t, float, true, false><<<g, SPMV_THREADS, 0, s>>>(
-        m, A->n, (const int32_t*)A->rowptr, (const int32_t*)A->colind,
-        (const float*)A->nzval, A->diag, x, nullptr, alpha, beta, y, t0), note_launch();
-  else
-    spmv_k<int64_t, float, true, false><<<g, SPMV_THREADS, 0, s>>>(
-        m, A->n, (const int64_t*)A->rowptr, (const int64_t*)A->colind,
-        (const float*)A->nzval, A->diag, x, nullptr, alpha, beta, y, t0), note_launch();
-  MB_CUDA(cudaGetLastError());
+  if(A->m > 0)
+    spmv_launch<float, true, false>(A, alpha, x, nullptr, beta, y, s, t0);
 }
 
 }  // namespace mb
@@ -219,24 +221,12 @@ extern "C" int macis_b200_spmv_mixed_noalloc(const macis_b200_csr* A,
                "holds (4,194,304)");
     mb::DeviceScope on(A->device);
     float* x32 = mb::noalloc_scratch(A->device);
-    const int64_t m = A->m;
     cudaStream_t s = A->stream;
-    if(m > 0) {
+    if(A->m > 0) {
       // the scratch is fully rewritten before it is read: nothing to clear
       mb::to_f32_k<<<mb::grid_for(size_t(A->n), 256, 8 * mb::num_sms()), 256,
                      0, s>>>(x, x32, A->n), mb::note_launch();
-      const unsigned g = mb::spmv_grid(m);
-      if(A->idx_bytes == 4)
-        mb::spmv_k<int32_t, float, true><<<g, mb::SPMV_THREADS, 0, s>>>(
-            m, A->n, (const int32_t*)A->rowptr, (const int32_t*)A->colind,
-            (const float*)A->nzval, A->diag, x, x32, alpha, beta, y, nullptr),
-            mb::note_launch();
-      else
-        mb::spmv_k<int64_t, float, true><<<g, mb::SPMV_THREADS, 0, s>>>(
-            m, A->n, (const int64_t*)A->rowptr, (const int64_t*)A->colind,
-            (const float*)A->nzval, A->diag, x, x32, alpha, beta, y, nullptr),
-            mb::note_launch();
-      MB_CUDA(cudaGetLastError());
+      mb::spmv_launch<float, true, true>(A, alpha, x, x32, beta, y, s);
     }
     MB_CUDA(cudaStreamSynchronize(s));
     return MACIS_B200_OK;

@@ -188,3 +188,23 @@ def test_product_time_leaves_host_work_out(stored):
     dev = sum(st[k] for k in ("apply_ms", "rayleigh_ms", "residual_ms",
                               "ortho_ms"))
     assert dev < st["wall_ms"]
+
+
+@pytest.mark.parametrize("rows", [1, 7, 32767, 32768, 32801])
+def test_spmv_at_the_block_shapes(rows):
+    """Products of row blocks below and above the length from which 32 and not
+    8 rows make a block, against numpy on the downloaded matrix: FP64, and
+    FP32 values with the FP32 copy of x. Sums of at most 876 terms: 1e-12 of
+    the largest."""
+    T, V, d = fci(10, 5, 5, 64, seed=0)
+    H = mb.HamiltonianGenerator(T, V, 64)
+    x = np.random.default_rng(1).standard_normal(len(d))
+    for vt in (np.float64, np.float32):
+        A = mb.make_csr_hamiltonian_block(d[:rows], d, H, 1e-14, value_t=vt)
+        rp, ci, nz = A.to_host()
+        xs = x if vt is np.float64 else x.astype(np.float32).astype(np.float64)
+        ref = np.add.reduceat(nz.astype(np.float64) * xs[ci], rp[:-1])
+        if vt is np.float32:
+            ref += A.diagonal() * x[:rows]
+        np.testing.assert_allclose(A.spmv(x), ref, rtol=0,
+                                   atol=1e-12 * np.abs(ref).max())
