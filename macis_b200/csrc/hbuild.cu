@@ -37,6 +37,8 @@ namespace mb {
 constexpr int HB_WARPS = 4;
 constexpr int HB_THREADS = 32 * HB_WARPS;
 constexpr int GEN_CAP = 1024;  // candidates sorted in shared memory per warp
+// bytes of candidate lists up to which the free memory is not asked for
+constexpr uint64_t GEN_LIST_ASK = uint64_t(256) << 20;
 
 template <int NSW>
 __device__ __forceinline__ int sp_cmp(const Spin<NSW>& a, const Spin<NSW>& b) {
@@ -2023,14 +2025,31 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     GenData gd = gen_plan<NBITS>(h, bra, nbra, ket, nket, sub, r0, A);
     const unsigned gr = grid_for(nbra, HB_WARPS, size_t(sms) * 16);
     // candidate lists of the rows, as far as a tenth of the memory holds
-    // them (4 B per candidate, at most GEN_CAP per row)
+    // them (4 B per candidate, at most GEN_CAP per row). What is free is asked
+    // for long lists alone: the query takes 60 us and, on a shared host, up to
+    // milliseconds, as much as the build of a few hundred determinants.
     unsigned* ctr = A.get<unsigned>(1);
     auto* used = A.get<unsigned long long>(1);
     int64_t* list_off = A.get<int64_t>(nbra);
-    const uint64_t cap = std::min<uint64_t>(
-        {uint64_t(nbra) * GEN_CAP, uint64_t(device_bytes_available() / 40),
-         candidate_list_limit()});
-    uint32_t* list = A.get<uint32_t>(cap);
+    uint64_t cap = std::min<uint64_t>(uint64_t(nbra) * GEN_CAP,
+                                      candidate_list_limit());
+    size_t avail = 0;
+    if(4 * cap > GEN_LIST_ASK) {
+      avail = device_bytes_available();
+      cap = std::min<uint64_t>(cap, avail / 40);
+    }
+    auto have = [](auto&& get) {  // memory that may be missing
+      try {
+        get();
+      } catch(const Error& e) {
+        if(e.code != MACIS_B200_ENOMEM) throw;
+        cudaGetLastError();  // the allocation's
+        return false;
+      }
+      return true;
+    };
+    uint32_t* list = nullptr;
+    if(!have([&] { list = A.get<uint32_t>(cap); })) cap = 0;
     MB_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), s));
     MB_CUDA(cudaMemsetAsync(used, 0, 8, s));
     gen_list_k<NBITS><<<gr, HB_THREADS, 0, s>>>(
@@ -2039,15 +2058,27 @@ static void build_impl(macis_b200_ham* h, const uint64_t* bra, size_t nbra,
     exclusive_scan<int64_t, int64_t>(rowcnt, rowptr64, nbra, rowptr64 + nbra, A);
     nnz_ub = to_host(rowptr64 + nbra, s);
     // a matrix that needs their memory goes without the lists
-    if(1.05 * double(nnz_ub) * (sizeof(CI) + sizeof(VT)) + 1073741824.0 >
-       double(device_bytes_available())) {
+    auto drop_list = [&] {
       A.release(list);
       list = nullptr;
       MB_CUDA(cudaMemsetAsync(list_off, 0xFF, nbra * 8, s));
-    }
+    };
+    if(list && avail &&
+       1.05 * double(nnz_ub) * (sizeof(CI) + sizeof(VT)) + 1073741824.0 +
+               4.0 * double(cap) > double(avail))
+      drop_list();
     out->nnz_candidates = nnz_ub;
-    colind = A.get<CI>(size_t(nnz_ub));
-    nzval = A.get<VT>(size_t(nnz_ub));
+    auto get_matrix = [&] {
+      colind = A.get<CI>(size_t(nnz_ub));
+      nzval = A.get<VT>(size_t(nnz_ub));
+    };
+    if(!list) {
+      get_matrix();
+    } else if(!have(get_matrix)) {
+      if(colind) A.release(colind);
+      drop_list();
+      get_matrix();
+    }
     // long rows
     uint32_t* lf = A.get<uint32_t>(nbra + 1);
     uint32_t* lpos = A.get<uint32_t>(nbra + 1);

@@ -159,7 +159,9 @@ def test_injected_int32_capacity(faults):
 def test_failed_builds_give_their_memory_back(faults, product):
     """A build that ends with ECAPACITY or, at any of its allocations, with
     ENOMEM holds nothing afterwards: the matrix part that it had is there for
-    the 64-bit build or the matrix-free operator that follows."""
+    the 64-bit build or the matrix-free operator that follows. Without the
+    memory for its candidate lists, or for the matrix beside them, a general
+    build goes on without the lists."""
     rt = pytest.importorskip("cuda.bindings.runtime")
     _, pool = rt.cudaDeviceGetDefaultMemPool(0)
     used = lambda: int(rt.cudaMemPoolGetAttribute(
@@ -175,12 +177,24 @@ def test_failed_builds_give_their_memory_back(faults, product):
         mb.make_csr_hamiltonian(d, H, 1e-3)
     assert e.value.code == _lib.ECAPACITY and used() == base
     faults(_lib.FAULT_NONE)
+    want = mb.make_csr_hamiltonian(d, H, 1e-3).to_host()
+    runs, good = [], 0       # lengths of the runs of builds that succeed
     for k in range(400):
         faults(_lib.FAULT_ALLOC, k)
         try:
             A = mb.make_csr_hamiltonian(d, H, 1e-3)
         except mb.MacisError as e:
             assert e.code == _lib.ENOMEM and used() == base, k
-        else:
+            good = 0
+            continue
+        for a, b in zip(A.to_host(), want):
+            assert np.array_equal(a, b)
+        del A
+        good += 1
+        if good == 1:
+            runs.append(0)
+        runs[-1] = good
+        if good == 5:        # beyond the last allocation
             break
-    assert 10 < k < 399 and A.nnz == nnz
+    # the lists and the two arrays beside them; then nothing fails any more
+    assert good == 5 and sum(runs[:-1]) == (0 if product else 3)
