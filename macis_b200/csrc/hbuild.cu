@@ -2565,10 +2565,12 @@ __global__ void __launch_bounds__(HB_THREADS)
 }
 
 // Diagonal branch: the rows' sums over the pairs of orbitals occupied in
-// them. A block takes DG_ROWS rows, its threads the orbital pairs, and adds
+// them. A block takes DG_ROWS rows and a pair of orbitals a thread, and adds
 // one partial sum per pair: atomics per orbital pair and block, not per row
-// (every row adds to the pairs of the deepest orbitals).
+// (every row adds to the pairs of the deepest orbitals). With all pairs in one
+// block, 300 determinants of 100 orbitals had 3 blocks for 10,000 pairs.
 constexpr int DG_ROWS = 128;
+constexpr int DG_THREADS = 256;
 template <int NBITS, bool DIRECT>
 __global__ void rdm_diag_k(const uint64_t* dets, int64_t n, const double* w,
                            int norb, double* ordm, int two, RdmSums S) {
@@ -2583,7 +2585,8 @@ __global__ void rdm_diag_k(const uint64_t* dets, int64_t n, const double* w,
   for(int i = threadIdx.x; i < nr; i += blockDim.x) sw[i] = w[r0 + i];
   __syncthreads();
   const int npair = two ? norb * norb : norb;
-  for(int x = threadIdx.x; x < npair; x += blockDim.x) {
+  const int x = blockIdx.y * blockDim.x + threadIdx.x;
+  if(x < npair) {
     const int p = two ? x % norb : x, q = two ? x / norb : x;
     double one = 0.0, ss = 0.0, os = 0.0;
     for(int r = 0; r < nr; ++r) {
@@ -2649,14 +2652,15 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
   S.trdm = trdm;
   S.diag = A.get<double>(n);
   const int two = trdm ? 1 : 0;
-  const unsigned gd = grid_for(n, DG_ROWS);
+  const dim3 gd(grid_for(n, DG_ROWS),
+                grid_for(two ? n1 * n1 : n1, DG_THREADS));
   // The sums are taken last, so that without the memory for them the pairs go
   // straight to the 2-RDM; so do those of short lists, where the passes over
   // the sums cost more than the additions that they save. Selected lists of
   // norb^2 / 20, 4 norb^2 and 16 norb^2 determinants, sums / straight: n = 24
-  // 0.37 / 0.34, 0.41 / 0.40, 0.57 / 0.58 ms; n = 48 0.50 / 0.39, 0.81 / 0.72,
-  // 1.55 / 1.76; n = 100 3.39 / 1.19, 7.9 / 6.0, 24.6 / 25.2. CAS spaces (more
-  // pairs a determinant) lie above the line: CAS(9,8) 0.87 / 1.32 ms.
+  // 0.36 / 0.32, 0.40 / 0.39, 0.53 / 0.55 ms; n = 48 0.44 / 0.33, 0.73 / 0.65,
+  // 1.47 / 1.72; n = 100 2.58 / 0.41, 6.5 / 4.6, 22.9 / 22.7. CAS spaces (more
+  // pairs a determinant) lie above the line: CAS(9,8) 0.81 / 1.32 ms.
   auto sums = [&] {
     const size_t tot = 2 * n4 + 2 * n3 + 2 * n1 * n1;
     if(!trdm || n <= 4 * n1 * n1) return false;
@@ -2680,8 +2684,8 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
       <<<gr, HB_THREADS, 0, s>>>(g, dets, int64_t(n), C, h->norb, ordm, two, \
                                  S, ctr),                                    \
       note_launch();                                                         \
-  rdm_diag_k<NB, DIRECT><<<gd, 256, 0, s>>>(dets, int64_t(n), S.diag,        \
-                                            h->norb, ordm, two, S),          \
+  rdm_diag_k<NB, DIRECT><<<gd, DG_THREADS, 0, s>>>(                          \
+      dets, int64_t(n), S.diag, h->norb, ordm, two, S),                      \
       note_launch();
 #define MB_RDM(NB)                                                           \
   {                                                                          \

@@ -192,3 +192,36 @@ def test_rdm_scratch_of_a_short_list():
     C = np.full(10, 10 ** -0.5)
     H.form_rdms(d, C)
     assert _peak_pool_bytes(lambda: H.form_rdms(d, C)) < 1.1 * 8 * n ** 4
+
+
+@pytest.mark.parametrize("n,ndets", [(16, 130), (17, 40), (17, 1200),
+                                     (33, 257)])
+def test_rdms_with_more_orbital_pairs_than_threads(n, ndets):
+    """Orbital pairs beyond one block's threads and rows beyond one block's,
+    straight to the 2-RDM and through the sums (17 orbitals, 1,200
+    determinants), against the pair sums in plain Python: 1e-12."""
+    rng = np.random.default_rng(n)
+    T, V = mb.synthetic_integrals(n, 2)
+    hf, words = 7, set()
+    while len(words) < ndets:
+        a, b = hf, hf
+        for _ in range(int(rng.integers(0, 3))):
+            i, v = rng.integers(0, 3), rng.integers(3, n)
+            x = (1 << int(i)) | (1 << int(v))
+            if rng.random() < 0.5:
+                a = a ^ x if a & x == 1 << int(i) else a
+            else:
+                b = b ^ x if b & x == 1 << int(i) else b
+        words.add((a, b))
+    words = sorted(words)
+    d = mb.sd.make_dets([a for a, _ in words], [b for _, b in words], 128)
+    d = shuffled(d, seed=1).copy()
+    C = rng.standard_normal(len(d))
+    C /= np.linalg.norm(C)
+    H = mb.HamiltonianGenerator(T, V, 128)
+    for two in (True, False):
+        o, t = H.form_rdms(d, C, two=two)
+        ro, rt = _rdms_by_pairs(d, C, n, two)
+        np.testing.assert_allclose(o, ro, rtol=0, atol=1e-12)
+        if two:
+            np.testing.assert_allclose(t, rt, rtol=0, atol=1e-12)
