@@ -1890,7 +1890,7 @@ static void asci_impl(macis_b200_ham* h, const macis_b200_asci_settings& st,
   }
   stats.screen_ms = ms_since(t_scr);
 
-  {
+  if(!st.just_singles) {  // units of doubles
     const size_t n2 = size_t(h->norb) * h->norb;
     uint8_t* full = A.get<uint8_t>(2 * n2);
     pair_full_k<<<grid_for(2 * n2 * 32, 256, 16 * sms), 256, 0, s>>>(
