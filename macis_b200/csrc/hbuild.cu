@@ -2654,7 +2654,7 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
   const int two = trdm ? 1 : 0;
   const dim3 gd(grid_for(n, DG_ROWS),
                 grid_for(two ? n1 * n1 : n1, DG_THREADS));
-  // The sums are taken last, so that without the memory for them the pairs go
+  // Without the memory for the sums, or for the plan beside them, the pairs go
   // straight to the 2-RDM; so do those of short lists, where the passes over
   // the sums cost more than the additions that they save. Selected lists of
   // norb^2 / 20, 4 norb^2 and 16 norb^2 determinants, sums / straight: n = 24
@@ -2689,19 +2689,35 @@ void form_rdms_device(macis_b200_ham* h, const uint64_t* dets, size_t n,
       note_launch();
 #define MB_RDM(NB)                                                           \
   {                                                                          \
-    const GenData g = gen_plan<NB>(h, dets, n, dets, n, true, 0, A);         \
-    if(sums() || !trdm) {                                                    \
+    const GenData g = gen_plan<NB>(h, dets, n, dets, n, true, 0, P);         \
+    if(S.os || !trdm) {                                                      \
       MB_RDM_RUN(NB, false)                                                  \
     } else {                                                                 \
       MB_RDM_RUN(NB, true)                                                   \
     }                                                                        \
   }
-  if(h->nbits == 64) {
-    MB_RDM(64)
-  } else if(h->nbits == 128) {
-    MB_RDM(128)
+  auto run = [&] {
+    Arena P(s);
+    if(h->nbits == 64) {
+      MB_RDM(64)
+    } else if(h->nbits == 128) {
+      MB_RDM(128)
+    } else {
+      MB_RDM(256)
+    }
+  };
+  if(!sums()) {
+    run();
   } else {
-    MB_RDM(256)
+    try {
+      run();
+    } catch(const Error& e) {  // the plan: nothing is added yet
+      if(e.code != MACIS_B200_ENOMEM) throw;
+      cudaGetLastError();
+      A.release(S.os);
+      S.os = nullptr;
+      run();
+    }
   }
   if(S.os)
     rdm_expand_k<<<grid_for(n4, 256, 16 * num_sms()), 256, 0, s>>>(
