@@ -153,8 +153,9 @@ __global__ void __launch_bounds__(DV_THREADS)
   }
   __threadfence_system();  // before the report of the last chunk
   if(last_block(done + gridDim.y, gridDim.y) && threadIdx.x == 0) {
-    rep->t_row0 = *static_cast<volatile unsigned long long*>(t0);
-    rep->t_app0 = *static_cast<volatile unsigned long long*>(t0 + 1);
+    const ulonglong2 t = __ldcg(reinterpret_cast<const ulonglong2*>(t0));
+    rep->t_row0 = t.x;
+    rep->t_app0 = t.y;
     rep->t_row1 = gpu_time_ns();
     __threadfence_system();
     rep->row_seq = seq;
