@@ -19,8 +19,8 @@
 //
 // When the raw contributions do not fit in HBM at once, the candidate
 // determinants are split into ranges by a hash of the determinant; each
-// range is generated, sorted and accumulated on its own (its sums are
-// complete) and merged into a running top-k.
+// range is generated, grouped and summed on its own (its sums are complete)
+// and merged into a running top-k.
 #include <algorithm>
 #include <chrono>
 #include <cstdlib>
@@ -295,7 +295,8 @@ struct AlphaLists {
 // list itself is the result the numbers are ranks in the sorted list of the
 // strings, so that the key sorts in the same order as the determinant's
 // bitset; a search only groups equal keys, and its numbers come from a hash
-// table (a sort of the 7e7 candidates of the 122 strings of an n = 100 core
+// table, arbitrary and not the same in every run, since only their equality
+// is used (a sort of the 7e7 candidates of the 122 strings of an n = 100 core
 // set cost 18 digit passes a spin). Per
 // distinct core string u of a spin the table R holds the ranks of its
 // M = 1 + N1 + N2 candidates: u itself, its N1 singles (index ii * nv + aa,
@@ -324,7 +325,7 @@ __device__ __forceinline__ int64_t double_row_base(int ii, int aa, int ne,
 }
 
 // The candidate strings of the distinct core strings, one thread per
-// (string, candidate): written with their index, for the rank sort.
+// (string, candidate): written, with their index where they will be sorted.
 template <int NSW>
 __global__ void cand_strings_k(const uint64_t* words, const uint8_t* occ,
                                const uint8_t* vir, size_t nu, int ne, int nv,
@@ -1735,8 +1736,9 @@ static int bits_for(size_t n) {
 
 // Rank tables of both spins (RankTables), when they fit: the tables and
 // the distinct candidate strings within 10 % of the free device memory,
-// the candidate sort within half of it, 32-bit candidate indices and
-// bits_a + bits_b <= 64. Returns the key width in bits, 0 when not built.
+// the candidates' sort or hash table within half of it, 32-bit candidate
+// indices and bits_a + bits_b <= 64. Returns the key width in bits, 0 when
+// not built.
 template <int NBITS>
 static int build_ranks(const SpinPlan& pa, const SpinPlan& pb, size_t ncdets,
                        bool ordered, Arena& A, cudaStream_t s,

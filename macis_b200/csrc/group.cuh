@@ -63,9 +63,10 @@ struct HashDigit {  // the byte of the key's hash at bit `shift`
 };
 
 // Hash digits for n records: 20 per bucket at most, of which a window of 32
-// still ends a whole bucket. A digit pass moves every record once (10.6 ms of
-// 1e9); for 2.9e8 records a fourth pass takes 3.1 ms and their sums 4.0 in
-// place of 6.5 ms, and fuller buckets are read one key after another.
+// still ends a whole bucket. A digit pass moves every record once (9.3 ms of
+// 1e9 16-byte records, 10.6 when the line was drawn: for 2.9e8 records a
+// fourth pass then took 3.1 ms and their sums 4.0 in place of 6.5 ms); fuller
+// buckets are read one key after another.
 inline int group_digits(size_t n) {
   int np = 1;
   while(np < 4 && (n >> (8 * np)) > 20) ++np;
@@ -75,7 +76,7 @@ inline int group_digits(size_t n) {
 constexpr int GS_THREADS = 128;
 constexpr int GS_WARPS = GS_THREADS / 32;
 template <int NW>
-struct GroupTile {  // 18 KB of keys and scores for the four warps
+struct GroupTile {  // 18 to 20 KB of keys and scores for the four warps
   static constexpr int IPT = NW == 1 ? 8 : NW == 2 ? 5 : 3;
   static constexpr int N = 32 * IPT;   // records per warp
   static constexpr int SPAN = N + 32;  // with those a last bucket may go on in

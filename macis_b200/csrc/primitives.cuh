@@ -1,9 +1,11 @@
 // Device-wide primitives written for this library: a workspace arena, an
 // exclusive scan and a stable LSD radix sort over multi-word keys.
 //
-// The radix sort is the dedup engine of the ASCI search (the reference's
-// std::sort by bitset_less, include/macis/asci/determinant_sort.hpp:40-57)
-// and the grouping step of the Hamiltonian build. Keys are NW little-endian
+// The radix sort orders the ASCI search's accumulated list and selections
+// (the reference's std::sort by bitset_less, include/macis/asci/
+// determinant_sort.hpp:40-57) and the determinants of the Hamiltonian build;
+// its digit passes also partition a search's contributions, which are not
+// sorted (group.cuh). Keys are NW little-endian
 // uint64 words stored item-contiguous; word NW-1 is the most significant
 // (the bitset_less order, bitset_operations.hpp:289-306). Only 8-bit digits
 // in which some key differs from the first key are sorted, so a 24-orbital
@@ -619,10 +621,10 @@ int radix_sort(uint64_t* keys, P* vals, uint64_t* keys_alt, P* vals_alt,
   auto classic_pass = [&](int shift) {
     classic.run(kin, vin, kout, vout, ShiftDigit<NW>{shift});
   };
-  // The one-sweep passes are opt-in (MACIS_B200_SORT_ONESWEEP=1): measured
-  // on the n = 48 ASCI searches with bin-grouped ranges, the classic passes
-  // were faster (1e5 core dets: 6.9 s against 8.1-11.3 s; 1e4: 0.64 s
-  // against 0.67-0.69 s) and steadier
+  // The one-sweep passes are opt-in (MACIS_B200_SORT_ONESWEEP=1): when the
+  // searches still sorted their contributions, the classic passes were faster
+  // (2.7e10 records in ranges: 6.9 s against 8.1-11.3 s; 2.7e9: 0.64 s against
+  // 0.67-0.69 s) and steadier
   const char* opt = getenv("MACIS_B200_SORT_ONESWEEP");
   const bool onesweep = n >= RS_ONESWEEP_MIN && np <= RS_MAX_PASSES &&
                         opt && opt[0] == '1';
